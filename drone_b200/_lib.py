@@ -112,6 +112,7 @@ def _declare(lib):
         "drone_pr_inceval": (i, [vp, C.POINTER(PRResponse), vp]),
         "drone_pr_power_iterate": (i, [vp, i, C.c_double, vp]),
         "drone_pr_step_local": (i, [i, C.POINTER(vp), i, C.POINTER(PRResponse), vp]),
+        "drone_pr_job_local": (i, [i, C.POINTER(vp), i, C.POINTER(i), vp, vp]),
         "drone_pr_power_iterate_local": (i, [i, C.POINTER(vp), i, C.c_double, vp]),
         "drone_pr_values": (i, [vp, vp, vp]),
         "drone_pr_set_isolated_count": (i, [vp, ll]),

@@ -224,6 +224,8 @@ int drone_xplan_create(drone_xplan **out, int rank, int nranks, int n_local, con
                   "drone_xplan_create: NULL routing table");
     drone_xplan *x = new (std::nothrow) drone_xplan();
     if (!x) return set_error(DRONE_E_INVALID, "drone_xplan_create: out of host memory");
+    static std::atomic<unsigned long long> plans_made{0};
+    x->uid = ++plans_made;
     x->rank = rank;
     x->nranks = nranks;
     x->n_local = n_local;

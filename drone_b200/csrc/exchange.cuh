@@ -13,6 +13,7 @@ struct drone_comm {
 };
 
 struct drone_xplan {
+    unsigned long long uid = 0;               // number of this plan in the process (addresses are reused, this is not)
     int rank = 0, nranks = 1, n_local = 0, max_features = 0;
     // host lists, grouped by peer (offsets have nranks+1 entries)
     std::vector<int> up_rows, up_off;        // my mirror rows, by owner, ascending global id

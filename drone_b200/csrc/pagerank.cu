@@ -10,11 +10,12 @@
 //
 // Where the reference pushes along out-edges with atomicAdd (pr.cu:14-87), this
 // implementation pulls along in-edges of the transposed local graph: every vertex
-// publishes {delta, pushed} once and every vertex sums what its in-neighbours
-// published.  Same arithmetic, no atomics on values, fixed summation order.
-// The boundary exchange is static and dense (all mirrors of a peer in one
-// message, ordered by global id); each entry carries the flag that the
-// reference expresses by sending or not sending the vertex, so the counts the
+// publishes its delta once (-0.0 for "did not push") and every vertex sums what its
+// in-neighbours published.  Same arithmetic, no atomics on values, fixed summation order.
+// Parts held by one process run all their supersteps in one launch (pr_run_kernel); between
+// processes the boundary exchange is static and dense (all mirrors of a peer in one
+// message, ordered by global id), each entry carrying the flag that the
+// reference expresses by sending or not sending the vertex.  Either way the counts the
 // caller uses to detect termination (Response, common.h:23-27) are reproduced.
 #include "exchange.cuh"
 #include "plan.cuh"
@@ -36,17 +37,26 @@ struct drone_pr {
     drone_xplan *xplan = nullptr;     // borrowed
     drone_comm *comm = nullptr;       // borrowed (may be NULL for a single part)
     int *out_degree = nullptr, *mirror2worker = nullptr;
-    void *pr = nullptr, *acc = nullptr, *diff = nullptr, *push = nullptr;   // real[n], real[n], real[n], real2[n]
-    // Large parts: where vertex i publishes its {delta, pushed} pair.  The pairs lie in the order of how often they are
-    // gathered (most gathered first) and the pull lists' columns are renumbered to match, so that the hot pairs are
-    // contiguous and stay in L2 (a pair is 8 bytes of a 32-byte sector).  NULL: pair i lies at i.
+    void *pr = nullptr, *acc = nullptr, *diff = nullptr, *push = nullptr;   // real[n] each
+    // Where vertex i publishes its delta.  The deltas lie in the order of how often they are gathered (most gathered
+    // first) and the pull lists' columns are renumbered to match, so that a prefix of the array, small enough for
+    // shared memory, serves most gathers.  NULL (few vertices): delta i lies at i.
     int *place = nullptr;
     int *active = nullptr, *ubm = nullptr;
-    void *scalars = nullptr;          // real[4]: globalDiff, globalAcc, dangling (power mode), spare
+    void *scalars = nullptr;          // real[4]: globalDiff, globalAcc, dangling (power mode), isolated value
     void *block_sums = nullptr;       // real[kReduceBlocks]
-    void *partials = nullptr;         // real2[n_partials]
+    void *partials = nullptr;         // Partial[n_partials]
+    int *slot_split = nullptr;        // [n_partials] split row a partial slot belongs to
+    int *arrived = nullptr;           // [n_split_rows] slots written so far in this pull (0 between pulls)
     void *send = nullptr, *recv = nullptr;   // real2[max(up, down)]
     int *counters = nullptr;          // [0..3] exchange counts, [4] active count
+    // parts held by one process: {part, row} of every contribution a master row takes, in m_pos order, and the plans
+    // it was made for
+    int2 *pairs = nullptr;
+    std::vector<unsigned long long> pairs_for;
+    char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
+    size_t control_bytes = 0;
+    int sms = 0;
     bool started = false;
     long long n_isolated = 0;         // vertex ids that occur in no part (power iteration treats them as dangling)
 };
@@ -55,7 +65,8 @@ namespace drone {
 
 static const int kReduceBlocks = 1024;
 
-template <typename R> struct alignas(2 * sizeof(R)) Pair { R val, flag; };
+template <typename R> struct alignas(2 * sizeof(R)) Pair { R val, flag; };          // one boundary entry of a message
+template <typename R> struct alignas(2 * sizeof(R)) Partial { R sum; int pushed; };   // one chunk of a split row
 template <typename R> struct NcclType;
 template <> struct NcclType<float> { static constexpr ncclDataType_t value = ncclFloat; };
 template <> struct NcclType<double> { static constexpr ncclDataType_t value = ncclDouble; };
@@ -63,6 +74,29 @@ template <> struct NcclType<double> { static constexpr ncclDataType_t value = nc
 template <typename R> __device__ __forceinline__ R fma_r(R a, R b, R c);
 template <> __device__ __forceinline__ float fma_r<float>(float a, float b, float c) { return fmaf(a, b, c); }
 template <> __device__ __forceinline__ double fma_r<double>(double a, double b, double c) { return fma(a, b, c); }
+
+// What a vertex that does not push publishes: -0.0.  A pushed delta is never -0.0 ((new - old) / outDegree gives +0.0
+// when nothing moved), and adding -0.0 changes no sum, so one word per vertex carries both the delta and the flag.
+__device__ __forceinline__ bool is_pushed(float v) { return __float_as_uint(v) != 0x80000000u; }
+__device__ __forceinline__ bool is_pushed(double v) { return __double_as_longlong(v) != (long long)0x8000000000000000ULL; }
+template <typename R> __device__ __forceinline__ R not_pushed() { return (R)-0.0; }
+
+// Device view of one part.
+template <typename R>
+struct PartView {
+    int n, global_v, n_chunks, n_ranges, n_masters, table_n;
+    const Chunk *chunks;
+    const int *col, *s_range_row, *s_rowptr, *s_rows, *s_col;
+    const SplitRow *split;
+    const int *slot_split;
+    int *arrived;
+    Partial<R> *partials;
+    R *pr, *acc, *diff, *push, *scalars;
+    int *active, *ubm;
+    const int *out_degree, *mirror2worker, *place;
+    const int *m_rows, *m_off;
+    const int2 *pairs;
+};
 
 // Sum of v over the block in a fixed order (tree over warps), result in thread 0.
 template <typename R>
@@ -79,40 +113,404 @@ __device__ R block_sum(R v) {
     return tot;
 }
 
-// pr = 1, acc = diff = 0, flags cleared; publish pr/outDegree; dangling mass of non-mirror vertices to block sums.
+// ---- per-vertex steps, shared by the kernels of one superstep and the persistent kernel.  `first` / `stride`: the
+// thread's share of the vertices, four of them at a time so that their loads are in flight together (a store between
+// two vertices' loads would keep the compiler from doing that itself).  Each returns the dangling mass it met. ----
+constexpr int kVertexBatch = 4;
+
+// pr = start, acc = diff = 0, flags cleared; publish start/outDegree.
 // (pr_init, DRONE/src/cuda/algorithm/pr.cu:14-37, plus the fills of PR_PEVal :391-394.)
 template <typename R>
-__global__ void pr_init_kernel(R *pr, R *acc, R *diff, Pair<R> *push, int *active, int *ubm,
-                               const int *__restrict__ out_degree, const int *__restrict__ mirror2worker, int n,
-                               int global_v, R start, R *block_sums, const int *__restrict__ place) {
+__device__ __forceinline__ R init_vertices(const PartView<R> &p, R start, bool power, int first, int stride) {
     R dangling = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        pr[i] = start;
-        acc[i] = 0;
-        diff[i] = 0;
-        active[i] = 0;
-        ubm[i] = 0;
-        Pair<R> p;
-        p.val = 0;
-        p.flag = 0;
-        const int od = out_degree[i];
-        if (od == 0) {
-            if (mirror2worker[i] == -1) dangling += start / global_v;
-        } else {
-            p.val = start / od;
-            p.flag = 1;
+#pragma unroll 1
+    for (int i0 = first; i0 < p.n; i0 += kVertexBatch * stride) {
+        int od[kVertexBatch], at[kVertexBatch];
+#pragma unroll
+        for (int b = 0; b < kVertexBatch; ++b) {
+            const int i = i0 + b * stride;
+            od[b] = i < p.n ? __ldg(p.out_degree + i) : 1;
+            at[b] = i < p.n && p.place ? __ldg(p.place + i) : i;
         }
-        push[place ? place[i] : i] = p;
+#pragma unroll
+        for (int b = 0; b < kVertexBatch; ++b) {
+            const int i = i0 + b * stride;
+            if (i >= p.n) break;
+            p.pr[i] = start;
+            p.acc[i] = 0;
+            p.diff[i] = 0;
+            p.active[i] = 0;
+            p.ubm[i] = 0;
+            if (od[b] == 0 && __ldg(p.mirror2worker + i) == -1) dangling += power ? start : start / p.global_v;
+            p.push[at[b]] = od[b] == 0 ? not_pushed<R>() : start / od[b];
+        }
     }
-    const R tot = block_sum<R>(dangling);
+    return dangling;
+}
+
+// pr_process_messages (pr.cu:430-448) fused with pr_increment (pr.cu:51-87).
+template <typename R>
+__device__ __forceinline__ R increment_vertices(const PartView<R> &p, R eps, R gacc, int first, int stride) {
+    const R alpha = (R)0.85f;                // pr.cu:12 declares a float constant
+    const R one_minus_alpha = (R)1 - alpha;
+    R dangling = 0;
+#pragma unroll 1
+    for (int i0 = first; i0 < p.n; i0 += kVertexBatch * stride) {
+        R a[kVertexBatch], old[kVertexBatch];
+        int od[kVertexBatch], at[kVertexBatch];
+#pragma unroll
+        for (int b = 0; b < kVertexBatch; ++b) {
+            const int i = i0 + b * stride;
+            a[b] = i < p.n ? p.acc[i] + p.diff[i] : (R)0;
+            old[b] = i < p.n ? p.pr[i] : (R)0;
+            od[b] = i < p.n ? __ldg(p.out_degree + i) : 1;
+            at[b] = i < p.n && p.place ? __ldg(p.place + i) : i;
+        }
+#pragma unroll
+        for (int b = 0; b < kVertexBatch; ++b) {
+            const int i = i0 + b * stride;
+            if (i >= p.n) break;
+            p.ubm[i] = 0;
+            p.acc[i] = a[b];                 // the pull that follows writes diff and active of every vertex
+            const R now = fma_r<R>(alpha, a[b] + gacc, one_minus_alpha);
+            R d = now - old[b];
+            if (d < 0) d = -d;
+            R out = not_pushed<R>();
+            if (!(d < eps)) {
+                if (od[b] == 0) {
+                    if (__ldg(p.mirror2worker + i) == -1) dangling += (now - old[b]) / p.global_v;
+                } else {
+                    out = (now - old[b]) / od[b];
+                }
+                p.pr[i] = now;
+            }
+            p.push[at[b]] = out;
+        }
+    }
+    return dangling;
+}
+
+// pr' = (1-d)/V + d * (sum over in-edges + dangling/V), published as pr'/outDegree for the next iteration; after the
+// last one (`last`) the value itself is stored instead: before that nobody can see it.
+template <typename R>
+__device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R dang, bool last, int first, int stride) {
+    const R base = ((R)1 - damping) / p.global_v;
+    const R share = dang / p.global_v;
+    R dangling = 0;
+#pragma unroll 1
+    for (int i0 = first; i0 < p.n; i0 += kVertexBatch * stride) {
+        R d[kVertexBatch];
+        int od[kVertexBatch], at[kVertexBatch];
+#pragma unroll
+        for (int b = 0; b < kVertexBatch; ++b) {
+            const int i = i0 + b * stride;
+            d[b] = i < p.n ? p.diff[i] : (R)0;
+            od[b] = i < p.n && !last ? __ldg(p.out_degree + i) : 1;
+            at[b] = i < p.n && !last && p.place ? __ldg(p.place + i) : i;
+        }
+#pragma unroll
+        for (int b = 0; b < kVertexBatch; ++b) {
+            const int i = i0 + b * stride;
+            if (i >= p.n) break;
+            const R now = base + damping * (d[b] + share);
+            if (last) {
+                p.pr[i] = now;
+                continue;
+            }
+            if (od[b] == 0 && __ldg(p.mirror2worker + i) == -1) dangling += now;
+            p.push[at[b]] = od[b] == 0 ? not_pushed<R>() : now / od[b];
+        }
+    }
+    return dangling;
+}
+
+// ---- pull along in-edges: diff[v] = sum of published deltas, active[v] = any in-neighbour pushed ----
+//
+// Bound: one scattered gather per edge.  A load of 32 scattered words from L2 costs the LSU 32 wavefronts whatever
+// its hit rate, which caps the whole part at about 2.9e11 gathers per second; a shared-memory load of 32 scattered
+// words costs 3 to 4.  So every block first copies the most gathered part of the array (a prefix, see `place`) into
+// shared memory and gathers from global memory only what lies behind it (R-MAT-22: 59 % of the gathers hit 51,200
+// floats).  Measured, R-MAT-22 float: 0.323 -> 0.256 ms per power iteration.
+//
+// `table`: the first p.table_n published values, in shared memory.  `warp` of `n_warps`: this warp's share of the work.
+
+// The value published at place c.  Both loads are predicated instead of branched around, so that the gathers of a batch
+// stay in flight together.  `table` is a shared-memory address.
+__device__ __forceinline__ float published(unsigned table, int table_n, const float *push, int c) {
+    float v;
+    asm volatile("{\n\t.reg .pred n;\n\t.reg .u32 s;\n\t.reg .u64 g;\n\t.reg .f32 a, b;\n\t"
+                 "setp.lt.s32 n, %1, %2;\n\t"
+                 "mad.lo.u32 s, %1, 4, %3;\n\t"
+                 "mad.wide.s32 g, %1, 4, %4;\n\t"
+                 "@n ld.shared.f32 a, [s];\n\t"
+                 "@!n ld.global.f32 b, [g];\n\t"
+                 "selp.f32 %0, a, b, n;\n\t}"
+                 : "=f"(v) : "r"(c), "r"(table_n), "r"(table), "l"(push) : "memory");
+    return v;
+}
+__device__ __forceinline__ double published(unsigned table, int table_n, const double *push, int c) {
+    double v;
+    asm volatile("{\n\t.reg .pred n;\n\t.reg .u32 s;\n\t.reg .u64 g;\n\t.reg .f64 a, b;\n\t"
+                 "setp.lt.s32 n, %1, %2;\n\t"
+                 "mad.lo.u32 s, %1, 8, %3;\n\t"
+                 "mad.wide.s32 g, %1, 8, %4;\n\t"
+                 "@n ld.shared.f64 a, [s];\n\t"
+                 "@!n ld.global.f64 b, [g];\n\t"
+                 "selp.f64 %0, a, b, n;\n\t}"
+                 : "=d"(v) : "r"(c), "r"(table_n), "r"(table), "l"(push) : "memory");
+    return v;
+}
+
+// 16 bytes a load and four loads in flight: the table is filled once per pull by every block.
+template <typename R>
+__device__ __forceinline__ void load_table(const PartView<R> &p, R *table) {
+    constexpr int W = 16 / sizeof(R);
+    const int n4 = p.table_n / W;
+    const float4 *src = reinterpret_cast<const float4 *>(p.push);
+    float4 *dst = reinterpret_cast<float4 *>(table);
+    int i = threadIdx.x;
+#pragma unroll 1
+    for (; i + 3 * (int)blockDim.x < n4; i += 4 * blockDim.x) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = src[i + u * blockDim.x];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) dst[i + u * blockDim.x] = v[u];
+    }
+    for (; i < n4; i += blockDim.x) dst[i] = src[i];
+    for (i = n4 * W + threadIdx.x; i < p.table_n; i += blockDim.x) table[i] = p.push[i];
+}
+
+// Split rows: the warps note the slots they filled and, 32 chunks at a time, make them visible with one fence and count
+// them in; the warp that counts in a row's last slot adds the row's slots, in slot order.  (A fence per chunk was 11 %
+// of the stall cycles of the whole kernel.)  `slot`: lane l's l-th noted slot, -1 for none.
+template <typename R, bool FLAGS>
+__device__ __forceinline__ void close_slots(const PartView<R> &p, int slot) {
+    const int lane = threadIdx.x & 31;
+    if (!__any_sync(0xffffffffu, slot >= 0)) return;
+    int at = 0, first = 0, n_slots = 0;
+    bool last = false;
+    __threadfence();
+    __syncwarp();
+    if (slot >= 0) {
+        at = __ldg(p.slot_split + slot);
+        const int4 sr = __ldg(reinterpret_cast<const int4 *>(p.split) + at);      // row, first slot, slots
+        first = sr.y;
+        n_slots = sr.z;
+        last = atomicAdd(p.arrived + at, 1) == n_slots - 1;
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, last);
+    if (todo) __threadfence();
+#pragma unroll 1
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int f = __shfl_sync(0xffffffffu, first, src), n = __shfl_sync(0xffffffffu, n_slots, src);
+        R sum = 0;
+        bool pushed = false;
+#pragma unroll 1
+        for (int k = lane; k < n; k += 32) {
+            const Partial<R> *q = p.partials + f + k;
+            sum += __ldcg(&q->sum);
+            if (FLAGS) pushed = pushed || __ldcg(&q->pushed) != 0;
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (FLAGS) pushed = __any_sync(0xffffffffu, pushed);
+        if (lane == src) {
+            const int row = __ldg(&p.split[at].row);
+            p.arrived[at] = 0;
+            p.diff[row] = sum;
+            if (FLAGS) p.active[row] = pushed ? 1 : 0;
+        }
+    }
+}
+
+template <typename R, bool FLAGS, int UN, int US>
+__device__ void pull_rows(const PartView<R> &p, const R *table_ptr, int warp, int n_warps) {
+    const int lane = threadIdx.x & 31;
+    // in registers: the gathers below are opaque to the compiler, which would fetch the view's fields again after each
+    const unsigned table = (unsigned)__cvta_generic_to_shared(table_ptr);
+    const int table_n = p.table_n, n_chunks = p.n_chunks;
+    const R *push = p.push;
+    // Long rows: one warp per chunk, UN gathers per lane in flight.  The next chunk's first columns and the descriptor of
+    // the one after it are requested before the gathers of the current one.  (The loops are kept rolled: unrolled by the
+    // compiler they spilled, which cost more than the loop.)
+    const int4 *chunks = reinterpret_cast<const int4 *>(p.chunks);
+    const int *cols = p.col + lane;
+    const int4 none = make_int4(0, 0, 0, -1);
+    int noted = 0, my_slot = -1;
+    int4 ch = warp < n_chunks ? __ldg(chunks + warp) : none;
+    int4 ahead = warp + n_warps < n_chunks ? __ldg(chunks + warp + n_warps) : none;
+    int c[UN];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) c[u] = u * 32 + lane < ch.z ? __ldcs(cols + ch.y + u * 32) : 0;
+#pragma unroll 1
+    for (int i = warp; i < n_chunks; i += n_warps) {
+        int cn[UN];
+#pragma unroll
+        for (int u = 0; u < UN; ++u) cn[u] = u * 32 + lane < ahead.z ? __ldcs(cols + ahead.y + u * 32) : 0;
+        const int4 after = i + 2 * n_warps < n_chunks ? __ldg(chunks + i + 2 * n_warps) : none;
+        R sum = 0;
+        bool pushed = false;
+#pragma unroll 1
+        for (int k = 0; k < ch.z; k += UN * 32) {
+            R v[UN];
+            if (k > 0) {
+#pragma unroll
+                for (int u = 0; u < UN; ++u) c[u] = k + u * 32 + lane < ch.z ? __ldcs(cols + ch.y + k + u * 32) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < UN; ++u) {      // lanes beyond the chunk read place 0 and count as not pushed
+                v[u] = published(table, table_n, push, c[u]);
+                if (k + u * 32 + lane >= ch.z) v[u] = not_pushed<R>();
+            }
+#pragma unroll
+            for (int u = 0; u < UN; ++u) {
+                sum += v[u];
+                if (FLAGS) pushed = pushed || is_pushed(v[u]);
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (FLAGS) pushed = __any_sync(0xffffffffu, pushed);
+        if (ch.w < 0) {
+            if (lane == 0) {
+                p.diff[ch.x] = sum;
+                if (FLAGS) p.active[ch.x] = pushed ? 1 : 0;
+            }
+        } else {
+            if (lane == 0) {
+                Partial<R> q;
+                q.sum = sum;
+                q.pushed = pushed ? 1 : 0;
+                p.partials[ch.w] = q;
+            }
+            if (lane == noted) my_slot = ch.w;
+            if (++noted == 32) {
+                close_slots<R, FLAGS>(p, my_slot);
+                noted = 0;
+                my_slot = -1;
+            }
+        }
+        ch = ahead;
+        ahead = after;
+#pragma unroll
+        for (int u = 0; u < UN; ++u) c[u] = cn[u];
+    }
+    close_slots<R, FLAGS>(p, my_slot);
+    // Short rows through the plan's stream (columns with an end-of-row flag, ranges of whole rows): a warp takes up to
+    // eight neighbouring ranges, one lane per entry and four entries per lane in flight, so the column reads are
+    // coalesced; the sums of the rows inside 32 entries come from a segmented scan (fixed tree order), a row that
+    // continues into the next 32 carries its sum over.  The warps go on where the chunks left off.
+    const int n_ranges = p.n_ranges, per_item = min(8, max(1, n_ranges / n_warps));
+    const int n_items = (n_ranges + per_item - 1) / per_item;
+    const int *range_row = p.s_range_row, *s_rowptr = p.s_rowptr, *s_rows = p.s_rows, *s_col = p.s_col;
+    R *diff = p.diff;
+    int *active = p.active;
+    int item = (warp - n_chunks) % n_warps;
+    if (item < 0) item += n_warps;
+#pragma unroll 1
+    for (; item < n_items; item += n_warps) {
+        int ri = __ldg(range_row + item * per_item);
+        const int k0 = __ldg(s_rowptr + ri), k1 = __ldg(s_rowptr + __ldg(range_row + min((item + 1) * per_item, n_ranges)));
+        R carry = 0;
+        bool carry_pushed = false;
+        unsigned e[US];
+#pragma unroll
+        for (int u = 0; u < US; ++u) e[u] = k0 + u * 32 + lane < k1 ? (unsigned)__ldcs(s_col + k0 + u * 32 + lane) : 0u;
+#pragma unroll 1
+        for (int base = k0; base < k1; base += US * 32) {
+            unsigned en[US];
+            R v[US];
+#pragma unroll
+            for (int u = 0; u < US; ++u) {
+                const int k = base + (US + u) * 32 + lane;
+                en[u] = k < k1 ? (unsigned)__ldcs(s_col + k) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < US; ++u) {
+                const bool live = base + u * 32 + lane < k1 && !(e[u] & kPlaceholder);
+                v[u] = published(table, table_n, push, live ? (int)(e[u] & kColMask) : 0);
+                if (!live) v[u] = not_pushed<R>();
+            }
+#pragma unroll
+            for (int u = 0; u < US; ++u) {
+                const bool end = base + u * 32 + lane < k1 && (e[u] & kLastInRow);
+                const unsigned ends = __ballot_sync(0xffffffffu, end);
+                const unsigned heads = (ends << 1) | 1u;                   // lane starts a row if the lane before ended one
+                const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+                const unsigned pushers = FLAGS ? __ballot_sync(0xffffffffu, is_pushed(v[u])) : 0u;
+                R s = v[u];
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const R t = __shfl_up_sync(0xffffffffu, s, d);
+                    if (lane - d >= start) s += t;
+                }
+                bool pushed = FLAGS && (pushers & (0xffffffffu >> (31 - lane)) & (0xffffffffu << start)) != 0;
+                if (start == 0) {                                          // the row open at the start of this batch
+                    s += carry;
+                    if (FLAGS) pushed = pushed || carry_pushed;
+                }
+                if (end) {
+                    const int row = __ldg(s_rows + ri + __popc(ends & ((1u << lane) - 1u)));
+                    diff[row] = s;
+                    if (FLAGS) active[row] = pushed ? 1 : 0;
+                }
+                const R last = __shfl_sync(0xffffffffu, s, 31);
+                const bool open = !(ends >> 31);
+                carry = open ? last : (R)0;
+                if (FLAGS) {
+                    const int last_pushed = __shfl_sync(0xffffffffu, (int)pushed, 31);
+                    carry_pushed = open && last_pushed != 0;
+                }
+                ri += __popc(ends);
+                e[u] = en[u];
+            }
+        }
+    }
+}
+
+// ---- the steps as kernels of their own, for one process per GPU (the exchange between them is the transport's) ----
+
+constexpr int kPullThreads = 768;      // most threads a block of the kernels below has
+
+template <typename R, bool FLAGS>
+__global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(PartView<R> p) {
+    extern __shared__ __align__(16) char table_bytes[];
+    R *table = reinterpret_cast<R *>(table_bytes);
+    load_table(p, table);
+    __syncthreads();
+    // warps numbered across the blocks first: neighbours in the work list go to different SMs
+    pull_rows<R, FLAGS, sizeof(R) == 4 ? 8 : 4, 4>(p, table, (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x),
+                                                   (int)((blockDim.x >> 5) * gridDim.x));
+}
+
+template <typename R>
+__global__ void pr_init_kernel(PartView<R> p, R start, int power, R *block_sums) {
+    const R tot = block_sum<R>(init_vertices(p, start, power != 0, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x));
     if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
 }
 
-// scalars[0] (globalDiff) += sum of block sums, in block order.
+template <typename R>
+__global__ void pr_increment_kernel(PartView<R> p, R eps, R *block_sums) {
+    const R tot = block_sum<R>(increment_vertices(p, eps, p.scalars[1], blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x));
+    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
+}
+
+template <typename R>
+__global__ void pr_power_apply_kernel(PartView<R> p, R damping, int store, R *block_sums) {
+    const R dang = p.scalars[2];
+    const R tot = block_sum<R>(power_vertices(p, damping, dang, store != 0, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x));
+    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.scalars[3] = ((R)1 - damping) / p.global_v + damping * (dang / p.global_v);
+}
+
+// scalars[slot] += sum of block sums, lane by lane, then a fixed tree.
 template <typename R>
 __global__ void pr_fold_block_sums_kernel(const R *block_sums, int n_blocks, R *scalars, int slot) {
     if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    R s = 0;                                          // lane l adds blocks l, l+32, ...; then a fixed tree
+    R s = 0;
     for (int i = threadIdx.x; i < n_blocks; i += 32) s += block_sums[i];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (threadIdx.x == 0) scalars[slot] += s;
@@ -124,160 +522,6 @@ __global__ void pr_roll_scalars_kernel(R *scalars) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         scalars[1] += scalars[0];
         scalars[0] = 0;
-    }
-}
-
-// pr_process_messages (pr.cu:430-448) fused with pr_increment (pr.cu:51-87).
-template <typename R>
-__global__ void pr_increment_kernel(R *pr, R *acc, R *diff, Pair<R> *push, int *active, int *ubm,
-                                    const int *__restrict__ out_degree, const int *__restrict__ mirror2worker, int n,
-                                    int global_v, R eps, const R *scalars, R *block_sums,
-                                    const int *__restrict__ place) {
-    const R alpha = (R)0.85f;                // pr.cu:12 declares a float constant
-    const R one_minus_alpha = (R)1 - alpha;
-    const R gacc = scalars[1];
-    R dangling = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        active[i] = 0;
-        ubm[i] = 0;
-        const R a = acc[i] + diff[i];
-        acc[i] = a;
-        diff[i] = 0;
-        const R old = pr[i];
-        const R now = fma_r<R>(alpha, a + gacc, one_minus_alpha);
-        R d = now - old;
-        if (d < 0) d = -d;
-        Pair<R> p;
-        p.val = 0;
-        p.flag = 0;
-        if (!(d < eps)) {
-            const int od = out_degree[i];
-            if (od == 0) {
-                if (mirror2worker[i] == -1) dangling += (now - old) / global_v;
-            } else {
-                p.val = (now - old) / od;
-                p.flag = 1;
-            }
-            pr[i] = now;
-        }
-        push[place ? place[i] : i] = p;
-    }
-    const R tot = block_sum<R>(dangling);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
-}
-
-// ---- pull along in-edges: diff[v] = sum of published deltas, active[v] = any in-neighbour pushed ----
-
-// Short rows through the plan's short-row stream (columns with an end-of-row flag, ranges of whole rows): one warp
-// per range, one lane per entry, so the column reads are coalesced and 32 gathers are in flight per warp; the sums of
-// the rows inside a batch come from a segmented scan (fixed tree order), rows that continue into the next batch
-// carry their partial sum over.
-template <typename R>
-__global__ void pr_pull_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, const int *__restrict__ s_rowptr,
-                                      const int *__restrict__ s_rows, const int *__restrict__ s_col,
-                                      const Pair<R> *__restrict__ push, R *diff, int *active) {
-    const int lane = threadIdx.x & 31;
-    const long long range = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    if (range >= n_ranges) return;
-    int ri = s_range_row[range];
-    const int k0 = s_rowptr[ri], k1 = s_rowptr[s_range_row[range + 1]];
-    R carry_v = 0, carry_f = 0;
-    unsigned c_next = (k0 + lane < k1) ? (unsigned)s_col[k0 + lane] : 0u;
-    for (int base = k0; base < k1; base += 32) {
-        const unsigned c = c_next;
-        const bool live = base + lane < k1;
-        c_next = (base + 32 + lane < k1) ? (unsigned)s_col[base + 32 + lane] : 0u;
-        R v = 0, f = 0;
-        if (live && !(c & kPlaceholder)) {
-            const Pair<R> p = push[c & kColMask];
-            v = p.val;
-            f = p.flag;
-        }
-        const bool end = live && (c & kLastInRow);
-        const unsigned ends = __ballot_sync(0xffffffffu, end);
-        const unsigned heads = (ends << 1) | 1u;                       // lane starts a row if the lane before ended one
-        const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const R tv = __shfl_up_sync(0xffffffffu, v, d);
-            const R tf = __shfl_up_sync(0xffffffffu, f, d);
-            if (lane - d >= start) { v += tv; f += tf; }
-        }
-        if (start == 0) { v += carry_v; f += carry_f; }                // the row open at the start of this batch
-        if (end) {
-            const int row = s_rows[ri + __popc(ends & ((1u << lane) - 1u))];
-            diff[row] = v;
-            active[row] = f > 0 ? 1 : 0;
-        }
-        const R last_v = __shfl_sync(0xffffffffu, v, 31), last_f = __shfl_sync(0xffffffffu, f, 31);
-        const bool open = !(ends >> 31);
-        carry_v = open ? last_v : (R)0;
-        carry_f = open ? last_f : (R)0;
-        ri += __popc(ends);
-    }
-}
-
-template <typename R>
-__global__ void pr_pull_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__restrict__ col,
-                                      const Pair<R> *__restrict__ push, R *diff, int *active, Pair<R> *partials) {
-    const int lane = threadIdx.x & 31;
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    if (warp >= n_chunks) return;
-    const Chunk ch = chunks[warp];
-    R sum = 0, flag = 0;
-    int k = lane;
-    for (; k + 96 < ch.len; k += 128) {          // four independent gathers in flight per lane
-        const int c0 = col[ch.k0 + k], c1 = col[ch.k0 + k + 32], c2 = col[ch.k0 + k + 64], c3 = col[ch.k0 + k + 96];
-        const Pair<R> p0 = push[c0], p1 = push[c1], p2 = push[c2], p3 = push[c3];
-        sum += p0.val; flag += p0.flag;
-        sum += p1.val; flag += p1.flag;
-        sum += p2.val; flag += p2.flag;
-        sum += p3.val; flag += p3.flag;
-    }
-    for (; k < ch.len; k += 32) {
-        const Pair<R> p = push[col[ch.k0 + k]];
-        sum += p.val;
-        flag += p.flag;
-    }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        flag += __shfl_xor_sync(0xffffffffu, flag, o);
-    }
-    if (lane == 0) {
-        if (ch.slot < 0) {
-            diff[ch.row] = sum;
-            active[ch.row] = flag > 0 ? 1 : 0;
-        } else {
-            Pair<R> p;
-            p.val = sum;
-            p.flag = flag;
-            partials[ch.slot] = p;
-        }
-    }
-}
-
-template <typename R>
-__global__ void pr_pull_reduce_kernel(const SplitRow *__restrict__ split, int n_split,
-                                      const Pair<R> *__restrict__ partials, R *diff, int *active) {
-    const int lane = threadIdx.x & 31;
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    if (warp >= n_split) return;
-    const SplitRow sr = split[warp];
-    R sum = 0, flag = 0;
-    for (int k = lane; k < sr.nslots; k += 32) {
-        const Pair<R> p = partials[sr.slot0 + k];
-        sum += p.val;
-        flag += p.flag;
-    }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        flag += __shfl_xor_sync(0xffffffffu, flag, o);
-    }
-    if (lane == 0) {
-        diff[sr.row] = sum;
-        active[sr.row] = flag > 0 ? 1 : 0;
     }
 }
 
@@ -366,31 +610,6 @@ __global__ void pr_count_active_kernel(const int *active, int n, int *counters) 
     if (cnt) atomicAdd(counters + 4, cnt);
 }
 
-// ---- power iteration ----
-
-// publish pr/outDegree, collect dangling mass (non-mirror copies only) into block sums
-template <typename R>
-__global__ void pr_power_prepare_kernel(const R *pr, Pair<R> *push, const int *__restrict__ out_degree,
-                                        const int *__restrict__ mirror2worker, int n, R *block_sums,
-                                        const int *__restrict__ place) {
-    R dangling = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        Pair<R> p;
-        p.val = 0;
-        p.flag = 0;
-        const int od = out_degree[i];
-        if (od == 0) {
-            if (mirror2worker[i] == -1) dangling += pr[i];
-        } else {
-            p.val = pr[i] / od;
-            p.flag = 1;
-        }
-        push[place ? place[i] : i] = p;
-    }
-    const R tot = block_sum<R>(dangling);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
-}
-
 // scalars[2] += n_isolated * (common value of the isolated vertices): ids that occur in no part have no
 // edges at all, so they are dangling and all hold scalars[3]; one rank adds their mass.
 template <typename R>
@@ -398,39 +617,296 @@ __global__ void pr_power_isolated_kernel(R *scalars, long long n_isolated) {
     if (threadIdx.x == 0 && blockIdx.x == 0) scalars[2] += (R)n_isolated * scalars[3];
 }
 
-// pr' = (1-d)/V + d * (sum over in-edges + dangling/V); the isolated vertices' value follows the same rule.
-// The same pass publishes pr'/outDegree and collects the dangling mass for the next iteration.
-template <typename R>
-__global__ void pr_power_apply_kernel(R *pr, const R *diff, Pair<R> *push, const int *__restrict__ out_degree,
-                                      const int *__restrict__ mirror2worker, int n, int global_v, R damping, R *scalars,
-                                      R *block_sums, const int *__restrict__ place) {
-    const R dang = scalars[2];
-    const R base = ((R)1 - damping) / global_v;
-    R dangling = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const R now = base + damping * (diff[i] + dang / global_v);
-        pr[i] = now;
-        Pair<R> p;
-        p.val = 0;
-        p.flag = 0;
-        const int od = out_degree[i];
-        if (od == 0) {
-            if (mirror2worker[i] == -1) dangling += now;
-        } else {
-            p.val = now / od;
-            p.flag = 1;
-        }
-        push[place ? place[i] : i] = p;
-    }
-    const R tot = block_sum<R>(dangling);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
-    if (blockIdx.x == 0 && threadIdx.x == 0) scalars[3] = base + damping * (dang / global_v);
-}
-
 template <typename R>
 __global__ void pr_set_scalar_kernel(R *scalars, int slot, R value) {
     if (threadIdx.x == 0 && blockIdx.x == 0) scalars[slot] = value;
 }
+
+// ---- all supersteps in one launch, for parts that one process holds on one device ----
+//
+// A superstep of a small graph is a few microseconds of work, so launches, copies between the parts and the host's
+// look at the counts used to be nearly all of its time (R-MAT-16, four parts: 310 us per superstep of the job, two
+// parts: 117 us per power iteration).  Here one cooperative launch, one block per SM, runs supersteps back to back
+// with a grid barrier between their phases; every block works for one part, blocks are dealt to the parts by their
+// number of edges, and boundary vertices are read and written where they lie instead of being packed and copied.
+// Measured on the same graphs: 33 us per superstep of the job, 22 us per power iteration.
+
+constexpr int kMaxLocalParts = 64;
+constexpr int kHistorySteps = 128;         // supersteps of the job per launch
+constexpr unsigned kBarrierPolls = 1u << 23;   // about five seconds: the barrier gives up instead of hanging
+
+struct RunControl {
+    unsigned arrived;                      // blocks that reached a barrier, over all barriers of the launch
+    int failed;                            // a wait ran out
+    int steps, done;                       // supersteps run; 1 when the last one exchanged nothing
+    unsigned long long t_start, t_pull, t_end;   // nanoseconds: start, end of the first pull, end
+    int visited[kMaxLocalParts];
+};
+
+template <typename R, int MAXP>
+struct RunArgs {
+    int n_parts;
+    int first_block[MAXP + 1];             // part q's blocks: first_block[q] .. first_block[q + 1]
+    PartView<R> part[MAXP];
+    R *block_sums;
+    RunControl *control;
+    int *history;                          // [max_steps][n_parts][4], zero at the start
+    // job
+    R eps;
+    int peval, max_steps, count_visited;
+    // power iteration
+    R damping;
+    int iterations;
+    long long n_isolated;
+};
+
+// Every thread of the grid arrives; false when a wait ran out (in some block), then everybody returns.
+__device__ inline bool grid_barrier(RunControl *c, unsigned &phase) {
+    __shared__ int ok;
+    phase += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&c->arrived, 1u);
+        unsigned seen = 0, polls = 0;
+        int failed = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&c->arrived) : "memory");
+            if (++polls >= kBarrierPolls) atomicExch(&c->failed, 1);
+            if ((polls & 255u) == 0) failed = *(volatile int *)&c->failed;
+        } while (seen < phase && !failed);
+        __threadfence();
+        ok = failed ? 0 : 1;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ unsigned long long now_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Sum of the blocks' sums in a fixed order, the same value in every thread.
+template <typename R>
+__device__ R fold_blocks(const R *block_sums) {
+    __shared__ double total;
+    if (threadIdx.x < 32) {
+        R s = 0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += 32) s += block_sums[i];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0) total = (double)s;
+    }
+    __syncthreads();
+    return (R)total;
+}
+
+// One entry that travelled from (which = 0) or to (3) part q: in registers for few parts, up in the low and down in the
+// high half (atomics of a whole warp on one word of shared memory took longer than the exchange itself).
+template <int MAXP>
+__device__ __forceinline__ void note_moved(unsigned *moved, int *counts, int q, int which) {
+    if (MAXP <= 8) {
+#pragma unroll
+        for (int i = 0; i < (MAXP <= 8 ? MAXP : 1); ++i) moved[i] += i == q ? (which == 0 ? 1u : 0x10000u) : 0u;
+    } else {
+        atomicAdd(counts + 4 * q + which, 1);
+    }
+}
+
+template <typename R, int MAXP, bool JOB>
+__global__ void __launch_bounds__(kPullThreads, 1) pr_run_kernel(const __grid_constant__ RunArgs<R, MAXP> a) {
+    extern __shared__ __align__(16) char table_bytes[];
+    R *table = reinterpret_cast<R *>(table_bytes);
+    __shared__ PartView<R> p;
+    __shared__ R *diff_of[MAXP];
+    __shared__ int *active_of[MAXP], *ubm_of[MAXP];
+    __shared__ int counts[MAXP * 4];
+    __shared__ int me_shared;
+    if (threadIdx.x == 0) {
+        int q = 0;
+        while (q + 1 < a.n_parts && (int)blockIdx.x >= a.first_block[q + 1]) ++q;
+        me_shared = q;
+        p = a.part[q];
+    }
+    for (int q = threadIdx.x; q < a.n_parts; q += blockDim.x) {
+        diff_of[q] = a.part[q].diff;
+        active_of[q] = a.part[q].active;
+        ubm_of[q] = a.part[q].ubm;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.control->t_start = now_ns();
+    __syncthreads();
+    const int me = me_shared;
+    const int block = (int)blockIdx.x - a.first_block[me], blocks = a.first_block[me + 1] - a.first_block[me];
+    const int first = block * blockDim.x + threadIdx.x, stride = blocks * blockDim.x;
+    const int warp = (threadIdx.x >> 5) * blocks + block, n_warps = (blockDim.x >> 5) * blocks;
+    unsigned phase = 0;
+
+    R gdiff = 0, gacc = 0, iso = 0, dangling = 0;
+    if (JOB) {
+        if (!a.peval) {
+            gdiff = p.scalars[0];
+            gacc = p.scalars[1];
+        }
+    } else {
+        iso = (R)1 / (R)p.global_v;
+        dangling = init_vertices(p, iso, true, first, stride);
+    }
+    const int n_steps = JOB ? a.max_steps : a.iterations;
+    for (int step = 0; step < n_steps; ++step) {
+        if (JOB) {
+            if (a.peval && step == 0) {
+                dangling = init_vertices(p, (R)1, false, first, stride);
+            } else {
+                gacc += gdiff;
+                dangling = increment_vertices(p, a.eps, gacc, first, stride);
+            }
+        }
+        const R mine = block_sum<R>(dangling);
+        if (threadIdx.x == 0) a.block_sums[blockIdx.x] = mine;
+        if (!grid_barrier(a.control, phase)) return;
+        load_table(p, table);
+        const R dang = fold_blocks<R>(a.block_sums);      // its barrier also closes the table
+        pull_rows<R, JOB, sizeof(R) == 4 ? 8 : 4, 4>(p, table, warp, n_warps);
+        if (JOB) gdiff = dang;
+        if (!grid_barrier(a.control, phase)) return;
+        if (JOB && step == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.control->t_pull = now_ns();
+        if (a.n_parts > 1) {
+            // a master takes what its mirrors hold, in ascending rank order, and hands the total back (Mirror2MasterSend,
+            // pr.cu:215-297, Master2MirrorSend, :299-373); in the job only flagged entries travel, and they are counted
+            if (JOB) {
+                for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x) counts[q] = 0;
+                __syncthreads();
+            }
+            int received = 0, sent = 0;
+            unsigned moved[MAXP <= 8 ? MAXP : 1] = {0};
+#pragma unroll 1
+            for (int m = first; m < p.n_masters; m += stride) {
+                const int row = __ldg(p.m_rows + m), k0 = __ldg(p.m_off + m), k1 = __ldg(p.m_off + m + 1);
+                R d = p.diff[row];
+                const int own = JOB ? p.active[row] : 0;
+                int got = 0;
+                // four mirrors at a time, their loads in flight together (most masters have fewer)
+                for (int k = k0; k < k1; k += 4) {
+                    int2 from[4];
+                    int flag[4];
+                    R v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) from[u] = k + u < k1 ? p.pairs[k + u] : make_int2(-1, 0);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        flag[u] = from[u].x < 0 ? 0 : JOB ? active_of[from[u].x][from[u].y] : 1;
+                        v[u] = from[u].x < 0 ? (R)0 : diff_of[from[u].x][from[u].y];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (flag[u] == 0) continue;
+                        d += v[u];
+                        if (JOB) {
+                            ++got;
+                            note_moved<MAXP>(moved, counts, from[u].x, 0);
+                        }
+                    }
+                }
+                if (JOB) {
+                    received += got;
+                    if (got) {
+                        p.diff[row] = d;
+                        p.ubm[row] = 1;
+                    }
+                    if (!got && own == 0) continue;
+                    sent += k1 - k0;
+                } else {
+                    p.diff[row] = d;
+                }
+                for (int k = k0; k < k1; ++k) {
+                    const int2 to = p.pairs[k];
+                    diff_of[to.x][to.y] = d;
+                    if (JOB) {
+                        ubm_of[to.x][to.y] = 1;
+                        note_moved<MAXP>(moved, counts, to.x, 3);
+                    }
+                }
+            }
+            if (JOB) {
+                received = __reduce_add_sync(0xffffffffu, received);
+                sent = __reduce_add_sync(0xffffffffu, sent);
+                if ((threadIdx.x & 31) == 0) {
+                    if (received) atomicAdd(&counts[4 * me + 1], received);
+                    if (sent) atomicAdd(&counts[4 * me + 2], sent);
+                }
+                if (MAXP <= 8) {
+#pragma unroll
+                    for (int q = 0; q < (MAXP <= 8 ? MAXP : 1); ++q) {
+                        const unsigned up = __reduce_add_sync(0xffffffffu, moved[q] & 0xffffu);
+                        const unsigned down = __reduce_add_sync(0xffffffffu, moved[q] >> 16);
+                        if ((threadIdx.x & 31) == 0 && up) atomicAdd(&counts[4 * q], (int)up);
+                        if ((threadIdx.x & 31) == 0 && down) atomicAdd(&counts[4 * q + 3], (int)down);
+                    }
+                }
+                __syncthreads();
+                int *h = a.history + (long long)step * a.n_parts * 4;
+                for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x)
+                    if (counts[q]) atomicAdd(h + q, counts[q]);
+            }
+            if (!grid_barrier(a.control, phase)) return;
+        }
+        if (JOB) {
+            int sent = 0;      // every block looks at the counts of all parts
+            if (a.n_parts > 1)
+                for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x) sent |= __ldcg(a.history + (long long)step * a.n_parts * 4 + q);
+            const bool done = __syncthreads_or(sent) == 0;
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                a.control->steps = step + 1;
+                a.control->done = done ? 1 : 0;
+            }
+            if (done) break;
+        } else {
+            const R all = dang + (R)a.n_isolated * iso;
+            const bool last = step + 1 == n_steps;
+            dangling = power_vertices(p, a.damping, all, last, first, stride);
+            iso = ((R)1 - a.damping) / p.global_v + a.damping * (all / p.global_v);
+        }
+    }
+    if (JOB) {
+        if (block == 0 && threadIdx.x == 0) {
+            p.scalars[0] = gdiff;
+            p.scalars[1] = gacc;
+        }
+        if (a.count_visited) {      // VisitedSize: the barrier after the pull made every block's flags visible
+            int seen = 0;
+            for (int i = first; i < p.n; i += stride) seen += p.active[i] != 0;
+            seen = __reduce_add_sync(0xffffffffu, seen);
+            if ((threadIdx.x & 31) == 0 && seen) atomicAdd(&a.control->visited[me], seen);
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.control->t_end = now_ns();
+}
+
+// slot_split[slot] = index of the split row the slot belongs to
+__global__ void pr_slot_split_kernel(const SplitRow *__restrict__ split, int n_split, int *slot_split) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_split; i += gridDim.x * blockDim.x)
+        for (int k = 0; k < split[i].nslots; ++k) slot_split[split[i].slot0 + k] = i;
+}
+
+// pairs[k] = {part, row} behind position m_pos[k] of part q's receive buffer: peer p's entries start at down_off[p]
+// there and are, in the same order, peer p's up list for q.
+struct PeerLists {
+    int down_off[kMaxLocalParts + 1];
+    const int *up_rows[kMaxLocalParts];    // start of each peer's list for this part
+};
+
+__global__ void pr_pairs_kernel(const int *__restrict__ m_pos, int n, const __grid_constant__ PeerLists peers, int n_parts,
+                                int2 *pairs) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int pos = m_pos[k];
+        int q = 0;
+        while (q + 1 < n_parts && pos >= peers.down_off[q + 1]) ++q;
+        pairs[k] = make_int2(q, peers.up_rows[q][pos - peers.down_off[q]]);
+    }
+}
+
+// ---- host side ----
 
 static inline int grid1d(long long n, int cap = 148 * 16) {
     long long g = (n + 255) / 256;
@@ -439,18 +915,75 @@ static inline int grid1d(long long n, int cap = 148 * 16) {
     return (int)g;
 }
 
-// Moves the packed boundary entries: up == true sends my `up` slices and receives `down` slices.
-struct Transport {
-    virtual int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, bool dbl, cudaStream_t st) = 0;
-    // where the entries sent to part p lie after move(): its receive buffer unless the transport delivers elsewhere
-    virtual const void *received(drone_pr *p) { return p->recv; }
-    virtual int allreduce(std::vector<drone_pr *> &parts, int slot, bool dbl, cudaStream_t st) = 0;
-    virtual ~Transport() {}
-};
+// Fewer vertices than this lie in local-id order: all their published values fit the table in either type, so ordering
+// them by how often they are gathered (a sort at creation) would gain nothing.
+constexpr long long kOrderMinRows = 16 << 10;
+constexpr int kTableBytes = 160 * 1024;        // shared memory for the table; the rest of the SM serves as L1, whose lines are
+                                               // what gathers in flight wait in (R-MAT-22: 5.3 ms with 64 to 160 KB, 7.0 with 200)
 
-struct NcclTransport : Transport {
-    int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, bool dbl, cudaStream_t st) override {
-        drone_pr *p = parts[0];
+// View of part p for a pull by `blocks` blocks.  The table holds no more values than a block has edges to gather for
+// (filling it costs a read per value, which a small graph's gathers would not pay back), and is left out where the
+// published values lie in no particular order and do not all fit.
+template <typename R>
+static PartView<R> part_view(const drone_pr *p, int blocks) {
+    const Side &s = p->plan->side[DRONE_OP_AT];
+    const drone_xplan *x = p->xplan;
+    PartView<R> v;
+    v.n = p->n_local;
+    v.global_v = p->global_v;
+    v.chunks = s.chunks;
+    v.n_chunks = s.n_chunks;
+    v.col = s.col;
+    v.s_range_row = s.s_range_row;
+    v.n_ranges = s.n_short_ranges;
+    v.s_rowptr = s.s_rowptr;
+    v.s_rows = s.s_rows;
+    v.s_col = s.s_col;
+    v.split = s.split;
+    v.slot_split = p->slot_split;
+    v.arrived = p->arrived;
+    v.partials = (Partial<R> *)p->partials;
+    v.pr = (R *)p->pr;
+    v.acc = (R *)p->acc;
+    v.diff = (R *)p->diff;
+    v.push = (R *)p->push;
+    v.scalars = (R *)p->scalars;
+    v.active = p->active;
+    v.ubm = p->ubm;
+    v.out_degree = p->out_degree;
+    v.mirror2worker = p->mirror2worker;
+    v.place = p->place;
+    v.m_rows = x->d_m_rows;
+    v.m_off = x->d_m_off;
+    v.n_masters = (int)x->m_rows.size();
+    v.pairs = p->pairs;
+    const long long capacity = kTableBytes / (long long)sizeof(R);
+    long long t = std::min<long long>(capacity, p->n_local);
+    if (!p->place && p->n_local > capacity) t = 0;
+    v.table_n = (int)std::min<long long>(t, p->nnz / std::max(blocks, 1));
+    return v;
+}
+
+template <typename Kernel>
+static int allow_table(Kernel kernel) {
+    DRONE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes));
+    return DRONE_OK;
+}
+
+template <typename R, bool FLAGS>
+static int pull(drone_pr *p, cudaStream_t st) {
+    if (p->n_local == 0) return DRONE_OK;
+    const PartView<R> v = part_view<R>(p, p->sms);
+    const int rc = allow_table(pr_pull_kernel<R, FLAGS>);
+    if (rc) return rc;
+    pr_pull_kernel<R, FLAGS><<<p->sms, kPullThreads, (size_t)v.table_n * sizeof(R), st>>>(v);
+    DRONE_LAUNCH_CHECK("pr_pull_kernel");
+    return DRONE_OK;
+}
+
+// Moves the packed boundary entries of one process per GPU: up == true sends my `up` slices and receives `down` slices.
+struct NcclTransport {
+    virtual int move(drone_pr *p, bool up, size_t pair_bytes, bool dbl, cudaStream_t st) {
         const drone_xplan *x = p->xplan;
         if (x->nranks == 1) return DRONE_OK;
         const std::vector<int> &s_off = up ? x->up_off : x->down_off;
@@ -466,21 +999,22 @@ struct NcclTransport : Transport {
         DRONE_NCCL(ncclGroupEnd());
         return DRONE_OK;
     }
-    int allreduce(std::vector<drone_pr *> &parts, int slot, bool dbl, cudaStream_t st) override {
-        drone_pr *p = parts[0];
+    // where the entries sent to part p lie after move(): its receive buffer unless the transport delivers elsewhere
+    virtual const void *received(drone_pr *p) { return p->recv; }
+    int allreduce(drone_pr *p, int slot, bool dbl, cudaStream_t st) {
         if (!p->comm || p->comm->nranks == 1) return DRONE_OK;
         char *ptr = (char *)p->scalars + (size_t)slot * (dbl ? 8 : 4);
         DRONE_NCCL(ncclAllReduce(ptr, ptr, 1, dbl ? ncclDouble : ncclFloat, ncclSum, p->comm->comm, st));
         return DRONE_OK;
     }
+    virtual ~NcclTransport() {}
 };
 
 // One process per GPU on one NVLink domain: entries are stored straight into the receiver's memory
 // (the exchange plan's peer-memory transport, exchange_p2p.cu); the scalar sums stay on NCCL.
 struct PeerTransport : NcclTransport {
     const void *landed = nullptr;
-    int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, bool, cudaStream_t st) override {
-        drone_pr *p = parts[0];
+    int move(drone_pr *p, bool up, size_t pair_bytes, bool, cudaStream_t st) override {
         if (p->xplan->nranks == 1) return DRONE_OK;
         return p2p_move_elements(p->xplan, p->send, pair_bytes, up, st, &landed);
     }
@@ -493,221 +1027,110 @@ static bool use_peer_transport(const drone_pr *p) {
     return p->xplan->p2p != nullptr && (size_t)p->xplan->max_features * 4 >= (p->dbl ? 16u : 8u);
 }
 
+// mirror -> master (add), master -> mirror (assign)
 template <typename R>
-__global__ void pr_sum_scalars_kernel(R **scalars, int n_parts, int slot) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        R s = 0;
-        for (int p = 0; p < n_parts; ++p) s += scalars[p][slot];
-        for (int p = 0; p < n_parts; ++p) scalars[p][slot] = s;
-    }
-}
-
-// all parts in one process on one device: messages are device-to-device copies
-struct LocalTransport : Transport {
-    void **d_ptrs = nullptr;
-    ~LocalTransport() override { cudaFree(d_ptrs); }
-    int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, bool, cudaStream_t st) override {
-        const int P = (int)parts.size();
-        for (int p = 0; p < P; ++p)
-            for (int q = 0; q < P; ++q) {
-                if (p == q) continue;
-                const std::vector<int> &s_off = up ? parts[p]->xplan->up_off : parts[p]->xplan->down_off;
-                const std::vector<int> &r_off = up ? parts[q]->xplan->down_off : parts[q]->xplan->up_off;
-                const size_t ns = (size_t)(s_off[q + 1] - s_off[q]), nr = (size_t)(r_off[p + 1] - r_off[p]);
-                if (ns != nr)
-                    return set_error(DRONE_E_STATE, "exchange plans disagree between parts %d and %d (%zu vs %zu rows)", p, q,
-                                     ns, nr);
-                if (ns)
-                    DRONE_CUDA(cudaMemcpyAsync((char *)parts[q]->recv + (size_t)r_off[p] * pair_bytes,
-                                               (char *)parts[p]->send + (size_t)s_off[q] * pair_bytes, ns * pair_bytes,
-                                               cudaMemcpyDeviceToDevice, st));
-            }
-        return DRONE_OK;
-    }
-    int allreduce(std::vector<drone_pr *> &parts, int slot, bool dbl, cudaStream_t st) override {
-        const int P = (int)parts.size();
-        if (!d_ptrs) DRONE_CUDA(cudaMalloc(&d_ptrs, sizeof(void *) * 64));
-        std::vector<void *> h(P);
-        for (int p = 0; p < P; ++p) h[p] = parts[p]->scalars;
-        DRONE_CUDA(cudaMemcpyAsync(d_ptrs, h.data(), sizeof(void *) * P, cudaMemcpyHostToDevice, st));
-        DRONE_CUDA(cudaStreamSynchronize(st));  // h goes out of scope
-        if (dbl) pr_sum_scalars_kernel<double><<<1, 32, 0, st>>>((double **)d_ptrs, P, slot);
-        else pr_sum_scalars_kernel<float><<<1, 32, 0, st>>>((float **)d_ptrs, P, slot);
-        DRONE_LAUNCH_CHECK("pr_sum_scalars_kernel");
-        return DRONE_OK;
-    }
-};
-
-template <typename R>
-static int pull(drone_pr *p, cudaStream_t st) {
-    const Side &s = p->plan->side[DRONE_OP_AT];
-    const int n = p->n_local;
-    (void)n;
-    if (s.n_short_ranges > 0) {
-        pr_pull_stream_kernel<R><<<ceil_div(s.n_short_ranges, 8), 256, 0, st>>>(
-            s.s_range_row, s.n_short_ranges, s.s_rowptr, s.s_rows, s.s_col, (const Pair<R> *)p->push, (R *)p->diff,
-            p->active);
-        DRONE_LAUNCH_CHECK("pr_pull_stream_kernel");
-    }
-    if (s.n_chunks > 0) {
-        pr_pull_chunks_kernel<R><<<ceil_div(s.n_chunks, 8), 256, 0, st>>>(s.chunks, s.n_chunks, s.col,
-                                                                           (const Pair<R> *)p->push, (R *)p->diff,
-                                                                           p->active, (Pair<R> *)p->partials);
-        DRONE_LAUNCH_CHECK("pr_pull_chunks_kernel");
-    }
-    if (s.n_split_rows > 0) {
-        pr_pull_reduce_kernel<R><<<ceil_div(s.n_split_rows, 8), 256, 0, st>>>(s.split, s.n_split_rows,
-                                                                               (const Pair<R> *)p->partials, (R *)p->diff,
-                                                                               p->active);
-        DRONE_LAUNCH_CHECK("pr_pull_reduce_kernel");
-    }
-    return DRONE_OK;
-}
-
-// mirror -> master (add), master -> mirror (assign), over all parts in the list
-template <typename R>
-static int exchange(std::vector<drone_pr *> &parts, Transport &tr, cudaStream_t st) {
+static int exchange(drone_pr *p, NcclTransport &tr, cudaStream_t st) {
     int rc;
-    for (drone_pr *p : parts) {
-        const drone_xplan *x = p->xplan;
-        const int n_up = (int)x->up_rows.size();
-        if (n_up) {
-            pr_pack_up_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const R *)p->diff, p->active,
-                                                              (Pair<R> *)p->send, p->counters);
-            DRONE_LAUNCH_CHECK("pr_pack_up_kernel");
-        }
+    const drone_xplan *x = p->xplan;
+    const int n_up = (int)x->up_rows.size(), n_m = (int)x->m_rows.size(), n_down = (int)x->down_rows.size();
+    if (n_up) {
+        pr_pack_up_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const R *)p->diff, p->active,
+                                                          (Pair<R> *)p->send, p->counters);
+        DRONE_LAUNCH_CHECK("pr_pack_up_kernel");
     }
-    if ((rc = tr.move(parts, true, sizeof(Pair<R>), sizeof(R) == 8, st))) return rc;
-    for (drone_pr *p : parts) {
-        const drone_xplan *x = p->xplan;
-        const int n_m = (int)x->m_rows.size(), n_down = (int)x->down_rows.size();
-        if (n_m) {
-            pr_apply_up_kernel<R><<<grid1d(n_m), 256, 0, st>>>(x->d_m_rows, x->d_m_off, x->d_m_pos, n_m,
-                                                              (const Pair<R> *)tr.received(p), (R *)p->diff, p->ubm, p->counters);
-            DRONE_LAUNCH_CHECK("pr_apply_up_kernel");
-        }
-        if (n_down) {
-            pr_pack_down_kernel<R><<<grid1d(n_down), 256, 0, st>>>(x->d_down_rows, n_down, (const R *)p->diff, p->active,
-                                                                  p->ubm, (Pair<R> *)p->send, p->counters);
-            DRONE_LAUNCH_CHECK("pr_pack_down_kernel");
-        }
+    if ((rc = tr.move(p, true, sizeof(Pair<R>), sizeof(R) == 8, st))) return rc;
+    if (n_m) {
+        pr_apply_up_kernel<R><<<grid1d(n_m), 256, 0, st>>>(x->d_m_rows, x->d_m_off, x->d_m_pos, n_m,
+                                                          (const Pair<R> *)tr.received(p), (R *)p->diff, p->ubm, p->counters);
+        DRONE_LAUNCH_CHECK("pr_apply_up_kernel");
     }
-    if ((rc = tr.move(parts, false, sizeof(Pair<R>), sizeof(R) == 8, st))) return rc;
-    for (drone_pr *p : parts) {
-        const drone_xplan *x = p->xplan;
-        const int n_up = (int)x->up_rows.size();
-        if (n_up) {
-            pr_apply_down_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const Pair<R> *)tr.received(p), (R *)p->diff,
-                                                                 p->ubm, p->counters);
-            DRONE_LAUNCH_CHECK("pr_apply_down_kernel");
-        }
+    if (n_down) {
+        pr_pack_down_kernel<R><<<grid1d(n_down), 256, 0, st>>>(x->d_down_rows, n_down, (const R *)p->diff, p->active,
+                                                              p->ubm, (Pair<R> *)p->send, p->counters);
+        DRONE_LAUNCH_CHECK("pr_pack_down_kernel");
+    }
+    if ((rc = tr.move(p, false, sizeof(Pair<R>), sizeof(R) == 8, st))) return rc;
+    if (n_up) {
+        pr_apply_down_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const Pair<R> *)tr.received(p), (R *)p->diff,
+                                                             p->ubm, p->counters);
+        DRONE_LAUNCH_CHECK("pr_apply_down_kernel");
     }
     return DRONE_OK;
 }
 
+// One superstep of the job on a rank whose boundary entries travel between GPUs.
 template <typename R>
-static int delta_step(std::vector<drone_pr *> &parts, bool peval, Transport &tr, drone_pr_response *res,
-                      cudaStream_t st) {
+static int delta_step(drone_pr *p, bool peval, NcclTransport &tr, drone_pr_response *res, cudaStream_t st) {
     using clock = std::chrono::steady_clock;
     const auto t0 = clock::now();
     int rc;
-    for (drone_pr *p : parts) {
-        if (!peval && !p->started) return set_error(DRONE_E_STATE, "PR_IncEVal called before PR_PEVal");
-        DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 8, st));
-        const int n = p->n_local;
-        const int grid = grid1d(n, kReduceBlocks);
-        if (peval) {
-            DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
-            pr_init_kernel<R><<<grid, 256, 0, st>>>((R *)p->pr, (R *)p->acc, (R *)p->diff, (Pair<R> *)p->push, p->active,
-                                                    p->ubm, p->out_degree, p->mirror2worker, n, p->global_v, (R)1,
-                                                    (R *)p->block_sums, p->place);
-            DRONE_LAUNCH_CHECK("pr_init_kernel");
-        } else {
-            pr_roll_scalars_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars);
-            DRONE_LAUNCH_CHECK("pr_roll_scalars_kernel");
-            pr_increment_kernel<R><<<grid, 256, 0, st>>>((R *)p->pr, (R *)p->acc, (R *)p->diff, (Pair<R> *)p->push,
-                                                         p->active, p->ubm, p->out_degree, p->mirror2worker, n,
-                                                         p->global_v, (R)p->eps, (const R *)p->scalars,
-                                                         (R *)p->block_sums, p->place);
-            DRONE_LAUNCH_CHECK("pr_increment_kernel");
-        }
-        pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 0);
-        DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
-        if ((rc = pull<R>(p, st))) return rc;
-        p->started = true;
+    DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 8, st));
+    const PartView<R> v = part_view<R>(p, p->sms);
+    const int grid = grid1d(p->n_local, kReduceBlocks);
+    if (peval) {
+        DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
+        pr_init_kernel<R><<<grid, 256, 0, st>>>(v, (R)1, 0, (R *)p->block_sums);
+        DRONE_LAUNCH_CHECK("pr_init_kernel");
+    } else {
+        pr_roll_scalars_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars);
+        DRONE_LAUNCH_CHECK("pr_roll_scalars_kernel");
+        pr_increment_kernel<R><<<grid, 256, 0, st>>>(v, (R)p->eps, (R *)p->block_sums);
+        DRONE_LAUNCH_CHECK("pr_increment_kernel");
     }
+    pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 0);
+    DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
+    if ((rc = pull<R, true>(p, st))) return rc;
+    p->started = true;
     DRONE_CUDA(cudaStreamSynchronize(st));
     const auto t1 = clock::now();
-    if ((rc = exchange<R>(parts, tr, st))) return rc;
-    if ((rc = tr.allreduce(parts, 0, sizeof(R) == 8, st))) return rc;
-    for (size_t i = 0; i < parts.size(); ++i) {
-        drone_pr *p = parts[i];
-        if (p->n_local > 0) {
-            pr_count_active_kernel<<<grid1d(p->n_local), 256, 0, st>>>(p->active, p->n_local, p->counters);
-            DRONE_LAUNCH_CHECK("pr_count_active_kernel");
-        }
+    if ((rc = exchange<R>(p, tr, st))) return rc;
+    if ((rc = tr.allreduce(p, 0, sizeof(R) == 8, st))) return rc;
+    if (p->n_local > 0) {
+        pr_count_active_kernel<<<grid1d(p->n_local), 256, 0, st>>>(p->active, p->n_local, p->counters);
+        DRONE_LAUNCH_CHECK("pr_count_active_kernel");
     }
-    std::vector<int> h(8 * parts.size());
-    for (size_t i = 0; i < parts.size(); ++i)
-        DRONE_CUDA(cudaMemcpyAsync(h.data() + 8 * i, parts[i]->counters, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
+    int h[8];
+    DRONE_CUDA(cudaMemcpyAsync(h, p->counters, sizeof(h), cudaMemcpyDeviceToHost, st));
     DRONE_CUDA(cudaStreamSynchronize(st));
     const auto t2 = clock::now();
-    for (size_t i = 0; i < parts.size(); ++i) {
-        drone_pr_response &r = res[i];
-        r.Mirror2MasterSendSize = h[8 * i + 0];
-        r.Mirror2MasterRecvSize = h[8 * i + 1];
-        r.Master2MirrorSendSize = h[8 * i + 2];
-        r.Master2MirrorRecvSize = h[8 * i + 3];
-        r.VisitedSize = h[8 * i + 4];
-        r.LocalVertexSize = parts[i]->n_local;
-        r.CalTime = std::chrono::duration<float>(t1 - t0).count();
-        r.SendTime = std::chrono::duration<float>(t2 - t1).count();
-    }
+    res->Mirror2MasterSendSize = h[0];
+    res->Mirror2MasterRecvSize = h[1];
+    res->Master2MirrorSendSize = h[2];
+    res->Master2MirrorRecvSize = h[3];
+    res->VisitedSize = h[4];
+    res->LocalVertexSize = p->n_local;
+    res->CalTime = std::chrono::duration<float>(t1 - t0).count();
+    res->SendTime = std::chrono::duration<float>(t2 - t1).count();
     return DRONE_OK;
 }
 
 template <typename R>
-static int power_iterations(std::vector<drone_pr *> &parts, int iterations, double damping, Transport &tr,
-                            cudaStream_t st) {
+static int power_iterations(drone_pr *p, int iterations, double damping, NcclTransport &tr, cudaStream_t st) {
     int rc;
-    for (drone_pr *p : parts) {
-        const int n = p->n_local;
-        DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
-        pr_init_kernel<R><<<grid1d(n, kReduceBlocks), 256, 0, st>>>(
-            (R *)p->pr, (R *)p->acc, (R *)p->diff, (Pair<R> *)p->push, p->active, p->ubm, p->out_degree,
-            p->mirror2worker, n, p->global_v, (R)1 / (R)p->global_v, (R *)p->block_sums, p->place);
-        DRONE_LAUNCH_CHECK("pr_init_kernel");
-        pr_set_scalar_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, 3, (R)1 / (R)p->global_v);
-        DRONE_LAUNCH_CHECK("pr_set_scalar_kernel");
-        p->started = false;
-    }
-    for (drone_pr *p : parts) {
-        pr_power_prepare_kernel<R><<<grid1d(p->n_local, kReduceBlocks), 256, 0, st>>>(
-            (const R *)p->pr, (Pair<R> *)p->push, p->out_degree, p->mirror2worker, p->n_local, (R *)p->block_sums,
-            p->place);
-        DRONE_LAUNCH_CHECK("pr_power_prepare_kernel");
-    }
+    const PartView<R> v = part_view<R>(p, p->sms);
+    const int grid = grid1d(p->n_local, kReduceBlocks);
+    const R start = (R)1 / (R)p->global_v;
+    DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
+    pr_init_kernel<R><<<grid, 256, 0, st>>>(v, start, 1, (R *)p->block_sums);
+    DRONE_LAUNCH_CHECK("pr_init_kernel");
+    pr_set_scalar_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, 3, start);
+    DRONE_LAUNCH_CHECK("pr_set_scalar_kernel");
+    p->started = false;
     for (int it = 0; it < iterations; ++it) {
-        for (drone_pr *p : parts) {
-            const int grid = grid1d(p->n_local, kReduceBlocks);
-            DRONE_CUDA(cudaMemsetAsync((char *)p->scalars + 2 * sizeof(R), 0, sizeof(R), st));
-            pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 2);
-            DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
-            if (p->xplan->rank == 0 && p->n_isolated > 0) {
-                pr_power_isolated_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, p->n_isolated);
-                DRONE_LAUNCH_CHECK("pr_power_isolated_kernel");
-            }
-            if ((rc = pull<R>(p, st))) return rc;
+        DRONE_CUDA(cudaMemsetAsync((char *)p->scalars + 2 * sizeof(R), 0, sizeof(R), st));
+        pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 2);
+        DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
+        if (p->xplan->rank == 0 && p->n_isolated > 0) {
+            pr_power_isolated_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, p->n_isolated);
+            DRONE_LAUNCH_CHECK("pr_power_isolated_kernel");
         }
-        if ((rc = exchange<R>(parts, tr, st))) return rc;
-        if ((rc = tr.allreduce(parts, 2, sizeof(R) == 8, st))) return rc;
-        for (drone_pr *p : parts) {
-            // new values, and what they publish for the next iteration, in one pass
-            pr_power_apply_kernel<R><<<grid1d(p->n_local, kReduceBlocks), 256, 0, st>>>(
-                (R *)p->pr, (const R *)p->diff, (Pair<R> *)p->push, p->out_degree, p->mirror2worker, p->n_local,
-                p->global_v, (R)damping, (R *)p->scalars, (R *)p->block_sums, p->place);
-            DRONE_LAUNCH_CHECK("pr_power_apply_kernel");
-        }
+        // with flags: the exchange's pack kernels send the rows that have some in-neighbour
+        if ((rc = pull<R, true>(p, st))) return rc;
+        if ((rc = exchange<R>(p, tr, st))) return rc;
+        if ((rc = tr.allreduce(p, 2, sizeof(R) == 8, st))) return rc;
+        // new values, and what they publish for the next iteration, in one pass
+        pr_power_apply_kernel<R><<<grid, 256, 0, st>>>(v, (R)damping, it + 1 == iterations, (R *)p->block_sums);
+        DRONE_LAUNCH_CHECK("pr_power_apply_kernel");
     }
     return DRONE_OK;
 }
@@ -720,6 +1143,164 @@ static int prepare_parts(std::vector<drone_pr *> &parts) {
     }
     return DRONE_OK;
 }
+
+// Where every part's master rows find their mirrors in the other parts' arrays; made once per set of exchange plans.
+static int prepare_pairs(std::vector<drone_pr *> &parts, cudaStream_t st) {
+    const int P = (int)parts.size();
+    std::vector<unsigned long long> key;
+    for (drone_pr *p : parts) key.push_back(p->xplan->uid);
+    for (int q = 0; q < P; ++q) {
+        drone_pr *me = parts[q];
+        const drone_xplan *x = me->xplan;
+        if (me->pairs_for == key || P == 1) continue;
+        PeerLists lists;
+        for (int p = 0; p <= P; ++p) lists.down_off[p] = x->down_off[p];
+        for (int p = 0; p < P; ++p) {
+            const drone_xplan *y = parts[p]->xplan;
+            const int ns = y->up_off[q + 1] - y->up_off[q], nr = x->down_off[p + 1] - x->down_off[p];
+            if (p != q && ns != nr)
+                return set_error(DRONE_E_STATE, "exchange plans disagree between parts %d and %d (%d vs %d rows)", p, q, ns, nr);
+            lists.up_rows[p] = y->d_up_rows + y->up_off[q];
+        }
+        const int n = (int)x->m_pos.size();
+        if (n > 0) {
+            if (!me->pairs) DRONE_CUDA(cudaMalloc(&me->pairs, sizeof(int2) * (size_t)n));
+            pr_pairs_kernel<<<grid1d(n), 256, 0, st>>>(x->d_m_pos, n, lists, P, me->pairs);
+            DRONE_LAUNCH_CHECK("pr_pairs_kernel");
+        }
+        me->pairs_for = key;
+    }
+    return DRONE_OK;
+}
+
+// What one persistent launch is asked to do.
+struct RunRequest {
+    bool job = false;              // supersteps of the job; otherwise the power iteration
+    bool peval = false, count_visited = false;
+    int max_steps = 0;
+    int iterations = 0;
+    double damping = 0;
+};
+
+template <typename R, int MAXP, bool JOB>
+static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaStream_t st) {
+    const int P = (int)parts.size();
+    drone_pr *lead = parts[0];
+    long long edges = 0;
+    for (drone_pr *p : parts) edges += (long long)p->nnz + p->n_local;
+    // A block has at least about 2048 edges and vertices to work through; more blocks only make the barriers longer.
+    const int grid = std::max(P, (int)std::min<long long>(lead->sms, (edges + 2047) / 2048));
+    // More warps hide more of a chunk's latencies (R-MAT-22: 6.5 ms with 512 threads, 5.3 with 768), fewer meet sooner at
+    // a barrier (R-MAT-16, two parts: 0.40 against 0.46 ms).
+    const int threads = edges / grid > 32768 ? kPullThreads : 512;
+    RunArgs<R, MAXP> a;
+    a.n_parts = P;
+    // blocks dealt to the parts by their share of the work, at least one each
+    long long before = 0;
+    a.first_block[0] = 0;
+    for (int q = 0; q < P; ++q) {
+        before += (long long)parts[q]->nnz + parts[q]->n_local;
+        int end = edges > 0 ? (int)((before * grid + edges / 2) / edges) : q + 1;
+        end = std::max(end, a.first_block[q] + 1);
+        end = std::min(end, grid - (P - 1 - q));
+        a.first_block[q + 1] = q + 1 == P ? grid : end;
+    }
+    size_t table = 0;
+    for (int q = 0; q < P; ++q) {
+        a.part[q] = part_view<R>(parts[q], a.first_block[q + 1] - a.first_block[q]);
+        table = std::max(table, (size_t)a.part[q].table_n * sizeof(R));
+    }
+    a.block_sums = (R *)lead->block_sums;
+    a.control = (RunControl *)lead->control;
+    a.history = (int *)(lead->control + sizeof(RunControl));
+    a.eps = (R)lead->eps;
+    a.peval = rq.peval;
+    a.max_steps = rq.max_steps;
+    a.count_visited = rq.count_visited;
+    a.damping = (R)rq.damping;
+    a.iterations = rq.iterations;
+    a.n_isolated = lead->n_isolated;
+    DRONE_CUDA(cudaMemsetAsync(lead->control, 0, sizeof(RunControl) + (JOB ? sizeof(int) * 4 * (size_t)P * rq.max_steps : 0), st));
+    const int rc = allow_table(pr_run_kernel<R, MAXP, JOB>);
+    if (rc) return rc;
+    void *args[] = {&a};
+    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)pr_run_kernel<R, MAXP, JOB>, dim3(grid), dim3(threads), args, table, st));
+    count_launch();
+    for (drone_pr *p : parts) p->started = JOB;
+    return DRONE_OK;
+}
+
+static int run_local(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaStream_t st) {
+    drone_pr *lead = parts[0];
+    const size_t need = sizeof(RunControl) + sizeof(int) * 4 * parts.size() * kHistorySteps;
+    if (need > lead->control_bytes) {      // handles of one part get theirs at creation
+        DRONE_CUDA(cudaStreamSynchronize(st));
+        cudaFree(lead->control);
+        lead->control = nullptr;
+        lead->control_bytes = 0;
+        DRONE_CUDA(cudaMalloc(&lead->control, need));
+        lead->control_bytes = need;
+    }
+    const int rc = prepare_pairs(parts, st);
+    if (rc) return rc;
+    const bool few = parts.size() <= 8;
+    if (lead->dbl) {
+        if (rq.job) return few ? launch_run<double, 8, true>(parts, rq, st) : launch_run<double, kMaxLocalParts, true>(parts, rq, st);
+        return few ? launch_run<double, 8, false>(parts, rq, st) : launch_run<double, kMaxLocalParts, false>(parts, rq, st);
+    }
+    if (rq.job) return few ? launch_run<float, 8, true>(parts, rq, st) : launch_run<float, kMaxLocalParts, true>(parts, rq, st);
+    return few ? launch_run<float, 8, false>(parts, rq, st) : launch_run<float, kMaxLocalParts, false>(parts, rq, st);
+}
+
+// What the persistent launch left: its control block and the counts of `steps` supersteps.
+static int read_control(drone_pr *lead, int n_parts, int steps, RunControl *c, int *history, cudaStream_t st) {
+    DRONE_CUDA(cudaMemcpyAsync(c, lead->control, sizeof(RunControl), cudaMemcpyDeviceToHost, st));
+    if (history)
+        DRONE_CUDA(cudaMemcpyAsync(history, lead->control + sizeof(RunControl), sizeof(int) * 4 * (size_t)n_parts * steps,
+                                   cudaMemcpyDeviceToHost, st));
+    DRONE_CUDA(cudaStreamSynchronize(st));
+    if (c->failed) return set_error(DRONE_E_STATE, "PageRank: a wait between the blocks of a superstep ran out");
+    return DRONE_OK;
+}
+
+// One superstep of all given parts.
+static int step_parts(std::vector<drone_pr *> &parts, bool peval, drone_pr_response *res, cudaStream_t st) {
+    for (drone_pr *p : parts)
+        if (!peval && !p->started) return set_error(DRONE_E_STATE, "PR_IncEVal called before PR_PEVal");
+    RunRequest rq;
+    rq.job = true;
+    rq.peval = peval;
+    rq.max_steps = 1;
+    rq.count_visited = true;
+    int rc = run_local(parts, rq, st);
+    if (rc) return rc;
+    RunControl c;
+    std::vector<int> h(4 * parts.size());
+    if ((rc = read_control(parts[0], (int)parts.size(), 1, &c, h.data(), st))) return rc;
+    for (size_t i = 0; i < parts.size(); ++i) {
+        drone_pr_response &r = res[i];
+        r.Mirror2MasterSendSize = h[4 * i + 0];
+        r.Mirror2MasterRecvSize = h[4 * i + 1];
+        r.Master2MirrorSendSize = h[4 * i + 2];
+        r.Master2MirrorRecvSize = h[4 * i + 3];
+        r.VisitedSize = c.visited[i];
+        r.LocalVertexSize = parts[i]->n_local;
+        r.CalTime = (float)((c.t_pull - c.t_start) * 1e-9);
+        r.SendTime = (float)((c.t_end - c.t_pull) * 1e-9);
+    }
+    return DRONE_OK;
+}
+
+struct OnDevice {      // the handle's device for the duration of a call
+    int prev = -1, mine = -1;
+    int enter(int device) {
+        mine = device;
+        DRONE_CUDA(cudaGetDevice(&prev));
+        if (prev != mine) DRONE_CUDA(cudaSetDevice(mine));
+        return DRONE_OK;
+    }
+    ~OnDevice() { if (prev >= 0 && prev != mine) cudaSetDevice(prev); }
+};
 
 }  // namespace drone
 
@@ -765,7 +1346,7 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         if (rc) break;
         {
             const char *v = getenv("DRONE_PR_ORDER_MIN_ROWS");
-            const long long min_rows = (v && *v) ? atoll(v) : (1LL << 22);
+            const long long min_rows = (v && *v) ? atoll(v) : kOrderMinRows;
             if (min_rows > 0 && n_local >= min_rows && nnz > 0) {
                 rc = plan_order_columns_by_frequency(p->plan, DRONE_OP_AT, d_index, &p->place, nullptr);
                 if (rc) break;
@@ -778,16 +1359,29 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         alloc(&p->pr, rs * n1);
         alloc(&p->acc, rs * n1);
         alloc(&p->diff, rs * n1);
-        alloc(&p->push, 2 * rs * n1);
+        alloc(&p->push, rs * n1);
         alloc((void **)&p->active, sizeof(int) * n1);
         alloc((void **)&p->ubm, sizeof(int) * n1);
         alloc(&p->scalars, 8 * 4);
         alloc(&p->block_sums, 8 * kReduceBlocks);
-        alloc(&p->partials, 2 * rs * (size_t)p->plan->side[DRONE_OP_AT].n_partials);
+        const Side &side = p->plan->side[DRONE_OP_AT];
+        alloc(&p->partials, 2 * rs * (size_t)side.n_partials);
+        alloc((void **)&p->slot_split, sizeof(int) * (size_t)side.n_partials);
+        alloc((void **)&p->arrived, sizeof(int) * (size_t)side.n_split_rows);
         const size_t nb = std::max(xplan->up_rows.size(), xplan->down_rows.size());
         alloc(&p->send, 2 * rs * nb);
         alloc(&p->recv, 2 * rs * nb);
         alloc((void **)&p->counters, sizeof(int) * 8);
+        p->control_bytes = sizeof(RunControl) + sizeof(int) * 4 * (size_t)xplan->nranks * kHistorySteps;
+        alloc((void **)&p->control, p->control_bytes);
+        if (e == cudaSuccess) e = cudaMemset(p->control, 0, p->control_bytes);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
+        if (e == cudaSuccess && side.n_split_rows > 0) {
+            e = cudaMemset(p->arrived, 0, sizeof(int) * (size_t)side.n_split_rows);
+            pr_slot_split_kernel<<<grid1d(side.n_split_rows), 256>>>(side.split, side.n_split_rows, p->slot_split);
+            if (e == cudaSuccess) e = cudaGetLastError();
+            count_launch();
+        }
         if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: cudaMalloc failed: %s", cudaGetErrorString(e)); break; }
         if (n_local > 0) {
             e = cudaMemcpy(p->out_degree, d_out_degree, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
@@ -813,67 +1407,88 @@ int drone_pr_destroy(drone_pr *p) {
     cudaFree(p->out_degree); cudaFree(p->mirror2worker); cudaFree(p->pr); cudaFree(p->acc); cudaFree(p->diff);
     cudaFree(p->push); cudaFree(p->active); cudaFree(p->ubm); cudaFree(p->scalars); cudaFree(p->block_sums);
     cudaFree(p->partials); cudaFree(p->send); cudaFree(p->recv); cudaFree(p->counters);
+    cudaFree(p->slot_split); cudaFree(p->arrived); cudaFree(p->pairs); cudaFree(p->control);
     if (prev >= 0) cudaSetDevice(prev);
     delete p;
     return DRONE_OK;
 }
 
-static int run_delta(std::vector<drone_pr *> &parts, bool peval, Transport &tr, drone_pr_response *res, void *stream) {
-    int rc = prepare_parts(parts);
+static int run_step(drone_pr *p, bool peval, drone_pr_response *res, void *stream) {
+    std::vector<drone_pr *> parts{p};
+    OnDevice dev;
+    int rc = dev.enter(p->device);
     if (rc) return rc;
-    int dev = -1;
-    DRONE_CUDA(cudaGetDevice(&dev));
-    if (dev != parts[0]->device) DRONE_CUDA(cudaSetDevice(parts[0]->device));
-    rc = parts[0]->dbl ? delta_step<double>(parts, peval, tr, res, (cudaStream_t)stream)
-                       : delta_step<float>(parts, peval, tr, res, (cudaStream_t)stream);
-    if (dev != parts[0]->device) cudaSetDevice(dev);
-    return rc;
+    if ((rc = prepare_parts(parts))) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (p->xplan->nranks == 1) return step_parts(parts, peval, res, st);
+    if (!peval && !p->started) return set_error(DRONE_E_STATE, "PR_IncEVal called before PR_PEVal");
+    PeerTransport peer;
+    NcclTransport nccl;
+    NcclTransport &tr = use_peer_transport(p) ? peer : nccl;
+    return p->dbl ? delta_step<double>(p, peval, tr, res, st) : delta_step<float>(p, peval, tr, res, st);
 }
 
 int drone_pr_peval(drone_pr *p, drone_pr_response *res, void *stream) {
     DRONE_REQUIRE(p && res, "drone_pr_peval: NULL argument");
     DRONE_REQUIRE(p->xplan->nranks == 1 || p->comm, "drone_pr_peval: %d ranks but no communicator", p->xplan->nranks);
-    std::vector<drone_pr *> parts{p};
-    if (use_peer_transport(p)) {
-        PeerTransport tr;
-        return run_delta(parts, true, tr, res, stream);
-    }
-    NcclTransport tr;
-    return run_delta(parts, true, tr, res, stream);
+    return run_step(p, true, res, stream);
 }
 
 int drone_pr_inceval(drone_pr *p, drone_pr_response *res, void *stream) {
     DRONE_REQUIRE(p && res, "drone_pr_inceval: NULL argument");
-    std::vector<drone_pr *> parts{p};
-    if (use_peer_transport(p)) {
-        PeerTransport tr;
-        return run_delta(parts, false, tr, res, stream);
+    DRONE_REQUIRE(p->xplan->nranks == 1 || p->comm, "drone_pr_inceval: %d ranks but no communicator", p->xplan->nranks);
+    return run_step(p, false, res, stream);
+}
+
+// The handles of all parts of one partition, as the *_local entry points take them.
+static int local_parts(const char *who, int n_parts, drone_pr **prs, std::vector<drone_pr *> *parts) {
+    DRONE_REQUIRE(n_parts >= 1 && n_parts <= kMaxLocalParts && prs, "%s: bad arguments", who);
+    parts->assign(prs, prs + n_parts);
+    for (int i = 0; i < n_parts; ++i) {
+        const drone_pr *p = (*parts)[i];
+        DRONE_REQUIRE(p && p->xplan->nranks == n_parts && p->xplan->rank == i && p->dbl == prs[0]->dbl && p->device == prs[0]->device,
+                      "%s: handle %d is not part %d of %d", who, i, i, n_parts);
     }
-    NcclTransport tr;
-    return run_delta(parts, false, tr, res, stream);
+    return DRONE_OK;
 }
 
 int drone_pr_step_local(int n_parts, drone_pr **prs, int is_peval, drone_pr_response *res, void *stream) {
-    DRONE_REQUIRE(n_parts >= 1 && n_parts <= 64 && prs && res, "drone_pr_step_local: bad arguments");
-    std::vector<drone_pr *> parts(prs, prs + n_parts);
-    for (int i = 0; i < n_parts; ++i)
-        DRONE_REQUIRE(parts[i] && parts[i]->xplan->nranks == n_parts && parts[i]->xplan->rank == i &&
-                          parts[i]->dbl == parts[0]->dbl,
-                      "drone_pr_step_local: handle %d is not part %d of %d", i, i, n_parts);
-    LocalTransport tr;
-    return run_delta(parts, is_peval != 0, tr, res, stream);
+    std::vector<drone_pr *> parts;
+    int rc = local_parts("drone_pr_step_local", n_parts, prs, &parts);
+    if (rc) return rc;
+    DRONE_REQUIRE(res != nullptr, "drone_pr_step_local: bad arguments");
+    OnDevice dev;
+    if ((rc = dev.enter(prs[0]->device)) || (rc = prepare_parts(parts))) return rc;
+    return step_parts(parts, is_peval != 0, res, (cudaStream_t)stream);
 }
 
-static int run_power(std::vector<drone_pr *> &parts, int iterations, double damping, Transport &tr, void *stream) {
-    int rc = prepare_parts(parts);
+int drone_pr_job_local(int n_parts, drone_pr **prs, int max_steps, int *n_steps, int *sizes, void *stream) {
+    std::vector<drone_pr *> parts;
+    int rc = local_parts("drone_pr_job_local", n_parts, prs, &parts);
     if (rc) return rc;
-    int dev = -1;
-    DRONE_CUDA(cudaGetDevice(&dev));
-    if (dev != parts[0]->device) DRONE_CUDA(cudaSetDevice(parts[0]->device));
-    rc = parts[0]->dbl ? power_iterations<double>(parts, iterations, damping, tr, (cudaStream_t)stream)
-                       : power_iterations<float>(parts, iterations, damping, tr, (cudaStream_t)stream);
-    if (dev != parts[0]->device) cudaSetDevice(dev);
-    return rc;
+    DRONE_REQUIRE(n_steps != nullptr && max_steps >= 1, "drone_pr_job_local: max_steps=%d, or a NULL step count", max_steps);
+    OnDevice dev;
+    if ((rc = dev.enter(prs[0]->device)) || (rc = prepare_parts(parts))) return rc;
+    RunRequest rq;
+    rq.job = true;
+    std::vector<int> h((size_t)kHistorySteps * n_parts * 4);
+    int total = 0;
+    for (RunControl c{}; !c.done && total < max_steps; total += c.steps) {
+        rq.peval = total == 0;
+        rq.max_steps = std::min(kHistorySteps, max_steps - total);
+        if ((rc = run_local(parts, rq, (cudaStream_t)stream))) return rc;
+        if ((rc = read_control(parts[0], n_parts, rq.max_steps, &c, h.data(), (cudaStream_t)stream))) return rc;
+        if (sizes) memcpy(sizes + (size_t)total * n_parts * 4, h.data(), sizeof(int) * 4 * (size_t)n_parts * c.steps);
+    }
+    *n_steps = total;
+    return DRONE_OK;
+}
+
+static int run_power(std::vector<drone_pr *> &parts, int iterations, double damping, cudaStream_t st) {
+    RunRequest rq;
+    rq.iterations = iterations;
+    rq.damping = damping;
+    return run_local(parts, rq, st);
 }
 
 int drone_pr_power_iterate(drone_pr *p, int iterations, double damping, void *stream) {
@@ -883,25 +1498,26 @@ int drone_pr_power_iterate(drone_pr *p, int iterations, double damping, void *st
     DRONE_REQUIRE(p->xplan->nranks == 1 || p->comm, "drone_pr_power_iterate: %d ranks but no communicator",
                   p->xplan->nranks);
     std::vector<drone_pr *> parts{p};
-    if (use_peer_transport(p)) {
-        PeerTransport tr;
-        return run_power(parts, iterations, damping, tr, stream);
-    }
-    NcclTransport tr;
-    return run_power(parts, iterations, damping, tr, stream);
+    OnDevice dev;
+    int rc = dev.enter(p->device);
+    if (rc || (rc = prepare_parts(parts))) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (p->xplan->nranks == 1) return run_power(parts, iterations, damping, st);
+    PeerTransport peer;
+    NcclTransport nccl;
+    NcclTransport &tr = use_peer_transport(p) ? peer : nccl;
+    return p->dbl ? power_iterations<double>(p, iterations, damping, tr, st) : power_iterations<float>(p, iterations, damping, tr, st);
 }
 
 int drone_pr_power_iterate_local(int n_parts, drone_pr **prs, int iterations, double damping, void *stream) {
-    DRONE_REQUIRE(n_parts >= 1 && n_parts <= 64 && prs, "drone_pr_power_iterate_local: bad arguments");
+    std::vector<drone_pr *> parts;
+    int rc = local_parts("drone_pr_power_iterate_local", n_parts, prs, &parts);
+    if (rc) return rc;
     DRONE_REQUIRE(iterations >= 0 && damping >= 0 && damping <= 1, "drone_pr_power_iterate_local: iterations=%d damping=%g",
                   iterations, damping);
-    std::vector<drone_pr *> parts(prs, prs + n_parts);
-    for (int i = 0; i < n_parts; ++i)
-        DRONE_REQUIRE(parts[i] && parts[i]->xplan->nranks == n_parts && parts[i]->xplan->rank == i &&
-                          parts[i]->dbl == parts[0]->dbl,
-                      "drone_pr_power_iterate_local: handle %d is not part %d of %d", i, i, n_parts);
-    LocalTransport tr;
-    return run_power(parts, iterations, damping, tr, stream);
+    OnDevice dev;
+    if ((rc = dev.enter(prs[0]->device)) || (rc = prepare_parts(parts))) return rc;
+    return run_power(parts, iterations, damping, (cudaStream_t)stream);
 }
 
 int drone_pr_set_isolated_count(drone_pr *p, long long n_isolated) {

@@ -85,18 +85,16 @@ def power_iterate_local(prs, iterations=20, damping=0.85, stream=None):
     check(_lib.lib().drone_pr_power_iterate_local(n, handles, int(iterations), float(damping), _stream_ptr(stream)))
 
 
-def run_job_local(prs, max_steps=10000):
-    """The master's loop for the job "pr_cuda" (no step cap; stops when no part exchanged anything)."""
-    res = step_local(prs, True)
-    steps = 1
-    sizes = [[(r.Mirror2MasterSendSize, r.Mirror2MasterRecvSize, r.Master2MirrorSendSize, r.Master2MirrorRecvSize)
-              for r in res]]
-    while not all(r.is_empty() for r in res) and steps < max_steps:
-        res = step_local(prs, False)
-        sizes.append([(r.Mirror2MasterSendSize, r.Mirror2MasterRecvSize, r.Master2MirrorSendSize,
-                       r.Master2MirrorRecvSize) for r in res])
-        steps += 1
-    return steps, sizes
+def run_job_local(prs, max_steps=10000, stream=None):
+    """The master's loop for the job "pr_cuda" (no step cap; stops when no part exchanged anything), inside the library.
+    Returns the number of supersteps and, per superstep, the four exchange sizes of every part."""
+    n = len(prs)
+    handles = (C.c_void_p * n)(*[p.handle for p in prs])
+    steps = C.c_int(0)
+    sizes = np.empty((max_steps, n, 4), np.int32)      # pages nobody writes cost nothing
+    check(_lib.lib().drone_pr_job_local(n, handles, int(max_steps), C.byref(steps), C.c_void_p(sizes.ctypes.data),
+                                        _stream_ptr(stream)))
+    return steps.value, [[tuple(part) for part in step] for step in sizes[:steps.value].tolist()]
 
 
 def gather_global(prs, graphs, global_v, replicas_owner=None):

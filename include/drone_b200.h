@@ -460,6 +460,10 @@ int drone_pr_set_isolated_count(drone_pr *pr, long long n_isolated);
 /* The same procedures over n_parts handles held by one process on one device
  * (prs[p] built with part p's exchange plan, comm NULL); res has n_parts entries. */
 int drone_pr_step_local(int n_parts, drone_pr **prs, int is_peval, drone_pr_response *res, void *stream);
+/* The whole job over such handles: PEval, then IncEval until no part exchanged anything (the master's stop rule,
+ * DRONE/src/master.go:430-463) or max_steps supersteps have run.  *n_steps receives their number; sizes, unless NULL,
+ * the four exchange sizes of every superstep and part, [n_steps][n_parts][4] (room for max_steps).  Synchronous. */
+int drone_pr_job_local(int n_parts, drone_pr **prs, int max_steps, int *n_steps, int *sizes, void *stream);
 int drone_pr_power_iterate_local(int n_parts, drone_pr **prs, int iterations, double damping, void *stream);
 
 /* Device arrays of the state, indexed by local id (float or double as chosen at creation): what

@@ -200,3 +200,29 @@ def test_pagerank_over_nccl_two_gpus():
     if torch.cuda.device_count() < 2:
         pytest.skip("needs two GPUs")
     run_ranks(_nccl_rank, 2, (29700 + os.getpid() % 2000,))
+
+
+@pytest.mark.parametrize("scale,parts,use_double", [(5, 2, True), (12, 12, True), (15, 9, False), (15, 1, True), (16, 3, False)])
+def test_supersteps_in_one_launch(cuda_device, oracle, scale, parts, use_double):
+    """The persistent kernel at its edges: fewer vertices than a block has threads, more than eight parts, values that do
+    and do not all fit the shared-memory table, rows of many partial sums.  The job in one launch takes the supersteps,
+    and sends the entries, that the same job driven one superstep at a time does."""
+    n, u, v, out_deg, part = pr_case(scale=scale, seed=50 + scale, parts=parts)
+    graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+    steps, sizes = prk.run_job_local(prs)
+    got = prk.gather_global(prs, graphs, n)
+    alone = [[(r.Mirror2MasterSendSize, r.Mirror2MasterRecvSize, r.Master2MirrorSendSize, r.Master2MirrorRecvSize)
+              for r in prk.step_local(prs, True)]]
+    while any(any(s) for s in alone[-1]):
+        alone.append([(r.Mirror2MasterSendSize, r.Mirror2MasterRecvSize, r.Master2MirrorSendSize, r.Master2MirrorRecvSize)
+                      for r in prk.step_local(prs, False)])
+    assert steps == len(alone) and sizes == alone
+    assert np.array_equal(got, prk.gather_global(prs, graphs, n))
+    capped, _ = prk.run_job_local(prs, max_steps=1)
+    assert capped == 1
+    prk.power_iterate_local(prs, 20, 0.85)
+    got = prk.gather_global(prs, graphs, n)
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
+    touched = part.replicas > 0
+    assert np.max(np.abs(got[touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
