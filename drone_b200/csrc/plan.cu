@@ -135,6 +135,12 @@ __global__ void fill_chunks_kernel(const int *__restrict__ rowptr, int n_rows, i
     }
 }
 
+// slot_split[slot] = index of the split row the slot belongs to
+__global__ void fill_slot_split_kernel(const SplitRow *__restrict__ split, int n_split, int *__restrict__ slot_split) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_split; i += (long long)gridDim.x * blockDim.x)
+        for (int k = 0; k < split[i].nslots; ++k) slot_split[split[i].slot0 + k] = (int)i;
+}
+
 // key[i] = first column of chunk i (tags removed), idx[i] = i
 __global__ void chunk_first_column_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__restrict__ col,
                                           int *__restrict__ key, int *__restrict__ idx) {
@@ -335,6 +341,8 @@ static void free_side(Side &s) {
     cudaFree(s.chunks);
     cudaFree(s.split);
     cudaFree(s.wide);
+    cudaFree(s.slot_split);
+    cudaFree(s.arrived);
     cudaFree(s.s_rows);
     cudaFree(s.s_rowptr);
     cudaFree(s.s_col);
@@ -409,11 +417,15 @@ static void free_lists(Side &s) {
     cudaFree(s.chunks);
     cudaFree(s.split);
     cudaFree(s.wide);
+    cudaFree(s.slot_split);
+    cudaFree(s.arrived);
     cudaFree(s.s_rows);
     cudaFree(s.s_rowptr);
     cudaFree(s.s_col);
     cudaFree(s.s_val);
     cudaFree(s.s_range_row);
+    s.slot_split = s.arrived = nullptr;
+    s.small = false;
     s.chunks = nullptr;
     s.split = s.wide = nullptr;
     s.s_rows = s.s_rowptr = s.s_col = s.s_range_row = nullptr;
@@ -476,6 +488,7 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     if ((rc = class_major_scan(p, cnt[1], off[1], scratch, tmp, tmp_bytes, slot_start, st))) return rc;
     if ((rc = class_major_scan(p, cnt[2], off[2], scratch, tmp, tmp_bytes, s.split_start, st))) return rc;
     if ((rc = class_major_scan(p, cnt[3], off[3], scratch, tmp, tmp_bytes, long_start, st))) return rc;
+    s.small = p->for_spmm && p->nnz <= env_int("DRONE_SMALL_NNZ", kSmallNnz) && s.hot_ids == nullptr;
     s.n_classes = K;
     s.n_chunks = s.chunk_start[K];
     s.n_partials = slot_start[K];
@@ -490,7 +503,13 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
         fill_chunks_kernel<<<grid_for(n), 256, 0, st>>>(s.rowptr, n, p->chunk_nnz, cnt[0], off[0], off[1], off[2],
                                                        s.chunks, s.split);
         DRONE_LAUNCH_CHECK("fill_chunks_kernel");
-        if (s.n_split_rows > 0) {
+        if (s.small && s.n_split_rows > 0) {
+            DRONE_CUDA(cudaMalloc(&s.slot_split, sizeof(int) * (size_t)s.n_partials));
+            DRONE_CUDA(cudaMalloc(&s.arrived, sizeof(int) * (size_t)s.n_split_rows));
+            DRONE_CUDA(cudaMemsetAsync(s.arrived, 0, sizeof(int) * (size_t)s.n_split_rows, st));
+            fill_slot_split_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, s.slot_split);
+            DRONE_LAUNCH_CHECK("fill_slot_split_kernel");
+        } else if (s.n_split_rows > 0) {
             int *d_max = scratch, *d_count = scratch + 1;
             DRONE_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(int), st));
             max_nslots_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, d_max);
@@ -560,8 +579,9 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     s.n_short_rows = srow_start[K];
     s.n_short_entries = sent_start[K];
     s.range_start[0] = 0;
+    const int range_nnz = s.small ? kSmallRangeNnz : kShortRangeNnz;
     for (int c = 0; c < K; ++c)
-        s.range_start[c + 1] = s.range_start[c] + ceil_div(sent_start[c + 1] - sent_start[c], kShortRangeNnz);
+        s.range_start[c + 1] = s.range_start[c] + ceil_div(sent_start[c + 1] - sent_start[c], range_nnz);
     s.n_short_ranges = s.range_start[K];
     if (s.n_short_rows > 0) {
         DRONE_CUDA(cudaMalloc(&s.s_rows, sizeof(int) * (size_t)s.n_short_rows));
@@ -579,7 +599,7 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
             const int nr = s.range_start[c + 1] - s.range_start[c];
             if (nr > 0) {
                 short_ranges_kernel<<<grid_for(nr), 256, 0, st>>>(s.s_rowptr, srow_start[c], srow_start[c + 1],
-                                                                 sent_start[c], nr, kShortRangeNnz,
+                                                                 sent_start[c], nr, range_nnz,
                                                                  s.s_range_row + s.range_start[c]);
                 DRONE_LAUNCH_CHECK("short_ranges_kernel");
             }
@@ -663,12 +683,13 @@ int validate_csr(const char *who, const int *d_index, const int *d_col, int n_ro
 
 static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_index, const int *d_dst,
                             const float *d_values, const int *d_in_degree, const int *d_out_degree,
-                            int orientations, cudaStream_t st, bool allow_tags) {
+                            int orientations, cudaStream_t st, bool for_spmm) {
     DRONE_CUDA(cudaGetDevice(&p->device));
     {
         const int rc = validate_csr("drone_plan_create", d_index, d_dst, n_rows, n_rows, nnz, st);
         if (rc) return rc;
     }
+    p->for_spmm = for_spmm;
     p->n_rows = n_rows;
     p->nnz = nnz;
     p->short_row_limit = env_int("DRONE_SHORT_ROW_LIMIT", 32);
@@ -721,7 +742,7 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
         const int min_rows = env_int("DRONE_HOT_MIN_ROWS", 1 << 23);
         long long n_hot = table_mb * (1LL << 20) / 128;
         if (n_hot > n_rows / 4) n_hot = n_rows / 4;
-        if (allow_tags && table_mb > 0 && n_rows >= min_rows && n_rows < (1 << 29) && nnz > 0 && n_hot > 0) {
+        if (for_spmm && table_mb > 0 && n_rows >= min_rows && n_rows < (1 << 29) && nnz > 0 && n_hot > 0) {
             Side &t = p->side[DRONE_OP_AT];
             int rc = DRONE_OK;
             if (orientations & DRONE_PLAN_AT) rc = tag_hot_columns(p, t, a.rowptr, (int)n_hot, st);
@@ -795,7 +816,7 @@ using namespace drone;
 extern "C" int drone_plan_destroy(drone_plan *p);
 static int plan_create_checked(drone_plan **out, int n_rows, int nnz, const int *d_index, const int *d_dst,
                                const float *d_values, const int *d_in_degree, const int *d_out_degree,
-                               int orientations, void *stream, bool allow_tags) {
+                               int orientations, void *stream, bool for_spmm) {
     DRONE_REQUIRE(out != nullptr, "drone_plan_create: out is NULL");
     *out = nullptr;
     DRONE_REQUIRE(n_rows >= 0 && nnz >= 0, "drone_plan_create: negative size (n_rows=%d, nnz=%d)", n_rows, nnz);
@@ -809,7 +830,7 @@ static int plan_create_checked(drone_plan **out, int n_rows, int nnz, const int 
     drone_plan *p = new (std::nothrow) drone_plan();
     if (!p) return set_error(DRONE_E_INVALID, "drone_plan_create: out of host memory");
     const int rc = plan_create_impl(p, n_rows, nnz, d_index, d_dst, d_values, d_in_degree, d_out_degree,
-                                    orientations, (cudaStream_t)stream, allow_tags);
+                                    orientations, (cudaStream_t)stream, for_spmm);
     if (rc != DRONE_OK) {
         drone_plan_destroy(p);
         return rc;

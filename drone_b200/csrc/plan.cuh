@@ -5,8 +5,13 @@
 
 namespace drone {
 
+// Plans with at most this many nonzeros run a call as one launch: up to here the launches of the separate kernels take
+// longer than what handing chunks out dynamically, and overlapping the two kinds of rows, gains (R-MAT directed + I, one
+// launch / separate kernels, us at F = 16 | 64: 4.3 M nonzeros 49 / 89 | 133 / 160, 8.5 M 88 / 110 | 246 / 192).
+constexpr int kSmallNnz = 6 << 20;
 constexpr int kWideSlots = 64;              // split rows above this many partial slots are reduced by a whole block
-constexpr int kShortRangeNnz = 64;          // stream entries per lane group (plus at most one more row)
+constexpr int kShortRangeNnz = 64;          // stream entries per lane group (plus at most one more row) ...
+constexpr int kSmallRangeNnz = 16;          // ... and in small plans, where one group's walk is the length of the call
 constexpr unsigned kLastInRow = 0x80000000u; // flag on s_col: last entry of its row
 constexpr unsigned kPlaceholder = 0x40000000u; // flag on s_col: row has no nonzeros, entry carries no data
 constexpr unsigned kColMask = 0x3fffffffu;
@@ -62,6 +67,11 @@ struct Side {
     int n_short_rows = 0;
     int n_short_entries = 0;
     int n_short_ranges = 0;
+    // Small plans (kSmallNnz): a call is one launch (spmm_small_kernel), in which split rows are closed by whoever
+    // arrives last; slot_split[slot] = the slot's entry of `split`, arrived[entry] = slots written so far (0 between calls)
+    bool small = false;
+    int *slot_split = nullptr; // [n_partials]
+    int *arrived = nullptr;    // [n_split_rows]
     int n_long_rows = 0;
     int n_chunks = 0;
     int n_split_rows = 0;
@@ -93,6 +103,7 @@ struct drone_plan {
     int device = 0;
     int n_rows = 0;
     int nnz = 0;
+    bool for_spmm = true;      // false: a plan whose lists other kernels of the library read (plan_create_untagged)
     int short_row_limit = 0;   // rows with deg <= this are summed by one lane group
     int chunk_nnz = 0;         // nonzeros per chunk of longer rows
     int last_slice_width = 0;  // what the most recent call used (reported by drone_plan_get_stats)
@@ -113,12 +124,11 @@ struct drone_plan {
     // tagged plans: the table of hot rows, refilled from X by every call
     float *hot_table = nullptr;
     size_t hot_table_bytes = 0;
-    // Staging for operands whose rows cannot be read as float4 (a width that is not a multiple of 4, odd leading
-    // dimensions or addresses): [pad_rows, pad_width] floats each, made by drone_plan_reserve on request.  When
-    // present and large enough, such a call copies X into pad_x with rows padded to a multiple of 4 floats, runs the
-    // float4 kernels on the padded copies and copies the result out of pad_y.
+    // Copies of X and Y with rows that can be accessed as float4, for operands whose rows cannot where they lie (a width
+    // that is not a multiple of 4, odd leading dimensions or addresses): made by drone_plan_reserve or by the first such
+    // call.  X is copied into pad_x before the kernels, the result out of pad_y after them.
     float *pad_x = nullptr, *pad_y = nullptr;
-    int pad_width = 0;
+    size_t pad_x_floats = 0, pad_y_floats = 0;
     int chunk_blocks_per_sm = 0;   // cap on resident blocks of the chunk kernel per SM (0: as many as fit)
     cudaStream_t own_stream = nullptr;
     // drone_spmm_host with pinned operands: second stream and one event per column half for the copy that runs ahead

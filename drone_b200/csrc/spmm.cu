@@ -31,24 +31,29 @@ __global__ void degree_scales_kernel(const int *__restrict__ in_deg, const int *
     out_scale[i] = out_deg[i] > 0 ? (float)(1.0 / sqrt((double)out_deg[i])) : 0.f;
 }
 
-// padded[r, 0:F] = X[r, 0:F], padded[r, F:Fp] = 0          (Fp = F rounded up to a multiple of 4)
-__global__ void pad_rows_kernel(const float *__restrict__ X, long long ldx, int n_rows, int F, int Fp,
+// padded[r, 0:F] = X[r, 0:F], padded[r, F:Fp] = 0          (Fp = F rounded up to a multiple of 4; rows `stride` floats apart)
+__global__ void pad_rows_kernel(const float *__restrict__ X, long long ldx, int n_rows, int F, int nvec, int stride,
                                 float *__restrict__ padded) {
-    const long long total = (long long)n_rows * Fp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(i / Fp), j = (int)(i - (long long)r * Fp);
-        padded[i] = j < F ? __ldg(X + (long long)r * ldx + j) : 0.f;
+    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (RowColumn at(first, step, nvec); at.row < n_rows; at.advance()) {
+        const float *x = X + (long long)at.row * ldx + 4 * at.col;
+        const int left = F - 4 * at.col;
+        float4 v;
+        v.x = left > 0 ? __ldg(x) : 0.f;
+        v.y = left > 1 ? __ldg(x + 1) : 0.f;
+        v.z = left > 2 ? __ldg(x + 2) : 0.f;
+        v.w = left > 3 ? __ldg(x + 3) : 0.f;
+        *reinterpret_cast<float4 *>(padded + (long long)at.row * stride + 4 * at.col) = v;
     }
 }
 
 // Y[row, 0:F] = padded[row, 0:F] for the rows of `rows` (rows == NULL: rows 0..n_rows-1)
 __global__ void unpad_rows_kernel(const float *__restrict__ padded, int Fp, const int *__restrict__ rows, int n_rows, int F,
                                   float *__restrict__ Y, long long ldy) {
-    const long long total = (long long)n_rows * F;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(i / F), j = (int)(i - (long long)k * F);
-        const int r = rows ? __ldg(rows + k) : k;
-        Y[(long long)r * ldy + j] = __ldcs(padded + (long long)r * Fp + j);
+    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (RowColumn at(first, step, F); at.row < n_rows; at.advance()) {
+        const int r = rows ? __ldg(rows + at.row) : at.row;
+        Y[(long long)r * ldy + at.col] = __ldcs(padded + (long long)r * Fp + at.col);
     }
 }
 
@@ -62,6 +67,48 @@ static int ensure_scratch(drone_plan *p, size_t bytes) {
     DRONE_CUDA(cudaMalloc(&p->scratch, bytes));
     p->scratch_bytes = bytes;
     return DRONE_OK;
+}
+
+// Floats between the rows of a padded copy.  A row that starts on a 128-byte line is read with one line less than one
+// that starts anywhere, and the gathers pay per line (Reddit-shaped, F = 41: 2.42 ms float by float, 1.70 copied to rows 44 apart, 1.52 to rows 64 apart), so rows wider than half a
+// line start on a line and shorter ones do not straddle one, as long as the copy then still fits the part of L2 the
+// gathers can count on; larger copies, whose rows come from HBM, start on the 64 bytes HBM delivers.
+static long long padded_stride(int n_rows, int F) {
+    const long long fp = (F + 3) & ~3;
+    long long lines = 4;
+    while (lines < fp && lines < 32) lines *= 2;
+    if (lines < fp) lines = (fp + 31) / 32 * 32;
+    if ((double)n_rows * lines * 4 <= 64e6) return lines;
+    return (fp + 15) / 16 * 16;
+}
+
+// The copies' buffers.  drone_plan_reserve makes them ahead of time; otherwise the first call that wants them does, unless
+// that call must not allocate, or they would take more than kPadBytes nobody asked for.
+constexpr size_t kPadBytes = (size_t)4 << 30;
+
+static int ensure_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
+    if (x_floats <= p->pad_x_floats && y_floats <= p->pad_y_floats) return DRONE_OK;
+    DRONE_CUDA(cudaDeviceSynchronize());      // calls in flight use the buffers about to be replaced
+    cudaFree(p->pad_x);
+    cudaFree(p->pad_y);
+    p->pad_x = p->pad_y = nullptr;
+    x_floats = std::max(x_floats, p->pad_x_floats);
+    y_floats = std::max(y_floats, p->pad_y_floats);
+    p->pad_x_floats = p->pad_y_floats = 0;
+    DRONE_CUDA(cudaMalloc(&p->pad_x, sizeof(float) * x_floats));
+    DRONE_CUDA(cudaMalloc(&p->pad_y, sizeof(float) * y_floats));
+    p->pad_x_floats = x_floats;
+    p->pad_y_floats = y_floats;
+    return DRONE_OK;
+}
+
+static bool may_allocate(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status == cudaStreamCaptureStatusNone;
 }
 
 // Width of the column slices a call is cut into (0 = no slicing).  Gathering a slice of w columns touches only
@@ -86,11 +133,12 @@ struct CallOptions {
     bool unit_values = false;
     Epilogue epi;
     drone_xplan *push_up_to = nullptr;   // the call also sends the mirror rows of Y to their owners
+    bool no_allocation = false;
 };
 
-static bool operands_allow_vec4(int F, long long ldx, long long ldy, const float *X, const float *Y) {
-    return (F % 4 == 0) && (ldx % 4 == 0) && (ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0) &&
-           ((reinterpret_cast<uintptr_t>(Y) & 15) == 0);
+// Whether rows of F floats, ld apart from base, can be accessed 16 bytes at a time.
+static bool rows_of_vectors(int F, long long ld, const float *base) {
+    return F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
 }
 
 // One launch sequence over columns [0, width) of the operands a.gather.X / a.Y point at.
@@ -116,31 +164,49 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
                      long long ldy, cudaStream_t st, const CallOptions &opt = CallOptions()) {
     const Side &s = p->side[orientation];
     if (p->n_rows == 0) return DRONE_OK;
-    bool vec4 = operands_allow_vec4(F, ldx, ldy, X, Y);
-    // Rows that cannot be read as float4 where they lie: with padded staging reserved, work on padded copies.
-    const int Fp = (F + 3) & ~3;
-    const bool padded = !vec4 && p->pad_x != nullptr && Fp <= p->pad_width && F >= 5;
+    // Operands whose rows cannot be accessed as float4 where they lie are copied to where they can (X before the kernels,
+    // Y after them): passes over [n, F] against a gather of every row as often as it has nonzeros.  Not in small plans,
+    // whose rows cost no more to read float by float than the launches of the copies.
     float *const caller_Y = Y;
     const long long caller_ldy = ldy;
     const int caller_F = F;
-    if (padded) {
-        const long long total = (long long)p->n_rows * Fp;
-        pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(X, ldx, p->n_rows, F, Fp, p->pad_x);
-        DRONE_LAUNCH_CHECK("pad_rows_kernel");
-        X = p->pad_x;
-        Y = p->pad_y;
-        ldx = ldy = F = Fp;
-        vec4 = true;
+    const bool copy_x = !rows_of_vectors(F, ldx, X), copy_y = !rows_of_vectors(F, ldy, Y);
+    bool vec4 = !copy_x && !copy_y;
+    if (!vec4 && F >= 5 && !s.small && p->nnz >= 2LL * p->n_rows) {
+        const int Fp = (F + 3) & ~3;
+        const long long stride = padded_stride(p->n_rows, F);
+        const size_t x_floats = (size_t)stride * (size_t)p->n_rows, y_floats = (size_t)Fp * (size_t)p->n_rows;
+        vec4 = x_floats <= p->pad_x_floats && y_floats <= p->pad_y_floats;
+        if (!vec4 && !opt.no_allocation && sizeof(float) * (x_floats + y_floats) <= kPadBytes && may_allocate(st)) {
+            vec4 = ensure_padding(p, x_floats, y_floats) == DRONE_OK;
+            if (!vec4) cudaGetLastError();      // no memory for the copies: the rows are accessed float by float
+        }
+        if (vec4) {
+            if (copy_x) {
+                const long long total = (long long)p->n_rows * (Fp / 4);
+                pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
+                    X, ldx, p->n_rows, F, Fp / 4, (int)stride, p->pad_x);
+                DRONE_LAUNCH_CHECK("pad_rows_kernel");
+                X = p->pad_x;
+                ldx = stride;
+            }
+            if (copy_y) {
+                Y = p->pad_y;
+                ldy = Fp;
+            }
+            F = Fp;
+        }
     }
+    const bool y_copied = vec4 && copy_y;
     // The upward half of the exchange inside this call: the kernels store mirror rows into their owners' memory
     // (rows read as float4 where they lie), or the copy kernel sends them afterwards (any other layout).
     bool routed = false, send_after = false;
     const int2 *route = nullptr;
     float *const *peer_rows = nullptr;
     if (opt.push_up_to) {
-        const int rc = p2p_route_begin(opt.push_up_to, p->n_rows, F, &route, &peer_rows);
+        const int rc = p2p_route_begin(opt.push_up_to, p->n_rows, caller_F, &route, &peer_rows);
         if (rc) return rc;
-        routed = route != nullptr && vec4 && !padded;
+        routed = route != nullptr && vec4 && !y_copied;
         send_after = route != nullptr && !routed;
     }
     const int slice = slice_width(p, F, vec4);
@@ -180,7 +246,7 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         const int rc = p2p_route_publish(opt.push_up_to, st);
         if (rc) return rc;
     }
-    if (padded) {
+    if (y_copied) {
         const int *rows = nullptr;
         int n_out = p->n_rows;
         if (opt.row_class >= 0 && p->row_order) {      // only the rows this call computed
@@ -190,7 +256,7 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         if (n_out > 0) {
             const long long total = (long long)n_out * caller_F;
             unpad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
-                p->pad_y, Fp, rows, n_out, caller_F, caller_Y, caller_ldy);
+                p->pad_y, F, rows, n_out, caller_F, caller_Y, caller_ldy);
             DRONE_LAUNCH_CHECK("unpad_rows_kernel");
         }
     }
@@ -378,18 +444,9 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
         if (!p->own_stream) DRONE_CUDA(cudaStreamCreateWithFlags(&p->own_stream, cudaStreamNonBlocking));
     }
     if ((what & DRONE_RESERVE_PADDED_ROWS) && p->n_rows > 0) {
-        const int width = (max_features + 3) & ~3;
-        if (width > p->pad_width) {
-            DRONE_CUDA(cudaDeviceSynchronize());
-            cudaFree(p->pad_x);
-            cudaFree(p->pad_y);
-            p->pad_x = p->pad_y = nullptr;
-            p->pad_width = 0;
-            const size_t bytes = sizeof(float) * (size_t)p->n_rows * (size_t)width;
-            DRONE_CUDA(cudaMalloc(&p->pad_x, bytes));
-            DRONE_CUDA(cudaMalloc(&p->pad_y, bytes));
-            p->pad_width = width;
-        }
+        long long stride = 0;      // of the widths up to max_features, the one whose copy is largest
+        for (int f = 5; f <= max_features; ++f) stride = std::max(stride, padded_stride(p->n_rows, f));
+        return ensure_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)((max_features + 3) & ~3) * (size_t)p->n_rows);
     }
     return DRONE_OK;
 }
@@ -543,7 +600,7 @@ extern "C" int drone_spmm_static_scratch(drone_plan *p, int orientation, int F, 
     if (p->n_rows == 0) return DRONE_OK;
     DRONE_REQUIRE(d_X && d_Y, "drone_spmm_static_scratch: NULL operand");
     DRONE_REQUIRE(d_X != d_Y, "drone_spmm_static_scratch: X and Y must not alias");
-    const size_t need = (size_t)s.n_partials * (size_t)((F + 3) & ~3);   // the width the kernels may run at (padded rows)
+    const size_t need = (size_t)s.n_partials * (size_t)((F + 3) & ~3);   // the width the kernels may run at (padded copy)
     if (need > drone::kStaticScratchFloats)
         return drone::set_error(DRONE_E_TOO_LARGE,
                                 "drone_spmm_static_scratch: this plan needs %zu bytes of partial sums at F=%d, the built-in "
@@ -555,15 +612,17 @@ extern "C" int drone_spmm_static_scratch(drone_plan *p, int orientation, int F, 
     float *partials = nullptr;
     int rc = drone::static_partials_address(p->device, &partials);
     if (rc == DRONE_OK) {
-        // same route as drone_spmm (padded staging when the plan has it, no column slices), with the partial sums in
-        // the built-in array: the plan's own scratch pointer is swapped for the duration of the call
+        // same route as drone_spmm (a padded copy where the plan already has room for it, no column slices), with the
+        // partial sums in the built-in array: the plan's own scratch pointer is swapped for the duration of the call
         float *const plan_scratch = p->scratch;
         const size_t plan_scratch_bytes = p->scratch_bytes;
         const int plan_slices = p->slice_forced;
         p->scratch = partials;
         p->scratch_bytes = DRONE_STATIC_SCRATCH_BYTES;
         p->slice_forced = 0;
-        rc = drone::spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream);
+        drone::CallOptions opt;
+        opt.no_allocation = true;
+        rc = drone::spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream, opt);
         p->scratch = plan_scratch;
         p->scratch_bytes = plan_scratch_bytes;
         p->slice_forced = plan_slices;

@@ -208,19 +208,16 @@ spmm_fill_hot_kernel(const int *__restrict__ hot_ids, int hot_rows, const float 
 //    its last entry has been added.  Entries of a row are added in CSR order
 //    into one accumulator.
 // ---------------------------------------------------------------------------
+// `range`: the lane group's range; groups beyond the last one only take part in the shuffles.
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
-__global__ void __launch_bounds__(256)
-spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, const int *__restrict__ s_rowptr,
-                         const int *__restrict__ s_rows, const int *__restrict__ s_col,
-                         const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec,
-                         Epilogue epi) {
+__device__ __forceinline__ void walk_short_range(long long range, const int *__restrict__ s_range_row, int n_ranges,
+                                                 const int *__restrict__ s_rowptr, const int *__restrict__ s_rows,
+                                                 const int *__restrict__ s_col, const float *__restrict__ s_val,
+                                                 const Gather &g, float *__restrict__ Y, long long ldy, int nvec,
+                                                 const Epilogue &epi) {
     using V = typename Vec<VEC>::type;
-    constexpr int RPW = 32 / G;
     constexpr int UU = MinOf<U, G>::value;
-    const int lane = threadIdx.x & 31;
-    const int gl = lane & (G - 1);
-    const int gi = lane / G;
-    const long long range = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * RPW + gi;
+    const int gl = threadIdx.x & (G - 1);
     int ri = 0, k = 0, kend = 0;
     if (range < n_ranges) {
         ri = s_range_row[range];
@@ -297,6 +294,17 @@ spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, cons
     }
 }
 
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
+__global__ void __launch_bounds__(256)
+spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, const int *__restrict__ s_rowptr,
+                         const int *__restrict__ s_rows, const int *__restrict__ s_col,
+                         const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec,
+                         Epilogue epi) {
+    const long long range = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * (32 / G) + (threadIdx.x & 31) / G;
+    walk_short_range<G, VPL, VEC, U, EXACT, UNIT, HOT>(range, s_range_row, n_ranges, s_rowptr, s_rows, s_col, s_val, g, Y,
+                                                       ldy, nvec, epi);
+}
+
 // ---------------------------------------------------------------------------
 // 2. chunks of long rows: one warp per chunk.  The warp loads 32 (col, val)
 //    pairs at a time; its 32/G lane groups take interleaved entries.  Warps take
@@ -308,14 +316,100 @@ spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, cons
 // ---------------------------------------------------------------------------
 constexpr int kChunkGroup = 4;
 
+// Sum of one chunk: nonzeros [k0, k0 + len), taken in interleaved order by the warp's lane groups; (c, v) hold the
+// lane's entry of the first 32.  Every lane group ends with the same totals in acc.
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
+__device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const int *__restrict__ col,
+                                          const float *__restrict__ val, const Gather &g, int k0, int len, int c, float v,
+                                          int nvec, unsigned long long pol_keep, unsigned long long pol_stream) {
+    using V = typename Vec<VEC>::type;
+    constexpr int RPW = 32 / G;
+    constexpr int UU = MinOf<U, G>::value;
+    const int lane = threadIdx.x & 31;
+    const int gl = lane & (G - 1);
+    const int gi = lane / G;
+#pragma unroll
+    for (int p = 0; p < VPL; ++p) acc[p] = Vec<VEC>::zero();
+
+    int base = 0;
+    // full batches of 32 entries: no bounds checks.  (col, val) of the next batch are requested before the
+    // gathers of the current one, so the dependent chain col -> X row costs one memory latency per batch
+    for (; base + 32 <= len; base += 32) {
+        int c_next = 0;
+        float v_next = UNIT ? 1.f : 0.f;
+        if (base + 32 + lane < len) {
+            c_next = ld_stream(col + k0 + base + 32 + lane, pol_stream);
+            if (!UNIT) v_next = ld_stream(val + k0 + base + 32 + lane, pol_stream);
+        }
+#pragma unroll
+        for (int t = 0; t < G; t += UU) {
+            int cc[UU];
+            float vv[UU];
+            V x[UU][VPL];
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+                cc[u] = __shfl_sync(0xffffffffu, c, (t + u) * RPW + gi);
+                vv[u] = UNIT ? 1.f : __shfl_sync(0xffffffffu, v, (t + u) * RPW + gi);
+            }
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+                const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
+#pragma unroll
+                for (int p = 0; p < VPL; ++p)
+                    x[u][p] = (EXACT || gl + p * G < nvec) ? ld_keep(xr + p * G, pol_keep)
+                                                           : Vec<VEC>::zero();
+            }
+#pragma unroll
+            for (int u = 0; u < UU; ++u)
+#pragma unroll
+                for (int p = 0; p < VPL; ++p) Vec<VEC>::fma(acc[p], vv[u], x[u][p]);
+        }
+        c = (int)resolve_column<HOT>(g, (unsigned)c_next);
+        v = v_next;
+    }
+    // last, partial batch (entries beyond the chunk were loaded as zeros)
+    if (base < len) {
+        const int cnt = len - base;
+        const int steps = (cnt + RPW - 1) / RPW;  // <= G
+        for (int t = 0; t < steps; t += UU) {
+            int cc[UU];
+            float vv[UU];
+            V x[UU][VPL];
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+                const int e = (t + u) * RPW + gi;
+                cc[u] = __shfl_sync(0xffffffffu, c, e & 31);
+                vv[u] = UNIT ? 1.f : __shfl_sync(0xffffffffu, v, e & 31);
+                if (e >= cnt) { vv[u] = 0.f; cc[u] = 0; }
+            }
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+                const bool live = (t + u) * RPW + gi < cnt;
+                const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
+#pragma unroll
+                for (int p = 0; p < VPL; ++p)
+                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_keep(xr + p * G, pol_keep)
+                                                                    : Vec<VEC>::zero();
+            }
+#pragma unroll
+            for (int u = 0; u < UU; ++u)
+#pragma unroll
+                for (int p = 0; p < VPL; ++p) Vec<VEC>::fma(acc[p], vv[u], x[u][p]);
+        }
+    }
+    // combine the lane groups (butterfly: every lane ends with the same total)
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1)
+#pragma unroll
+        for (int p = 0; p < VPL; ++p) Vec<VEC>::add(acc[p], Vec<VEC>::shfl_xor(acc[p], o));
+}
+
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
 __global__ void __launch_bounds__(256)
 spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__restrict__ col,
                    const float *__restrict__ val, Gather g, float *__restrict__ Y, long long ldy,
                    float *__restrict__ partials, int nvec, Epilogue epi, unsigned *counter) {
     using V = typename Vec<VEC>::type;
-    constexpr int RPW = 32 / G;
-    constexpr int UU = MinOf<U, G>::value;
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gi = lane / G;
@@ -358,80 +452,7 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
             }
 
             V acc[VPL];
-#pragma unroll
-            for (int p = 0; p < VPL; ++p) acc[p] = Vec<VEC>::zero();
-
-            int base = 0;
-            // full batches of 32 entries: no bounds checks.  (col, val) of the next batch are requested before the
-            // gathers of the current one, so the dependent chain col -> X row costs one memory latency per batch
-            for (; base + 32 <= len; base += 32) {
-                int c_next = 0;
-                float v_next = UNIT ? 1.f : 0.f;
-                if (base + 32 + lane < len) {
-                    c_next = ld_stream(col + k0 + base + 32 + lane, pol_stream);
-                    if (!UNIT) v_next = ld_stream(val + k0 + base + 32 + lane, pol_stream);
-                }
-#pragma unroll
-                for (int t = 0; t < G; t += UU) {
-                    int cc[UU];
-                    float vv[UU];
-                    V x[UU][VPL];
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        cc[u] = __shfl_sync(0xffffffffu, c, (t + u) * RPW + gi);
-                        vv[u] = UNIT ? 1.f : __shfl_sync(0xffffffffu, v, (t + u) * RPW + gi);
-                    }
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
-#pragma unroll
-                        for (int p = 0; p < VPL; ++p)
-                            x[u][p] = (EXACT || gl + p * G < nvec) ? ld_keep(xr + p * G, pol_keep)
-                                                                   : Vec<VEC>::zero();
-                    }
-#pragma unroll
-                    for (int u = 0; u < UU; ++u)
-#pragma unroll
-                        for (int p = 0; p < VPL; ++p) Vec<VEC>::fma(acc[p], vv[u], x[u][p]);
-                }
-                c = (int)resolve_column<HOT>(g, (unsigned)c_next);
-                v = v_next;
-            }
-            // last, partial batch (entries beyond the chunk were loaded as zeros)
-            if (base < len) {
-                const int cnt = len - base;
-                const int steps = (cnt + RPW - 1) / RPW;  // <= G
-                for (int t = 0; t < steps; t += UU) {
-                    int cc[UU];
-                    float vv[UU];
-                    V x[UU][VPL];
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        const int e = (t + u) * RPW + gi;
-                        cc[u] = __shfl_sync(0xffffffffu, c, e & 31);
-                        vv[u] = UNIT ? 1.f : __shfl_sync(0xffffffffu, v, e & 31);
-                        if (e >= cnt) { vv[u] = 0.f; cc[u] = 0; }
-                    }
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        const bool live = (t + u) * RPW + gi < cnt;
-                        const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
-#pragma unroll
-                        for (int p = 0; p < VPL; ++p)
-                            x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_keep(xr + p * G, pol_keep)
-                                                                            : Vec<VEC>::zero();
-                    }
-#pragma unroll
-                    for (int u = 0; u < UU; ++u)
-#pragma unroll
-                        for (int p = 0; p < VPL; ++p) Vec<VEC>::fma(acc[p], vv[u], x[u][p]);
-                }
-            }
-            // combine the lane groups (butterfly: every lane ends with the same total)
-#pragma unroll
-            for (int o = G; o < 32; o <<= 1)
-#pragma unroll
-                for (int p = 0; p < VPL; ++p) Vec<VEC>::add(acc[p], Vec<VEC>::shfl_xor(acc[p], o));
+            sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
 
             if (gi == 0) {
                 if (slot < 0) {
@@ -544,6 +565,105 @@ spmm_reduce_partials_kernel(const SplitRow *__restrict__ split, int n_split,
 }
 
 // ---------------------------------------------------------------------------
+// 4. small plans: the three steps in one launch.  Blocks below `chunk_blocks` take one chunk per warp, the others walk
+//    the short-row stream; the warp that writes the last partial sum of a split row (counted in `arrived`, which it
+//    sets back to 0) adds the row's slots, lane groups taking interleaved slots.  A call on such a plan is a few
+//    microseconds of work, so the memset, the four launches and the fork and join of the big plans' path used to be
+//    most of it (R-MAT-12 symmetrised, F = 16: 24 us of GPU and host time per call, 10 with this kernel; F = 64: 44, 10).
+// ---------------------------------------------------------------------------
+template <int VEC>
+__device__ __forceinline__ void store_vector(const RowDestination<VEC> &dest, int vi, const typename Vec<VEC>::type &v,
+                                             unsigned long long pol) {
+    if (dest.remote) dest.ptr[vi] = v;
+    else st_stream(dest.ptr + vi, v, pol);
+}
+
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT>
+__global__ void __launch_bounds__(256)
+spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_blocks, const int *__restrict__ col,
+                  const float *__restrict__ val, const SplitRow *__restrict__ split, const int *__restrict__ slot_split,
+                  int *arrived, float *partials, const int *__restrict__ s_range_row, int n_ranges,
+                  const int *__restrict__ s_rowptr, const int *__restrict__ s_rows, const int *__restrict__ s_col,
+                  const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec, Epilogue epi) {
+    using V = typename Vec<VEC>::type;
+    constexpr int RPW = 32 / G;
+    const int lane = threadIdx.x & 31;
+    const int gl = lane & (G - 1);
+    const int gi = lane / G;
+    if ((int)blockIdx.x >= chunk_blocks) {
+        const long long warp = (((int)blockIdx.x - chunk_blocks) * (long long)blockDim.x + threadIdx.x) >> 5;
+        walk_short_range<G, VPL, VEC, U, EXACT, UNIT, false>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
+                                                             s_val, g, Y, ldy, nvec, epi);
+        return;
+    }
+    const int at = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (at >= n_chunks) return;
+    const unsigned long long pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
+    const int4 ch = __ldg(reinterpret_cast<const int4 *>(chunks) + at);      // row, first nonzero, length, slot
+    int c = 0;
+    float v = UNIT ? 1.f : 0.f;
+    if (lane < ch.z) {
+        c = ld_stream(col + ch.y + lane, pol_stream);
+        if (!UNIT) v = ld_stream(val + ch.y + lane, pol_stream);
+    }
+    V acc[VPL];
+    sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
+    int row = ch.x;
+    if (ch.w >= 0) {
+        if (gi == 0) {
+            V *out = reinterpret_cast<V *>(partials + (long long)ch.w * nvec * VEC) + gl;
+#pragma unroll
+            for (int p = 0; p < VPL; ++p)
+                if (EXACT || gl + p * G < nvec) out[p * G] = acc[p];
+        }
+        const int which = __ldg(slot_split + ch.w);
+        const int4 sr = __ldg(reinterpret_cast<const int4 *>(split) + which);      // row, first slot, slots
+        __threadfence();
+        __syncwarp();
+        int last = 0;
+        if (lane == 0) last = atomicAdd(arrived + which, 1) == sr.z - 1;
+        if (!__shfl_sync(0xffffffffu, last, 0)) return;
+        __threadfence();
+        if (lane == 0) arrived[which] = 0;
+        // the order of spmm_reduce_partials_kernel: one pass over interleaved slots, or for many slots its eight warps'
+        // shares one after the other
+        const int shares = sr.z > kWideSlots ? 8 : 1;
+        V tot[VPL];
+        for (int w = 0; w < shares; ++w) {
+#pragma unroll
+            for (int p = 0; p < VPL; ++p) acc[p] = Vec<VEC>::zero();
+#pragma unroll 4
+            for (int sidx = w * RPW + gi; sidx < sr.z; sidx += shares * RPW) {
+                const V *pr = reinterpret_cast<const V *>(partials + (long long)(sr.y + sidx) * nvec * VEC);
+#pragma unroll
+                for (int p = 0; p < VPL; ++p)
+                    if (EXACT || gl + p * G < nvec) Vec<VEC>::add(acc[p], __ldcg(pr + gl + p * G));
+            }
+#pragma unroll
+            for (int o = G; o < 32; o <<= 1)
+#pragma unroll
+                for (int p = 0; p < VPL; ++p) Vec<VEC>::add(acc[p], Vec<VEC>::shfl_xor(acc[p], o));
+#pragma unroll
+            for (int p = 0; p < VPL; ++p) {
+                if (w == 0) tot[p] = acc[p];
+                else Vec<VEC>::add(tot[p], acc[p]);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < VPL; ++p) acc[p] = tot[p];
+        row = sr.x;
+    }
+    if (gi == 0) {
+        const float scale = epi.row_scale ? __ldg(epi.row_scale + row) : 1.f;
+        const RowDestination<VEC> dest = row_destination<VEC>(epi, Y, ldy, row);
+#pragma unroll
+        for (int p = 0; p < VPL; ++p)
+            if (EXACT || gl + p * G < nvec)
+                store_vector<VEC>(dest, gl + p * G, finish_row<VEC>(acc[p], epi, scale), pol_stream);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // dispatch
 // ---------------------------------------------------------------------------
 struct SpmmArgs {
@@ -591,6 +711,15 @@ static int launch_all(const SpmmArgs &a) {
     class_range(a.row_class, s.n_classes, s.chunk_start, &chunk_lo, &n_chunks);
     class_range(a.row_class, s.n_classes, s.split_start, &split_lo, &n_split);
     class_range(a.row_class, s.n_classes, s.wide_start, &wide_lo, &n_wide);
+    if (!HOT && s.small) {
+        const int chunk_blocks = ceil_div(n_chunks, 8), short_blocks = ceil_div(n_ranges, 8 * RPW);
+        if (chunk_blocks + short_blocks == 0) return DRONE_OK;
+        spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT><<<chunk_blocks + short_blocks, 256, 0, a.st>>>(
+            s.chunks + chunk_lo, n_chunks, chunk_blocks, s.col, s.val, s.split, s.slot_split, s.arrived, a.partials,
+            s.s_range_row + range_lo, n_ranges, s.s_rowptr, s.s_rows, s.s_col, s.s_val, a.gather, a.Y, a.ldy, a.nvec, a.epi);
+        DRONE_LAUNCH_CHECK("spmm_small_kernel");
+        return DRONE_OK;
+    }
     if (HOT && a.gather.hot_rows > 0) {
         const long long total = (long long)a.gather.hot_rows * a.nvec;
         const int grid = (int)std::min<long long>((total + 255) / 256, 148 * 16);
@@ -645,25 +774,42 @@ static int launch_exact(const SpmmArgs &a) {
     return a.nvec == G * VPL ? launch_all<G, VPL, VEC, U, true, UNIT, HOT>(a) : launch_all<G, VPL, VEC, U, false, UNIT, HOT>(a);
 }
 
-// Entry of a translation unit: picks the lane-group shape for the width (nvec vectors of VEC floats per row).
-template <int VEC, bool UNIT, bool HOT>
-static int dispatch_width(const SpmmArgs &a) {
+// Entries of a translation unit: pick the lane-group shape for the width (nvec vectors of four floats, or floats, per row).
+template <bool UNIT, bool HOT>
+static int dispatch_vectors(const SpmmArgs &a) {
     const int nv = a.nvec;
-    if (nv <= 1) return launch_exact<1, 1, VEC, 4, UNIT, HOT>(a);
-    if (nv <= 2) return launch_exact<2, 1, VEC, 4, UNIT, HOT>(a);
-    if (nv <= 4) return launch_exact<4, 1, VEC, 4, UNIT, HOT>(a);
-    if (nv <= 8) return launch_exact<8, 1, VEC, 4, UNIT, HOT>(a);
-    if (nv <= 16) return launch_exact<16, 1, VEC, 4, UNIT, HOT>(a);
-    if (nv <= 32) return launch_exact<32, 1, VEC, 4, UNIT, HOT>(a);
-    if (nv <= 64) return launch_exact<32, 2, VEC, 2, UNIT, HOT>(a);
-    if (nv <= 96) return launch_exact<32, 3, VEC, 2, UNIT, HOT>(a);
-    if (nv <= 128) return launch_exact<32, 4, VEC, 1, UNIT, HOT>(a);
-    if (nv <= 256) return launch_exact<32, 8, VEC, 1, UNIT, HOT>(a);
-    if (VEC == 1) {
-        if (nv <= 512) return launch_exact<32, 16, 1, 1, UNIT, HOT>(a);
-        if (nv <= 1024) return launch_exact<32, 32, 1, 1, UNIT, HOT>(a);
-    }
-    return set_error(DRONE_E_INVALID, "drone_spmm: feature width %d is above 1024", nv * VEC);
+    if (nv <= 1) return launch_exact<1, 1, 4, 4, UNIT, HOT>(a);
+    if (nv <= 2) return launch_exact<2, 1, 4, 4, UNIT, HOT>(a);
+    if (nv <= 4) return launch_exact<4, 1, 4, 4, UNIT, HOT>(a);
+    if (nv <= 8) return launch_exact<8, 1, 4, 4, UNIT, HOT>(a);
+    if (nv <= 16) return launch_exact<16, 1, 4, 4, UNIT, HOT>(a);
+    if (nv <= 32) return launch_exact<32, 1, 4, 4, UNIT, HOT>(a);
+    if (nv <= 64) return launch_exact<32, 2, 4, 2, UNIT, HOT>(a);
+    if (nv <= 96) return launch_exact<32, 3, 4, 2, UNIT, HOT>(a);
+    if (nv <= 128) return launch_exact<32, 4, 4, 1, UNIT, HOT>(a);
+    if (nv <= 256) return launch_exact<32, 8, 4, 1, UNIT, HOT>(a);
+    return set_error(DRONE_E_INVALID, "drone_spmm: feature width %d is above 1024", nv * 4);
+}
+
+// Rows that are read float by float: widths below 4, and wider ones for which there is no padded copy.  The latter take
+// the lane groups the padded copy would (four floats for every vector of a lane), so that a row's nonzeros are added
+// in the same order and the result has the same bits by either route.
+template <bool UNIT, bool HOT>
+static int dispatch_floats(const SpmmArgs &a) {
+    const int f = a.nvec, nv = (f + 3) / 4;
+    if (f <= 1) return launch_all<1, 1, 1, 4, true, UNIT, HOT>(a);
+    if (f <= 2) return launch_all<2, 1, 1, 4, true, UNIT, HOT>(a);
+    if (f <= 4) return launch_all<4, 1, 1, 4, false, UNIT, HOT>(a);
+    if (nv <= 2) return launch_all<2, 4, 1, 2, false, UNIT, HOT>(a);
+    if (nv <= 4) return launch_all<4, 4, 1, 2, false, UNIT, HOT>(a);
+    if (nv <= 8) return launch_all<8, 4, 1, 2, false, UNIT, HOT>(a);
+    if (nv <= 16) return launch_all<16, 4, 1, 2, false, UNIT, HOT>(a);
+    if (nv <= 32) return launch_all<32, 4, 1, 2, false, UNIT, HOT>(a);
+    if (nv <= 64) return launch_all<32, 8, 1, 1, false, UNIT, HOT>(a);
+    if (nv <= 96) return launch_all<32, 12, 1, 1, false, UNIT, HOT>(a);
+    if (nv <= 128) return launch_all<32, 16, 1, 1, false, UNIT, HOT>(a);
+    if (nv <= 256) return launch_all<32, 32, 1, 1, false, UNIT, HOT>(a);
+    return set_error(DRONE_E_INVALID, "drone_spmm: feature width %d is above 1024", f);
 }
 
 // The four combinations, each defined in a translation unit of its own (spmm_variants_*.cu).

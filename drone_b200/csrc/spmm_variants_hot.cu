@@ -7,7 +7,7 @@
 namespace drone {
 
 int spmm_dispatch_hot(const SpmmArgs &a, bool vec4) {
-    return vec4 ? dispatch_width<4, false, true>(a) : dispatch_width<1, false, true>(a);
+    return vec4 ? dispatch_vectors<false, true>(a) : dispatch_floats<false, true>(a);
 }
 
 }  // namespace drone

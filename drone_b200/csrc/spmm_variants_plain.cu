@@ -7,7 +7,7 @@
 namespace drone {
 
 int spmm_dispatch_plain(const SpmmArgs &a, bool vec4) {
-    return vec4 ? dispatch_width<4, false, false>(a) : dispatch_width<1, false, false>(a);
+    return vec4 ? dispatch_vectors<false, false>(a) : dispatch_floats<false, false>(a);
 }
 
 }  // namespace drone

@@ -7,7 +7,7 @@
 namespace drone {
 
 int spmm_dispatch_unit(const SpmmArgs &a, bool vec4) {
-    return vec4 ? dispatch_width<4, true, false>(a) : dispatch_width<1, true, false>(a);
+    return vec4 ? dispatch_vectors<true, false>(a) : dispatch_floats<true, false>(a);
 }
 
 }  // namespace drone

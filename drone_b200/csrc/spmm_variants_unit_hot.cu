@@ -7,7 +7,7 @@
 namespace drone {
 
 int spmm_dispatch_unit_hot(const SpmmArgs &a, bool vec4) {
-    return vec4 ? dispatch_width<4, true, true>(a) : dispatch_width<1, true, true>(a);
+    return vec4 ? dispatch_vectors<true, true>(a) : dispatch_floats<true, true>(a);
 }
 
 }  // namespace drone

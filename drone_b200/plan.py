@@ -105,7 +105,7 @@ class AggregationPlan:
 
     def reserve(self, max_features, host_operands=False, padded_rows=False):
         """Allocate now what calls with F <= max_features would allocate on first use (partial sums of split rows;
-        with host_operands the device staging of spmm_host; with padded_rows the staging that lets widths which are
+        with host_operands the device staging of spmm_host; with padded_rows the copy through which widths that are
         not multiples of 4 run on the float4 kernels)."""
         with torch.cuda.device(self.device):
             check(_lib.lib().drone_plan_reserve(self._h, int(max_features),
@@ -140,22 +140,24 @@ class AggregationPlan:
             raise ValueError("out must be a [n_rows, F] float32 CUDA tensor with unit inner stride")
         ldx = x.stride(0) if self.n_rows > 1 else max(f, x.stride(0))
         ldy = out.stride(0) if self.n_rows > 1 else max(f, out.stride(0))
-        with torch.cuda.device(self.device):
-            if relu or row_scale is not None or unit_values or push_up_to is not None:
-                if row_scale is not None and not (row_scale.is_cuda and row_scale.dtype == torch.float32 and
-                                                  row_scale.is_contiguous() and row_scale.numel() == self.n_rows):
-                    raise ValueError("row_scale must be a contiguous float32 CUDA tensor with one entry per row")
-                opts = SpmmOpts(EPILOGUE_RELU if relu else EPILOGUE_NONE, -1 if row_class is None else int(row_class),
-                                1 if unit_values else 0, 0, row_scale.data_ptr() if row_scale is not None else None,
-                                getattr(push_up_to, "value", push_up_to))
-                check(_lib.lib().drone_spmm_ex(self._h, int(orientation), f, _ptr(x), int(ldx), _ptr(out), int(ldy),
-                                               C.byref(opts), _stream_ptr(stream)))
-            elif row_class is None:
-                check(_lib.lib().drone_spmm(self._h, int(orientation), f, _ptr(x), int(ldx), _ptr(out), int(ldy),
-                                            _stream_ptr(stream)))
-            else:
-                check(_lib.lib().drone_spmm_rows(self._h, int(orientation), int(row_class), f, _ptr(x), int(ldx),
-                                                 _ptr(out), int(ldy), _stream_ptr(stream)))
+        # plain integers for pointers and no device context around the call (the library switches to the plan's device
+        # itself): this runs once per layer and direction, and small layers take a few microseconds on the GPU
+        lib = _lib.lib()
+        sp = stream.cuda_stream if stream is not None else torch._C._cuda_getCurrentRawStream(self.device.index)
+        if relu or row_scale is not None or unit_values or push_up_to is not None:
+            if row_scale is not None and not (row_scale.is_cuda and row_scale.dtype == torch.float32 and
+                                              row_scale.is_contiguous() and row_scale.numel() == self.n_rows):
+                raise ValueError("row_scale must be a contiguous float32 CUDA tensor with one entry per row")
+            opts = SpmmOpts(EPILOGUE_RELU if relu else EPILOGUE_NONE, -1 if row_class is None else int(row_class),
+                            1 if unit_values else 0, 0, row_scale.data_ptr() if row_scale is not None else None,
+                            getattr(push_up_to, "value", push_up_to))
+            rc = lib.drone_spmm_ex(self._h, orientation, f, x.data_ptr(), ldx, out.data_ptr(), ldy, C.byref(opts), sp)
+        elif row_class is None:
+            rc = lib.drone_spmm(self._h, orientation, f, x.data_ptr(), ldx, out.data_ptr(), ldy, sp)
+        else:
+            rc = lib.drone_spmm_rows(self._h, orientation, row_class, f, x.data_ptr(), ldx, out.data_ptr(), ldy, sp)
+        if rc:
+            check(rc)
         return out
 
     def spmm_host(self, orientation, x_host, out_host):

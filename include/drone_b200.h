@@ -194,13 +194,14 @@ int drone_spmm_rows(drone_plan *plan, int orientation, int row_class, int F,
  * Allocates, ahead of time, everything later calls of this plan would otherwise allocate on first use: the
  * partial-sum buffer of split rows for feature widths up to max_features and, as `what` asks,
  *   DRONE_RESERVE_HOST_OPERANDS  the device staging of drone_spmm_host for [n_rows, max_features] operands;
- *   DRONE_RESERVE_PADDED_ROWS    two [n_rows, max_features rounded up to 4] buffers for operands whose rows cannot
- *                                be read 16 bytes at a time where they lie (a width that is not a multiple of 4 such
- *                                as the class widths 41 and 47, odd leading dimensions, unaligned addresses).  With
- *                                them, such calls copy X into rows padded to a multiple of 4 floats, run the float4
- *                                kernels and copy the result out (two extra passes over [n_rows, F], small beside the
- *                                gathers); without them the scalar kernels run.  The two routes add in different
- *                                (each fixed) orders, so they agree to rounding, not bit for bit.
+ *   DRONE_RESERVE_PADDED_ROWS    room for copies of X and Y with padded rows, for operands whose rows cannot be accessed
+ *                                16 bytes at a time where they lie (a width that is not a multiple of 4 such as the
+ *                                class widths 41 and 47, odd leading dimensions, unaligned addresses).  Such calls copy
+ *                                X, run the float4 kernels and copy the result out (two extra passes over [n_rows, F],
+ *                                small beside the gathers); without the reservation the first such call makes the room
+ *                                itself, unless it takes more than 4 GB or the stream is being captured, and then, as
+ *                                on small graphs, the rows are accessed float by float.  Both routes add in the same
+ *                                order.
  * After it, drone_spmm / drone_spmm_rows / drone_spmm_host with F <= max_features reach neither cudaMalloc nor a
  * device-wide synchronisation.
  * Stands where the reference sizes its cuSPARSE workspace on the first training step,
@@ -250,6 +251,8 @@ int drone_spmm_host_wait(drone_plan *plan, long long ticket);
  * drone_spmm: the same kernels run in the same order, so the output is
  * bit-identical.
  * Limits and rules:
+ *  - a padded copy of X (see drone_plan_reserve) is made only where the plan
+ *    already has room for it;
  *  - a call whose plan needs more than DRONE_STATIC_SCRATCH_BYTES of partial
  *    sums (n_partials[orientation] * F * 4 bytes, see drone_plan_get_stats)
  *    fails with DRONE_E_TOO_LARGE and launches nothing;

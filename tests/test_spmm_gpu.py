@@ -552,3 +552,50 @@ def test_device_graph_build_matches_the_host_builder(cuda_device, scale, parts):
     bad = torch.tensor([3, 99], dtype=torch.int32, device=cuda_device)
     with pytest.raises(db.DroneError, match="outside"):
         pt.device_local_graph(bad, bad, 16)
+
+
+@pytest.mark.parametrize("f", [1, 3, 4, 16, 41, 63, 64, 128, 260])
+def test_one_launch_and_separate_kernels(cuda_device, oracle, f):
+    """A small plan's call is one launch; the same graph with that switched off takes the separate kernels.  Both against
+    the double oracle, repeatable, with rows of one chunk, of many (closed by the last to arrive) and without nonzeros,
+    in row classes, and in the value-free form."""
+    n, u, v = gg.rmat_graph(12, 16, seed=61, symmetrise=False, self_loops="drop")
+    index, dst, in_deg, out_deg, val = graph_case(gg, oracle, n, u.numpy(), v.numpy())
+    x = torch.as_tensor(gg.seeded_normal(300 + f, (n, f)), device=cuda_device)
+    scale = torch.as_tensor(gg.seeded_normal(5, (n, 1)), device=cuda_device)[:, 0].contiguous()
+    cls = torch.as_tensor((np.arange(n) * 7 % 3).astype(np.int32), device=cuda_device)
+    for env in ({}, {"DRONE_SMALL_NNZ": 1}, {"DRONE_SHORT_ROW_LIMIT": 4, "DRONE_CHUNK_NNZ": 8}):
+        plan = make_plan(cuda_device, index, dst, in_deg, out_deg, **env)
+        assert plan.stats().n_split_rows[db.OP_AT] > 0
+        check_both_orientations(plan, oracle, index, dst, val, x.cpu().numpy(), cuda_device)
+        whole = plan.spmm(db.OP_AT, x)
+        assert torch.equal(plan.spmm(db.OP_AT, x), whole)
+        assert torch.equal(plan.spmm(db.OP_AT, x, relu=True, row_scale=scale), torch.clamp_min(whole * scale[:, None], 0.0))
+        ones = plan.spmm(db.OP_AT, x, unit_values=True)
+        want = oracle.spmm_csr_f64(*oracle.transpose_csr(n, n, index, dst, np.ones_like(val)), x.cpu().numpy(), with_abs=True)
+        assert_close_to_oracle(ones.cpu().numpy(), *want)
+        plan.set_row_classes(cls, 3)
+        y = torch.empty_like(whole)
+        for c in (2, 0, 1):
+            plan.spmm(db.OP_AT, x, out=y, row_class=c)
+        assert torch.equal(y, whole)
+
+
+@pytest.mark.parametrize("f", [5, 13, 41, 62, 100, 127, 255, 383, 511, 1021])
+def test_copied_and_uncopied_rows_have_the_same_bits(cuda_device, oracle, f):
+    """Rows that cannot be read 16 bytes at a time, through the padded copy (drone_spmm on a plan that is not small) and
+    float by float (a small plan; the entry point that may not allocate, on a plan that has no copy yet): one order of
+    additions, so the same bits."""
+    import ctypes as C
+    n, u, v = gg.rmat_graph(10, 16, seed=62, symmetrise=False, self_loops="add")
+    index, dst, in_deg, out_deg, val = graph_case(gg, oracle, n, u.numpy(), v.numpy())
+    x = torch.as_tensor(gg.seeded_normal(400 + f, (n, f)), device=cuda_device)
+    for env in ({}, {"DRONE_SMALL_NNZ": 1}):
+        plan = make_plan(cuda_device, index, dst, in_deg, out_deg, **env)
+        y = torch.empty_like(x)
+        rc = db.lib().drone_spmm_static_scratch(plan.handle, db.OP_AT, f, C.c_void_p(x.data_ptr()), f, C.c_void_p(y.data_ptr()),
+                                                f, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0, db.lib().drone_last_error()
+        assert torch.equal(plan.spmm(db.OP_AT, x), y)
+        want, mag = oracle.spmm_csr_f64(*oracle.transpose_csr(n, n, index, dst, val), x.cpu().numpy(), with_abs=True)
+        assert_close_to_oracle(y.cpu().numpy(), want, mag)
