@@ -5,18 +5,19 @@
 // DRONE/src/cuda/algorithm/cc.cu and sssp.cu (PEval / IncEval and their helper kernels) with these changes:
 //   * one state, one set of kernels for both jobs: distances are non-negative floats, whose bit patterns order like
 //     unsigned integers, so both kinds are "atomicMin on a 32-bit word";
-//   * a warp works on 32 vertices; rows above kSerialDegree edges are spread over the warp's lanes, and rows above
-//     kHeavyDegree are cut into chunks that a second kernel hands to all warps of the grid (the reference walks
-//     every row with one thread, which a hub row turns into one long serial loop);
+//   * a local run is one launch: its rounds follow one another with a grid barrier between them instead of one or two
+//     launches each and a look from the host, and vertices wait with large values until the small ones have spread;
+//   * short rows of a frontier are walked as one flat list of edges, long ones in pieces handed to the whole grid (the
+//     reference walks every row with one thread, which a hub row turns into one long serial loop);
 //   * the exchange uses the static plan (rows in a fixed order, no ids on the wire, no allocation per superstep);
 //     every boundary vertex travels as {value, flag} and only flagged entries count and are applied, which gives the
-//     same values and the same Response sizes as the reference's lists of changed vertices;
-//   * several relaxation steps are launched per look at the "anything changed" word.
+//     same values and the same Response sizes as the reference's lists of changed vertices.
 // Labels start as GLOBAL vertex ids (the CPU job's choice, DRONE/src/algorithm/CC.go:73-79; cc_init writes the local
 // index, cc.cu:14, which cannot be compared between workers).  A shorter distance always re-activates its vertex
 // (sssp_exec asks for an improvement above 1e-6, sssp.cu:67; with the unit lengths build_graph stores both agree).
 #include "exchange.cuh"
 
+#include <algorithm>
 #include <chrono>
 #include <new>
 #include <vector>
@@ -28,28 +29,29 @@ int xplan_ensure_device(drone_xplan *x);
 }
 
 struct drone_mp {
-    int device = 0, kind = 0, n_local = 0, nnz = 0;
+    int device = 0, kind = 0, n_local = 0, nnz = 0, sms = 0;
     const int *index = nullptr, *dst = nullptr, *l2g = nullptr;   // borrowed device arrays
     const float *len = nullptr;                                   // borrowed, NULL = 1.0
     drone_xplan *xplan = nullptr;                                 // borrowed
     drone_comm *comm = nullptr;                                   // borrowed, may be NULL for one part
     unsigned *value = nullptr;     // [n] label, or the bits of a non-negative float distance
-    int *active = nullptr;         // [n] -1 idle, s = in the frontier of step s; > 0 after a run: lowered in that run
+    int *state = nullptr;          // [n] -1 idle, r = waiting to offer its value since round r
+    int *active = nullptr;         // [n] after a run: 1 lowered in it, 0 in its first frontier and not lowered, -1 neither
     int *ubm = nullptr;            // [n] lowered by a received message since the last sweep
     uint2 *send = nullptr, *recv = nullptr;   // [max(up, down)] {value, flag}
-    int *counters = nullptr;       // [0..3] exchange sizes, [4] VisitedSize, [5] "a step lowered something",
-                                   // [6] entries in `heavy`
-    int2 *heavy = nullptr;         // [heavy_cap] {vertex, chunk}: this step's chunks of frontier rows above kHeavyDegree
-    int heavy_cap = 0;
+    int *counters = nullptr;       // [0..3] exchange sizes, [4] VisitedSize; the run's control block follows them
+    int4 *items = nullptr;         // [item_cap] {first edge, edges, value, 0}: pieces of the long rows of a round's frontier
+    int item_cap = 0;
     bool started = false;
 };
 
 namespace drone {
 
-constexpr int kSerialDegree = 8;     // rows up to this many edges are walked by their own lane
-constexpr int kHeavyDegree = 4096;   // rows above this many edges are cut into chunks for the whole grid
-constexpr int kHeavyChunk = 2048;    // edges per chunk
-constexpr int kStepsPerLook = 4;     // relaxation steps launched between two reads of the changed word
+constexpr int kWarpRow = 64;         // rows up to this many edges are walked by the warp that finds them in the frontier
+constexpr int kItemEdges = 512;      // longer ones are cut into pieces of this many edges for the whole grid
+constexpr int kRunThreads = 1024;
+constexpr int kRoundsPerLaunch = 4096;
+constexpr unsigned kMpPolls = 1u << 23;      // about five seconds: the grid barrier gives up instead of hanging
 constexpr unsigned kFarBits = 0x4CBEBC20u;   // 1e8f, the reference's "not reached" (sssp.cu:33)
 
 static inline int grid_mp(long long n, int cap = 148 * 16) {
@@ -59,110 +61,295 @@ static inline int grid_mp(long long n, int cap = 148 * 16) {
     return (int)g;
 }
 
-// PEval start.  Labels: every vertex is in the frontier of step 0 with its global id.  Distances: only the source.
-__global__ void mp_init_kernel(int kind, unsigned *value, int *active, int *ubm, const int *__restrict__ l2g, int n,
-                               int source_global, int *counters) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        ubm[i] = 0;
-        if (kind == DRONE_MP_CC) {
-            value[i] = (unsigned)l2g[i];
-            active[i] = 0;
-            counters[5] = 1;
-        } else if (l2g[i] == source_global) {
-            value[i] = 0u;      // 0.0f
-            active[i] = 0;
-            counters[5] = 1;
-        } else {
-            value[i] = kFarBits;
-            active[i] = -1;
-        }
+struct MpRound {
+    int items;             // pieces of long rows in the queue
+    int offered;           // 1: some vertex of the round's frontier offered its value
+    unsigned nearest_left; // complement of the least value among the waiting vertices that lay above the limit (0: none)
+    int pad;
+};
+
+struct MpControl {
+    unsigned arrived;      // blocks that reached a barrier, over all barriers of the launch
+    int failed;            // a wait ran out
+    int unfinished;        // 1: the launch stopped after kRoundsPerLaunch rounds
+    int round;             // where the next launch goes on
+    unsigned limit;
+    int pad[3];
+    MpRound rounds[4];     // round r uses rounds[r & 3]
+};
+
+enum MpStart { kMpPeval = 0, kMpIncEval = 1, kMpContinue = 2 };
+
+struct MpArgs {
+    int n, start, source_global, item_cap;
+    const int *index, *dst, *l2g;
+    const float *len;
+    unsigned *value;
+    int *state, *active, *ubm, *counters;
+    int4 *items;
+    MpControl *control;
+};
+
+// Every thread of the grid arrives; false when a wait ran out (in some block), then everybody returns.
+__device__ inline bool mp_barrier(MpControl *c, unsigned &phase) {
+    __shared__ int ok;
+    phase += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&c->arrived, 1u);
+        unsigned seen = 0, polls = 0;
+        int failed = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&c->arrived) : "memory");
+            if (++polls >= kMpPolls) atomicExch(&c->failed, 1);
+            if ((polls & 255u) == 0) failed = *(volatile int *)&c->failed;
+        } while (seen < phase && !failed);
+        __threadfence();
+        ok = failed ? 0 : 1;
     }
+    __syncthreads();
+    return ok != 0;
 }
 
-// IncEval start: vertices lowered by a message form the frontier of step 0 (cc_process_messages, cc.cu:385-398).
-__global__ void mp_sweep_kernel(int *active, int *ubm, int n, int *counters) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        if (ubm[i] != 0) {
-            active[i] = 0;
-            ubm[i] = 0;
-            counters[5] = 1;
-        } else {
-            active[i] = -1;
-        }
-    }
-}
-
+// The value an edge offers: a label as it is, a distance plus the edge's length.
 template <int KIND>
-__device__ __forceinline__ void mp_relax_edge(unsigned now, int k, const int *__restrict__ dst, const float *__restrict__ len,
-                                              unsigned *value, int *active, int step, int *counters) {
-    const int w = dst[k];
-    unsigned nv = now;
-    if (KIND == DRONE_MP_SSSP) nv = __float_as_uint(__uint_as_float(now) + (len ? len[k] : 1.0f));
-    if (nv < value[w]) {                       // cheap filter; the atomic decides
-        const unsigned old = atomicMin(value + w, nv);
-        if (old > nv) {
-            active[w] = step + 1;
-            counters[5] = 1;
-        }
+__device__ __forceinline__ unsigned mp_offer(unsigned now, const float *len, int k) {
+    if (KIND == DRONE_MP_CC) return now;
+    return __float_as_uint(__uint_as_float(now) + (len ? __ldg(len + k) : 1.0f));
+}
+
+// `held`: value[w] read before, possibly out of date (values only fall, so it can only be too high); the atomic decides.
+__device__ __forceinline__ void mp_lower(const MpArgs &a, int w, unsigned offer, unsigned held, int round) {
+    if (offer < held && atomicMin(a.value + w, offer) > offer) {
+        a.state[w] = round + 1;
+        a.active[w] = 1;
     }
 }
 
-// One step: every vertex in the frontier of `step` offers its value to its out-neighbours (cc_exec, cc.cu:21-46;
-// sssp_exec, sssp.cu:41-74).
+// Values up to which waiting vertices offer theirs, given the least of them.  Labels: powers of 32, so that the vertices
+// with the smallest labels, one of which will be nearly everybody's in the end, spread theirs before the others have
+// offered labels that nobody keeps.  Distances: twice the least, so that few vertices offer a distance that a shorter
+// path still replaces.
 template <int KIND>
-__global__ void __launch_bounds__(256)
-mp_relax_kernel(const int *__restrict__ index, const int *__restrict__ dst, const float *__restrict__ len,
-                unsigned *value, int *active, int n, int step, int *counters, int2 *heavy, int heavy_cap) {
+__device__ __forceinline__ unsigned mp_limit(unsigned least) {
+    if (KIND == DRONE_MP_SSSP) return __float_as_uint(2.0f * __uint_as_float(least));
+    unsigned limit = 0;
+    while (limit < least) {
+        if (limit >= 1u << 26) return 0xfffffffeu;
+        limit = limit * 32 + 31;
+    }
+    return limit;
+}
+
+// One local run, all rounds in one launch (cc_exec, cc.cu:21-46; sssp_exec, sssp.cu:41-74, until nothing changes).
+//
+// A round: every warp looks at 128 vertices at a time; those that wait and lie within the limit offer their value to
+// their out-neighbours, short rows at once (the 32 rows of a step as one flat list of edges, so that lanes stay busy
+// whatever the degrees), long rows as pieces in a queue that the whole grid works off after a barrier.  When a round
+// finds nobody within the limit, the limit moves up to the least value that waits.
+//
+// Bound: one scattered 4-byte read of the neighbour's value per edge offered, 32 LSU wavefronts a load instruction; the
+// order above lets nearly every vertex offer once.  A step used to be two launches over all vertices, every label went
+// out before the small ones had spread, and the host looked in every fourth step (R-MAT-20 symmetrised labels: 5.08 ms,
+// MP_CC here; R-MAT-22 unit distances: 4.03 ms, MP_SSSP here).
+template <int KIND>
+__global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) {
     const int lane = threadIdx.x & 31;
-    const long long warp0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long base = warp0 * 32; base < n; base += n_warps * 32) {
-        const long long v = base + lane;
-        bool front = v < n && active[v] == step;
-        int beg = 0, end = 0;
-        unsigned now = 0;
-        if (front) {
-            beg = index[v];
-            end = index[v + 1];
-            now = value[v];
-            if (end - beg <= kSerialDegree) {
-                for (int k = beg; k < end; ++k) mp_relax_edge<KIND>(now, k, dst, len, value, active, step, counters);
-                front = false;
-            } else if (end - beg > kHeavyDegree) {
-                const int n_chunks = (end - beg + kHeavyChunk - 1) / kHeavyChunk;
-                const int at = atomicAdd(counters + 6, n_chunks);
-                if (at + n_chunks <= heavy_cap) {          // always true: the capacity covers every row at once
-                    for (int c = 0; c < n_chunks; ++c) heavy[at + c] = make_int2((int)v, c);
-                    front = false;
+    const int warp = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x), n_warps = (int)((blockDim.x >> 5) * gridDim.x);
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    __shared__ unsigned block_least;
+    __shared__ int block_offered;
+    unsigned phase = 0;
+    int round = 1;
+    unsigned limit = 0;
+    if (a.start == kMpContinue) {
+        round = a.control->round;
+        limit = a.control->limit;
+    } else {
+        // PEval: every label waits, or only the source.  IncEval: vertices lowered by a message (cc_process_messages,
+        // cc.cu:385-398).
+        for (int i = first; i < a.n; i += stride) {
+            bool waits;
+            if (a.start == kMpPeval) {
+                const int gid = __ldg(a.l2g + i);
+                waits = KIND == DRONE_MP_CC || gid == a.source_global;
+                a.value[i] = KIND == DRONE_MP_CC ? (unsigned)gid : waits ? 0u : kFarBits;
+            } else {
+                waits = a.ubm[i] != 0;
+            }
+            a.ubm[i] = 0;
+            a.state[i] = waits ? 0 : -1;
+            a.active[i] = waits ? 0 : -1;
+        }
+        if (!mp_barrier(a.control, phase)) return;
+    }
+    const int last_round = round + kRoundsPerLaunch;
+    bool finished = false;
+    while (!finished && round < last_round) {
+        MpRound *now_round = a.control->rounds + (round & 3);
+        if (threadIdx.x == 0) {
+            block_least = 0xffffffffu;
+            block_offered = 0;
+        }
+        __syncthreads();
+        unsigned least = 0xffffffffu;
+        bool offered = false;
+#pragma unroll 1
+        for (long long base = (long long)warp * 128; base < a.n; base += (long long)n_warps * 128) {
+            int st[4];
+            const int v0 = (int)base + lane * 4;
+            if (base + 128 <= a.n) {
+                const int4 s4 = *reinterpret_cast<const int4 *>(a.state + v0);
+                st[0] = s4.x; st[1] = s4.y; st[2] = s4.z; st[3] = s4.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) st[j] = v0 + j < a.n ? a.state[v0 + j] : -1;
+            }
+            if (!__any_sync(0xffffffffu, st[0] >= 0 || st[1] >= 0 || st[2] >= 0 || st[3] >= 0)) continue;
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {
+                const int v = v0 + j;
+                const int mark = j == 0 ? st[0] : j == 1 ? st[1] : j == 2 ? st[2] : st[3];
+                // a mark of this round's making (round + 1) waits for the next one
+                bool front = mark >= 0 && mark <= round;
+                unsigned now = 0;
+                if (front) {
+                    now = __ldcg(a.value + v);
+                    if (now > limit) {
+                        least = min(least, now);
+                        front = false;
+                    }
+                }
+                if (!__any_sync(0xffffffffu, front)) continue;
+                offered = true;
+                int beg = 0, deg = 0;
+                if (front) {
+                    // taken off the list unless somebody lowers it right now, which leaves round + 1 there; the value is
+                    // read (again) after that, so that what it was lowered to before goes out with this offer
+                    atomicCAS(a.state + v, mark, -1);
+                    now = __ldcg(a.value + v);
+                    beg = __ldg(a.index + v);
+                    deg = __ldg(a.index + v + 1) - beg;
+                }
+                // long rows: pieces into the queue
+                int pieces = deg > kWarpRow ? (deg + kItemEdges - 1) / kItemEdges : 0;
+                if (__any_sync(0xffffffffu, pieces > 0)) {
+                    int before = pieces;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int t = __shfl_up_sync(0xffffffffu, before, d);
+                        if (lane >= d) before += t;
+                    }
+                    int at = 0;
+                    if (lane == 31) at = atomicAdd(&now_round->items, before);
+                    at = __shfl_sync(0xffffffffu, at, 31) + before - pieces;
+                    if (at + pieces <= a.item_cap)      // always true: the capacity covers every long row at once
+                        for (int i = 0; i < pieces; ++i)
+                            a.items[at + i] = make_int4(beg + i * kItemEdges, min(kItemEdges, deg - i * kItemEdges), (int)now, 0);
+                    if (pieces > 0) deg = 0;
+                }
+                // short rows: edge e of the step belongs to the lane whose inclusive sum of degrees first exceeds e
+                int upto = deg;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d) upto += t;
+                }
+                const int total = __shfl_sync(0xffffffffu, upto, 31);
+                const int row0 = beg - (upto - deg);      // edge e of this lane's row is edge row0 + e of the graph
+                constexpr int UE = 4;
+#pragma unroll 1
+                for (int e0 = 0; e0 < total; e0 += 32 * UE) {
+                    int k[UE], w[UE];
+                    unsigned offer[UE], held[UE];
+#pragma unroll
+                    for (int u = 0; u < UE; ++u) {
+                        const int e = e0 + u * 32 + lane;
+                        int owner = 0;
+#pragma unroll
+                        for (int d = 16; d > 0; d >>= 1) {
+                            const int t = __shfl_sync(0xffffffffu, upto, owner + d - 1);
+                            if (t <= e) owner += d;
+                        }
+                        k[u] = __shfl_sync(0xffffffffu, row0, owner & 31) + e;
+                        offer[u] = __shfl_sync(0xffffffffu, now, owner & 31);
+                        w[u] = e < total ? __ldcs(a.dst + k[u]) : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < UE; ++u)
+                        if (w[u] >= 0) {
+                            offer[u] = mp_offer<KIND>(offer[u], a.len, k[u]);
+                            held[u] = a.value[w[u]];
+                        }
+#pragma unroll
+                    for (int u = 0; u < UE; ++u)
+                        if (w[u] >= 0) mp_lower(a, w[u], offer[u], held[u], round);
                 }
             }
         }
-        unsigned todo = __ballot_sync(0xffffffffu, front);
-        while (todo) {
-            const int src = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int b = __shfl_sync(0xffffffffu, beg, src), e = __shfl_sync(0xffffffffu, end, src);
-            const unsigned x = __shfl_sync(0xffffffffu, now, src);
-            for (int k = b + lane; k < e; k += 32) mp_relax_edge<KIND>(x, k, dst, len, value, active, step, counters);
+        least = __reduce_min_sync(0xffffffffu, least);
+        if (lane == 0) {
+            if (least != 0xffffffffu) atomicMin(&block_least, least);
+            if (offered) block_offered = 1;
         }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (block_least != 0xffffffffu) atomicMax(&now_round->nearest_left, ~block_least);
+            if (block_offered) now_round->offered = 1;
+        }
+        if (!mp_barrier(a.control, phase)) return;
+        const int n_items = min(__ldcg(&now_round->items), a.item_cap);
+        if (n_items > 0) {
+            // pieces of long rows: a warp each, four edges a lane in flight
+#pragma unroll 1
+            for (int i = warp; i < n_items; i += n_warps) {
+                const int4 it = __ldcg(a.items + i);
+#pragma unroll 1
+                for (int e0 = 0; e0 < it.y; e0 += 128) {
+                    int w[4];
+                    unsigned offer[4], held[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int e = e0 + u * 32 + lane;
+                        w[u] = e < it.y ? __ldcs(a.dst + it.x + e) : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (w[u] >= 0) {
+                            offer[u] = mp_offer<KIND>((unsigned)it.z, a.len, it.x + e0 + u * 32 + lane);
+                            held[u] = a.value[w[u]];
+                        }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (w[u] >= 0) mp_lower(a, w[u], offer[u], held[u], round);
+                }
+            }
+            if (!mp_barrier(a.control, phase)) return;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {      // used next two rounds from now; its last readers are behind the barrier
+            MpRound *later = a.control->rounds + ((round + 2) & 3);
+            later->items = 0;
+            later->offered = 0;
+            later->nearest_left = 0;
+        }
+        if (!__ldcg(&now_round->offered)) {
+            const unsigned left = ~__ldcg(&now_round->nearest_left);
+            if (left == 0xffffffffu) finished = true;
+            else limit = mp_limit<KIND>(left);
+        }
+        ++round;
     }
-}
-
-// The chunks queued by mp_relax_kernel in the same step, one warp per chunk.
-template <int KIND>
-__global__ void __launch_bounds__(256)
-mp_relax_heavy_kernel(const int *__restrict__ index, const int *__restrict__ dst, const float *__restrict__ len,
-                      unsigned *value, int *active, int step, int *counters, const int2 *heavy, int heavy_cap) {
-    const int lane = threadIdx.x & 31;
-    const int count = min(counters[6], heavy_cap);
-    const long long warp0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long i = warp0; i < count; i += n_warps) {
-        const int2 item = heavy[i];
-        const int b = index[item.x] + item.y * kHeavyChunk;
-        const int e = min(b + kHeavyChunk, index[item.x + 1]);
-        const unsigned x = value[item.x];
-        for (int k = b + lane; k < e; k += 32) mp_relax_edge<KIND>(x, k, dst, len, value, active, step, counters);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.control->unfinished = finished ? 0 : 1;
+        a.control->round = round;
+        a.control->limit = limit;
+    }
+    if (finished) {      // VisitedSize as the reference counts it: entries of `active` that are not 0 (countActive, common.cu:6-16)
+        int seen = 0;
+        for (int i = first; i < a.n; i += stride) seen += a.active[i] != 0;
+        seen = __reduce_add_sync(0xffffffffu, seen);
+        if (lane == 0 && seen) atomicAdd(a.counters + 4, seen);
     }
 }
 
@@ -225,14 +412,6 @@ __global__ void mp_apply_down_kernel(const int *__restrict__ up_rows, int n_up, 
     if (got) atomicAdd(counters + 3, got);
 }
 
-// VisitedSize as the reference counts it: entries of `active` that are not 0 (countActive, common.cu:6-16).
-__global__ void mp_count_visited_kernel(const int *active, int n, int *counters) {
-    int mine = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        mine += active[i] != 0;
-    if (mine) atomicAdd(counters + 4, mine);
-}
-
 // Moves the packed boundary entries of all parts: over NCCL (one part per process) or as device-to-device copies
 // (all parts in this process).
 static int mp_move(std::vector<drone_mp *> &parts, bool up, bool local, cudaStream_t st) {
@@ -268,35 +447,58 @@ static int mp_move(std::vector<drone_mp *> &parts, bool up, bool local, cudaStre
     return DRONE_OK;
 }
 
-// Relaxation steps until a whole group of kStepsPerLook steps lowers nothing.
-static int mp_local_run(drone_mp *p, cudaStream_t st) {
-    const int n = p->n_local;
-    if (n == 0) return DRONE_OK;
-    int step = 0, changed = 0;
-    DRONE_CUDA(cudaMemcpyAsync(&changed, p->counters + 5, sizeof(int), cudaMemcpyDeviceToHost, st));
-    DRONE_CUDA(cudaStreamSynchronize(st));
-    const int grid = grid_mp((long long)n, 148 * 8);
-    while (changed) {
-        DRONE_CUDA(cudaMemsetAsync(p->counters + 5, 0, sizeof(int), st));
-        for (int i = 0; i < kStepsPerLook; ++i, ++step) {
-            DRONE_CUDA(cudaMemsetAsync(p->counters + 6, 0, sizeof(int), st));
-            if (p->kind == DRONE_MP_CC) {
-                mp_relax_kernel<DRONE_MP_CC><<<grid, 256, 0, st>>>(p->index, p->dst, nullptr, p->value, p->active, n, step,
-                                                                   p->counters, p->heavy, p->heavy_cap);
-                DRONE_LAUNCH_CHECK("mp_relax_kernel");
-                mp_relax_heavy_kernel<DRONE_MP_CC><<<grid, 256, 0, st>>>(p->index, p->dst, nullptr, p->value, p->active, step,
-                                                                         p->counters, p->heavy, p->heavy_cap);
-            } else {
-                mp_relax_kernel<DRONE_MP_SSSP><<<grid, 256, 0, st>>>(p->index, p->dst, p->len, p->value, p->active, n, step,
-                                                                     p->counters, p->heavy, p->heavy_cap);
-                DRONE_LAUNCH_CHECK("mp_relax_kernel");
-                mp_relax_heavy_kernel<DRONE_MP_SSSP><<<grid, 256, 0, st>>>(p->index, p->dst, p->len, p->value, p->active, step,
-                                                                           p->counters, p->heavy, p->heavy_cap);
-            }
-            DRONE_LAUNCH_CHECK("mp_relax_heavy_kernel");
-        }
-        DRONE_CUDA(cudaMemcpyAsync(&changed, p->counters + 5, sizeof(int), cudaMemcpyDeviceToHost, st));
+// Counters and control block of a handle lie in one piece, so that one memset and one copy serve both.
+struct MpReport {
+    int counters[8];
+    MpControl control;
+};
+
+// Launches (or continues) the local run of one part.
+static int mp_launch(drone_mp *p, int start, int source_global, cudaStream_t st) {
+    MpArgs a;
+    a.n = p->n_local;
+    a.start = start;
+    a.source_global = source_global;
+    a.item_cap = p->item_cap;
+    a.index = p->index;
+    a.dst = p->dst;
+    a.l2g = p->l2g;
+    a.len = p->len;
+    a.value = p->value;
+    a.state = p->state;
+    a.active = p->active;
+    a.ubm = p->ubm;
+    a.counters = p->counters;
+    a.items = p->items;
+    a.control = &reinterpret_cast<MpReport *>(p->counters)->control;
+    if (start == kMpContinue) DRONE_CUDA(cudaMemsetAsync(&a.control->arrived, 0, sizeof(unsigned), st));
+    else DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(MpReport), st));
+    // a block has at least about 4096 edges and vertices to look at; more blocks only make the barriers longer
+    const int grid = std::max(1, (int)std::min<long long>(p->sms, ((long long)p->n_local + p->nnz + 4095) / 4096));
+    void *args[] = {&a};
+    const void *kernel = p->kind == DRONE_MP_CC ? (const void *)mp_run_kernel<DRONE_MP_CC> : (const void *)mp_run_kernel<DRONE_MP_SSSP>;
+    DRONE_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kRunThreads), args, 0, st));
+    count_launch();
+    return DRONE_OK;
+}
+
+// Local runs of all parts; on return they have finished and reports[i] is what part i's left.
+static int mp_local_runs(std::vector<drone_mp *> &parts, bool peval, int source_global, std::vector<MpReport> &reports,
+                         cudaStream_t st) {
+    int rc;
+    for (drone_mp *p : parts)
+        if ((rc = mp_launch(p, peval ? kMpPeval : kMpIncEval, source_global, st))) return rc;
+    for (bool again = true; again;) {
+        for (size_t i = 0; i < parts.size(); ++i)
+            DRONE_CUDA(cudaMemcpyAsync(&reports[i], parts[i]->counters, sizeof(MpReport), cudaMemcpyDeviceToHost, st));
         DRONE_CUDA(cudaStreamSynchronize(st));
+        again = false;
+        for (size_t i = 0; i < parts.size(); ++i) {
+            if (reports[i].control.failed) return set_error(DRONE_E_STATE, "a wait between the blocks of a local run ran out");
+            if (!reports[i].control.unfinished) continue;
+            again = true;
+            if ((rc = mp_launch(parts[i], kMpContinue, source_global, st))) return rc;
+        }
     }
     return DRONE_OK;
 }
@@ -344,43 +546,26 @@ static int mp_step(std::vector<drone_mp *> &parts, bool peval, int source_global
     using clock = std::chrono::steady_clock;
     const auto t0 = clock::now();
     int rc;
-    for (drone_mp *p : parts) {
-        if (!peval && !p->started) return set_error(DRONE_E_STATE, "IncEVal called before PEVal");
-        DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 8, st));
-        const int n = p->n_local;
-        if (n > 0) {
-            if (peval) {
-                mp_init_kernel<<<grid_mp(n), 256, 0, st>>>(p->kind, p->value, p->active, p->ubm, p->l2g, n, source_global,
-                                                          p->counters);
-                DRONE_LAUNCH_CHECK("mp_init_kernel");
-            } else {
-                mp_sweep_kernel<<<grid_mp(n), 256, 0, st>>>(p->active, p->ubm, n, p->counters);
-                DRONE_LAUNCH_CHECK("mp_sweep_kernel");
-            }
-        }
-        if ((rc = mp_local_run(p, st))) return rc;
-        p->started = true;
-    }
-    DRONE_CUDA(cudaStreamSynchronize(st));
-    const auto t1 = clock::now();
-    if ((rc = mp_exchange(parts, local, st))) return rc;
     for (drone_mp *p : parts)
-        if (p->n_local > 0) {
-            mp_count_visited_kernel<<<grid_mp(p->n_local), 256, 0, st>>>(p->active, p->n_local, p->counters);
-            DRONE_LAUNCH_CHECK("mp_count_visited_kernel");
-        }
-    std::vector<int> h(8 * parts.size());
-    for (size_t i = 0; i < parts.size(); ++i)
-        DRONE_CUDA(cudaMemcpyAsync(h.data() + 8 * i, parts[i]->counters, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
-    DRONE_CUDA(cudaStreamSynchronize(st));
+        if (!peval && !p->started) return set_error(DRONE_E_STATE, "IncEVal called before PEVal");
+    std::vector<MpReport> reports(parts.size());
+    if ((rc = mp_local_runs(parts, peval, source_global, reports, st))) return rc;
+    for (drone_mp *p : parts) p->started = true;
+    const auto t1 = clock::now();
+    if (parts[0]->xplan->nranks > 1) {
+        if ((rc = mp_exchange(parts, local, st))) return rc;
+        for (size_t i = 0; i < parts.size(); ++i)
+            DRONE_CUDA(cudaMemcpyAsync(reports[i].counters, parts[i]->counters, sizeof(reports[i].counters), cudaMemcpyDeviceToHost, st));
+        DRONE_CUDA(cudaStreamSynchronize(st));
+    }
     const auto t2 = clock::now();
     for (size_t i = 0; i < parts.size(); ++i) {
         drone_pr_response &r = res[i];
-        r.Mirror2MasterSendSize = h[8 * i + 0];
-        r.Mirror2MasterRecvSize = h[8 * i + 1];
-        r.Master2MirrorSendSize = h[8 * i + 2];
-        r.Master2MirrorRecvSize = h[8 * i + 3];
-        r.VisitedSize = h[8 * i + 4];
+        r.Mirror2MasterSendSize = reports[i].counters[0];
+        r.Mirror2MasterRecvSize = reports[i].counters[1];
+        r.Master2MirrorSendSize = reports[i].counters[2];
+        r.Master2MirrorRecvSize = reports[i].counters[3];
+        r.VisitedSize = reports[i].counters[4];
         r.LocalVertexSize = parts[i]->n_local;
         r.CalTime = std::chrono::duration<float>(t1 - t0).count();
         r.SendTime = std::chrono::duration<float>(t2 - t1).count();
@@ -437,15 +622,16 @@ int drone_mp_create(drone_mp **out, int kind, int n_local, int nnz, const int *d
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
     const size_t nb = std::max<size_t>(std::max(xplan->up_rows.size(), xplan->down_rows.size()), 1);
     if (err == cudaSuccess) err = cudaMalloc(&p->value, sizeof(unsigned) * n1);
+    if (err == cudaSuccess) err = cudaMalloc(&p->state, sizeof(int) * (n1 + 3));      // read four at a time
     if (err == cudaSuccess) err = cudaMalloc(&p->active, sizeof(int) * n1);
     if (err == cudaSuccess) err = cudaMalloc(&p->ubm, sizeof(int) * n1);
     if (err == cudaSuccess) err = cudaMalloc(&p->send, sizeof(uint2) * nb);
     if (err == cudaSuccess) err = cudaMalloc(&p->recv, sizeof(uint2) * nb);
-    if (err == cudaSuccess) err = cudaMalloc(&p->counters, sizeof(int) * 8);
-    // every row above kHeavyDegree in the frontier at once: at most nnz / kHeavyChunk full chunks plus one partial
-    // chunk per such row, of which there are fewer than nnz / kHeavyDegree
-    p->heavy_cap = nnz / kHeavyChunk + nnz / kHeavyDegree + 16;
-    if (err == cudaSuccess) err = cudaMalloc(&p->heavy, sizeof(int2) * (size_t)p->heavy_cap);
+    if (err == cudaSuccess) err = cudaMalloc(&p->counters, sizeof(MpReport));
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
+    // every row above kWarpRow in the frontier at once: full pieces, and one partial piece per such row
+    p->item_cap = nnz / kItemEdges + nnz / kWarpRow + 16;
+    if (err == cudaSuccess) err = cudaMalloc(&p->items, sizeof(int4) * (size_t)p->item_cap);
     if (err != cudaSuccess) {
         drone_mp_destroy(p);
         return set_error(DRONE_E_CUDA, "drone_mp_create: %s", cudaGetErrorString(err));
@@ -460,7 +646,7 @@ int drone_mp_destroy(drone_mp *p) {
     cudaGetDevice(&prev);
     cudaSetDevice(p->device);
     cudaFree(p->value); cudaFree(p->active); cudaFree(p->ubm); cudaFree(p->send); cudaFree(p->recv); cudaFree(p->counters);
-    cudaFree(p->heavy);
+    cudaFree(p->state); cudaFree(p->items);
     if (prev >= 0) cudaSetDevice(prev);
     delete p;
     return DRONE_OK;

@@ -160,3 +160,43 @@ def test_jobs_over_nccl_two_gpus():
     if torch.cuda.device_count() < 2:
         pytest.skip("needs two GPUs")
     run_ranks(_rank, 2, (29300 + os.getpid() % 2000,))
+
+
+@pytest.mark.parametrize("shape", ["chain", "stars", "rmat15", "far_labels"])
+@pytest.mark.parametrize("kind", ["labels", "unit", "weighted"])
+def test_run_at_its_edges(cuda_device, oracle, shape, kind):
+    """One part, run in one launch: a chain that needs more rounds than a launch runs, hubs whose rows are cut into many
+    pieces (and rows of exactly one and of one more than a warp's own), a graph of many warps, and labels whose
+    smallest is a vertex that reaches nobody."""
+    import types
+    rng = np.random.default_rng(9)
+    if shape == "chain":
+        n = 4500
+        u, v = np.arange(n - 1, dtype=np.int32), np.arange(1, n, dtype=np.int32)
+    elif shape == "stars":
+        n = 6000
+        hubs = [(3, 5000), (7, 64), (11, 65), (13, 512), (17, 513), (19, 1)]
+        u = np.concatenate([np.full(d, h, np.int32) for h, d in hubs] + [np.arange(20, 3000, dtype=np.int32)])
+        v = np.concatenate([(h + 1 + np.arange(d, dtype=np.int32)) % n for h, d in hubs] + [np.arange(20, 3000, dtype=np.int32) % 20])
+    else:
+        n, u, v = gg.rmat_graph(15, 8, seed=71, symmetrise=shape == "far_labels", self_loops="drop")
+        u, v = u.numpy(), v.numpy()
+        if shape == "far_labels":      # the low ids keep no edge: every component's smallest label is a large one
+            keep = (u >= 3000) & (v >= 3000)
+            u, v = u[keep], v[keep]
+    rowptr, col, _ = csr(n, u, v)
+    length = rng.uniform(0.01, 1.0, len(col)).astype(np.float32) if kind == "weighted" else None
+    index, dst = torch.as_tensor(np.asarray(rowptr, np.int32), device=cuda_device), torch.as_tensor(np.asarray(col, np.int32), device=cuda_device)
+    host = types.SimpleNamespace(rank=0, n_parts=1, n_local=n, l2g=np.arange(n, dtype=np.int32), mirror2worker=np.full(n, -1, np.int32),
+                                 master_worker_index=np.zeros(n + 1, np.int32), master2workers=np.zeros(0, np.int32))
+    graph = types.SimpleNamespace(host=host, n_local=n, device=cuda_device, index=index, dst=dst, xplan=pt.ExchangePlan(host, 1))
+    source = 0 if shape == "chain" else int(np.argmax(np.diff(rowptr)))
+    lens = torch.as_tensor(length, device=cuda_device) if length is not None else None
+    job = mp.MinProp(graph, mp.CC if kind == "labels" else mp.SSSP, edge_len=lens)
+    want = oracle.cc_fixed_point(rowptr, col) if kind == "labels" else oracle.sssp_f32(rowptr, col, source, length)
+    for _ in range(2):
+        res = job.peval(source)
+        assert np.array_equal(job.values(), want)
+        # all but the vertices that started in the frontier and were never lowered
+        still = int((want == np.arange(n)).sum()) if kind == "labels" else 1
+        assert res.VisitedSize == n - still and res.is_empty()
