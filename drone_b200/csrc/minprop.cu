@@ -63,8 +63,8 @@ static inline int grid_mp(long long n, int cap = 148 * 16) {
 
 struct MpRound {
     int items;             // pieces of long rows in the queue
-    int offered;           // 1: some vertex of the round's frontier offered its value
-    unsigned nearest_left; // complement of the least value among the waiting vertices that lay above the limit (0: none)
+    int waiting;           // vertices left waiting above the limit, not counting those lowered in this round
+    unsigned nearest;      // complement of the least value that waits after the round (0: nobody waits)
     int pad;
 };
 
@@ -119,21 +119,27 @@ __device__ __forceinline__ unsigned mp_offer(unsigned now, const float *len, int
     return __float_as_uint(__uint_as_float(now) + (len ? __ldg(len + k) : 1.0f));
 }
 
-// `held`: value[w] read before, possibly out of date (values only fall, so it can only be too high); the atomic decides.
-__device__ __forceinline__ void mp_lower(const MpArgs &a, int w, unsigned offer, unsigned held, int round) {
-    if (offer < held && atomicMin(a.value + w, offer) > offer) {
+// `held`: value[w] as some moment of this run had it; values only fall, so it can only be too high.  Nobody waits for the
+// atomic's result: whoever finds held > offer marks the vertex, and rightly so, since its value then was, or had been in
+// this run, lowered to the offer or below.  (A vertex lowered further by somebody else may offer once more for nothing.)
+// `least` keeps the least value offered this way.
+__device__ __forceinline__ void mp_lower(const MpArgs &a, int w, unsigned offer, unsigned held, int round, unsigned &least) {
+    if (offer < held) {
+        atomicMin(a.value + w, offer);
         a.state[w] = round + 1;
         a.active[w] = 1;
+        least = min(least, offer);
     }
 }
 
 // Values up to which waiting vertices offer theirs, given the least of them.  Labels: powers of 32, so that the vertices
 // with the smallest labels, one of which will be nearly everybody's in the end, spread theirs before the others have
 // offered labels that nobody keeps.  Distances: twice the least, so that few vertices offer a distance that a shorter
-// path still replaces.
+// path still replaces.  All labels, once few are left (distances have no such end: few wait at the start as well).
 template <int KIND>
-__device__ __forceinline__ unsigned mp_limit(unsigned least) {
+__device__ __forceinline__ unsigned mp_limit(unsigned least, bool few) {
     if (KIND == DRONE_MP_SSSP) return __float_as_uint(2.0f * __uint_as_float(least));
+    if (few) return 0xfffffffeu;
     unsigned limit = 0;
     while (limit < least) {
         if (limit >= 1u << 26) return 0xfffffffeu;
@@ -142,24 +148,55 @@ __device__ __forceinline__ unsigned mp_limit(unsigned least) {
     return limit;
 }
 
+constexpr int kGroup = 128;          // vertices a warp looks at together
+constexpr int kEdgesInFlight = 8;    // edges a lane reads together: their ends, then the values there (through L1: a value that
+                                     // is out of date there costs an offer for nothing, reading past it 40 % on R-MAT-20)
+struct MpGroupRows {                 // the rows of a group: row i's edges are entries upto[i-1] .. upto[i] of one flat list
+    int upto[kGroup];
+    int row0[kGroup];                // entry e of the list is edge row0[i] + e of the graph
+    unsigned value[kGroup];          // what the row's vertex offers
+};
+
+// Reduces the least waiting value and the number of waiting vertices of a block into the round's word.
+__device__ __forceinline__ void mp_note_round(MpRound *r, unsigned least, int waiting, unsigned *block_nearest, int *block_waiting) {
+    const unsigned nearest = __reduce_max_sync(0xffffffffu, ~least);
+    waiting = __reduce_add_sync(0xffffffffu, waiting);
+    if (threadIdx.x == 0) {
+        *block_nearest = 0;
+        *block_waiting = 0;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        if (nearest) atomicMax(block_nearest, nearest);
+        if (waiting) atomicAdd(block_waiting, waiting);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (*block_nearest) atomicMax(&r->nearest, *block_nearest);
+        if (*block_waiting) atomicAdd(&r->waiting, *block_waiting);
+    }
+}
+
 // One local run, all rounds in one launch (cc_exec, cc.cu:21-46; sssp_exec, sssp.cu:41-74, until nothing changes).
 //
 // A round: every warp looks at 128 vertices at a time; those that wait and lie within the limit offer their value to
-// their out-neighbours, short rows at once (the 32 rows of a step as one flat list of edges, so that lanes stay busy
-// whatever the degrees), long rows as pieces in a queue that the whole grid works off after a barrier.  When a round
-// finds nobody within the limit, the limit moves up to the least value that waits.
+// their out-neighbours, short rows at once (the rows of the group as one flat list of edges, so that lanes stay busy
+// whatever the degrees), long rows as pieces in a queue that the whole grid works off after a barrier.  The limit follows
+// the least value that waits after the round.
 //
-// Bound: one scattered 4-byte read of the neighbour's value per edge offered, 32 LSU wavefronts a load instruction; the
-// order above lets nearly every vertex offer once.  A step used to be two launches over all vertices, every label went
-// out before the small ones had spread, and the host looked in every fourth step (R-MAT-20 symmetrised labels: 5.08 ms,
-// MP_CC here; R-MAT-22 unit distances: 4.03 ms, MP_SSSP here).
+// Bound: one scattered 4-byte read of the neighbour's value per edge offered, up to 32 LSU wavefronts a load instruction
+// (about 2.8e11 a second on the whole part); the order above lets nearly every vertex offer once.  A step used to be two
+// launches over all vertices, every label went out before the small ones had spread, and the host looked in every fourth
+// step.  R-MAT-20 symmetrised, labels: 5.13 -> 0.27 ms; R-MAT-22, unit distances: 4.02 -> 0.62, weighted: 7.90 -> 1.44.
 template <int KIND>
 __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) {
+    extern __shared__ __align__(16) char group_bytes[];
     const int lane = threadIdx.x & 31;
+    MpGroupRows &rows = reinterpret_cast<MpGroupRows *>(group_bytes)[threadIdx.x >> 5];
     const int warp = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x), n_warps = (int)((blockDim.x >> 5) * gridDim.x);
     const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    __shared__ unsigned block_least;
-    __shared__ int block_offered;
+    __shared__ unsigned block_nearest;
+    __shared__ int block_waiting;
     unsigned phase = 0;
     int round = 1;
     unsigned limit = 0;
@@ -168,176 +205,180 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
         limit = a.control->limit;
     } else {
         // PEval: every label waits, or only the source.  IncEval: vertices lowered by a message (cc_process_messages,
-        // cc.cu:385-398).
+        // cc.cu:385-398).  A vertex without out-edges has nobody to offer to.
         for (int i = first; i < a.n; i += stride) {
-            bool waits;
+            bool front;
             if (a.start == kMpPeval) {
                 const int gid = __ldg(a.l2g + i);
-                waits = KIND == DRONE_MP_CC || gid == a.source_global;
-                a.value[i] = KIND == DRONE_MP_CC ? (unsigned)gid : waits ? 0u : kFarBits;
+                front = KIND == DRONE_MP_CC || gid == a.source_global;
+                a.value[i] = KIND == DRONE_MP_CC ? (unsigned)gid : front ? 0u : kFarBits;
             } else {
-                waits = a.ubm[i] != 0;
+                front = a.ubm[i] != 0;
             }
             a.ubm[i] = 0;
-            a.state[i] = waits ? 0 : -1;
-            a.active[i] = waits ? 0 : -1;
+            a.state[i] = front && __ldg(a.index + i + 1) > __ldg(a.index + i) ? 0 : -1;
+            a.active[i] = front ? 0 : -1;
         }
         if (!mp_barrier(a.control, phase)) return;
     }
     const int last_round = round + kRoundsPerLaunch;
+    const int few = max(1024, a.n / 64);
     bool finished = false;
     while (!finished && round < last_round) {
-        MpRound *now_round = a.control->rounds + (round & 3);
-        if (threadIdx.x == 0) {
-            block_least = 0xffffffffu;
-            block_offered = 0;
-        }
-        __syncthreads();
+        MpRound *this_round = a.control->rounds + (round & 3);
         unsigned least = 0xffffffffu;
-        bool offered = false;
+        int waiting = 0;
 #pragma unroll 1
-        for (long long base = (long long)warp * 128; base < a.n; base += (long long)n_warps * 128) {
-            int st[4];
+        for (long long base = (long long)warp * kGroup; base < a.n; base += (long long)n_warps * kGroup) {
+            int mark[4];
             const int v0 = (int)base + lane * 4;
-            if (base + 128 <= a.n) {
+            if (base + kGroup <= a.n) {
                 const int4 s4 = *reinterpret_cast<const int4 *>(a.state + v0);
-                st[0] = s4.x; st[1] = s4.y; st[2] = s4.z; st[3] = s4.w;
+                mark[0] = s4.x; mark[1] = s4.y; mark[2] = s4.z; mark[3] = s4.w;
             } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) st[j] = v0 + j < a.n ? a.state[v0 + j] : -1;
+                for (int j = 0; j < 4; ++j) mark[j] = v0 + j < a.n ? a.state[v0 + j] : -1;
             }
-            if (!__any_sync(0xffffffffu, st[0] >= 0 || st[1] >= 0 || st[2] >= 0 || st[3] >= 0)) continue;
-#pragma unroll 1
-            for (int j = 0; j < 4; ++j) {
-                const int v = v0 + j;
-                const int mark = j == 0 ? st[0] : j == 1 ? st[1] : j == 2 ? st[2] : st[3];
-                // a mark of this round's making (round + 1) waits for the next one
-                bool front = mark >= 0 && mark <= round;
-                unsigned now = 0;
-                if (front) {
-                    now = __ldcg(a.value + v);
-                    if (now > limit) {
-                        least = min(least, now);
-                        front = false;
-                    }
-                }
-                if (!__any_sync(0xffffffffu, front)) continue;
-                offered = true;
-                int beg = 0, deg = 0;
-                if (front) {
-                    // taken off the list unless somebody lowers it right now, which leaves round + 1 there; the value is
-                    // read (again) after that, so that what it was lowered to before goes out with this offer
-                    atomicCAS(a.state + v, mark, -1);
-                    now = __ldcg(a.value + v);
-                    beg = __ldg(a.index + v);
-                    deg = __ldg(a.index + v + 1) - beg;
-                }
-                // long rows: pieces into the queue
-                int pieces = deg > kWarpRow ? (deg + kItemEdges - 1) / kItemEdges : 0;
-                if (__any_sync(0xffffffffu, pieces > 0)) {
-                    int before = pieces;
+            // a mark of this round's making (round + 1) waits for the next one
+            bool any = false;
 #pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const int t = __shfl_up_sync(0xffffffffu, before, d);
-                        if (lane >= d) before += t;
-                    }
-                    int at = 0;
-                    if (lane == 31) at = atomicAdd(&now_round->items, before);
-                    at = __shfl_sync(0xffffffffu, at, 31) + before - pieces;
-                    if (at + pieces <= a.item_cap)      // always true: the capacity covers every long row at once
-                        for (int i = 0; i < pieces; ++i)
-                            a.items[at + i] = make_int4(beg + i * kItemEdges, min(kItemEdges, deg - i * kItemEdges), (int)now, 0);
-                    if (pieces > 0) deg = 0;
+            for (int j = 0; j < 4; ++j) {
+                if (mark[j] > round) mark[j] = -1;
+                any = any || mark[j] >= 0;
+            }
+            if (!__any_sync(0xffffffffu, any)) continue;
+            unsigned now[4];
+            int begin[5];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) now[j] = mark[j] >= 0 ? __ldcg(a.value + v0 + j) : 0u;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) begin[j] = any ? __ldg(a.index + min(v0 + j, a.n)) : 0;
+            int deg[4], pieces = 0, sum = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                deg[j] = 0;
+                if (mark[j] < 0) continue;
+                if (now[j] > limit) {
+                    least = min(least, now[j]);
+                    ++waiting;
+                    continue;
                 }
-                // short rows: edge e of the step belongs to the lane whose inclusive sum of degrees first exceeds e
-                int upto = deg;
+                // Off the list, unless somebody lowers the vertex just now: that leaves round + 1 there, before or after.
+                // Whether the value read above was the one from before or after does not matter then.
+                atomicCAS(a.state + v0 + j, mark[j], -1);
+                deg[j] = begin[j + 1] - begin[j];
+                if (deg[j] > kWarpRow) pieces += (deg[j] + kItemEdges - 1) / kItemEdges;
+                else sum += deg[j];
+            }
+            // long rows: pieces into the queue
+            if (__any_sync(0xffffffffu, pieces > 0)) {
+                int before = pieces;
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, upto, d);
-                    if (lane >= d) upto += t;
+                    const int t = __shfl_up_sync(0xffffffffu, before, d);
+                    if (lane >= d) before += t;
                 }
-                const int total = __shfl_sync(0xffffffffu, upto, 31);
-                const int row0 = beg - (upto - deg);      // edge e of this lane's row is edge row0 + e of the graph
-                constexpr int UE = 4;
-#pragma unroll 1
-                for (int e0 = 0; e0 < total; e0 += 32 * UE) {
-                    int k[UE], w[UE];
-                    unsigned offer[UE], held[UE];
+                int at = 0;
+                if (lane == 31) at = atomicAdd(&this_round->items, before);
+                at = __shfl_sync(0xffffffffu, at, 31) + before - pieces;
+                if (pieces > 0 && at + pieces <= a.item_cap) {      // always: the capacity covers every long row at once
 #pragma unroll
-                    for (int u = 0; u < UE; ++u) {
-                        const int e = e0 + u * 32 + lane;
-                        int owner = 0;
-#pragma unroll
-                        for (int d = 16; d > 0; d >>= 1) {
-                            const int t = __shfl_sync(0xffffffffu, upto, owner + d - 1);
-                            if (t <= e) owner += d;
+                    for (int j = 0; j < 4; ++j)
+                        if (deg[j] > kWarpRow) {
+                            for (int i = 0; i < deg[j]; i += kItemEdges)
+                                a.items[at++] = make_int4(begin[j] + i, min(kItemEdges, deg[j] - i), (int)now[j], 0);
+                            deg[j] = 0;
                         }
-                        k[u] = __shfl_sync(0xffffffffu, row0, owner & 31) + e;
-                        offer[u] = __shfl_sync(0xffffffffu, now, owner & 31);
-                        w[u] = e < total ? __ldcs(a.dst + k[u]) : -1;
-                    }
-#pragma unroll
-                    for (int u = 0; u < UE; ++u)
-                        if (w[u] >= 0) {
-                            offer[u] = mp_offer<KIND>(offer[u], a.len, k[u]);
-                            held[u] = a.value[w[u]];
-                        }
-#pragma unroll
-                    for (int u = 0; u < UE; ++u)
-                        if (w[u] >= 0) mp_lower(a, w[u], offer[u], held[u], round);
                 }
             }
+            // short rows
+            int upto = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += t;
+            }
+            const int total = __shfl_sync(0xffffffffu, upto, 31);
+            if (total == 0) continue;
+            __syncwarp();      // the previous group's list has been read
+            int end = upto - sum;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                rows.row0[lane * 4 + j] = begin[j] - end;
+                end += deg[j];
+                rows.upto[lane * 4 + j] = end;
+                rows.value[lane * 4 + j] = now[j];
+            }
+            __syncwarp();
+            constexpr int UE = kEdgesInFlight;
+#pragma unroll 1
+            for (int e0 = 0; e0 < total; e0 += 32 * UE) {
+                int k[UE], w[UE];
+                unsigned offer[UE], held[UE];
+#pragma unroll
+                for (int u = 0; u < UE; ++u) {
+                    const int e = e0 + u * 32 + lane;
+                    int i = 0;      // the first row whose end lies beyond e
+#pragma unroll
+                    for (int d = kGroup / 2; d > 0; d >>= 1)
+                        if (rows.upto[i + d - 1] <= e) i += d;
+                    k[u] = rows.row0[i] + e;
+                    offer[u] = rows.value[i];
+                    w[u] = e < total ? __ldcs(a.dst + k[u]) : -1;
+                }
+#pragma unroll
+                for (int u = 0; u < UE; ++u)
+                    if (w[u] >= 0) {
+                        offer[u] = mp_offer<KIND>(offer[u], a.len, k[u]);
+                        held[u] = a.value[w[u]];
+                    }
+#pragma unroll
+                for (int u = 0; u < UE; ++u)
+                    if (w[u] >= 0) mp_lower(a, w[u], offer[u], held[u], round, least);
+            }
         }
-        least = __reduce_min_sync(0xffffffffu, least);
-        if (lane == 0) {
-            if (least != 0xffffffffu) atomicMin(&block_least, least);
-            if (offered) block_offered = 1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (block_least != 0xffffffffu) atomicMax(&now_round->nearest_left, ~block_least);
-            if (block_offered) now_round->offered = 1;
-        }
+        mp_note_round(this_round, least, waiting, &block_nearest, &block_waiting);
         if (!mp_barrier(a.control, phase)) return;
-        const int n_items = min(__ldcg(&now_round->items), a.item_cap);
+        const int n_items = min(__ldcg(&this_round->items), a.item_cap);
         if (n_items > 0) {
-            // pieces of long rows: a warp each, four edges a lane in flight
+            // pieces of long rows: a warp each
+            constexpr int UE = kEdgesInFlight;
+            least = 0xffffffffu;
 #pragma unroll 1
             for (int i = warp; i < n_items; i += n_warps) {
                 const int4 it = __ldcg(a.items + i);
 #pragma unroll 1
-                for (int e0 = 0; e0 < it.y; e0 += 128) {
-                    int w[4];
-                    unsigned offer[4], held[4];
+                for (int e0 = 0; e0 < it.y; e0 += 32 * UE) {
+                    int w[UE];
+                    unsigned offer[UE], held[UE];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < UE; ++u) {
                         const int e = e0 + u * 32 + lane;
                         w[u] = e < it.y ? __ldcs(a.dst + it.x + e) : -1;
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < UE; ++u)
                         if (w[u] >= 0) {
                             offer[u] = mp_offer<KIND>((unsigned)it.z, a.len, it.x + e0 + u * 32 + lane);
                             held[u] = a.value[w[u]];
                         }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (w[u] >= 0) mp_lower(a, w[u], offer[u], held[u], round);
+                    for (int u = 0; u < UE; ++u)
+                        if (w[u] >= 0) mp_lower(a, w[u], offer[u], held[u], round, least);
                 }
             }
+            mp_note_round(this_round, least, 0, &block_nearest, &block_waiting);
             if (!mp_barrier(a.control, phase)) return;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {      // used next two rounds from now; its last readers are behind the barrier
             MpRound *later = a.control->rounds + ((round + 2) & 3);
             later->items = 0;
-            later->offered = 0;
-            later->nearest_left = 0;
+            later->waiting = 0;
+            later->nearest = 0;
         }
-        if (!__ldcg(&now_round->offered)) {
-            const unsigned left = ~__ldcg(&now_round->nearest_left);
-            if (left == 0xffffffffu) finished = true;
-            else limit = mp_limit<KIND>(left);
-        }
+        const unsigned nearest = __ldcg(&this_round->nearest);
+        if (nearest == 0) finished = true;
+        else if (~nearest > limit) limit = mp_limit<KIND>(~nearest, __ldcg(&this_round->waiting) <= few);
         ++round;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -476,8 +517,10 @@ static int mp_launch(drone_mp *p, int start, int source_global, cudaStream_t st)
     // a block has at least about 4096 edges and vertices to look at; more blocks only make the barriers longer
     const int grid = std::max(1, (int)std::min<long long>(p->sms, ((long long)p->n_local + p->nnz + 4095) / 4096));
     void *args[] = {&a};
+    const size_t smem = sizeof(MpGroupRows) * (kRunThreads / 32);
     const void *kernel = p->kind == DRONE_MP_CC ? (const void *)mp_run_kernel<DRONE_MP_CC> : (const void *)mp_run_kernel<DRONE_MP_SSSP>;
-    DRONE_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kRunThreads), args, 0, st));
+    DRONE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DRONE_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kRunThreads), args, smem, st));
     count_launch();
     return DRONE_OK;
 }
