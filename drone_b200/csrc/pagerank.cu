@@ -714,8 +714,8 @@ __device__ __forceinline__ void note_moved(unsigned *moved, int *counts, int q, 
     }
 }
 
-template <typename R, int MAXP, bool JOB>
-__global__ void __launch_bounds__(kPullThreads, 1) pr_run_kernel(const __grid_constant__ RunArgs<R, MAXP> a) {
+template <typename R, int MAXP, bool JOB, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constant__ RunArgs<R, MAXP> a) {
     extern __shared__ __align__(16) char table_bytes[];
     R *table = reinterpret_cast<R *>(table_bytes);
     __shared__ PartView<R> p;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_run_kernel(const __grid_co
         if (!grid_barrier(a.control, phase)) return;
         load_table(p, table);
         const R dang = fold_blocks<R>(a.block_sums);      // its barrier also closes the table
-        pull_rows<R, JOB, sizeof(R) == 4 ? 8 : 4, 4>(p, table, warp, n_warps);
+        pull_rows<R, JOB, sizeof(R) == 4 || THREADS <= 512 ? 8 : 4, 4>(p, table, warp, n_warps);
         if (JOB) gdiff = dang;
         if (!grid_barrier(a.control, phase)) return;
         if (JOB && step == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.control->t_pull = now_ns();
@@ -1190,8 +1190,8 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     for (drone_pr *p : parts) edges += (long long)p->nnz + p->n_local;
     // A block has at least about 2048 edges and vertices to work through; more blocks only make the barriers longer.
     const int grid = std::max(P, (int)std::min<long long>(lead->sms, (edges + 2047) / 2048));
-    // More warps hide more of a chunk's latencies (R-MAT-22: 6.5 ms with 512 threads, 5.3 with 768), fewer meet sooner at
-    // a barrier (R-MAT-16, two parts: 0.40 against 0.46 ms).
+    // More warps hide more of a chunk's latencies (R-MAT-22: 6.5 ms with 512 threads, 5.3 with 768); fewer meet sooner at
+    // a barrier and have the registers for more gathers each (R-MAT-16, two parts: 0.40 against 0.46 ms).
     const int threads = edges / grid > 32768 ? kPullThreads : 512;
     RunArgs<R, MAXP> a;
     a.n_parts = P;
@@ -1221,10 +1221,11 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     a.iterations = rq.iterations;
     a.n_isolated = lead->n_isolated;
     DRONE_CUDA(cudaMemsetAsync(lead->control, 0, sizeof(RunControl) + (JOB ? sizeof(int) * 4 * (size_t)P * rq.max_steps : 0), st));
-    const int rc = allow_table(pr_run_kernel<R, MAXP, JOB>);
+    auto kernel = threads == 512 ? pr_run_kernel<R, MAXP, JOB, 512> : pr_run_kernel<R, MAXP, JOB, kPullThreads>;
+    const int rc = allow_table(kernel);
     if (rc) return rc;
     void *args[] = {&a};
-    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)pr_run_kernel<R, MAXP, JOB>, dim3(grid), dim3(threads), args, table, st));
+    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(threads), args, table, st));
     count_launch();
     for (drone_pr *p : parts) p->started = JOB;
     return DRONE_OK;
