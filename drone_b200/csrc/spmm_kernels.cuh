@@ -57,6 +57,22 @@ __device__ __forceinline__ float ld_keep(const float *ptr, unsigned long long po
     asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(ptr), "l"(pol));
     return v;
 }
+// The same through the coherent path, for kernels that start before the one that writes X has finished (EARLY below).
+__device__ __forceinline__ float4 ld_coherent(const float4 *ptr, unsigned long long pol) {
+    float4 v;
+    asm volatile("ld.global.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(ptr), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float ld_coherent(const float *ptr, unsigned long long pol) {
+    float v;
+    asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(ptr), "l"(pol));
+    return v;
+}
+template <bool EARLY, typename T>
+__device__ __forceinline__ T ld_gathered(const T *ptr, unsigned long long pol) {
+    return EARLY ? ld_coherent(ptr, pol) : ld_keep(ptr, pol);
+}
 __device__ __forceinline__ int ld_stream(const int *ptr, unsigned long long pol) {
     int v;
     asm("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(ptr), "l"(pol));
@@ -186,6 +202,18 @@ __device__ __forceinline__ const typename Vec<VEC>::type *row_address(const Gath
     return base + (long long)(c & kHotMask) * stride + gl;
 }
 
+// Programmatic dependent launch: the next kernel of the stream may start once every block of this one has, and waits
+// (wait_for_operands) until this one has finished and its results are visible.
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_operands() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <bool EARLY>
+__device__ __forceinline__ float row_scale_of(const Epilogue &e, int row) {
+    if (e.row_scale == nullptr) return 1.f;
+    if (!EARLY) return __ldg(e.row_scale + row);
+    return ld_coherent(e.row_scale + row, l2_policy_keep());
+}
+
 // ---------------------------------------------------------------------------
 // 0. table of hot rows: hot[pos, :] = X[hot_ids[pos], :] for pos < hot_rows (dense, nvec vectors per row).
 // ---------------------------------------------------------------------------
@@ -208,8 +236,9 @@ spmm_fill_hot_kernel(const int *__restrict__ hot_ids, int hot_rows, const float 
 //    its last entry has been added.  Entries of a row are added in CSR order
 //    into one accumulator.
 // ---------------------------------------------------------------------------
-// `range`: the lane group's range; groups beyond the last one only take part in the shuffles.
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
+// `range`: the lane group's range; groups beyond the last one only take part in the shuffles.  EARLY: the kernel may have
+// started before its operands were complete; the plan's lists are read before it waits for them.
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT, bool EARLY>
 __device__ __forceinline__ void walk_short_range(long long range, const int *__restrict__ s_range_row, int n_ranges,
                                                  const int *__restrict__ s_rowptr, const int *__restrict__ s_rows,
                                                  const int *__restrict__ s_col, const float *__restrict__ s_val,
@@ -240,6 +269,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
         c_next = (unsigned)ld_stream(s_col + k + gl, pol_stream);
         if (!UNIT) v_next = ld_stream(s_val + k + gl, pol_stream);
     }
+    if (EARLY) wait_for_operands();
     for (int base = 0; base < maxlen; base += G) {
         const unsigned c = (c_next & ~kColMask) | resolve_column<HOT>(g, c_next & kColMask);
         const float v = v_next;
@@ -265,7 +295,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
                 const V *xr = row_address<VEC, HOT>(g, live ? (cc[u] & kColMask) : 0u, gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_keep(xr + p * G, pol_keep)
+                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_gathered<EARLY>(xr + p * G, pol_keep)
                                                                     : Vec<VEC>::zero();
             }
 #pragma unroll
@@ -274,7 +304,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
                 for (int p = 0; p < VPL; ++p) Vec<VEC>::fma(acc[p], vv[u], x[u][p]);
                 if ((cc[u] & kLastInRow) && (k + base + j + u < kend)) {
                     const int row = s_rows[ri];
-                    const float scale = epi.row_scale ? __ldg(epi.row_scale + row) : 1.f;
+                    const float scale = row_scale_of<EARLY>(epi, row);
                     const RowDestination<VEC> dest = row_destination<VEC>(epi, Y, ldy, row);
                     const bool remote = dest.remote;
                     V *yr = dest.ptr + gl;
@@ -301,7 +331,7 @@ spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, cons
                          const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec,
                          Epilogue epi) {
     const long long range = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * (32 / G) + (threadIdx.x & 31) / G;
-    walk_short_range<G, VPL, VEC, U, EXACT, UNIT, HOT>(range, s_range_row, n_ranges, s_rowptr, s_rows, s_col, s_val, g, Y,
+    walk_short_range<G, VPL, VEC, U, EXACT, UNIT, HOT, false>(range, s_range_row, n_ranges, s_rowptr, s_rows, s_col, s_val, g, Y,
                                                        ldy, nvec, epi);
 }
 
@@ -318,7 +348,7 @@ constexpr int kChunkGroup = 4;
 
 // Sum of one chunk: nonzeros [k0, k0 + len), taken in interleaved order by the warp's lane groups; (c, v) hold the
 // lane's entry of the first 32.  Every lane group ends with the same totals in acc.
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT, bool EARLY>
 __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const int *__restrict__ col,
                                           const float *__restrict__ val, const Gather &g, int k0, int len, int c, float v,
                                           int nvec, unsigned long long pol_keep, unsigned long long pol_stream) {
@@ -356,7 +386,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = (EXACT || gl + p * G < nvec) ? ld_keep(xr + p * G, pol_keep)
+                    x[u][p] = (EXACT || gl + p * G < nvec) ? ld_gathered<EARLY>(xr + p * G, pol_keep)
                                                            : Vec<VEC>::zero();
             }
 #pragma unroll
@@ -388,7 +418,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_keep(xr + p * G, pol_keep)
+                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_gathered<EARLY>(xr + p * G, pol_keep)
                                                                     : Vec<VEC>::zero();
             }
 #pragma unroll
@@ -452,7 +482,7 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
             }
 
             V acc[VPL];
-            sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
+            sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT, false>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
 
             if (gi == 0) {
                 if (slot < 0) {
@@ -569,7 +599,9 @@ spmm_reduce_partials_kernel(const SplitRow *__restrict__ split, int n_split,
 //    the short-row stream; the warp that writes the last partial sum of a split row (counted in `arrived`, which it
 //    sets back to 0) adds the row's slots, lane groups taking interleaved slots.  A call on such a plan is a few
 //    microseconds of work, so the memset, the four launches and the fork and join of the big plans' path used to be
-//    most of it (R-MAT-12 symmetrised, F = 16: 24 us of GPU and host time per call, 10 with this kernel; F = 64: 44, 10).
+//    most of it (R-MAT-12 symmetrised, F = 16: 24 us of GPU and host time per call, 8 with this kernel; F = 64: 44, 12).
+//    The kernel starts while the one before it in the stream still runs, reads the plan's lists, and only then waits for
+//    the operands (9.2 -> 8.0 us a call in a row of calls).
 // ---------------------------------------------------------------------------
 template <int VEC>
 __device__ __forceinline__ void store_vector(const RowDestination<VEC> &dest, int vi, const typename Vec<VEC>::type &v,
@@ -590,9 +622,10 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gi = lane / G;
+    let_next_kernel_start();
     if ((int)blockIdx.x >= chunk_blocks) {
         const long long warp = (((int)blockIdx.x - chunk_blocks) * (long long)blockDim.x + threadIdx.x) >> 5;
-        walk_short_range<G, VPL, VEC, U, EXACT, UNIT, false>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
+        walk_short_range<G, VPL, VEC, U, EXACT, UNIT, false, true>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
                                                              s_val, g, Y, ldy, nvec, epi);
         return;
     }
@@ -606,8 +639,11 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
         c = ld_stream(col + ch.y + lane, pol_stream);
         if (!UNIT) v = ld_stream(val + ch.y + lane, pol_stream);
     }
+    const int which = ch.w >= 0 ? __ldg(slot_split + ch.w) : 0;
+    const int4 sr = ch.w >= 0 ? __ldg(reinterpret_cast<const int4 *>(split) + which) : ch;      // row, first slot, slots
     V acc[VPL];
-    sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
+    wait_for_operands();
+    sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false, true>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
     int row = ch.x;
     if (ch.w >= 0) {
         if (gi == 0) {
@@ -616,8 +652,6 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
             for (int p = 0; p < VPL; ++p)
                 if (EXACT || gl + p * G < nvec) out[p * G] = acc[p];
         }
-        const int which = __ldg(slot_split + ch.w);
-        const int4 sr = __ldg(reinterpret_cast<const int4 *>(split) + which);      // row, first slot, slots
         __threadfence();
         __syncwarp();
         int last = 0;
@@ -654,7 +688,7 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
         row = sr.x;
     }
     if (gi == 0) {
-        const float scale = epi.row_scale ? __ldg(epi.row_scale + row) : 1.f;
+        const float scale = row_scale_of<true>(epi, row);
         const RowDestination<VEC> dest = row_destination<VEC>(epi, Y, ldy, row);
 #pragma unroll
         for (int p = 0; p < VPL; ++p)
@@ -714,10 +748,21 @@ static int launch_all(const SpmmArgs &a) {
     if (!HOT && s.small) {
         const int chunk_blocks = ceil_div(n_chunks, 8), short_blocks = ceil_div(n_ranges, 8 * RPW);
         if (chunk_blocks + short_blocks == 0) return DRONE_OK;
-        spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT><<<chunk_blocks + short_blocks, 256, 0, a.st>>>(
-            s.chunks + chunk_lo, n_chunks, chunk_blocks, s.col, s.val, s.split, s.slot_split, s.arrived, a.partials,
-            s.s_range_row + range_lo, n_ranges, s.s_rowptr, s.s_rows, s.s_col, s.s_val, a.gather, a.Y, a.ldy, a.nvec, a.epi);
-        DRONE_LAUNCH_CHECK("spmm_small_kernel");
+        cudaLaunchAttribute early;
+        early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        early.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(chunk_blocks + short_blocks);
+        cfg.blockDim = dim3(256);
+        cfg.stream = a.st;
+        cfg.attrs = &early;
+        cfg.numAttrs = 1;
+        DRONE_CUDA(cudaLaunchKernelEx(&cfg, spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT>, (const Chunk *)s.chunks + chunk_lo, n_chunks,
+                                      chunk_blocks, (const int *)s.col, (const float *)s.val, (const SplitRow *)s.split,
+                                      (const int *)s.slot_split, s.arrived, a.partials, (const int *)s.s_range_row + range_lo,
+                                      n_ranges, (const int *)s.s_rowptr, (const int *)s.s_rows, (const int *)s.s_col,
+                                      (const float *)s.s_val, a.gather, a.Y, a.ldy, a.nvec, a.epi));
+        count_launch();
         return DRONE_OK;
     }
     if (HOT && a.gather.hot_rows > 0) {
