@@ -513,41 +513,50 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
 
 // ---------------------------------------------------------------------------
 // 3. split rows: add the partial slots of a row in slot order.
-//    WIDE = false: one warp per split row (eight rows per block), its lane groups take interleaved slots; rows
-//    with more than max_slots slots are left to the wide launch.
-//    WIDE = true: one block per entry of the plan's list of wide rows, all eight warps share the row and their
-//    sums are added in warp order through shared memory.
+//    The first n_wide blocks take one entry each of the plan's list of wide rows, all eight warps share the row and
+//    their sums are added in warp order through shared memory; the other blocks take eight rows each, one per warp,
+//    leaving rows with more than kWideSlots slots to the first ones.  A warp's lane groups take interleaved slots.
+//    Bound: latency, since a row is a handful of loads; four of them are in flight per lane, and both kinds of rows share
+//    one launch (R-MAT-20 symmetrised, F = 64: 18 + 13 us in two launches -> TIME_REDUCE).
 // ---------------------------------------------------------------------------
-template <int G, int VPL, int VEC, bool WIDE>
+template <int G, int VPL, int VEC>
 __global__ void __launch_bounds__(256)
-spmm_reduce_partials_kernel(const SplitRow *__restrict__ split, int n_split,
-                            const float *__restrict__ partials, float *__restrict__ Y, long long ldy,
-                            int nvec, int max_slots, Epilogue epi) {
+spmm_reduce_partials_kernel(const SplitRow *__restrict__ split, int n_split, const SplitRow *__restrict__ wide, int n_wide,
+                            const float *__restrict__ partials, float *__restrict__ Y, long long ldy, int nvec, Epilogue epi) {
     using V = typename Vec<VEC>::type;
     constexpr int RPW = 32 / G;
-    extern __shared__ float smem[];  // [8][nvec*VEC] for the wide launch
+    extern __shared__ float smem[];  // [8][nvec*VEC] for the wide rows
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     const int gl = lane & (G - 1);
     const int gi = lane / G;
-    const long long entry = WIDE ? (long long)blockIdx.x : (long long)blockIdx.x * 8 + w;
-    if (entry >= n_split) return;
-    const int4 raw = __ldg(reinterpret_cast<const int4 *>(split) + entry);
+    const bool is_wide = (int)blockIdx.x < n_wide;
+    const long long entry = is_wide ? (long long)blockIdx.x : ((long long)blockIdx.x - n_wide) * 8 + w;
+    if (!is_wide && entry >= n_split) return;
+    const int4 raw = __ldg(reinterpret_cast<const int4 *>(is_wide ? wide : split) + entry);
     const int row = raw.x, slot0 = raw.y, nslots = raw.z;
-    if (!WIDE && nslots > max_slots) return;
+    if (!is_wide && nslots > kWideSlots) return;
 
     V acc[VPL];
 #pragma unroll
     for (int p = 0; p < VPL; ++p) acc[p] = Vec<VEC>::zero();
-    const int first = WIDE ? w * RPW + gi : gi;
-    const int stride = WIDE ? 8 * RPW : RPW;
-    for (int sidx = first; sidx < nslots; sidx += stride) {
-        const V *pr = reinterpret_cast<const V *>(partials + (long long)(slot0 + sidx) * nvec * VEC);
+    const int first = is_wide ? w * RPW + gi : gi;
+    const int stride = is_wide ? 8 * RPW : RPW;
+    constexpr int UR = VPL <= 2 ? 4 : 1;
+    for (int sidx = first; sidx < nslots; sidx += UR * stride) {
+        V x[UR][VPL];
 #pragma unroll
-        for (int p = 0; p < VPL; ++p) {
-            const int vi = gl + p * G;
-            if (vi < nvec) Vec<VEC>::add(acc[p], pr[vi]);
+        for (int u = 0; u < UR; ++u) {
+            const V *pr = reinterpret_cast<const V *>(partials + (long long)(slot0 + sidx + u * stride) * nvec * VEC);
+#pragma unroll
+            for (int p = 0; p < VPL; ++p)
+                x[u][p] = sidx + u * stride < nslots && gl + p * G < nvec ? pr[gl + p * G] : Vec<VEC>::zero();
         }
+#pragma unroll
+        for (int u = 0; u < UR; ++u)
+#pragma unroll
+            for (int p = 0; p < VPL; ++p)
+                if (sidx + u * stride < nslots) Vec<VEC>::add(acc[p], x[u][p]);
     }
 #pragma unroll
     for (int o = G; o < 32; o <<= 1)
@@ -558,7 +567,7 @@ spmm_reduce_partials_kernel(const SplitRow *__restrict__ split, int n_split,
     const RowDestination<VEC> dest = row_destination<VEC>(epi, Y, ldy, row);
     const bool remote = dest.remote;
     V *yr = dest.ptr;
-    if (!WIDE) {
+    if (!is_wide) {
         if (gi == 0) {
 #pragma unroll
             for (int p = 0; p < VPL; ++p) {
@@ -800,15 +809,10 @@ static int launch_all(const SpmmArgs &a) {
         DRONE_LAUNCH_CHECK("spmm_chunks_kernel");
     }
     if (n_split > 0) {
-        spmm_reduce_partials_kernel<G, VPL, VEC, false><<<ceil_div(n_split, 8), 256, 0, a.st>>>(
-            s.split + split_lo, n_split, a.partials, a.Y, a.ldy, a.nvec, kWideSlots, a.epi);
+        const size_t smem = n_wide > 0 ? sizeof(float) * 8 * (size_t)a.nvec * VEC : 0;
+        spmm_reduce_partials_kernel<G, VPL, VEC><<<n_wide + ceil_div(n_split, 8), 256, smem, a.st>>>(
+            s.split + split_lo, n_split, s.wide + wide_lo, n_wide, a.partials, a.Y, a.ldy, a.nvec, a.epi);
         DRONE_LAUNCH_CHECK("spmm_reduce_partials_kernel");
-        if (n_wide > 0) {
-            const size_t smem = sizeof(float) * 8 * (size_t)a.nvec * VEC;
-            spmm_reduce_partials_kernel<G, VPL, VEC, true><<<n_wide, 256, smem, a.st>>>(
-                s.wide + wide_lo, n_wide, a.partials, a.Y, a.ldy, a.nvec, 0, a.epi);
-            DRONE_LAUNCH_CHECK("spmm_reduce_partials_kernel(wide)");
-        }
     }
     if (overlap) DRONE_CUDA(cudaStreamWaitEvent(a.st, a.join, 0));
     return DRONE_OK;
