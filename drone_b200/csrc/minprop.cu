@@ -35,7 +35,8 @@ struct drone_mp {
     drone_xplan *xplan = nullptr;                                 // borrowed
     drone_comm *comm = nullptr;                                   // borrowed, may be NULL for one part
     unsigned *value = nullptr;     // [n] label, or the bits of a non-negative float distance
-    int *state = nullptr;          // [n] -1 idle, r = waiting to offer its value since round r
+    int *state = nullptr;          // [n] during a run: r >= 0 waits to offer its value since round r (0: from the start),
+                                   // kOffered after it did, kOfferedFirst the same but only from the start, kIdle neither
     int *active = nullptr;         // [n] after a run: 1 lowered in it, 0 in its first frontier and not lowered, -1 neither
     int *ubm = nullptr;            // [n] lowered by a received message since the last sweep
     uint2 *send = nullptr, *recv = nullptr;   // [max(up, down)] {value, flag}
@@ -48,7 +49,8 @@ struct drone_mp {
 namespace drone {
 
 constexpr int kWarpRow = 64;         // rows up to this many edges are walked by the warp that finds them in the frontier
-constexpr int kItemEdges = 512;      // longer ones are cut into pieces of this many edges for the whole grid
+constexpr int kIdle = -1, kOffered = -2, kOfferedFirst = -3;
+constexpr int kItemEdges = 256;      // longer ones are cut into pieces of this many edges for the whole grid
 constexpr int kRunThreads = 1024;
 constexpr int kRoundsPerLaunch = 4096;
 constexpr unsigned kMpPolls = 1u << 23;      // about five seconds: the grid barrier gives up instead of hanging
@@ -127,7 +129,6 @@ __device__ __forceinline__ void mp_lower(const MpArgs &a, int w, unsigned offer,
     if (offer < held) {
         atomicMin(a.value + w, offer);
         a.state[w] = round + 1;
-        a.active[w] = 1;
         least = min(least, offer);
     }
 }
@@ -187,7 +188,7 @@ __device__ __forceinline__ void mp_note_round(MpRound *r, unsigned least, int wa
 // Bound: one scattered 4-byte read of the neighbour's value per edge offered, up to 32 LSU wavefronts a load instruction
 // (about 2.8e11 a second on the whole part); the order above lets nearly every vertex offer once.  A step used to be two
 // launches over all vertices, every label went out before the small ones had spread, and the host looked in every fourth
-// step.  R-MAT-20 symmetrised, labels: 5.13 -> 0.27 ms; R-MAT-22, unit distances: 4.02 -> 0.62, weighted: 7.90 -> 1.44.
+// step.  R-MAT-20 symmetrised, labels: 5.13 -> 0.26 ms; R-MAT-22, unit distances: 4.02 -> 0.58, weighted: 7.90 -> 1.34.
 template <int KIND>
 __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) {
     extern __shared__ __align__(16) char group_bytes[];
@@ -216,8 +217,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
                 front = a.ubm[i] != 0;
             }
             a.ubm[i] = 0;
-            a.state[i] = front && __ldg(a.index + i + 1) > __ldg(a.index + i) ? 0 : -1;
-            a.active[i] = front ? 0 : -1;
+            a.state[i] = !front ? kIdle : __ldg(a.index + i + 1) > __ldg(a.index + i) ? 0 : kOfferedFirst;
         }
         if (!mp_barrier(a.control, phase)) return;
     }
@@ -237,13 +237,13 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
                 mark[0] = s4.x; mark[1] = s4.y; mark[2] = s4.z; mark[3] = s4.w;
             } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) mark[j] = v0 + j < a.n ? a.state[v0 + j] : -1;
+                for (int j = 0; j < 4; ++j) mark[j] = v0 + j < a.n ? a.state[v0 + j] : kIdle;
             }
             // a mark of this round's making (round + 1) waits for the next one
             bool any = false;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (mark[j] > round) mark[j] = -1;
+                if (mark[j] > round) mark[j] = kIdle;
                 any = any || mark[j] >= 0;
             }
             if (!__any_sync(0xffffffffu, any)) continue;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
                 }
                 // Off the list, unless somebody lowers the vertex just now: that leaves round + 1 there, before or after.
                 // Whether the value read above was the one from before or after does not matter then.
-                atomicCAS(a.state + v0 + j, mark[j], -1);
+                atomicCAS(a.state + v0 + j, mark[j], mark[j] > 0 ? kOffered : kOfferedFirst);
                 deg[j] = begin[j + 1] - begin[j];
                 if (deg[j] > kWarpRow) pieces += (deg[j] + kItemEdges - 1) / kItemEdges;
                 else sum += deg[j];
@@ -388,7 +388,12 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
     }
     if (finished) {      // VisitedSize as the reference counts it: entries of `active` that are not 0 (countActive, common.cu:6-16)
         int seen = 0;
-        for (int i = first; i < a.n; i += stride) seen += a.active[i] != 0;
+        for (int i = first; i < a.n; i += stride) {
+            const int st = a.state[i];
+            const int active = st == kIdle ? -1 : st == kOfferedFirst ? 0 : 1;
+            a.active[i] = active;
+            seen += active != 0;
+        }
         seen = __reduce_add_sync(0xffffffffu, seen);
         if (lane == 0 && seen) atomicAdd(a.counters + 4, seen);
     }
