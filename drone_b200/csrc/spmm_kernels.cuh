@@ -69,6 +69,38 @@ __device__ __forceinline__ float ld_coherent(const float *ptr, unsigned long lon
     asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(ptr), "l"(pol));
     return v;
 }
+// A gathered vector, or zeros where `live` is false.  The load is predicated inside one volatile statement: written as a
+// conditional expression it became a branch, which the compiler moved down to the multiply-add that uses the value, so
+// that the loads of a batch followed one another instead of being in flight together (R-MAT-16, F = 160: 597 us a call,
+// against 333 at F = 256, where no lane's vectors run past the row and the loads need no condition).
+template <bool EARLY>
+__device__ __forceinline__ float4 ld_gathered_if(const float4 *ptr, unsigned long long pol, bool live) {
+    float4 v;
+    if (EARLY)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %6, 0;\n\t"
+                     "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+                     "@q ld.global.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;\n\t}"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(ptr), "l"(pol), "r"((int)live));
+    else
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %6, 0;\n\t"
+                     "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+                     "@q ld.global.nc.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;\n\t}"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(ptr), "l"(pol), "r"((int)live));
+    return v;
+}
+template <bool EARLY>
+__device__ __forceinline__ float ld_gathered_if(const float *ptr, unsigned long long pol, bool live) {
+    float v;
+    if (EARLY)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.b32 %0, 0;\n\t"
+                     "@q ld.global.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
+                     : "=f"(v) : "l"(ptr), "l"(pol), "r"((int)live));
+    else
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.b32 %0, 0;\n\t"
+                     "@q ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
+                     : "=f"(v) : "l"(ptr), "l"(pol), "r"((int)live));
+    return v;
+}
 template <bool EARLY, typename T>
 __device__ __forceinline__ T ld_gathered(const T *ptr, unsigned long long pol) {
     return EARLY ? ld_coherent(ptr, pol) : ld_keep(ptr, pol);
@@ -230,6 +262,20 @@ spmm_fill_hot_kernel(const int *__restrict__ hot_ids, int hot_rows, const float 
     }
 }
 
+// Blocks per SM the two kernels of large plans are compiled for.  Left to itself (0) the compiler aims at 40 registers in
+// the chunk kernel, which hold five of a batch's eight row vectors and fewer where the loads are predicated; 64 registers
+// hold all eight, and 32 warps with eight loads each are worth more than 48 with four or five (R-MAT-24, F = 32: 4.69 ->
+// 4.37 ms; R-MAT-20 symmetrised: F = 64 599 -> 574 us, F = 100 1427 -> 984; products-shaped, F = 47: 6.7 -> 4.6 ms).  Wider
+// rows need more registers for the same (F = 400 on R-MAT-20: 7.8 -> 4.4 ms, F = 1000: 23.6 -> 13.0); where all of a lane's
+// vectors lie inside the row the compiler's own choice was the better one above one vector a lane.
+constexpr int chunk_blocks_per_sm(int G, int VPL, int VEC, bool EXACT) {
+    if (VEC != 4 || G < 8) return 0;
+    if (VPL == 1) return 4;
+    if (EXACT) return 0;
+    return VPL == 2 ? 4 : VPL <= 4 ? 3 : 2;
+}
+constexpr int short_blocks_per_sm(int VPL, int VEC, bool EXACT) { return VEC != 4 || VPL > 1 ? 0 : EXACT ? 4 : 5; }
+
 // ---------------------------------------------------------------------------
 // 1. short rows: one lane group walks a range of the short-row stream
 //    (about kShortRangeNnz entries, whole rows only) and writes each row when
@@ -295,8 +341,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
                 const V *xr = row_address<VEC, HOT>(g, live ? (cc[u] & kColMask) : 0u, gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_gathered<EARLY>(xr + p * G, pol_keep)
-                                                                    : Vec<VEC>::zero();
+                    x[u][p] = ld_gathered_if<EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u) {
@@ -325,7 +370,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
 }
 
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, short_blocks_per_sm(VPL, VEC, EXACT))
 spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, const int *__restrict__ s_rowptr,
                          const int *__restrict__ s_rows, const int *__restrict__ s_col,
                          const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec,
@@ -386,8 +431,8 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = (EXACT || gl + p * G < nvec) ? ld_gathered<EARLY>(xr + p * G, pol_keep)
-                                                           : Vec<VEC>::zero();
+                    x[u][p] = EXACT ? ld_gathered<EARLY>(xr + p * G, pol_keep)
+                                    : ld_gathered_if<EARLY>(xr + p * G, pol_keep, gl + p * G < nvec);
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u)
@@ -418,8 +463,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = (live && (EXACT || gl + p * G < nvec)) ? ld_gathered<EARLY>(xr + p * G, pol_keep)
-                                                                    : Vec<VEC>::zero();
+                    x[u][p] = ld_gathered_if<EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u)
@@ -435,7 +479,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
 }
 
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, chunk_blocks_per_sm(G, VPL, VEC, EXACT))
 spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__restrict__ col,
                    const float *__restrict__ val, Gather g, float *__restrict__ Y, long long ldy,
                    float *__restrict__ partials, int nvec, Epilogue epi, unsigned *counter) {
