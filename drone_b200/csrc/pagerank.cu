@@ -934,8 +934,8 @@ static PartView<R> part_view(const drone_pr *p, int blocks) {
     v.chunks = s.chunks;
     v.n_chunks = s.n_chunks;
     v.col = s.col;
-    v.s_range_row = s.s_range_row;
-    v.n_ranges = s.n_short_ranges;
+    v.s_range_row = s.ranges.row;
+    v.n_ranges = s.ranges.n;
     v.s_rowptr = s.s_rowptr;
     v.s_rows = s.s_rows;
     v.s_col = s.s_col;

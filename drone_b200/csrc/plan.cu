@@ -347,7 +347,8 @@ static void free_side(Side &s) {
     cudaFree(s.s_rowptr);
     cudaFree(s.s_col);
     cudaFree(s.s_val);
-    cudaFree(s.s_range_row);
+    cudaFree(s.ranges.row);
+    cudaFree(s.fine.row);
     s = Side();
 }
 
@@ -423,12 +424,14 @@ static void free_lists(Side &s) {
     cudaFree(s.s_rowptr);
     cudaFree(s.s_col);
     cudaFree(s.s_val);
-    cudaFree(s.s_range_row);
+    cudaFree(s.ranges.row);
+    cudaFree(s.fine.row);
     s.slot_split = s.arrived = nullptr;
     s.small = false;
     s.chunks = nullptr;
     s.split = s.wide = nullptr;
-    s.s_rows = s.s_rowptr = s.s_col = s.s_range_row = nullptr;
+    s.s_rows = s.s_rowptr = s.s_col = nullptr;
+    s.ranges = s.fine = Ranges();
     s.s_val = nullptr;
     s.ready = false;
 }
@@ -457,6 +460,28 @@ static int class_major_scan(const drone_plan *p, const int *cnt, int *off, int *
     for (int c = 0; c <= p->n_classes; ++c)
         DRONE_CUDA(cudaMemcpyAsync(&starts[c], permuted_off + p->class_start[c], sizeof(int), cudaMemcpyDeviceToHost, st));
     DRONE_CUDA(cudaStreamSynchronize(st));
+    return DRONE_OK;
+}
+
+// Cuts the stream of short rows into ranges of about range_nnz entries.  K row classes, class c's short rows starting at
+// row_start[c] of s_rows and its entries at entry_start[c]; both arrays stay alive until the caller has synchronised st.
+static int cut_ranges(const Side &s, Ranges &out, int range_nnz, int K, const int *row_start, const int *entry_start,
+                      cudaStream_t st) {
+    out.start[0] = 0;
+    for (int c = 0; c < K; ++c) out.start[c + 1] = out.start[c] + ceil_div(entry_start[c + 1] - entry_start[c], range_nnz);
+    out.n = out.start[K];
+    DRONE_CUDA(cudaMalloc(&out.row, sizeof(int) * (size_t)(out.n + 1)));
+    // ranges never straddle two classes; entry start[c] is also the end of class c-1's last range
+    for (int c = 0; c < K; ++c) {
+        const int nr = out.start[c + 1] - out.start[c];
+        if (nr > 0) {
+            short_ranges_kernel<<<grid_for(nr), 256, 0, st>>>(s.s_rowptr, row_start[c], row_start[c + 1], entry_start[c], nr,
+                                                             range_nnz, out.row + out.start[c]);
+            DRONE_LAUNCH_CHECK("short_ranges_kernel");
+        }
+    }
+    for (int c = 1; c <= K; ++c)   // after the kernels in stream order: the closing entry of every class
+        DRONE_CUDA(cudaMemcpyAsync(out.row + out.start[c], &row_start[c], sizeof(int), cudaMemcpyHostToDevice, st));
     return DRONE_OK;
 }
 
@@ -509,7 +534,8 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
             DRONE_CUDA(cudaMemsetAsync(s.arrived, 0, sizeof(int) * (size_t)s.n_split_rows, st));
             fill_slot_split_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, s.slot_split);
             DRONE_LAUNCH_CHECK("fill_slot_split_kernel");
-        } else if (s.n_split_rows > 0) {
+        }
+        if (s.n_split_rows > 0 && (!s.small || p->nnz > kSmallNnzMostFloats)) {   // for the separate kernels
             int *d_max = scratch, *d_count = scratch + 1;
             DRONE_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(int), st));
             max_nslots_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, d_max);
@@ -578,35 +604,18 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     if ((rc = class_major_scan(p, cnt[1], off[1], scratch, tmp, tmp_bytes, sent_start, st))) return rc;
     s.n_short_rows = srow_start[K];
     s.n_short_entries = sent_start[K];
-    s.range_start[0] = 0;
-    const int range_nnz = s.small ? kSmallRangeNnz : kShortRangeNnz;
-    for (int c = 0; c < K; ++c)
-        s.range_start[c + 1] = s.range_start[c] + ceil_div(sent_start[c + 1] - sent_start[c], range_nnz);
-    s.n_short_ranges = s.range_start[K];
     if (s.n_short_rows > 0) {
         DRONE_CUDA(cudaMalloc(&s.s_rows, sizeof(int) * (size_t)s.n_short_rows));
         DRONE_CUDA(cudaMalloc(&s.s_rowptr, sizeof(int) * (size_t)(s.n_short_rows + 1)));
         DRONE_CUDA(cudaMalloc(&s.s_col, sizeof(int) * (size_t)s.n_short_entries));
         DRONE_CUDA(cudaMalloc(&s.s_val, sizeof(float) * (size_t)s.n_short_entries));
-        DRONE_CUDA(cudaMalloc(&s.s_range_row, sizeof(int) * (size_t)(s.n_short_ranges + 1)));
         fill_short_kernel<<<grid_for(n), 256, 0, st>>>(s.rowptr, s.col, s.val, n, p->short_row_limit, off[0], off[1],
                                                       s.s_rows, s.s_rowptr, s.s_col, s.s_val);
         DRONE_LAUNCH_CHECK("fill_short_kernel");
         DRONE_CUDA(cudaMemcpyAsync(s.s_rowptr + s.n_short_rows, &s.n_short_entries, sizeof(int),
                                    cudaMemcpyHostToDevice, st));
-        // ranges never straddle two classes; entry range_start[c] is also the end of class c-1's last range
-        for (int c = 0; c < K; ++c) {
-            const int nr = s.range_start[c + 1] - s.range_start[c];
-            if (nr > 0) {
-                short_ranges_kernel<<<grid_for(nr), 256, 0, st>>>(s.s_rowptr, srow_start[c], srow_start[c + 1],
-                                                                 sent_start[c], nr, range_nnz,
-                                                                 s.s_range_row + s.range_start[c]);
-                DRONE_LAUNCH_CHECK("short_ranges_kernel");
-            }
-        }
-        for (int c = 1; c <= K; ++c)   // after the kernels in stream order: the closing entry of every class
-            DRONE_CUDA(cudaMemcpyAsync(s.s_range_row + s.range_start[c], &srow_start[c], sizeof(int),
-                                       cudaMemcpyHostToDevice, st));
+        if ((rc = cut_ranges(s, s.ranges, kShortRangeNnz, K, srow_start, sent_start, st))) return rc;
+        if (s.small && (rc = cut_ranges(s, s.fine, kFineRangeNnz, K, srow_start, sent_start, st))) return rc;
         DRONE_CUDA(cudaStreamSynchronize(st));
     }
     s.ready = true;

@@ -9,9 +9,15 @@ namespace drone {
 // longer than what handing chunks out dynamically, and overlapping the two kinds of rows, gains (R-MAT directed + I, one
 // launch / separate kernels, us at F = 16 | 64: 4.3 M nonzeros 49 / 89 | 133 / 160, 8.5 M 88 / 110 | 246 / 192).
 constexpr int kSmallNnz = 6 << 20;
+constexpr int kSmallNnzManyFloats = 1 << 20, kSmallNnzMostFloats = 1 << 15;   // the same with 8 or 16 floats of a row per lane
 constexpr int kWideSlots = 64;              // split rows above this many partial slots are reduced by a whole block
 constexpr int kShortRangeNnz = 64;          // stream entries per lane group (plus at most one more row) ...
-constexpr int kSmallRangeNnz = 16;          // ... and in small plans, where one group's walk is the length of the call
+// ... and in small plans, where one group's walk is the length of the call, as long as the stream's entries times the lanes of
+// a group stay below kFineRangeLanes: above it the longer ranges fill the GPU too and their rows stay closer together
+// (us a call, ranges of 16 / 64; power law, 1.2 M rows of 5: F = 8 69 / 100, F = 16 110 / 104, F = 64 354 / 291; power law,
+// 270,000 rows of 9: F = 8 27 / 44, F = 16 33 / 28, F = 64 114 / 87; R-MAT-18 + I: F = 16 52 / 59, F = 128 198 / 179).
+constexpr int kFineRangeNnz = 16;
+constexpr long long kFineRangeLanes = 6LL << 20;
 constexpr unsigned kLastInRow = 0x80000000u; // flag on s_col: last entry of its row
 constexpr unsigned kPlaceholder = 0x40000000u; // flag on s_col: row has no nonzeros, entry carries no data
 constexpr unsigned kColMask = 0x3fffffffu;
@@ -40,6 +46,13 @@ struct SplitRow {
     int pad;
 };
 
+// A cut of the short-row stream at row boundaries: range i starts at row row[i].
+struct Ranges {
+    int *row = nullptr;         // [n + 1]
+    int n = 0;
+    int start[kMaxRowClasses + 1] = {0};   // with row classes, class c's ranges are [start[c], start[c + 1])
+};
+
 // CSR of one orientation plus the work lists of its long rows.
 struct Side {
     bool ready = false;
@@ -58,15 +71,14 @@ struct Side {
     // Short rows (at most short_row_limit nonzeros) as one contiguous stream: their nonzeros copied
     // in row order, bit 31 of the column marking the last nonzero of a row.  A row without nonzeros
     // contributes one placeholder entry (bit 30) so that it is still written.  The stream is cut into
-    // ranges of about kShortRangeNnz entries at row boundaries; range i starts at row s_range_row[i].
+    // ranges of about kShortRangeNnz entries, in small plans also into ranges of about kFineRangeNnz.
     int *s_rows = nullptr;      // [n_short_rows] row id of each short row
     int *s_rowptr = nullptr;    // [n_short_rows + 1] start of each short row in the stream
     int *s_col = nullptr;       // [n_short_entries] column | flags
     float *s_val = nullptr;     // [n_short_entries]
-    int *s_range_row = nullptr; // [n_short_ranges + 1]
+    Ranges ranges, fine;
     int n_short_rows = 0;
     int n_short_entries = 0;
-    int n_short_ranges = 0;
     // Small plans (kSmallNnz): a call is one launch (spmm_small_kernel), in which split rows are closed by whoever
     // arrives last; slot_split[slot] = the slot's entry of `split`, arrived[entry] = slots written so far (0 between calls)
     bool small = false;
@@ -80,7 +92,7 @@ struct Side {
     // With row classes the four lists are class-major (all work of class 0 first, then class 1, ...; rows ascending
     // inside a class) and list x of class c is [x_start[c], x_start[c+1]).  Without classes everything is class 0.
     int n_classes = 1;
-    int range_start[kMaxRowClasses + 1] = {0}, chunk_start[kMaxRowClasses + 1] = {0};
+    int chunk_start[kMaxRowClasses + 1] = {0};
     int split_start[kMaxRowClasses + 1] = {0}, wide_start[kMaxRowClasses + 1] = {0};
 };
 

@@ -102,6 +102,19 @@ static int ensure_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
     return DRONE_OK;
 }
 
+// The copies are passes over [n, F]; what they save is in the gathers, so the line lies at a number of nonzeros per row.
+// us float by float / copied: power-law graphs of 270,000 rows and 9, 17, 33 nonzeros a row, F = 13: 57 / 52, 94 / 76,
+// 139 / 113, F = 63: 158 / 180, 264 / 258, 300 / 287, F = 401: 815 / 1192, 1310 / 1849, 2514 / 3113; R-MAT-22 (17 a row),
+// F = 41: 1710 / 2175; Reddit-shaped (491 a row), F = 41: 2410 / 1512.  On the smallest graphs the launches alone cost more
+// (5,000 rows, 33 a row, F = 41: 11 / 15), except where a lane would hold many single floats: above F = 128 operands that
+// stay in L2 with their copies are copied from 12 nonzeros a row on (F = 401: 108 / 42; 40,000 rows, F = 201: 153 / 144; but
+// 60,000 rows, 60 a row: 307 / 334).
+static bool worth_copying(const drone_plan *p, int F) {
+    const double per_row = (double)p->nnz / p->n_rows;
+    if (F > 128) return per_row >= 64 || (per_row >= 12 && (double)p->n_rows * F * 4 <= 40e6);
+    return p->nnz >= 1 << 20 && per_row >= (F <= 32 ? 16 : 32);
+}
+
 static bool may_allocate(cudaStream_t st) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
@@ -165,16 +178,13 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     const Side &s = p->side[orientation];
     if (p->n_rows == 0) return DRONE_OK;
     // Operands whose rows cannot be accessed as float4 where they lie are copied to where they can (X before the kernels,
-    // Y after them): passes over [n, F] against a gather of every row as often as it has nonzeros.  Not on the smallest
-    // graphs, where reading narrow rows float by float costs no more than the launches of the copies (R-MAT directed + I,
-    // F = 31, us: 0.3 M nonzeros 16 against 17, 2.1 M 53 against 44; F = 401, 1 M: 897 against 170).
+    // Y after them), where that is worth it.
     float *const caller_Y = Y;
     const long long caller_ldy = ldy;
     const int caller_F = F;
     const bool copy_x = !rows_of_vectors(F, ldx, X), copy_y = !rows_of_vectors(F, ldy, Y);
     bool vec4 = !copy_x && !copy_y;
-    const bool by_floats = s.small && F <= 128 && p->nnz <= 1 << 20;
-    if (!vec4 && F >= 5 && !by_floats && p->nnz >= 2LL * p->n_rows) {
+    if (!vec4 && F > 8 && worth_copying(p, F)) {
         const int Fp = (F + 3) & ~3;
         const long long stride = padded_stride(p->n_rows, F);
         const size_t x_floats = (size_t)stride * (size_t)p->n_rows, y_floats = (size_t)Fp * (size_t)p->n_rows;
@@ -221,6 +231,7 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     SpmmArgs a;
     a.side = &s;
     a.n_rows = p->n_rows;
+    a.nnz = p->nnz;
     a.ldy = ldy;
     a.partials = p->scratch;
     a.counter = p->counter;
@@ -447,7 +458,7 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
     }
     if ((what & DRONE_RESERVE_PADDED_ROWS) && p->n_rows > 0) {
         long long stride = 0;      // of the widths up to max_features, the one whose copy is largest
-        for (int f = 5; f <= max_features; ++f) stride = std::max(stride, padded_stride(p->n_rows, f));
+        for (int f = 9; f <= max_features; ++f) stride = std::max(stride, padded_stride(p->n_rows, f));
         return ensure_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)((max_features + 3) & ~3) * (size_t)p->n_rows);
     }
     return DRONE_OK;

@@ -160,6 +160,15 @@ template <> struct Vec<1> {
     }
 };
 
+// One of a lane's VPL vectors of a gathered row.  In the separate kernels, lanes with many single floats of a row (VEC = 1,
+// VPL >= 8: odd widths above 128) are bound by instructions, and nearly all of their loads are live: those keep the
+// branch, which costs them less than the zeroing of the predicated form.
+template <int VEC, int VPL, bool EARLY>
+__device__ __forceinline__ typename Vec<VEC>::type ld_row_if(const typename Vec<VEC>::type *ptr, unsigned long long pol, bool live) {
+    if (VEC == 1 && VPL >= 8 && !EARLY) return live ? ld_gathered<EARLY>(ptr, pol) : Vec<VEC>::zero();
+    return ld_gathered_if<EARLY>(ptr, pol, live);
+}
+
 template <int A, int B> struct MinOf { static constexpr int value = A < B ? A : B; };
 
 // What happens to a finished row before it is stored: Y[r,:] = act(row_scale[r] * sum).  Without a scale array the
@@ -274,7 +283,12 @@ constexpr int chunk_blocks_per_sm(int G, int VPL, int VEC, bool EXACT) {
     if (EXACT) return 0;
     return VPL == 2 ? 4 : VPL <= 4 ? 3 : 2;
 }
-constexpr int short_blocks_per_sm(int VPL, int VEC, bool EXACT) { return VEC != 4 || VPL > 1 ? 0 : EXACT ? 4 : 5; }
+// Short rows: five blocks leave 48 registers, enough for the four row vectors of a step (56 / 48 / 40 registers, us: power law,
+// 1.2 M rows of 17, F = 32 417 / 388 / 461, F = 64 765 / 713 / 799; R-MAT-22 F = 32 865 / 838 / 897).  Groups of one or two
+// lanes take 44 or fewer anyway, and with the bound at five came out slower (1.2 M rows of 9, F = 8: 129 / 156).
+constexpr int short_blocks_per_sm(int G, int VPL, int VEC, bool EXACT) {
+    return VEC != 4 || VPL > 1 ? 0 : EXACT && G < 4 ? 4 : 5;
+}
 
 // ---------------------------------------------------------------------------
 // 1. short rows: one lane group walks a range of the short-row stream
@@ -341,7 +355,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
                 const V *xr = row_address<VEC, HOT>(g, live ? (cc[u] & kColMask) : 0u, gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = ld_gathered_if<EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
+                    x[u][p] = ld_row_if<VEC, VPL, EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u) {
@@ -370,7 +384,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
 }
 
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
-__global__ void __launch_bounds__(256, short_blocks_per_sm(VPL, VEC, EXACT))
+__global__ void __launch_bounds__(256, short_blocks_per_sm(G, VPL, VEC, EXACT))
 spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, const int *__restrict__ s_rowptr,
                          const int *__restrict__ s_rows, const int *__restrict__ s_col,
                          const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec,
@@ -432,7 +446,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
                     x[u][p] = EXACT ? ld_gathered<EARLY>(xr + p * G, pol_keep)
-                                    : ld_gathered_if<EARLY>(xr + p * G, pol_keep, gl + p * G < nvec);
+                                    : ld_row_if<VEC, VPL, EARLY>(xr + p * G, pol_keep, gl + p * G < nvec);
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u)
@@ -463,7 +477,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = ld_gathered_if<EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
+                    x[u][p] = ld_row_if<VEC, VPL, EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u)
@@ -663,8 +677,8 @@ __device__ __forceinline__ void store_vector(const RowDestination<VEC> &dest, in
     else st_stream(dest.ptr + vi, v, pol);
 }
 
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT>
-__global__ void __launch_bounds__(256)
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, int BLOCKS_PER_SM>
+__global__ void __launch_bounds__(256, BLOCKS_PER_SM)
 spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_blocks, const int *__restrict__ col,
                   const float *__restrict__ val, const SplitRow *__restrict__ split, const int *__restrict__ slot_split,
                   int *arrived, float *partials, const int *__restrict__ s_range_row, int n_ranges,
@@ -756,6 +770,7 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
 struct SpmmArgs {
     const Side *side;
     int n_rows;
+    int nnz;
     int nvec;
     Gather gather;
     float *Y;
@@ -794,11 +809,17 @@ static int launch_all(const SpmmArgs &a) {
     constexpr int RPW = 32 / G;
     const Side &s = *a.side;
     int range_lo, n_ranges, chunk_lo, n_chunks, split_lo, n_split, wide_lo, n_wide;
-    class_range(a.row_class, s.n_classes, s.range_start, &range_lo, &n_ranges);
+    const bool fine = s.fine.row != nullptr && (G <= 2 || (long long)s.n_short_entries * G < kFineRangeLanes);
+    const Ranges &ranges = fine ? s.fine : s.ranges;
+    class_range(a.row_class, s.n_classes, ranges.start, &range_lo, &n_ranges);
     class_range(a.row_class, s.n_classes, s.chunk_start, &chunk_lo, &n_chunks);
     class_range(a.row_class, s.n_classes, s.split_start, &split_lo, &n_split);
     class_range(a.row_class, s.n_classes, s.wide_start, &wide_lo, &n_wide);
-    if (!HOT && s.small) {
+    // Lanes with many single floats of a row (odd widths above 128) keep few warps resident, so that one launch covers less
+    // (power-law graphs, one launch / separate kernels, us: F = 201 0.7 M nonzeros 75 / 107, 1.3 M 184 / 153; F = 401
+    // 0.02 M 14 / 31, 0.05 M 41 / 38).
+    const bool one_launch = s.small && (VEC == 4 || VPL < 8 || a.nnz <= (VPL < 16 ? kSmallNnzManyFloats : kSmallNnzMostFloats));
+    if (!HOT && one_launch) {
         const int chunk_blocks = ceil_div(n_chunks, 8), short_blocks = ceil_div(n_ranges, 8 * RPW);
         if (chunk_blocks + short_blocks == 0) return DRONE_OK;
         cudaLaunchAttribute early;
@@ -810,9 +831,17 @@ static int launch_all(const SpmmArgs &a) {
         cfg.stream = a.st;
         cfg.attrs = &early;
         cfg.numAttrs = 1;
-        DRONE_CUDA(cudaLaunchKernelEx(&cfg, spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT>, (const Chunk *)s.chunks + chunk_lo, n_chunks,
+        // Chunks want 64 registers, short rows want warps: 48 registers where most nonzeros lie in short rows and these are
+        // more than four blocks per SM work on at a time (64 / 48 registers, us: power law, 270,000 rows of 5, F = 32
+        // 39 / 30, F = 64 65 / 50; of 17, F = 128 275 / 246; but R-MAT-16 + I, F = 64, three quarters in chunks: 29 / 38, and
+        // 120,000 rows of 5, F = 64, one wave: 22 / 25).
+        auto kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0>;
+        if constexpr (VEC == 4 && VPL == 1 && G >= 4 && EXACT) {
+            if (short_blocks > 148 * 4 && s.n_short_entries >= a.nnz / 2) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 5>;
+        }
+        DRONE_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const Chunk *)s.chunks + chunk_lo, n_chunks,
                                       chunk_blocks, (const int *)s.col, (const float *)s.val, (const SplitRow *)s.split,
-                                      (const int *)s.slot_split, s.arrived, a.partials, (const int *)s.s_range_row + range_lo,
+                                      (const int *)s.slot_split, s.arrived, a.partials, (const int *)ranges.row + range_lo,
                                       n_ranges, (const int *)s.s_rowptr, (const int *)s.s_rows, (const int *)s.s_col,
                                       (const float *)s.s_val, a.gather, a.Y, a.ldy, a.nvec, a.epi));
         count_launch();
@@ -835,7 +864,7 @@ static int launch_all(const SpmmArgs &a) {
         }
         const int grid = ceil_div(n_ranges, 8 * RPW);
         spmm_short_stream_kernel<G, VPL, VEC, U, EXACT, UNIT, HOT><<<grid, 256, 0, short_stream>>>(
-            s.s_range_row + range_lo, n_ranges, s.s_rowptr, s.s_rows, s.s_col, s.s_val, a.gather, a.Y, a.ldy, a.nvec, a.epi);
+            ranges.row + range_lo, n_ranges, s.s_rowptr, s.s_rows, s.s_col, s.s_val, a.gather, a.Y, a.ldy, a.nvec, a.epi);
         DRONE_LAUNCH_CHECK("spmm_short_stream_kernel");
         if (overlap) DRONE_CUDA(cudaEventRecord(a.join, a.side_stream));
     }
@@ -893,6 +922,7 @@ static int dispatch_floats(const SpmmArgs &a) {
     if (f <= 1) return launch_all<1, 1, 1, 4, true, UNIT, HOT>(a);
     if (f <= 2) return launch_all<2, 1, 1, 4, true, UNIT, HOT>(a);
     if (f <= 4) return launch_all<4, 1, 1, 4, false, UNIT, HOT>(a);
+    if (f <= 8 && !a.side->small) return launch_all<8, 1, 1, 4, false, UNIT, HOT>(a);
     if (nv <= 2) return launch_all<2, 4, 1, 2, false, UNIT, HOT>(a);
     if (nv <= 4) return launch_all<4, 4, 1, 2, false, UNIT, HOT>(a);
     if (nv <= 8) return launch_all<8, 4, 1, 2, false, UNIT, HOT>(a);

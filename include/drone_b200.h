@@ -196,12 +196,12 @@ int drone_spmm_rows(drone_plan *plan, int orientation, int row_class, int F,
  *   DRONE_RESERVE_HOST_OPERANDS  the device staging of drone_spmm_host for [n_rows, max_features] operands;
  *   DRONE_RESERVE_PADDED_ROWS    room for copies of X and Y with padded rows, for operands whose rows cannot be accessed
  *                                16 bytes at a time where they lie (a width that is not a multiple of 4 such as the
- *                                class widths 41 and 47, odd leading dimensions, unaligned addresses).  Such calls copy
- *                                X, run the float4 kernels and copy the result out (two extra passes over [n_rows, F],
- *                                small beside the gathers); without the reservation the first such call makes the room
- *                                itself, unless it takes more than 4 GB or the stream is being captured, and then, as
- *                                on small graphs, the rows are accessed float by float.  Both routes add in the same
- *                                order.
+ *                                class widths 41 and 47, odd leading dimensions, unaligned addresses).  Where the graph
+ *                                has enough nonzeros per row, calls of more than 8 columns on such operands copy X, run
+ *                                the float4 kernels and copy the result out: two extra passes over [n_rows, F], made up
+ *                                for in the gathers.  Without the reservation the first such call makes the room itself,
+ *                                unless it takes more than 4 GB or the stream is being captured.  Everywhere else such
+ *                                rows are accessed float by float; either way adds in the same order.
  * After it, drone_spmm / drone_spmm_rows / drone_spmm_host with F <= max_features reach neither cudaMalloc nor a
  * device-wide synchronisation.
  * Stands where the reference sizes its cuSPARSE workspace on the first training step,

@@ -599,3 +599,29 @@ def test_copied_and_uncopied_rows_have_the_same_bits(cuda_device, oracle, f):
         assert torch.equal(plan.spmm(db.OP_AT, x), y)
         want, mag = oracle.spmm_csr_f64(*oracle.transpose_csr(n, n, index, dst, val), x.cpu().numpy(), with_abs=True)
         assert_close_to_oracle(y.cpu().numpy(), want, mag)
+
+
+@pytest.mark.parametrize("n,per_row,f", [(200000, 4, 8), (200000, 4, 16), (200000, 4, 64), (200000, 4, 100), (200000, 4, 128),
+                                         (30000, 40, 16), (30000, 40, 41), (30000, 40, 201), (5000, 40, 7), (5000, 40, 401)])
+def test_larger_one_launch_plans(cuda_device, oracle, n, per_row, f):
+    """Either side of the lines that a small plan's call is divided by: short ranges or long ones, registers for short rows or
+    for chunks, rows copied or read float by float.  None of them changes the order of a row's additions at these widths."""
+    import ctypes as C
+    rng = np.random.default_rng(n + f)
+    u, v = np.unique(rng.integers(0, n, size=(n * per_row, 2), dtype=np.int32), axis=0).T
+    index, dst, in_deg, out_deg, val = graph_case(gg, oracle, n, u.copy(), v.copy())
+    x = torch.as_tensor(gg.seeded_normal(500 + f, (n, f)), device=cuda_device)
+    plan = make_plan(cuda_device, index, dst, in_deg, out_deg)
+    y = plan.spmm(db.OP_AT, x)
+    want, mag = oracle.spmm_csr_f64(*oracle.transpose_csr(n, n, index, dst, val), x.cpu().numpy(), with_abs=True)
+    assert_close_to_oracle(y.cpu().numpy(), want, mag)
+    separate = make_plan(cuda_device, index, dst, in_deg, out_deg, DRONE_SMALL_NNZ=1)
+    if f > 8 or f % 4 == 0:
+        assert torch.equal(separate.spmm(db.OP_AT, x), y)
+    uncopied = torch.empty_like(y)
+    other = make_plan(cuda_device, index, dst, in_deg, out_deg)
+    rc = db.lib().drone_spmm_static_scratch(other.handle, db.OP_AT, f, C.c_void_p(x.data_ptr()), f,
+                                            C.c_void_p(uncopied.data_ptr()), f,
+                                            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, db.lib().drone_last_error()
+    assert torch.equal(uncopied, y)
