@@ -20,6 +20,7 @@
 #include "exchange.cuh"
 #include "plan.cuh"
 
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <new>
@@ -30,6 +31,7 @@ int xplan_ensure_device(drone_xplan *x);
 }
 
 struct drone_pr {
+    unsigned long long uid = 0;       // number of this handle in the process (addresses are reused, this is not)
     int device = 0, n_local = 0, global_v = 0, nnz = 0;
     bool dbl = false;
     double eps = 1e-6;
@@ -50,10 +52,11 @@ struct drone_pr {
     int *arrived = nullptr;           // [n_split_rows] slots written so far in this pull (0 between pulls)
     void *send = nullptr, *recv = nullptr;   // real2[max(up, down)]
     int *counters = nullptr;          // [0..3] exchange counts, [4] active count
-    // parts held by one process: {part, row} of every contribution a master row takes, in m_pos order, and the plans
-    // it was made for
-    int2 *pairs = nullptr;
+    // parts held by one process: {part, row} of every contribution a master row takes, in m_pos order, {place, out
+    // degree} of that row in its part, and the plans they were made for
+    int2 *pairs = nullptr, *targets = nullptr;
     std::vector<unsigned long long> pairs_for;
+    unsigned char *shared = nullptr;  // [n_local] 1 for rows that other parts hold too
     char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
     size_t control_bytes = 0;
     int sms = 0;
@@ -95,7 +98,8 @@ struct PartView {
     int *active, *ubm;
     const int *out_degree, *mirror2worker, *place;
     const int *m_rows, *m_off;
-    const int2 *pairs;
+    const int2 *pairs, *targets;
+    const unsigned char *shared;           // power iteration over several parts: 1 where the vertex is on others too
 };
 
 // Sum of v over the block in a fixed order (tree over warps), result in thread 0.
@@ -191,8 +195,9 @@ __device__ __forceinline__ R increment_vertices(const PartView<R> &p, R eps, R g
 }
 
 // pr' = (1-d)/V + d * (sum over in-edges + dangling/V), published as pr'/outDegree for the next iteration; after the
-// last one (`last`) the value itself is stored instead: before that nobody can see it.
-template <typename R>
+// last one (`last`) the value itself is stored instead: before that nobody can see it.  Leaves out the vertices that
+// p.shared marks (SHARED).
+template <typename R, bool SHARED>
 __device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R dang, bool last, int first, int stride) {
     const R base = ((R)1 - damping) / p.global_v;
     const R share = dang / p.global_v;
@@ -200,10 +205,11 @@ __device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R d
 #pragma unroll 1
     for (int i0 = first; i0 < p.n; i0 += kVertexBatch * stride) {
         R d[kVertexBatch];
-        int od[kVertexBatch], at[kVertexBatch];
+        int od[kVertexBatch], at[kVertexBatch], skip[kVertexBatch];
 #pragma unroll
         for (int b = 0; b < kVertexBatch; ++b) {
             const int i = i0 + b * stride;
+            skip[b] = i >= p.n ? 1 : SHARED ? (int)__ldg(p.shared + i) : 0;
             d[b] = i < p.n ? p.diff[i] : (R)0;
             od[b] = i < p.n && !last ? __ldg(p.out_degree + i) : 1;
             at[b] = i < p.n && !last && p.place ? __ldg(p.place + i) : i;
@@ -211,7 +217,7 @@ __device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R d
 #pragma unroll
         for (int b = 0; b < kVertexBatch; ++b) {
             const int i = i0 + b * stride;
-            if (i >= p.n) break;
+            if (skip[b]) continue;
             const R now = base + damping * (d[b] + share);
             if (last) {
                 p.pr[i] = now;
@@ -501,7 +507,7 @@ __global__ void pr_increment_kernel(PartView<R> p, R eps, R *block_sums) {
 template <typename R>
 __global__ void pr_power_apply_kernel(PartView<R> p, R damping, int store, R *block_sums) {
     const R dang = p.scalars[2];
-    const R tot = block_sum<R>(power_vertices(p, damping, dang, store != 0, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x));
+    const R tot = block_sum<R>(power_vertices<R, false>(p, damping, dang, store != 0, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x));
     if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
     if (blockIdx.x == 0 && threadIdx.x == 0) p.scalars[3] = ((R)1 - damping) / p.global_v + damping * (dang / p.global_v);
 }
@@ -629,7 +635,7 @@ __global__ void pr_set_scalar_kernel(R *scalars, int slot, R value) {
 // parts: 117 us per power iteration).  Here one cooperative launch, one block per SM, runs supersteps back to back
 // with a grid barrier between their phases; every block works for one part, blocks are dealt to the parts by their
 // number of edges, and boundary vertices are read and written where they lie instead of being packed and copied.
-// Measured on the same graphs: 33 us per superstep of the job, 22 us per power iteration.
+// Measured on the same graphs: 29 us per superstep of the job, 20 us per power iteration.
 
 constexpr int kMaxLocalParts = 64;
 constexpr int kHistorySteps = 128;         // supersteps of the job per launch
@@ -714,13 +720,81 @@ __device__ __forceinline__ void note_moved(unsigned *moved, int *counts, int q, 
     }
 }
 
+// The other parts' arrays, by part.
+template <typename R, int MAXP>
+struct PartArrays {
+    R *diff[MAXP], *push[MAXP], *pr[MAXP];
+    int *active[MAXP], *ubm[MAXP];
+};
+
+// power_vertices for the vertices that several parts hold, exchange included: a master adds what its mirrors' parts summed
+// (ascending rank order), and publishes the new value in every part that holds the vertex.  The mirrors' sums are only
+// read and the published values only written between two barriers, so that the exchange needs none of its own (us per
+// iteration with / without one; R-MAT-16: two parts, double 20.4 / 20.1, four, float 22.6 / 20.8, eight, double 27.7 / 27.0;
+// R-MAT-18, two parts, float 36.7 / 34.3).  Where a mirror publishes lies beside its row in a list of its own: looked up in
+// the mirror's part it was one scattered load more and made eight parts slower (28.4).
+template <typename R, int MAXP>
+__device__ __noinline__ R power_shared_vertices(const PartView<R> &p, const PartArrays<R, MAXP> &of, R damping, R dang, bool last,
+                                                   int first, int stride) {
+    const R base = ((R)1 - damping) / p.global_v;
+    const R share = dang / p.global_v;
+    R dangling = 0;
+#pragma unroll 1
+    for (int m = first; m < p.n_masters; m += stride) {
+        const int row = __ldg(p.m_rows + m), k0 = __ldg(p.m_off + m), k1 = __ldg(p.m_off + m + 1);
+        R d = p.diff[row];
+        const int od = last ? 1 : __ldg(p.out_degree + row), at = !last && p.place ? __ldg(p.place + row) : row;
+        // four mirrors at a time, their loads in flight together (most masters have fewer); the last four stay in registers
+        int2 to[4], where[4];
+        int k = k0;
+        while (true) {
+            R v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                to[u] = k + u < k1 ? p.pairs[k + u] : make_int2(-1, 0);
+                where[u] = k + u < k1 ? p.targets[k + u] : make_int2(0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = to[u].x < 0 ? (R)0 : of.diff[to[u].x][to[u].y];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (to[u].x >= 0) d += v[u];
+            if (k + 4 >= k1) break;
+            k += 4;
+        }
+        const R now = base + damping * (d + share);
+        if (last) {
+            p.pr[row] = now;
+        } else {
+            if (od == 0 && __ldg(p.mirror2worker + row) == -1) dangling += now;
+            p.push[at] = od == 0 ? not_pushed<R>() : now / od;
+        }
+        while (true) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int q = to[u].x;
+                if (q < 0) continue;
+                if (last) of.pr[q][to[u].y] = now;
+                else of.push[q][where[u].x] = where[u].y == 0 ? not_pushed<R>() : now / where[u].y;
+            }
+            k -= 4;
+            if (k < k0) break;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                to[u] = p.pairs[k + u];
+                where[u] = p.targets[k + u];
+            }
+        }
+    }
+    return dangling;
+}
+
 template <typename R, int MAXP, bool JOB, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constant__ RunArgs<R, MAXP> a) {
     extern __shared__ __align__(16) char table_bytes[];
     R *table = reinterpret_cast<R *>(table_bytes);
     __shared__ PartView<R> p;
-    __shared__ R *diff_of[MAXP];
-    __shared__ int *active_of[MAXP], *ubm_of[MAXP];
+    __shared__ PartArrays<R, MAXP> of;
     __shared__ int counts[MAXP * 4];
     __shared__ int me_shared;
     if (threadIdx.x == 0) {
@@ -730,9 +804,11 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
         p = a.part[q];
     }
     for (int q = threadIdx.x; q < a.n_parts; q += blockDim.x) {
-        diff_of[q] = a.part[q].diff;
-        active_of[q] = a.part[q].active;
-        ubm_of[q] = a.part[q].ubm;
+        of.diff[q] = a.part[q].diff;
+        of.push[q] = a.part[q].push;
+        of.pr[q] = a.part[q].pr;
+        of.active[q] = a.part[q].active;
+        of.ubm[q] = a.part[q].ubm;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) a.control->t_start = now_ns();
     __syncthreads();
@@ -771,20 +847,18 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
         if (JOB) gdiff = dang;
         if (!grid_barrier(a.control, phase)) return;
         if (JOB && step == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.control->t_pull = now_ns();
-        if (a.n_parts > 1) {
+        if (JOB && a.n_parts > 1) {
             // a master takes what its mirrors hold, in ascending rank order, and hands the total back (Mirror2MasterSend,
-            // pr.cu:215-297, Master2MirrorSend, :299-373); in the job only flagged entries travel, and they are counted
-            if (JOB) {
-                for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x) counts[q] = 0;
-                __syncthreads();
-            }
+            // pr.cu:215-297, Master2MirrorSend, :299-373); only flagged entries travel, and they are counted
+            for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x) counts[q] = 0;
+            __syncthreads();
             int received = 0, sent = 0;
             unsigned moved[MAXP <= 8 ? MAXP : 1] = {0};
 #pragma unroll 1
             for (int m = first; m < p.n_masters; m += stride) {
                 const int row = __ldg(p.m_rows + m), k0 = __ldg(p.m_off + m), k1 = __ldg(p.m_off + m + 1);
                 R d = p.diff[row];
-                const int own = JOB ? p.active[row] : 0;
+                const int own = p.active[row];
                 int got = 0;
                 // four mirrors at a time, their loads in flight together (most masters have fewer)
                 for (int k = k0; k < k1; k += 4) {
@@ -795,60 +869,50 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
                     for (int u = 0; u < 4; ++u) from[u] = k + u < k1 ? p.pairs[k + u] : make_int2(-1, 0);
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        flag[u] = from[u].x < 0 ? 0 : JOB ? active_of[from[u].x][from[u].y] : 1;
-                        v[u] = from[u].x < 0 ? (R)0 : diff_of[from[u].x][from[u].y];
+                        flag[u] = from[u].x < 0 ? 0 : of.active[from[u].x][from[u].y];
+                        v[u] = from[u].x < 0 ? (R)0 : of.diff[from[u].x][from[u].y];
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         if (flag[u] == 0) continue;
                         d += v[u];
-                        if (JOB) {
-                            ++got;
-                            note_moved<MAXP>(moved, counts, from[u].x, 0);
-                        }
+                        ++got;
+                        note_moved<MAXP>(moved, counts, from[u].x, 0);
                     }
                 }
-                if (JOB) {
-                    received += got;
-                    if (got) {
-                        p.diff[row] = d;
-                        p.ubm[row] = 1;
-                    }
-                    if (!got && own == 0) continue;
-                    sent += k1 - k0;
-                } else {
+                received += got;
+                if (got) {
                     p.diff[row] = d;
+                    p.ubm[row] = 1;
                 }
+                if (!got && own == 0) continue;
+                sent += k1 - k0;
                 for (int k = k0; k < k1; ++k) {
                     const int2 to = p.pairs[k];
-                    diff_of[to.x][to.y] = d;
-                    if (JOB) {
-                        ubm_of[to.x][to.y] = 1;
-                        note_moved<MAXP>(moved, counts, to.x, 3);
-                    }
+                    of.diff[to.x][to.y] = d;
+                    of.ubm[to.x][to.y] = 1;
+                    note_moved<MAXP>(moved, counts, to.x, 3);
                 }
             }
-            if (JOB) {
-                received = __reduce_add_sync(0xffffffffu, received);
-                sent = __reduce_add_sync(0xffffffffu, sent);
-                if ((threadIdx.x & 31) == 0) {
-                    if (received) atomicAdd(&counts[4 * me + 1], received);
-                    if (sent) atomicAdd(&counts[4 * me + 2], sent);
-                }
-                if (MAXP <= 8) {
+            received = __reduce_add_sync(0xffffffffu, received);
+            sent = __reduce_add_sync(0xffffffffu, sent);
+            if ((threadIdx.x & 31) == 0) {
+                if (received) atomicAdd(&counts[4 * me + 1], received);
+                if (sent) atomicAdd(&counts[4 * me + 2], sent);
+            }
+            if (MAXP <= 8) {
 #pragma unroll
-                    for (int q = 0; q < (MAXP <= 8 ? MAXP : 1); ++q) {
-                        const unsigned up = __reduce_add_sync(0xffffffffu, moved[q] & 0xffffu);
-                        const unsigned down = __reduce_add_sync(0xffffffffu, moved[q] >> 16);
-                        if ((threadIdx.x & 31) == 0 && up) atomicAdd(&counts[4 * q], (int)up);
-                        if ((threadIdx.x & 31) == 0 && down) atomicAdd(&counts[4 * q + 3], (int)down);
-                    }
+                for (int q = 0; q < (MAXP <= 8 ? MAXP : 1); ++q) {
+                    const unsigned up = __reduce_add_sync(0xffffffffu, moved[q] & 0xffffu);
+                    const unsigned down = __reduce_add_sync(0xffffffffu, moved[q] >> 16);
+                    if ((threadIdx.x & 31) == 0 && up) atomicAdd(&counts[4 * q], (int)up);
+                    if ((threadIdx.x & 31) == 0 && down) atomicAdd(&counts[4 * q + 3], (int)down);
                 }
-                __syncthreads();
-                int *h = a.history + (long long)step * a.n_parts * 4;
-                for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x)
-                    if (counts[q]) atomicAdd(h + q, counts[q]);
             }
+            __syncthreads();
+            int *h = a.history + (long long)step * a.n_parts * 4;
+            for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x)
+                if (counts[q]) atomicAdd(h + q, counts[q]);
             if (!grid_barrier(a.control, phase)) return;
         }
         if (JOB) {
@@ -864,7 +928,8 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
         } else {
             const R all = dang + (R)a.n_isolated * iso;
             const bool last = step + 1 == n_steps;
-            dangling = power_vertices(p, a.damping, all, last, first, stride);
+            dangling = power_vertices<R, (MAXP > 1)>(p, a.damping, all, last, first, stride);
+            if (MAXP > 1) dangling += power_shared_vertices<R, MAXP>(p, of, a.damping, all, last, first, stride);
             iso = ((R)1 - a.damping) / p.global_v + a.damping * (all / p.global_v);
         }
     }
@@ -889,21 +954,28 @@ __global__ void pr_slot_split_kernel(const SplitRow *__restrict__ split, int n_s
         for (int k = 0; k < split[i].nslots; ++k) slot_split[split[i].slot0 + k] = i;
 }
 
-// pairs[k] = {part, row} behind position m_pos[k] of part q's receive buffer: peer p's entries start at down_off[p]
-// there and are, in the same order, peer p's up list for q.
+// pairs[k] = {part, row} (and targets[k] = {place, out degree} of that row) behind position m_pos[k] of part q's receive
+// buffer: peer p's entries start at down_off[p] there and are, in the same order, peer p's up list for q.
 struct PeerLists {
     int down_off[kMaxLocalParts + 1];
     const int *up_rows[kMaxLocalParts];    // start of each peer's list for this part
+    const int *place[kMaxLocalParts], *out_degree[kMaxLocalParts];
 };
 
 __global__ void pr_pairs_kernel(const int *__restrict__ m_pos, int n, const __grid_constant__ PeerLists peers, int n_parts,
-                                int2 *pairs) {
+                                int2 *pairs, int2 *targets) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int pos = m_pos[k];
         int q = 0;
         while (q + 1 < n_parts && pos >= peers.down_off[q + 1]) ++q;
-        pairs[k] = make_int2(q, peers.up_rows[q][pos - peers.down_off[q]]);
+        const int row = peers.up_rows[q][pos - peers.down_off[q]];
+        pairs[k] = make_int2(q, row);
+        targets[k] = make_int2(peers.place[q] ? peers.place[q][row] : row, peers.out_degree[q][row]);
     }
+}
+
+__global__ void pr_mark_rows_kernel(const int *__restrict__ rows, int n, unsigned char *mark) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) mark[rows[i]] = 1;
 }
 
 // ---- host side ----
@@ -957,6 +1029,8 @@ static PartView<R> part_view(const drone_pr *p, int blocks) {
     v.m_off = x->d_m_off;
     v.n_masters = (int)x->m_rows.size();
     v.pairs = p->pairs;
+    v.targets = p->targets;
+    v.shared = nullptr;
     const long long capacity = kTableBytes / (long long)sizeof(R);
     long long t = std::min<long long>(capacity, p->n_local);
     if (!p->place && p->n_local > capacity) t = 0;
@@ -1144,11 +1218,14 @@ static int prepare_parts(std::vector<drone_pr *> &parts) {
     return DRONE_OK;
 }
 
-// Where every part's master rows find their mirrors in the other parts' arrays; made once per set of exchange plans.
+// Where every part's master rows find their mirrors in the other parts' arrays; made once per set of handles.
 static int prepare_pairs(std::vector<drone_pr *> &parts, cudaStream_t st) {
     const int P = (int)parts.size();
     std::vector<unsigned long long> key;
-    for (drone_pr *p : parts) key.push_back(p->xplan->uid);
+    for (drone_pr *p : parts) {
+        key.push_back(p->xplan->uid);
+        key.push_back(p->uid);
+    }
     for (int q = 0; q < P; ++q) {
         drone_pr *me = parts[q];
         const drone_xplan *x = me->xplan;
@@ -1161,12 +1238,28 @@ static int prepare_pairs(std::vector<drone_pr *> &parts, cudaStream_t st) {
             if (p != q && ns != nr)
                 return set_error(DRONE_E_STATE, "exchange plans disagree between parts %d and %d (%d vs %d rows)", p, q, ns, nr);
             lists.up_rows[p] = y->d_up_rows + y->up_off[q];
+            lists.place[p] = parts[p]->place;
+            lists.out_degree[p] = parts[p]->out_degree;
         }
         const int n = (int)x->m_pos.size();
         if (n > 0) {
             if (!me->pairs) DRONE_CUDA(cudaMalloc(&me->pairs, sizeof(int2) * (size_t)n));
-            pr_pairs_kernel<<<grid1d(n), 256, 0, st>>>(x->d_m_pos, n, lists, P, me->pairs);
+            if (!me->targets) DRONE_CUDA(cudaMalloc(&me->targets, sizeof(int2) * (size_t)n));
+            pr_pairs_kernel<<<grid1d(n), 256, 0, st>>>(x->d_m_pos, n, lists, P, me->pairs, me->targets);
             DRONE_LAUNCH_CHECK("pr_pairs_kernel");
+        }
+        if (me->n_local > 0) {
+            if (!me->shared) DRONE_CUDA(cudaMalloc(&me->shared, (size_t)me->n_local));
+            DRONE_CUDA(cudaMemsetAsync(me->shared, 0, (size_t)me->n_local, st));
+            const int up = (int)x->up_rows.size(), masters = (int)x->m_rows.size();
+            if (up > 0) {
+                pr_mark_rows_kernel<<<grid1d(up), 256, 0, st>>>(x->d_up_rows, up, me->shared);
+                DRONE_LAUNCH_CHECK("pr_mark_rows_kernel");
+            }
+            if (masters > 0) {
+                pr_mark_rows_kernel<<<grid1d(masters), 256, 0, st>>>(x->d_m_rows, masters, me->shared);
+                DRONE_LAUNCH_CHECK("pr_mark_rows_kernel");
+            }
         }
         me->pairs_for = key;
     }
@@ -1208,6 +1301,7 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     size_t table = 0;
     for (int q = 0; q < P; ++q) {
         a.part[q] = part_view<R>(parts[q], a.first_block[q + 1] - a.first_block[q]);
+        a.part[q].shared = parts[q]->shared;
         table = std::max(table, (size_t)a.part[q].table_n * sizeof(R));
     }
     a.block_sums = (R *)lead->block_sums;
@@ -1247,9 +1341,11 @@ static int run_local(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaS
     const bool few = parts.size() <= 8;
     if (lead->dbl) {
         if (rq.job) return few ? launch_run<double, 8, true>(parts, rq, st) : launch_run<double, kMaxLocalParts, true>(parts, rq, st);
+        if (parts.size() == 1) return launch_run<double, 1, false>(parts, rq, st);
         return few ? launch_run<double, 8, false>(parts, rq, st) : launch_run<double, kMaxLocalParts, false>(parts, rq, st);
     }
     if (rq.job) return few ? launch_run<float, 8, true>(parts, rq, st) : launch_run<float, kMaxLocalParts, true>(parts, rq, st);
+    if (parts.size() == 1) return launch_run<float, 1, false>(parts, rq, st);
     return few ? launch_run<float, 8, false>(parts, rq, st) : launch_run<float, kMaxLocalParts, false>(parts, rq, st);
 }
 
@@ -1326,6 +1422,8 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
     DRONE_REQUIRE(eps >= 0, "drone_pr_create: eps=%g is negative", eps);
     drone_pr *p = new (std::nothrow) drone_pr();
     if (!p) return set_error(DRONE_E_INVALID, "drone_pr_create: out of host memory");
+    static std::atomic<unsigned long long> created{0};
+    p->uid = ++created;
     p->n_local = n_local;
     p->global_v = global_v;
     p->nnz = nnz;
@@ -1408,7 +1506,8 @@ int drone_pr_destroy(drone_pr *p) {
     cudaFree(p->out_degree); cudaFree(p->mirror2worker); cudaFree(p->pr); cudaFree(p->acc); cudaFree(p->diff);
     cudaFree(p->push); cudaFree(p->active); cudaFree(p->ubm); cudaFree(p->scalars); cudaFree(p->block_sums);
     cudaFree(p->partials); cudaFree(p->send); cudaFree(p->recv); cudaFree(p->counters);
-    cudaFree(p->slot_split); cudaFree(p->arrived); cudaFree(p->pairs); cudaFree(p->control);
+    cudaFree(p->slot_split); cudaFree(p->arrived); cudaFree(p->pairs); cudaFree(p->targets); cudaFree(p->shared);
+    cudaFree(p->control);
     if (prev >= 0) cudaSetDevice(prev);
     delete p;
     return DRONE_OK;
