@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "../../include/drone_b200.h"
 
@@ -22,6 +23,32 @@ extern std::atomic<long long> g_kernel_launches;
 inline void count_launch(int n = 1) { g_kernel_launches.fetch_add(n, std::memory_order_relaxed); }
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+// Several device arrays as pieces of one allocation: cudaMalloc and above all cudaFree cost the same few hundred
+// microseconds for each of a handle's arrays that they cost for all of them together (graph and plan of R-MAT-22 + I, from
+// generator to ready: 61 -> 49 ms; Reddit-shaped 72 -> 62; PageRank handle of R-MAT-22 with its graph 65 -> 50).
+struct DeviceBlock {
+    void *base = nullptr;
+    template <typename T>
+    void add(T **array, size_t bytes) {
+        pieces.push_back({(void **)array, total});
+        total += (bytes + 255) / 256 * 256;
+    }
+    cudaError_t make() {
+        const cudaError_t e = cudaMalloc(&base, total > 0 ? total : 256);
+        if (e == cudaSuccess)
+            for (const Piece &p : pieces) *p.array = (char *)base + p.offset;
+        return e;
+    }
+    void release() {
+        cudaFree(base);
+        base = nullptr;
+    }
+private:
+    struct Piece { void **array; size_t offset; };
+    std::vector<Piece> pieces;
+    size_t total = 0;
+};
 
 // Device-side check of a CSR given by the caller (defined with the plan builder): DRONE_E_INVALID naming the first
 // bad row pointer or column, DRONE_OK for a well-formed input.  Synchronises `st`.

@@ -43,6 +43,7 @@ struct drone_mp {
     int *counters = nullptr;       // [0..3] exchange sizes, [4] VisitedSize; the run's control block follows them
     int4 *items = nullptr;         // [item_cap] {first edge, edges, value, 0}: pieces of the long rows of a round's frontier
     int item_cap = 0;
+    drone::DeviceBlock block;             // what the arrays above are pieces of
     bool started = false;
 };
 
@@ -669,17 +670,18 @@ int drone_mp_create(drone_mp **out, int kind, int n_local, int nnz, const int *d
     cudaError_t err = cudaGetDevice(&p->device);
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
     const size_t nb = std::max<size_t>(std::max(xplan->up_rows.size(), xplan->down_rows.size()), 1);
-    if (err == cudaSuccess) err = cudaMalloc(&p->value, sizeof(unsigned) * n1);
-    if (err == cudaSuccess) err = cudaMalloc(&p->state, sizeof(int) * (n1 + 3));      // read four at a time
-    if (err == cudaSuccess) err = cudaMalloc(&p->active, sizeof(int) * n1);
-    if (err == cudaSuccess) err = cudaMalloc(&p->ubm, sizeof(int) * n1);
-    if (err == cudaSuccess) err = cudaMalloc(&p->send, sizeof(uint2) * nb);
-    if (err == cudaSuccess) err = cudaMalloc(&p->recv, sizeof(uint2) * nb);
-    if (err == cudaSuccess) err = cudaMalloc(&p->counters, sizeof(MpReport));
+    p->block.add(&p->value, sizeof(unsigned) * n1);
+    p->block.add(&p->state, sizeof(int) * (n1 + 3));      // read four at a time
+    p->block.add(&p->active, sizeof(int) * n1);
+    p->block.add(&p->ubm, sizeof(int) * n1);
+    p->block.add(&p->send, sizeof(uint2) * nb);
+    p->block.add(&p->recv, sizeof(uint2) * nb);
+    p->block.add(&p->counters, sizeof(MpReport));
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
     // every row above kWarpRow in the frontier at once: full pieces, and one partial piece per such row
     p->item_cap = nnz / kItemEdges + nnz / kWarpRow + 16;
-    if (err == cudaSuccess) err = cudaMalloc(&p->items, sizeof(int4) * (size_t)p->item_cap);
+    p->block.add(&p->items, sizeof(int4) * (size_t)p->item_cap);
+    if (err == cudaSuccess) err = p->block.make();
     if (err != cudaSuccess) {
         drone_mp_destroy(p);
         return set_error(DRONE_E_CUDA, "drone_mp_create: %s", cudaGetErrorString(err));
@@ -693,8 +695,7 @@ int drone_mp_destroy(drone_mp *p) {
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(p->device);
-    cudaFree(p->value); cudaFree(p->active); cudaFree(p->ubm); cudaFree(p->send); cudaFree(p->recv); cudaFree(p->counters);
-    cudaFree(p->state); cudaFree(p->items);
+    p->block.release();
     if (prev >= 0) cudaSetDevice(prev);
     delete p;
     return DRONE_OK;

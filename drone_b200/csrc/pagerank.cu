@@ -59,6 +59,7 @@ struct drone_pr {
     unsigned char *shared = nullptr;  // [n_local] 1 for rows that other parts hold too
     char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
     size_t control_bytes = 0;
+    drone::DeviceBlock block;                // what the arrays made at creation are pieces of
     int sms = 0;
     bool started = false;
     long long n_isolated = 0;         // vertex ids that occur in no part (power iteration treats them as dangling)
@@ -1436,12 +1437,10 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
     int rc = DRONE_OK;
     do {
-        // transposed graph and the split of long rows: reuse the aggregation plan (coefficients unused)
-        float *ones = nullptr;
-        if (cudaMalloc(&ones, sizeof(float) * (size_t)(nnz > 0 ? nnz : 1)) != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: out of device memory"); break; }
-        cudaMemset(ones, 0, sizeof(float) * (size_t)(nnz > 0 ? nnz : 1));
-        rc = plan_create_untagged(&p->plan, n_local, nnz, d_index, d_dst, ones, nullptr, nullptr, DRONE_PLAN_AT, nullptr);
-        cudaFree(ones);
+        // transposed graph and the split of long rows: reuse the aggregation plan, whose coefficients are never read here, so
+        // any nnz words do
+        rc = plan_create_untagged(&p->plan, n_local, nnz, d_index, d_dst, reinterpret_cast<const float *>(d_dst), nullptr, nullptr,
+                                  DRONE_PLAN_AT, nullptr);
         if (rc) break;
         {
             const char *v = getenv("DRONE_PR_ORDER_MIN_ROWS");
@@ -1452,27 +1451,27 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
             }
         }
         cudaError_t e = cudaSuccess;
-        auto alloc = [&](void **ptr, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(ptr, bytes > 0 ? bytes : 16); };
-        alloc((void **)&p->out_degree, sizeof(int) * n1);
-        alloc((void **)&p->mirror2worker, sizeof(int) * n1);
-        alloc(&p->pr, rs * n1);
-        alloc(&p->acc, rs * n1);
-        alloc(&p->diff, rs * n1);
-        alloc(&p->push, rs * n1);
-        alloc((void **)&p->active, sizeof(int) * n1);
-        alloc((void **)&p->ubm, sizeof(int) * n1);
-        alloc(&p->scalars, 8 * 4);
-        alloc(&p->block_sums, 8 * kReduceBlocks);
+        p->block.add(&p->out_degree, sizeof(int) * n1);
+        p->block.add(&p->mirror2worker, sizeof(int) * n1);
+        p->block.add(&p->pr, rs * n1);
+        p->block.add(&p->acc, rs * n1);
+        p->block.add(&p->diff, rs * n1);
+        p->block.add(&p->push, rs * n1);
+        p->block.add(&p->active, sizeof(int) * n1);
+        p->block.add(&p->ubm, sizeof(int) * n1);
+        p->block.add(&p->scalars, 8 * 4);
+        p->block.add(&p->block_sums, 8 * kReduceBlocks);
         const Side &side = p->plan->side[DRONE_OP_AT];
-        alloc(&p->partials, 2 * rs * (size_t)side.n_partials);
-        alloc((void **)&p->slot_split, sizeof(int) * (size_t)side.n_partials);
-        alloc((void **)&p->arrived, sizeof(int) * (size_t)side.n_split_rows);
+        p->block.add(&p->partials, 2 * rs * (size_t)side.n_partials);
+        p->block.add(&p->slot_split, sizeof(int) * (size_t)side.n_partials);
+        p->block.add(&p->arrived, sizeof(int) * (size_t)side.n_split_rows);
         const size_t nb = std::max(xplan->up_rows.size(), xplan->down_rows.size());
-        alloc(&p->send, 2 * rs * nb);
-        alloc(&p->recv, 2 * rs * nb);
-        alloc((void **)&p->counters, sizeof(int) * 8);
+        p->block.add(&p->send, 2 * rs * nb);
+        p->block.add(&p->recv, 2 * rs * nb);
+        p->block.add(&p->counters, sizeof(int) * 8);
+        if (e == cudaSuccess) e = p->block.make();
         p->control_bytes = sizeof(RunControl) + sizeof(int) * 4 * (size_t)xplan->nranks * kHistorySteps;
-        alloc((void **)&p->control, p->control_bytes);
+        if (e == cudaSuccess) e = cudaMalloc(&p->control, p->control_bytes);
         if (e == cudaSuccess) e = cudaMemset(p->control, 0, p->control_bytes);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
         if (e == cudaSuccess && side.n_split_rows > 0) {
@@ -1503,10 +1502,8 @@ int drone_pr_destroy(drone_pr *p) {
     cudaSetDevice(p->device);
     drone_plan_destroy(p->plan);
     cudaFree(p->place);
-    cudaFree(p->out_degree); cudaFree(p->mirror2worker); cudaFree(p->pr); cudaFree(p->acc); cudaFree(p->diff);
-    cudaFree(p->push); cudaFree(p->active); cudaFree(p->ubm); cudaFree(p->scalars); cudaFree(p->block_sums);
-    cudaFree(p->partials); cudaFree(p->send); cudaFree(p->recv); cudaFree(p->counters);
-    cudaFree(p->slot_split); cudaFree(p->arrived); cudaFree(p->pairs); cudaFree(p->targets); cudaFree(p->shared);
+    p->block.release();
+    cudaFree(p->pairs); cudaFree(p->targets); cudaFree(p->shared);
     cudaFree(p->control);
     if (prev >= 0) cudaSetDevice(prev);
     delete p;

@@ -338,17 +338,9 @@ static void free_side(Side &s) {
     cudaFree(s.rowptr);
     cudaFree(s.col);
     cudaFree(s.val);
-    cudaFree(s.chunks);
-    cudaFree(s.split);
+    s.lists.release();
     cudaFree(s.wide);
-    cudaFree(s.slot_split);
-    cudaFree(s.arrived);
-    cudaFree(s.s_rows);
-    cudaFree(s.s_rowptr);
-    cudaFree(s.s_col);
-    cudaFree(s.s_val);
-    cudaFree(s.ranges.row);
-    cudaFree(s.fine.row);
+    s.stream.release();
     s = Side();
 }
 
@@ -361,77 +353,65 @@ static int build_transpose(drone_plan *p, cudaStream_t st) {
     DRONE_CUDA(cudaMalloc(&t.col, sizeof(int) * (size_t)(nnz > 0 ? nnz : 1)));
     DRONE_CUDA(cudaMalloc(&t.val, sizeof(float) * (size_t)(nnz > 0 ? nnz : 1)));
 
+    int end_bit = 1;
+    while (end_bit < 31 && (1LL << end_bit) < (long long)n) ++end_bit;
+    // scratch, one allocation; the sort's keys lie in what becomes the column array
+    struct Temp {
+        DeviceBlock block;
+        ~Temp() { block.release(); }
+    } scratch;
+    int *counts = nullptr, *src = nullptr, *keys_alt = nullptr, *perm = nullptr, *perm_alt = nullptr;
+    void *tmp = nullptr;
+    const size_t words = sizeof(int) * (size_t)nnz;
+    scratch.block.add(&counts, sizeof(int) * (size_t)(n + 1));
+    scratch.block.add(&src, words);
+    scratch.block.add(&keys_alt, words);
+    scratch.block.add(&perm, words);
+    scratch.block.add(&perm_alt, words);
+    cub::DoubleBuffer<int> keys(t.col, nullptr), edges(nullptr, nullptr);
+    size_t scan_bytes = 0, sort_bytes = 0;
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, counts, t.rowptr, n + 1, st));
+    if (nnz > 0) DRONE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, edges, nnz, 0, end_bit, st));
+    scratch.block.add(&tmp, std::max(scan_bytes, sort_bytes));
+    DRONE_CUDA(scratch.block.make());
+
     // row pointer of the transpose: histogram of destinations, then exclusive scan
-    int *counts = nullptr;
-    DRONE_CUDA(cudaMalloc(&counts, sizeof(int) * (size_t)(n + 1)));
     DRONE_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)(n + 1), st));
     if (nnz > 0) {
         histogram_kernel<<<grid_for(nnz), 256, 0, st>>>(a.col, nnz, counts);
         DRONE_LAUNCH_CHECK("histogram_kernel");
     }
-    size_t tmp_bytes = 0;
-    void *tmp = nullptr;
-    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, counts, t.rowptr, n + 1, st));
-    DRONE_CUDA(cudaMalloc(&tmp, tmp_bytes > 0 ? tmp_bytes : 1));
-    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, t.rowptr, n + 1, st));
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, counts, t.rowptr, n + 1, st));
     count_launch();
-    DRONE_CUDA(cudaStreamSynchronize(st));
-    cudaFree(tmp);
-    cudaFree(counts);
-
     if (nnz > 0) {
         // stable sort of edge ids by destination: sources stay ascending inside a row
-        int *src = nullptr, *keys_alt = nullptr, *perm = nullptr, *perm_alt = nullptr, *keys = nullptr;
-        DRONE_CUDA(cudaMalloc(&src, sizeof(int) * (size_t)nnz));
-        DRONE_CUDA(cudaMalloc(&keys, sizeof(int) * (size_t)nnz));
-        DRONE_CUDA(cudaMalloc(&keys_alt, sizeof(int) * (size_t)nnz));
-        DRONE_CUDA(cudaMalloc(&perm, sizeof(int) * (size_t)nnz));
-        DRONE_CUDA(cudaMalloc(&perm_alt, sizeof(int) * (size_t)nnz));
         expand_rows_kernel<<<grid_for(nnz), 256, 0, st>>>(a.rowptr, n, nnz, src);
         DRONE_LAUNCH_CHECK("expand_rows_kernel");
         iota_kernel<<<grid_for(nnz), 256, 0, st>>>(perm, nnz);
         DRONE_LAUNCH_CHECK("iota_kernel");
-        DRONE_CUDA(cudaMemcpyAsync(keys, a.col, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToDevice, st));
-        int end_bit = 1;
-        while (end_bit < 31 && (1LL << end_bit) < (long long)n) ++end_bit;
-        cub::DoubleBuffer<int> kb(keys, keys_alt);
-        cub::DoubleBuffer<int> vb(perm, perm_alt);
-        tmp_bytes = 0;
-        DRONE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, kb, vb, nnz, 0, end_bit, st));
-        DRONE_CUDA(cudaMalloc(&tmp, tmp_bytes > 0 ? tmp_bytes : 1));
-        DRONE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, nnz, 0, end_bit, st));
+        DRONE_CUDA(cudaMemcpyAsync(t.col, a.col, words, cudaMemcpyDeviceToDevice, st));
+        keys = cub::DoubleBuffer<int>(t.col, keys_alt);
+        edges = cub::DoubleBuffer<int>(perm, perm_alt);
+        DRONE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, keys, edges, nnz, 0, end_bit, st));
         count_launch();
-        gather_transposed_kernel<<<grid_for(nnz), 256, 0, st>>>(vb.Current(), src, a.val, nnz, t.col, t.val);
+        gather_transposed_kernel<<<grid_for(nnz), 256, 0, st>>>(edges.Current(), src, a.val, nnz, t.col, t.val);
         DRONE_LAUNCH_CHECK("gather_transposed_kernel");
-        DRONE_CUDA(cudaStreamSynchronize(st));
-        cudaFree(tmp);
-        cudaFree(src);
-        cudaFree(keys);
-        cudaFree(keys_alt);
-        cudaFree(perm);
-        cudaFree(perm_alt);
     }
+    DRONE_CUDA(cudaStreamSynchronize(st));
     return DRONE_OK;
 }
 
 static void free_lists(Side &s) {
-    cudaFree(s.chunks);
-    cudaFree(s.split);
+    s.lists.release();
     cudaFree(s.wide);
-    cudaFree(s.slot_split);
-    cudaFree(s.arrived);
-    cudaFree(s.s_rows);
-    cudaFree(s.s_rowptr);
-    cudaFree(s.s_col);
-    cudaFree(s.s_val);
-    cudaFree(s.ranges.row);
-    cudaFree(s.fine.row);
+    s.stream.release();
     s.slot_split = s.arrived = nullptr;
     s.small = false;
     s.chunks = nullptr;
     s.split = s.wide = nullptr;
     s.s_rows = s.s_rowptr = s.s_col = nullptr;
     s.ranges = s.fine = Ranges();
+    s.stream = s.lists = DeviceBlock();
     s.s_val = nullptr;
     s.ready = false;
 }
@@ -463,14 +443,17 @@ static int class_major_scan(const drone_plan *p, const int *cnt, int *off, int *
     return DRONE_OK;
 }
 
-// Cuts the stream of short rows into ranges of about range_nnz entries.  K row classes, class c's short rows starting at
-// row_start[c] of s_rows and its entries at entry_start[c]; both arrays stay alive until the caller has synchronised st.
-static int cut_ranges(const Side &s, Ranges &out, int range_nnz, int K, const int *row_start, const int *entry_start,
-                      cudaStream_t st) {
+// The cut of the stream of short rows into ranges of about range_nnz entries.  K row classes, class c's short rows starting
+// at row_start[c] of s_rows and its entries at entry_start[c]; both arrays stay alive until the caller has synchronised st.
+static void add_ranges(Side &s, Ranges &out, int range_nnz, int K, const int *entry_start) {
     out.start[0] = 0;
     for (int c = 0; c < K; ++c) out.start[c + 1] = out.start[c] + ceil_div(entry_start[c + 1] - entry_start[c], range_nnz);
     out.n = out.start[K];
-    DRONE_CUDA(cudaMalloc(&out.row, sizeof(int) * (size_t)(out.n + 1)));
+    s.stream.add(&out.row, sizeof(int) * (size_t)(out.n + 1));
+}
+
+static int cut_ranges(const Side &s, const Ranges &out, int range_nnz, int K, const int *row_start, const int *entry_start,
+                      cudaStream_t st) {
     // ranges never straddle two classes; entry start[c] is also the end of class c-1's last range
     for (int c = 0; c < K; ++c) {
         const int nr = out.start[c + 1] - out.start[c];
@@ -492,10 +475,15 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     struct Temp {        // freed on every way out
         int *buf = nullptr;
         void *scan = nullptr;
-        ~Temp() { cudaFree(buf); cudaFree(scan); }
+        DeviceBlock block;
+        ~Temp() { block.release(); }
     } t;
     const size_t stride = (size_t)(n + 1);
-    DRONE_CUDA(cudaMalloc(&t.buf, sizeof(int) * stride * 10));  // 10 arrays of n+1 ints: counts x4, offsets x4, scratch x2
+    size_t tmp_bytes = 0;
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, t.buf, t.buf, n + 1, st));
+    t.block.add(&t.buf, sizeof(int) * stride * 10);  // 10 arrays of n+1 ints: counts x4, offsets x4, scratch x2
+    t.block.add(&t.scan, tmp_bytes);
+    DRONE_CUDA(t.block.make());
     int *buf = t.buf;
     int *cnt[4] = {buf, buf + stride, buf + 2 * stride, buf + 3 * stride};
     int *off[4] = {buf + 4 * stride, buf + 5 * stride, buf + 6 * stride, buf + 7 * stride};
@@ -503,9 +491,6 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     count_chunks_kernel<<<grid_for(n + 1), 256, 0, st>>>(s.rowptr, n, p->short_row_limit, p->chunk_nnz,
                                                         cnt[0], cnt[1], cnt[2], cnt[3]);
     DRONE_LAUNCH_CHECK("count_chunks_kernel");
-    size_t tmp_bytes = 0;
-    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt[0], off[0], n + 1, st));
-    DRONE_CUDA(cudaMalloc(&t.scan, tmp_bytes > 0 ? tmp_bytes : 1));
     void *tmp = t.scan;
     int rc;
     int slot_start[kMaxRowClasses + 1], long_start[kMaxRowClasses + 1];
@@ -523,14 +508,17 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     s.n_wide_rows = 0;
     for (int c = 0; c <= K; ++c) s.wide_start[c] = 0;
     if (s.n_chunks > 0) {
-        DRONE_CUDA(cudaMalloc(&s.chunks, sizeof(Chunk) * (size_t)s.n_chunks));
-        DRONE_CUDA(cudaMalloc(&s.split, sizeof(SplitRow) * (size_t)(s.n_split_rows > 0 ? s.n_split_rows : 1)));
+        s.lists.add(&s.chunks, sizeof(Chunk) * (size_t)s.n_chunks);
+        s.lists.add(&s.split, sizeof(SplitRow) * (size_t)s.n_split_rows);
+        if (s.small && s.n_split_rows > 0) {
+            s.lists.add(&s.slot_split, sizeof(int) * (size_t)s.n_partials);
+            s.lists.add(&s.arrived, sizeof(int) * (size_t)s.n_split_rows);
+        }
+        DRONE_CUDA(s.lists.make());
         fill_chunks_kernel<<<grid_for(n), 256, 0, st>>>(s.rowptr, n, p->chunk_nnz, cnt[0], off[0], off[1], off[2],
                                                        s.chunks, s.split);
         DRONE_LAUNCH_CHECK("fill_chunks_kernel");
         if (s.small && s.n_split_rows > 0) {
-            DRONE_CUDA(cudaMalloc(&s.slot_split, sizeof(int) * (size_t)s.n_partials));
-            DRONE_CUDA(cudaMalloc(&s.arrived, sizeof(int) * (size_t)s.n_split_rows));
             DRONE_CUDA(cudaMemsetAsync(s.arrived, 0, sizeof(int) * (size_t)s.n_split_rows, st));
             fill_slot_split_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, s.slot_split);
             DRONE_LAUNCH_CHECK("fill_slot_split_kernel");
@@ -575,19 +563,21 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
                 int *key = nullptr, *idx = nullptr, *key2 = nullptr, *idx2 = nullptr;
                 Chunk *sorted = nullptr;
                 void *tmp = nullptr;
-                ~Sort() { cudaFree(key); cudaFree(idx); cudaFree(key2); cudaFree(idx2); cudaFree(tmp); cudaFree(sorted); }
+                DeviceBlock block;
+                ~Sort() { block.release(); }
             } o;
             const size_t nb = sizeof(int) * (size_t)s.n_chunks;
-            DRONE_CUDA(cudaMalloc(&o.key, nb));
-            DRONE_CUDA(cudaMalloc(&o.idx, nb));
-            DRONE_CUDA(cudaMalloc(&o.key2, nb));
-            DRONE_CUDA(cudaMalloc(&o.idx2, nb));
-            DRONE_CUDA(cudaMalloc(&o.sorted, sizeof(Chunk) * (size_t)s.n_chunks));
-            chunk_first_column_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, s.n_chunks, s.col, o.key, o.idx);
-            DRONE_LAUNCH_CHECK("chunk_first_column_kernel");
             size_t sort_bytes = 0;
             DRONE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, o.key, o.key2, o.idx, o.idx2, s.n_chunks, 0, 30, st));
-            DRONE_CUDA(cudaMalloc(&o.tmp, sort_bytes > 0 ? sort_bytes : 1));
+            o.block.add(&o.key, nb);
+            o.block.add(&o.idx, nb);
+            o.block.add(&o.key2, nb);
+            o.block.add(&o.idx2, nb);
+            o.block.add(&o.sorted, sizeof(Chunk) * (size_t)s.n_chunks);
+            o.block.add(&o.tmp, sort_bytes);
+            DRONE_CUDA(o.block.make());
+            chunk_first_column_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, s.n_chunks, s.col, o.key, o.idx);
+            DRONE_LAUNCH_CHECK("chunk_first_column_kernel");
             DRONE_CUDA(cub::DeviceRadixSort::SortPairs(o.tmp, sort_bytes, o.key, o.key2, o.idx, o.idx2, s.n_chunks, 0, 30, st));
             count_launch();
             permute_chunks_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, o.idx2, s.n_chunks, o.sorted);
@@ -605,10 +595,13 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
     s.n_short_rows = srow_start[K];
     s.n_short_entries = sent_start[K];
     if (s.n_short_rows > 0) {
-        DRONE_CUDA(cudaMalloc(&s.s_rows, sizeof(int) * (size_t)s.n_short_rows));
-        DRONE_CUDA(cudaMalloc(&s.s_rowptr, sizeof(int) * (size_t)(s.n_short_rows + 1)));
-        DRONE_CUDA(cudaMalloc(&s.s_col, sizeof(int) * (size_t)s.n_short_entries));
-        DRONE_CUDA(cudaMalloc(&s.s_val, sizeof(float) * (size_t)s.n_short_entries));
+        s.stream.add(&s.s_rows, sizeof(int) * (size_t)s.n_short_rows);
+        s.stream.add(&s.s_rowptr, sizeof(int) * (size_t)(s.n_short_rows + 1));
+        s.stream.add(&s.s_col, sizeof(int) * (size_t)s.n_short_entries);
+        s.stream.add(&s.s_val, sizeof(float) * (size_t)s.n_short_entries);
+        add_ranges(s, s.ranges, kShortRangeNnz, K, sent_start);
+        if (s.small) add_ranges(s, s.fine, kFineRangeNnz, K, sent_start);
+        DRONE_CUDA(s.stream.make());
         fill_short_kernel<<<grid_for(n), 256, 0, st>>>(s.rowptr, s.col, s.val, n, p->short_row_limit, off[0], off[1],
                                                       s.s_rows, s.s_rowptr, s.s_col, s.s_val);
         DRONE_LAUNCH_CHECK("fill_short_kernel");
@@ -786,21 +779,23 @@ int plan_order_columns_by_frequency(drone_plan *p, int orientation, const int *d
     struct Temp {
         int *freq = nullptr, *ids = nullptr, *freq_sorted = nullptr, *ids_sorted = nullptr, *place = nullptr;
         void *sort = nullptr;
-        ~Temp() { cudaFree(freq); cudaFree(ids); cudaFree(freq_sorted); cudaFree(ids_sorted); cudaFree(place); cudaFree(sort); }
+        DeviceBlock block;
+        ~Temp() { cudaFree(place); block.release(); }
     } t;
     const size_t bytes = sizeof(int) * (size_t)(n + 1);
-    DRONE_CUDA(cudaMalloc(&t.freq, bytes));
-    DRONE_CUDA(cudaMalloc(&t.ids, bytes));
-    DRONE_CUDA(cudaMalloc(&t.freq_sorted, bytes));
-    DRONE_CUDA(cudaMalloc(&t.ids_sorted, bytes));
+    size_t tmp_bytes = 0;
+    DRONE_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_bytes, t.freq, t.freq_sorted, t.ids, t.ids_sorted, n, 0, 32, st));
+    t.block.add(&t.freq, bytes);
+    t.block.add(&t.ids, bytes);
+    t.block.add(&t.freq_sorted, bytes);
+    t.block.add(&t.ids_sorted, bytes);
+    t.block.add(&t.sort, tmp_bytes);
+    DRONE_CUDA(t.block.make());
     DRONE_CUDA(cudaMalloc(&t.place, bytes));
     row_lengths_kernel<<<grid_for(n), 256, 0, st>>>(d_other_rowptr, n, t.freq);
     DRONE_LAUNCH_CHECK("row_lengths_kernel");
     iota_kernel<<<grid_for(n), 256, 0, st>>>(t.ids, n);
     DRONE_LAUNCH_CHECK("iota_kernel");
-    size_t tmp_bytes = 0;
-    DRONE_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_bytes, t.freq, t.freq_sorted, t.ids, t.ids_sorted, n, 0, 32, st));
-    DRONE_CUDA(cudaMalloc(&t.sort, tmp_bytes > 0 ? tmp_bytes : 1));
     DRONE_CUDA(cub::DeviceRadixSort::SortPairsDescending(t.sort, tmp_bytes, t.freq, t.freq_sorted, t.ids, t.ids_sorted, n, 0, 32, st));
     count_launch();
     scatter_positions_kernel<<<grid_for(n), 256, 0, st>>>(t.ids_sorted, n, t.place);

@@ -77,6 +77,7 @@ struct Side {
     int *s_col = nullptr;       // [n_short_entries] column | flags
     float *s_val = nullptr;     // [n_short_entries]
     Ranges ranges, fine;
+    DeviceBlock stream, lists;  // what the arrays of the short rows, and those of the chunks, are pieces of
     int n_short_rows = 0;
     int n_short_entries = 0;
     // Small plans (kSmallNnz): a call is one launch (spmm_small_kernel), in which split rows are closed by whoever
