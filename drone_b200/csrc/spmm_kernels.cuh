@@ -160,12 +160,22 @@ template <> struct Vec<1> {
     }
 };
 
-// One of a lane's VPL vectors of a gathered row.  In the separate kernels, lanes with many single floats of a row (VEC = 1,
-// VPL >= 8: odd widths above 128) are bound by instructions, and nearly all of their loads are live: those keep the
-// branch, which costs them less than the zeroing of the predicated form.
-template <int VEC, int VPL, bool EARLY>
+// Of a lane's VPL vectors, how many lie inside the row at every width that the shape is used for (dispatch_floats: a shape
+// of 32 x VPL single floats starts where the next smaller one ends).  Their loads need no test against the width (us with a
+// test per vector / without, power law: 90,000 rows of 41, F = 131 268 / 248, F = 401 868 / 730; 250,000 rows of 7, F = 95
+// 155 / 128).  Above 512 floats half of the tests stay, and without the other half F = 601 was slower: 60,000 rows of 13,
+// 419 / 463.
+constexpr int sure_vectors(int G, int VPL, int VEC) {
+    if (VEC != 1 || G != 32) return 0;
+    return VPL == 4 ? 2 : VPL == 8 ? 4 : VPL == 12 ? 8 : VPL == 16 ? 12 : 0;
+}
+
+// The condition of a lane's vector p of a row.  BRANCH: lanes with many single floats of a row (odd widths above 128) in the
+// short-row kernel, and above 512 everywhere, are bound by instructions, and nearly all of their loads are live: a branch
+// costs them less than the zeroing of the predicated form.
+template <bool BRANCH, int VEC, bool EARLY>
 __device__ __forceinline__ typename Vec<VEC>::type ld_row_if(const typename Vec<VEC>::type *ptr, unsigned long long pol, bool live) {
-    if (VEC == 1 && VPL >= 8 && !EARLY) return live ? ld_gathered<EARLY>(ptr, pol) : Vec<VEC>::zero();
+    if (BRANCH) return live ? ld_gathered<EARLY>(ptr, pol) : Vec<VEC>::zero();
     return ld_gathered_if<EARLY>(ptr, pol, live);
 }
 
@@ -306,6 +316,8 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
                                                  const Epilogue &epi) {
     using V = typename Vec<VEC>::type;
     constexpr int UU = MinOf<U, G>::value;
+    constexpr bool BRANCH = VEC == 1 && VPL >= 8 && !EARLY;
+    constexpr int SURE = VPL == 8 || VPL == 12 ? 0 : sure_vectors(G, VPL, VEC);      // those two lost by it here
     const int gl = threadIdx.x & (G - 1);
     int ri = 0, k = 0, kend = 0;
     if (range < n_ranges) {
@@ -355,7 +367,7 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
                 const V *xr = row_address<VEC, HOT>(g, live ? (cc[u] & kColMask) : 0u, gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = ld_row_if<VEC, VPL, EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
+                    x[u][p] = ld_row_if<BRANCH, VEC, EARLY>(xr + p * G, pol_keep, live && (EXACT || p < SURE || gl + p * G < nvec));
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u) {
@@ -414,6 +426,8 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
     using V = typename Vec<VEC>::type;
     constexpr int RPW = 32 / G;
     constexpr int UU = MinOf<U, G>::value;
+    constexpr bool BRANCH = VEC == 1 && VPL == 32 && !EARLY;
+    constexpr int SURE = VPL == 4 && EARLY ? 0 : sure_vectors(G, VPL, VEC);      // F = 95, 10,000 rows of 81: 37 / 39 us with it
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gi = lane / G;
@@ -445,8 +459,8 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = EXACT ? ld_gathered<EARLY>(xr + p * G, pol_keep)
-                                    : ld_row_if<VEC, VPL, EARLY>(xr + p * G, pol_keep, gl + p * G < nvec);
+                    x[u][p] = EXACT || p < SURE ? ld_gathered<EARLY>(xr + p * G, pol_keep)
+                                                : ld_row_if<BRANCH, VEC, EARLY>(xr + p * G, pol_keep, gl + p * G < nvec);
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u)
@@ -477,7 +491,7 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
                 const V *xr = row_address<VEC, HOT>(g, (unsigned)cc[u], gl, nvec);
 #pragma unroll
                 for (int p = 0; p < VPL; ++p)
-                    x[u][p] = ld_row_if<VEC, VPL, EARLY>(xr + p * G, pol_keep, live && (EXACT || gl + p * G < nvec));
+                    x[u][p] = ld_row_if<BRANCH, VEC, EARLY>(xr + p * G, pol_keep, live && (EXACT || p < SURE || gl + p * G < nvec));
             }
 #pragma unroll
             for (int u = 0; u < UU; ++u)

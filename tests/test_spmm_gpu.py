@@ -625,3 +625,35 @@ def test_larger_one_launch_plans(cuda_device, oracle, n, per_row, f):
                                             C.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert rc == 0, db.lib().drone_last_error()
     assert torch.equal(uncopied, y)
+
+
+@pytest.mark.parametrize("n,per_row,f,copied", [(40000, 12, 131, False), (30000, 40, 131, True), (30000, 40, 255, True), (40000, 70, 129, True),
+                                                (41000, 60, 161, False), (41000, 62, 253, True), (40000, 33, 95, False),
+                                                (40000, 33, 63, True), (10000, 20, 383, False), (10000, 20, 401, True),
+                                                (9000, 10, 513, False), (210000, 33, 65, True), (210000, 31, 129, False)])
+def test_both_sides_of_the_copy_rule(cuda_device, n, per_row, f, copied):
+    """Which calls on rows that cannot be read 16 bytes at a time go through the padded copies (whose buffers the first such
+    call makes), and that both routes leave the same bits: the widths at which the shapes of single floats begin and end, whose lanes read some
+    of their floats without a test against the width, among them."""
+    import ctypes as C
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(n + f)
+    h = torch.unique(torch.randint(0, n * n, (n * per_row,), device=cuda_device, generator=gen))
+    u, v = (h // n).to(torch.int32), (h % n).to(torch.int32)
+    index, dst = gg.csr_by_source(u, v, n)
+    in_deg, out_deg = (d.clamp_(min=1) for d in gg.degrees(u, v, n))
+    x = torch.randn((n, f), device=cuda_device, generator=gen)
+    lib, stream = db.lib(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    plan, fresh = (db.AggregationPlan(index, dst, in_degree=in_deg, out_degree=out_deg) for _ in range(2))
+    wide = torch.zeros((n, f + 3 & ~3), device=cuda_device)
+    y, uncopied = torch.empty_like(x), torch.full_like(x, float("nan"))
+    for op in (db.OP_AT, db.OP_A):
+        plan.spmm(op, wide, out=torch.empty_like(wide))                   # makes the partial sums, and needs no copies
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info(cuda_device)[0]
+    for op in (db.OP_AT, db.OP_A):
+        plan.spmm(op, x, out=y)
+        rc = lib.drone_spmm_static_scratch(fresh.handle, op, f, C.c_void_p(x.data_ptr()), f, C.c_void_p(uncopied.data_ptr()), f, stream)
+        assert rc == 0, lib.drone_last_error()
+        assert torch.equal(uncopied, y)
+    assert copied == (torch.cuda.mem_get_info(cuda_device)[0] < free)
