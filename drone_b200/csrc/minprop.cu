@@ -16,6 +16,7 @@
 // index, cc.cu:14, which cannot be compared between workers).  A shorter distance always re-activates its vertex
 // (sssp_exec asks for an improvement above 1e-6, sssp.cu:67; with the unit lengths build_graph stores both agree).
 #include "exchange.cuh"
+#include "grid_sync.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -44,6 +45,7 @@ struct drone_mp {
     int4 *items = nullptr;         // [item_cap] {first edge, edges, value, 0}: pieces of the long rows of a round's frontier
     int item_cap = 0;
     drone::DeviceBlock block;             // what the arrays above are pieces of
+    unsigned barrier_start = 0;    // what the grid barrier's count starts at
     bool started = false;
 };
 
@@ -54,7 +56,6 @@ constexpr int kIdle = -1, kOffered = -2, kOfferedFirst = -3;
 constexpr int kItemEdges = 256;      // longer ones are cut into pieces of this many edges for the whole grid
 constexpr int kRunThreads = 1024;
 constexpr int kRoundsPerLaunch = 4096;
-constexpr unsigned kMpPolls = 1u << 23;      // about five seconds: the grid barrier gives up instead of hanging
 constexpr unsigned kFarBits = 0x4CBEBC20u;   // 1e8f, the reference's "not reached" (sssp.cu:33)
 
 static inline int grid_mp(long long n, int cap = 148 * 16) {
@@ -72,8 +73,7 @@ struct MpRound {
 };
 
 struct MpControl {
-    unsigned arrived;      // blocks that reached a barrier, over all barriers of the launch
-    int failed;            // a wait ran out
+    GridBarrier barrier;
     int unfinished;        // 1: the launch stopped after kRoundsPerLaunch rounds
     int round;             // where the next launch goes on
     unsigned limit;
@@ -85,6 +85,7 @@ enum MpStart { kMpPeval = 0, kMpIncEval = 1, kMpContinue = 2 };
 
 struct MpArgs {
     int n, start, source_global, item_cap;
+    unsigned barrier_start;
     const int *index, *dst, *l2g;
     const float *len;
     unsigned *value;
@@ -92,28 +93,6 @@ struct MpArgs {
     int4 *items;
     MpControl *control;
 };
-
-// Every thread of the grid arrives; false when a wait ran out (in some block), then everybody returns.
-__device__ inline bool mp_barrier(MpControl *c, unsigned &phase) {
-    __shared__ int ok;
-    phase += gridDim.x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&c->arrived, 1u);
-        unsigned seen = 0, polls = 0;
-        int failed = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&c->arrived) : "memory");
-            if (++polls >= kMpPolls) atomicExch(&c->failed, 1);
-            if ((polls & 255u) == 0) failed = *(volatile int *)&c->failed;
-        } while (seen < phase && !failed);
-        __threadfence();
-        ok = failed ? 0 : 1;
-    }
-    __syncthreads();
-    return ok != 0;
-}
 
 // The value an edge offers: a label as it is, a distance plus the edge's length.
 template <int KIND>
@@ -199,7 +178,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
     const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     __shared__ unsigned block_nearest;
     __shared__ int block_waiting;
-    unsigned phase = 0;
+    unsigned phase = a.barrier_start;
     int round = 1;
     unsigned limit = 0;
     if (a.start == kMpContinue) {
@@ -220,7 +199,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
             a.ubm[i] = 0;
             a.state[i] = !front ? kIdle : __ldg(a.index + i + 1) > __ldg(a.index + i) ? 0 : kOfferedFirst;
         }
-        if (!mp_barrier(a.control, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase)) return;
     }
     const int last_round = round + kRoundsPerLaunch;
     const int few = max(1024, a.n / 64);
@@ -339,7 +318,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
             }
         }
         mp_note_round(this_round, least, waiting, &block_nearest, &block_waiting);
-        if (!mp_barrier(a.control, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase)) return;
         const int n_items = min(__ldcg(&this_round->items), a.item_cap);
         if (n_items > 0) {
             // pieces of long rows: a warp each
@@ -369,7 +348,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
                 }
             }
             mp_note_round(this_round, least, 0, &block_nearest, &block_waiting);
-            if (!mp_barrier(a.control, phase)) return;
+            if (!grid_barrier(&a.control->barrier, phase)) return;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {      // used next two rounds from now; its last readers are behind the barrier
             MpRound *later = a.control->rounds + ((round + 2) & 3);
@@ -518,8 +497,11 @@ static int mp_launch(drone_mp *p, int start, int source_global, cudaStream_t st)
     a.counters = p->counters;
     a.items = p->items;
     a.control = &reinterpret_cast<MpReport *>(p->counters)->control;
-    if (start == kMpContinue) DRONE_CUDA(cudaMemsetAsync(&a.control->arrived, 0, sizeof(unsigned), st));
+    a.barrier_start = p->barrier_start;
+    if (start == kMpContinue) DRONE_CUDA(cudaMemsetAsync(&a.control->barrier.arrived, 0, sizeof(unsigned), st));
     else DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(MpReport), st));
+    if (p->barrier_start != 0)
+        DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &p->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
     // a block has at least about 4096 edges and vertices to look at; more blocks only make the barriers longer
     const int grid = std::max(1, (int)std::min<long long>(p->sms, ((long long)p->n_local + p->nnz + 4095) / 4096));
     void *args[] = {&a};
@@ -543,7 +525,7 @@ static int mp_local_runs(std::vector<drone_mp *> &parts, bool peval, int source_
         DRONE_CUDA(cudaStreamSynchronize(st));
         again = false;
         for (size_t i = 0; i < parts.size(); ++i) {
-            if (reports[i].control.failed) return set_error(DRONE_E_STATE, "a wait between the blocks of a local run ran out");
+            if (reports[i].control.barrier.failed) return set_error(DRONE_E_STATE, "a wait between the blocks of a local run ran out");
             if (!reports[i].control.unfinished) continue;
             again = true;
             if ((rc = mp_launch(parts[i], kMpContinue, source_global, st))) return rc;
@@ -667,6 +649,7 @@ int drone_mp_create(drone_mp **out, int kind, int n_local, int nnz, const int *d
     p->l2g = d_local2global;
     p->xplan = xplan;
     p->comm = comm;
+    p->barrier_start = barrier_start();
     cudaError_t err = cudaGetDevice(&p->device);
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
     const size_t nb = std::max<size_t>(std::max(xplan->up_rows.size(), xplan->down_rows.size()), 1);

@@ -18,6 +18,7 @@
 // reference expresses by sending or not sending the vertex.  Either way the counts the
 // caller uses to detect termination (Response, common.h:23-27) are reproduced.
 #include "exchange.cuh"
+#include "grid_sync.cuh"
 #include "plan.cuh"
 
 #include <atomic>
@@ -61,6 +62,7 @@ struct drone_pr {
     size_t control_bytes = 0;
     drone::DeviceBlock block;                // what the arrays made at creation are pieces of
     int sms = 0;
+    unsigned barrier_start = 0;       // what the grid barrier's count starts at
     bool started = false;
     long long n_isolated = 0;         // vertex ids that occur in no part (power iteration treats them as dangling)
 };
@@ -640,11 +642,9 @@ __global__ void pr_set_scalar_kernel(R *scalars, int slot, R value) {
 
 constexpr int kMaxLocalParts = 64;
 constexpr int kHistorySteps = 128;         // supersteps of the job per launch
-constexpr unsigned kBarrierPolls = 1u << 23;   // about five seconds: the barrier gives up instead of hanging
 
 struct RunControl {
-    unsigned arrived;                      // blocks that reached a barrier, over all barriers of the launch
-    int failed;                            // a wait ran out
+    GridBarrier barrier;
     int steps, done;                       // supersteps run; 1 when the last one exchanged nothing
     unsigned long long t_start, t_pull, t_end;   // nanoseconds: start, end of the first pull, end
     int visited[kMaxLocalParts];
@@ -657,6 +657,7 @@ struct RunArgs {
     PartView<R> part[MAXP];
     R *block_sums;
     RunControl *control;
+    unsigned barrier_start;
     int *history;                          // [max_steps][n_parts][4], zero at the start
     // job
     R eps;
@@ -666,28 +667,6 @@ struct RunArgs {
     int iterations;
     long long n_isolated;
 };
-
-// Every thread of the grid arrives; false when a wait ran out (in some block), then everybody returns.
-__device__ inline bool grid_barrier(RunControl *c, unsigned &phase) {
-    __shared__ int ok;
-    phase += gridDim.x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&c->arrived, 1u);
-        unsigned seen = 0, polls = 0;
-        int failed = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&c->arrived) : "memory");
-            if (++polls >= kBarrierPolls) atomicExch(&c->failed, 1);
-            if ((polls & 255u) == 0) failed = *(volatile int *)&c->failed;
-        } while (seen < phase && !failed);
-        __threadfence();
-        ok = failed ? 0 : 1;
-    }
-    __syncthreads();
-    return ok != 0;
-}
 
 __device__ __forceinline__ unsigned long long now_ns() {
     unsigned long long t;
@@ -817,7 +796,7 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
     const int block = (int)blockIdx.x - a.first_block[me], blocks = a.first_block[me + 1] - a.first_block[me];
     const int first = block * blockDim.x + threadIdx.x, stride = blocks * blockDim.x;
     const int warp = (threadIdx.x >> 5) * blocks + block, n_warps = (blockDim.x >> 5) * blocks;
-    unsigned phase = 0;
+    unsigned phase = a.barrier_start;
 
     R gdiff = 0, gacc = 0, iso = 0, dangling = 0;
     if (JOB) {
@@ -841,12 +820,12 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
         }
         const R mine = block_sum<R>(dangling);
         if (threadIdx.x == 0) a.block_sums[blockIdx.x] = mine;
-        if (!grid_barrier(a.control, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase)) return;
         load_table(p, table);
         const R dang = fold_blocks<R>(a.block_sums);      // its barrier also closes the table
         pull_rows<R, JOB, sizeof(R) == 4 || THREADS <= 512 ? 8 : 4, 4>(p, table, warp, n_warps);
         if (JOB) gdiff = dang;
-        if (!grid_barrier(a.control, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase)) return;
         if (JOB && step == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.control->t_pull = now_ns();
         if (JOB && a.n_parts > 1) {
             // a master takes what its mirrors hold, in ascending rank order, and hands the total back (Mirror2MasterSend,
@@ -914,7 +893,7 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
             int *h = a.history + (long long)step * a.n_parts * 4;
             for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x)
                 if (counts[q]) atomicAdd(h + q, counts[q]);
-            if (!grid_barrier(a.control, phase)) return;
+            if (!grid_barrier(&a.control->barrier, phase)) return;
         }
         if (JOB) {
             int sent = 0;      // every block looks at the counts of all parts
@@ -1307,6 +1286,7 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     }
     a.block_sums = (R *)lead->block_sums;
     a.control = (RunControl *)lead->control;
+    a.barrier_start = lead->barrier_start;
     a.history = (int *)(lead->control + sizeof(RunControl));
     a.eps = (R)lead->eps;
     a.peval = rq.peval;
@@ -1316,6 +1296,8 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     a.iterations = rq.iterations;
     a.n_isolated = lead->n_isolated;
     DRONE_CUDA(cudaMemsetAsync(lead->control, 0, sizeof(RunControl) + (JOB ? sizeof(int) * 4 * (size_t)P * rq.max_steps : 0), st));
+    if (lead->barrier_start != 0)
+        DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &lead->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
     auto kernel = threads == 512 ? pr_run_kernel<R, MAXP, JOB, 512> : pr_run_kernel<R, MAXP, JOB, kPullThreads>;
     const int rc = allow_table(kernel);
     if (rc) return rc;
@@ -1357,7 +1339,7 @@ static int read_control(drone_pr *lead, int n_parts, int steps, RunControl *c, i
         DRONE_CUDA(cudaMemcpyAsync(history, lead->control + sizeof(RunControl), sizeof(int) * 4 * (size_t)n_parts * steps,
                                    cudaMemcpyDeviceToHost, st));
     DRONE_CUDA(cudaStreamSynchronize(st));
-    if (c->failed) return set_error(DRONE_E_STATE, "PageRank: a wait between the blocks of a superstep ran out");
+    if (c->barrier.failed) return set_error(DRONE_E_STATE, "PageRank: a wait between the blocks of a superstep ran out");
     return DRONE_OK;
 }
 
@@ -1432,6 +1414,7 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
     p->eps = eps;
     p->xplan = xplan;
     p->comm = comm;
+    p->barrier_start = barrier_start();
     cudaGetDevice(&p->device);
     const size_t rs = p->dbl ? 8 : 4;
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);

@@ -200,3 +200,18 @@ def test_run_at_its_edges(cuda_device, oracle, shape, kind):
         # all but the vertices that started in the frontier and were never lowered
         still = int((want == np.arange(n)).sum()) if kind == "labels" else 1
         assert res.VisitedSize == n - still and res.is_empty()
+
+
+@pytest.mark.parametrize("kind", [mp.CC, mp.SSSP])
+def test_barrier_count_passes_its_end(cuda_device, monkeypatch, kind):
+    """The count of arrivals at the barriers of a launch is modulo 2^32: started just below that it changes nothing."""
+    n, u, v = graph_case(14, 8, 37, True)
+    part = pt.ebv_partition(n, u, v, 1, keep_self_loops=False)
+    graphs, _ = build(part, cuda_device)
+    results = []
+    for start in ("0", str(2 ** 32 - 20)):
+        monkeypatch.setenv("DRONE_BARRIER_START", start)
+        job = mp.MinProp(graphs[0], kind)
+        res = job.peval(int(u[0]))
+        results.append((res.VisitedSize, job.values()))
+    assert results[0][0] == results[1][0] and np.array_equal(results[0][1], results[1][1])

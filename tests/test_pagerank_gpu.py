@@ -226,3 +226,19 @@ def test_supersteps_in_one_launch(cuda_device, oracle, scale, parts, use_double)
     want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
     touched = part.replicas > 0
     assert np.max(np.abs(got[touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
+
+
+def test_barrier_count_passes_its_end(cuda_device, monkeypatch):
+    """The count of arrivals at the barriers of a launch is modulo 2^32: started just below that it changes nothing."""
+    n, u, v, out_deg, part = pr_case(scale=13, seed=70, parts=2)
+    results = []
+    for start in ("0", str(2 ** 32 - 100)):
+        monkeypatch.setenv("DRONE_BARRIER_START", start)
+        graphs, prs = build_parts(part, n, u, v, cuda_device, True, 1e-6)
+        steps, sizes = prk.run_job_local(prs)
+        delta = prk.gather_global(prs, graphs, n)
+        prk.power_iterate_local(prs, 20, 0.85)
+        results.append((steps, sizes, delta, prk.gather_global(prs, graphs, n)))
+    assert results[0][:2] == results[1][:2] and results[0][0] > 3
+    assert np.array_equal(results[0][2], results[1][2]) and np.array_equal(results[0][3], results[1][3])
+    assert np.ptp(results[1][3]) > 0                    # not the start values
