@@ -13,7 +13,13 @@ struct GridBarrier {
     int failed;            // a wait ran out
 };
 
-constexpr unsigned kBarrierPolls = 1u << 23;   // about five seconds
+// How often a block looks at the count before it gives up: kBarrierPolls (about five seconds), or DRONE_BARRIER_POLLS, read when
+// a handle is made (0: every block gives up at its first barrier, which is how the failure is tested).
+constexpr unsigned kBarrierPolls = 1u << 23;
+inline unsigned barrier_polls() {
+    const char *v = getenv("DRONE_BARRIER_POLLS");
+    return v && *v ? (unsigned)strtoul(v, nullptr, 10) : kBarrierPolls;
+}
 
 // What `arrived` starts at: 0, or DRONE_BARRIER_START, read when a handle is made (a start just below 2^32 takes a short run
 // over the end of the count, which otherwise 14 million iterations on a full grid reach).
@@ -25,20 +31,25 @@ inline unsigned barrier_start() {
 // Every thread of the grid arrives; false when a wait ran out (in some block), then everybody returns.  `phase`: what
 // `arrived` has to reach, at first its start.  The count only grows, so that a barrier is one atomic and one comparison
 // modulo 2^32 (the blocks of a grid are far closer together than 2^31); a count of 64 bits took 0.2 us more per barrier.
-__device__ inline bool grid_barrier(GridBarrier *b, unsigned &phase) {
+__device__ inline bool grid_barrier(GridBarrier *b, unsigned &phase, unsigned poll_limit) {
     __shared__ int ok;
     phase += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(&b->arrived, 1u);
-        unsigned seen = 0, polls = 0;
         int failed = 0;
-        do {
+        for (unsigned polls = 0;; ) {
+            unsigned seen;
+            if (polls >= poll_limit) {
+                atomicExch(&b->failed, 1);
+                failed = 1;
+                break;
+            }
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&b->arrived) : "memory");
-            if (++polls >= kBarrierPolls) atomicExch(&b->failed, 1);
-            if ((polls & 255u) == 0) failed = *(volatile int *)&b->failed;
-        } while ((int)(seen - phase) < 0 && !failed);
+            if ((int)(seen - phase) >= 0) break;
+            if ((++polls & 255u) == 0 && (failed = *(volatile int *)&b->failed) != 0) break;
+        }
         __threadfence();
         ok = failed ? 0 : 1;
     }

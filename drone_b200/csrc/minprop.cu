@@ -45,7 +45,7 @@ struct drone_mp {
     int4 *items = nullptr;         // [item_cap] {first edge, edges, value, 0}: pieces of the long rows of a round's frontier
     int item_cap = 0;
     drone::DeviceBlock block;             // what the arrays above are pieces of
-    unsigned barrier_start = 0;    // what the grid barrier's count starts at
+    unsigned barrier_start = 0, barrier_polls = 0;   // what the grid barrier's count starts at, and when its waits run out
     bool started = false;
 };
 
@@ -85,7 +85,7 @@ enum MpStart { kMpPeval = 0, kMpIncEval = 1, kMpContinue = 2 };
 
 struct MpArgs {
     int n, start, source_global, item_cap;
-    unsigned barrier_start;
+    unsigned barrier_start, barrier_polls;
     const int *index, *dst, *l2g;
     const float *len;
     unsigned *value;
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
             a.ubm[i] = 0;
             a.state[i] = !front ? kIdle : __ldg(a.index + i + 1) > __ldg(a.index + i) ? 0 : kOfferedFirst;
         }
-        if (!grid_barrier(&a.control->barrier, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) return;
     }
     const int last_round = round + kRoundsPerLaunch;
     const int few = max(1024, a.n / 64);
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
             }
         }
         mp_note_round(this_round, least, waiting, &block_nearest, &block_waiting);
-        if (!grid_barrier(&a.control->barrier, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) return;
         const int n_items = min(__ldcg(&this_round->items), a.item_cap);
         if (n_items > 0) {
             // pieces of long rows: a warp each
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) mp_run_kernel(const MpArgs a) 
                 }
             }
             mp_note_round(this_round, least, 0, &block_nearest, &block_waiting);
-            if (!grid_barrier(&a.control->barrier, phase)) return;
+            if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) return;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {      // used next two rounds from now; its last readers are behind the barrier
             MpRound *later = a.control->rounds + ((round + 2) & 3);
@@ -498,6 +498,7 @@ static int mp_launch(drone_mp *p, int start, int source_global, cudaStream_t st)
     a.items = p->items;
     a.control = &reinterpret_cast<MpReport *>(p->counters)->control;
     a.barrier_start = p->barrier_start;
+    a.barrier_polls = p->barrier_polls;
     if (start == kMpContinue) DRONE_CUDA(cudaMemsetAsync(&a.control->barrier.arrived, 0, sizeof(unsigned), st));
     else DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(MpReport), st));
     if (p->barrier_start != 0)
@@ -525,7 +526,10 @@ static int mp_local_runs(std::vector<drone_mp *> &parts, bool peval, int source_
         DRONE_CUDA(cudaStreamSynchronize(st));
         again = false;
         for (size_t i = 0; i < parts.size(); ++i) {
-            if (reports[i].control.barrier.failed) return set_error(DRONE_E_STATE, "a wait between the blocks of a local run ran out");
+            if (reports[i].control.barrier.failed) {
+                for (drone_mp *p : parts) p->started = false;
+                return set_error(DRONE_E_STATE, "a wait between the blocks of a local run ran out");
+            }
             if (!reports[i].control.unfinished) continue;
             again = true;
             if ((rc = mp_launch(parts[i], kMpContinue, source_global, st))) return rc;
@@ -650,6 +654,7 @@ int drone_mp_create(drone_mp **out, int kind, int n_local, int nnz, const int *d
     p->xplan = xplan;
     p->comm = comm;
     p->barrier_start = barrier_start();
+    p->barrier_polls = barrier_polls();
     cudaError_t err = cudaGetDevice(&p->device);
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
     const size_t nb = std::max<size_t>(std::max(xplan->up_rows.size(), xplan->down_rows.size()), 1);

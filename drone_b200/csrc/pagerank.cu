@@ -62,7 +62,9 @@ struct drone_pr {
     size_t control_bytes = 0;
     drone::DeviceBlock block;                // what the arrays made at creation are pieces of
     int sms = 0;
-    unsigned barrier_start = 0;       // what the grid barrier's count starts at
+    unsigned barrier_start = 0, barrier_polls = 0;   // what the grid barrier's count starts at, and when its waits run out
+    unsigned run = 0;                 // number (in the process) of the launch that made the values; 0: the separate kernels did
+    unsigned *unfinished = nullptr;   // device: number of the last launch that gave up
     bool started = false;
     long long n_isolated = 0;         // vertex ids that occur in no part (power iteration treats them as dangling)
 };
@@ -102,6 +104,7 @@ struct PartView {
     const int *out_degree, *mirror2worker, *place;
     const int *m_rows, *m_off;
     const int2 *pairs, *targets;
+    unsigned *unfinished;
     const unsigned char *shared;           // power iteration over several parts: 1 where the vertex is on others too
 };
 
@@ -657,7 +660,7 @@ struct RunArgs {
     PartView<R> part[MAXP];
     R *block_sums;
     RunControl *control;
-    unsigned barrier_start;
+    unsigned barrier_start, barrier_polls, run;
     int *history;                          // [max_steps][n_parts][4], zero at the start
     // job
     R eps;
@@ -769,6 +772,15 @@ __device__ __noinline__ R power_shared_vertices(const PartView<R> &p, const Part
     return dangling;
 }
 
+// A block whose wait at a barrier ran out: the run is marked as unfinished in every part, since any of them may lack what this
+// block would have stored, and the block's share of the values becomes NaN, so that nobody takes the start values, or those
+// of some superstep, for a result.
+template <typename R, int MAXP>
+__device__ __noinline__ void give_up(const RunArgs<R, MAXP> &a, R *pr, int n, int first, int stride) {
+    for (int q = threadIdx.x; q < a.n_parts; q += blockDim.x) *a.part[q].unfinished = a.run;
+    for (int i = first; i < n; i += stride) pr[i] = (R)NAN;
+}
+
 template <typename R, int MAXP, bool JOB, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constant__ RunArgs<R, MAXP> a) {
     extern __shared__ __align__(16) char table_bytes[];
@@ -820,12 +832,12 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
         }
         const R mine = block_sum<R>(dangling);
         if (threadIdx.x == 0) a.block_sums[blockIdx.x] = mine;
-        if (!grid_barrier(&a.control->barrier, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) return give_up(a, p.pr, p.n, first, stride);
         load_table(p, table);
         const R dang = fold_blocks<R>(a.block_sums);      // its barrier also closes the table
         pull_rows<R, JOB, sizeof(R) == 4 || THREADS <= 512 ? 8 : 4, 4>(p, table, warp, n_warps);
         if (JOB) gdiff = dang;
-        if (!grid_barrier(&a.control->barrier, phase)) return;
+        if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) return give_up(a, p.pr, p.n, first, stride);
         if (JOB && step == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.control->t_pull = now_ns();
         if (JOB && a.n_parts > 1) {
             // a master takes what its mirrors hold, in ascending rank order, and hands the total back (Mirror2MasterSend,
@@ -893,7 +905,7 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
             int *h = a.history + (long long)step * a.n_parts * 4;
             for (int q = threadIdx.x; q < a.n_parts * 4; q += blockDim.x)
                 if (counts[q]) atomicAdd(h + q, counts[q]);
-            if (!grid_barrier(&a.control->barrier, phase)) return;
+            if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) return give_up(a, p.pr, p.n, first, stride);
         }
         if (JOB) {
             int sent = 0;      // every block looks at the counts of all parts
@@ -1010,6 +1022,7 @@ static PartView<R> part_view(const drone_pr *p, int blocks) {
     v.n_masters = (int)x->m_rows.size();
     v.pairs = p->pairs;
     v.targets = p->targets;
+    v.unfinished = p->unfinished;
     v.shared = nullptr;
     const long long capacity = kTableBytes / (long long)sizeof(R);
     long long t = std::min<long long>(capacity, p->n_local);
@@ -1119,6 +1132,7 @@ static int delta_step(drone_pr *p, bool peval, NcclTransport &tr, drone_pr_respo
     const auto t0 = clock::now();
     int rc;
     DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 8, st));
+    p->run = 0;
     const PartView<R> v = part_view<R>(p, p->sms);
     const int grid = grid1d(p->n_local, kReduceBlocks);
     if (peval) {
@@ -1162,6 +1176,7 @@ template <typename R>
 static int power_iterations(drone_pr *p, int iterations, double damping, NcclTransport &tr, cudaStream_t st) {
     int rc;
     const PartView<R> v = part_view<R>(p, p->sms);
+    p->run = 0;
     const int grid = grid1d(p->n_local, kReduceBlocks);
     const R start = (R)1 / (R)p->global_v;
     DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
@@ -1286,7 +1301,11 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     }
     a.block_sums = (R *)lead->block_sums;
     a.control = (RunControl *)lead->control;
+    static std::atomic<unsigned> runs{0};
+    do a.run = ++runs;
+    while (a.run == 0);
     a.barrier_start = lead->barrier_start;
+    a.barrier_polls = lead->barrier_polls;
     a.history = (int *)(lead->control + sizeof(RunControl));
     a.eps = (R)lead->eps;
     a.peval = rq.peval;
@@ -1304,7 +1323,10 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     void *args[] = {&a};
     DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(threads), args, table, st));
     count_launch();
-    for (drone_pr *p : parts) p->started = JOB;
+    for (drone_pr *p : parts) {
+        p->started = JOB;
+        p->run = a.run;
+    }
     return DRONE_OK;
 }
 
@@ -1333,14 +1355,16 @@ static int run_local(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaS
 }
 
 // What the persistent launch left: its control block and the counts of `steps` supersteps.
-static int read_control(drone_pr *lead, int n_parts, int steps, RunControl *c, int *history, cudaStream_t st) {
+static int read_control(std::vector<drone_pr *> &parts, int steps, RunControl *c, int *history, cudaStream_t st) {
+    const drone_pr *lead = parts[0];
     DRONE_CUDA(cudaMemcpyAsync(c, lead->control, sizeof(RunControl), cudaMemcpyDeviceToHost, st));
     if (history)
-        DRONE_CUDA(cudaMemcpyAsync(history, lead->control + sizeof(RunControl), sizeof(int) * 4 * (size_t)n_parts * steps,
+        DRONE_CUDA(cudaMemcpyAsync(history, lead->control + sizeof(RunControl), sizeof(int) * 4 * parts.size() * steps,
                                    cudaMemcpyDeviceToHost, st));
     DRONE_CUDA(cudaStreamSynchronize(st));
-    if (c->barrier.failed) return set_error(DRONE_E_STATE, "PageRank: a wait between the blocks of a superstep ran out");
-    return DRONE_OK;
+    if (!c->barrier.failed) return DRONE_OK;
+    for (drone_pr *p : parts) p->started = false;
+    return set_error(DRONE_E_STATE, "PageRank: a wait between the blocks of a superstep ran out");
 }
 
 // One superstep of all given parts.
@@ -1356,7 +1380,7 @@ static int step_parts(std::vector<drone_pr *> &parts, bool peval, drone_pr_respo
     if (rc) return rc;
     RunControl c;
     std::vector<int> h(4 * parts.size());
-    if ((rc = read_control(parts[0], (int)parts.size(), 1, &c, h.data(), st))) return rc;
+    if ((rc = read_control(parts, 1, &c, h.data(), st))) return rc;
     for (size_t i = 0; i < parts.size(); ++i) {
         drone_pr_response &r = res[i];
         r.Mirror2MasterSendSize = h[4 * i + 0];
@@ -1415,6 +1439,7 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
     p->xplan = xplan;
     p->comm = comm;
     p->barrier_start = barrier_start();
+    p->barrier_polls = barrier_polls();
     cudaGetDevice(&p->device);
     const size_t rs = p->dbl ? 8 : 4;
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
@@ -1452,10 +1477,12 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         p->block.add(&p->send, 2 * rs * nb);
         p->block.add(&p->recv, 2 * rs * nb);
         p->block.add(&p->counters, sizeof(int) * 8);
+        p->block.add(&p->unfinished, sizeof(unsigned));
         if (e == cudaSuccess) e = p->block.make();
         p->control_bytes = sizeof(RunControl) + sizeof(int) * 4 * (size_t)xplan->nranks * kHistorySteps;
         if (e == cudaSuccess) e = cudaMalloc(&p->control, p->control_bytes);
         if (e == cudaSuccess) e = cudaMemset(p->control, 0, p->control_bytes);
+        if (e == cudaSuccess) e = cudaMemset(p->unfinished, 0, sizeof(unsigned));
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
         if (e == cudaSuccess && side.n_split_rows > 0) {
             e = cudaMemset(p->arrived, 0, sizeof(int) * (size_t)side.n_split_rows);
@@ -1557,7 +1584,7 @@ int drone_pr_job_local(int n_parts, drone_pr **prs, int max_steps, int *n_steps,
         rq.peval = total == 0;
         rq.max_steps = std::min(kHistorySteps, max_steps - total);
         if ((rc = run_local(parts, rq, (cudaStream_t)stream))) return rc;
-        if ((rc = read_control(parts[0], n_parts, rq.max_steps, &c, h.data(), (cudaStream_t)stream))) return rc;
+        if ((rc = read_control(parts, rq.max_steps, &c, h.data(), (cudaStream_t)stream))) return rc;
         if (sizes) memcpy(sizes + (size_t)total * n_parts * 4, h.data(), sizeof(int) * 4 * (size_t)n_parts * c.steps);
     }
     *n_steps = total;
@@ -1620,9 +1647,13 @@ int drone_pr_device_arrays(drone_pr *p, void **d_pr, void **d_acc, void **d_diff
 int drone_pr_values(drone_pr *p, void *h_out, void *stream) {
     DRONE_REQUIRE(p && (h_out || p->n_local == 0), "drone_pr_values: NULL argument");
     if (p->n_local == 0) return DRONE_OK;
+    unsigned unfinished = 0;
     DRONE_CUDA(cudaMemcpyAsync(h_out, p->pr, (p->dbl ? 8 : 4) * (size_t)p->n_local, cudaMemcpyDeviceToHost,
                                (cudaStream_t)stream));
+    DRONE_CUDA(cudaMemcpyAsync(&unfinished, p->unfinished, sizeof(unsigned), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     DRONE_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    if (p->run != 0 && unfinished == p->run)
+        return set_error(DRONE_E_STATE, "drone_pr_values: a wait between the blocks of the run that should have made the values ran out");
     return DRONE_OK;
 }
 

@@ -452,7 +452,8 @@ int drone_pr_inceval(drone_pr *pr, drone_pr_response *res, void *stream);
 
 /* Synchronous power iteration: pr = 1/|V|, then `iterations` times
  * pr' = (1-d)/|V| + d * (sum over in-edges of pr[u]/outDegree[u] + dangling/|V|),
- * with the same boundary exchange.  Collective; asynchronous on `stream`. */
+ * with the same boundary exchange.  Collective; asynchronous on `stream`.  The waits between the iterations' blocks are
+ * bounded (about five seconds): a run that one of them ended leaves NaN, and drone_pr_values returns DRONE_E_STATE. */
 int drone_pr_power_iterate(drone_pr *pr, int iterations, double damping, void *stream);
 
 /* Number of vertex ids in 0..|V|-1 that occur in no part (no edge at all).  The power iteration counts
@@ -475,7 +476,8 @@ int drone_pr_power_iterate_local(int n_parts, drone_pr **prs, int iterations, do
 int drone_pr_device_arrays(drone_pr *pr, void **d_pr, void **d_acc, void **d_diff, int **d_active,
                            int **d_update_by_message);
 
-/* Current values by local id into h_out (n_local floats or doubles); synchronises. */
+/* Current values by local id into h_out (n_local floats or doubles); synchronises.  DRONE_E_STATE when the run that should
+ * have made them did not finish. */
 int drone_pr_values(drone_pr *pr, void *h_out, void *stream);
 
 /* ------------------------------------------------------------------------- */

@@ -215,3 +215,20 @@ def test_barrier_count_passes_its_end(cuda_device, monkeypatch, kind):
         res = job.peval(int(u[0]))
         results.append((res.VisitedSize, job.values()))
     assert results[0][0] == results[1][0] and np.array_equal(results[0][1], results[1][1])
+
+
+def test_a_wait_that_runs_out_is_reported(cuda_device, monkeypatch):
+    """The barrier between the rounds of a local run gives up after a bounded number of looks (here: none), and the call that
+    waited for the run says so; IncEval is refused until a PEval has finished."""
+    n, u, v = graph_case(14, 8, 38, False)
+    part = pt.ebv_partition(n, u, v, 2, keep_self_loops=False)
+    graphs, _ = build(part, cuda_device)
+    monkeypatch.setenv("DRONE_BARRIER_POLLS", "0")
+    jobs = [mp.MinProp(g, mp.CC) for g in graphs]
+    with pytest.raises(db.DroneError, match="ran out"):
+        mp.step_local(jobs, True)
+    with pytest.raises(db.DroneError, match="before PEVal"):
+        mp.step_local(jobs, False)
+    monkeypatch.delenv("DRONE_BARRIER_POLLS")
+    jobs = [mp.MinProp(g, mp.CC) for g in graphs]
+    assert all(r.LocalVertexSize == g.n_local for r, g in zip(mp.step_local(jobs, True), graphs))

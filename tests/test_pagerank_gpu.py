@@ -242,3 +242,33 @@ def test_barrier_count_passes_its_end(cuda_device, monkeypatch):
     assert results[0][:2] == results[1][:2] and results[0][0] > 3
     assert np.array_equal(results[0][2], results[1][2]) and np.array_equal(results[0][3], results[1][3])
     assert np.ptp(results[1][3]) > 0                    # not the start values
+
+
+@pytest.mark.parametrize("parts,use_double", [(1, False), (3, True), (12, False)])
+def test_a_wait_that_runs_out_is_reported(cuda_device, oracle, monkeypatch, parts, use_double):
+    """A barrier between the blocks of a run gives up after a bounded number of looks (here: none).  The synchronous calls
+    report that themselves, the asynchronous power iteration through drone_pr_values of every part; a run that should have
+    finished leaves no plausible values; the handle and the device stay usable."""
+    n, u, v, out_deg, part = pr_case(scale=13, seed=71, parts=parts)
+    monkeypatch.setenv("DRONE_BARRIER_POLLS", "0")
+    graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+    prk.power_iterate_local(prs, 20, 0.85)
+    for pr_ in prs:
+        with pytest.raises(db.DroneError, match="ran out"):
+            pr_.values()
+    out = np.zeros(prs[0].n_local, np.float64 if use_double else np.float32)
+    assert db.lib().drone_pr_values(prs[0].handle, out.ctypes.data, None) == -4 and np.isnan(out).all()
+    with pytest.raises(db.DroneError, match="ran out"):
+        prk.step_local(prs, True)
+    with pytest.raises(db.DroneError, match="before PR_PEVal"):
+        prk.step_local(prs, False)
+    with pytest.raises(db.DroneError, match="ran out"):
+        prk.run_job_local(prs)
+    monkeypatch.delenv("DRONE_BARRIER_POLLS")
+    graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+    prk.power_iterate_local(prs, 20, 0.85)
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
+    got = prk.gather_global(prs, graphs, n)
+    touched = part.replicas > 0
+    assert np.max(np.abs(got[touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
