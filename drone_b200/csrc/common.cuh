@@ -34,11 +34,14 @@ struct DeviceBlock {
         pieces.push_back({(void **)array, total});
         total += (bytes + 255) / 256 * 256;
     }
+    size_t size() const { return total; }
     cudaError_t make() {
         const cudaError_t e = cudaMalloc(&base, total > 0 ? total : 256);
-        if (e == cudaSuccess)
-            for (const Piece &p : pieces) *p.array = (char *)base + p.offset;
+        if (e == cudaSuccess) place(base);
         return e;
+    }
+    void place(void *at) const {
+        for (const Piece &p : pieces) *p.array = (char *)at + p.offset;
     }
     void release() {
         cudaFree(base);

@@ -68,10 +68,9 @@ __global__ void histogram_kernel(const int *__restrict__ keys, int n, int *__res
         atomicAdd(counts + keys[k], 1);
 }
 
-// colT[i] = src[perm[i]], valT[i] = val[perm[i]]
-__global__ void gather_transposed_kernel(const int *__restrict__ perm, const int *__restrict__ src,
-                                         const float *__restrict__ val, int nnz,
-                                         int *__restrict__ col_t, float *__restrict__ val_t) {
+// colT[i] = src[perm[i]], valT[i] = val[perm[i]]; perm may lie in valT's memory (entry i is read before it is written)
+__global__ void gather_transposed_kernel(const int *perm, const int *__restrict__ src, const float *__restrict__ val, int nnz,
+                                         int *__restrict__ col_t, float *val_t) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nnz;
          i += (long long)gridDim.x * blockDim.x) {
         const int p = perm[i];
@@ -332,6 +331,57 @@ static int env_int(const char *name, int dflt) {
     return v > 0 ? v : dflt;
 }
 
+// Scratch of making a plan, one allocation for all of its steps: cudaMalloc of a few hundred kilobytes takes 3 us where the
+// driver has room in a mapping, and 300 us, and as much again to free, where it has to map some.  Kept to the end, it also holds
+// the mapping that the lists then find room in (ms to make a plan, an allocation per step / one for all; R-MAT-12 sym 2.65 / 2.2,
+// with other plans alive 1.8 / 1.1 to 1.5; R-MAT-14 3.25 / 2.65, -16 5.7 / 4.45, -18 7.9 / 5.4, -20 10.8 / 7.8).  Steps take
+// their pieces from it like from a stack; what does not fit gets an allocation of its own.
+struct PlanScratch {
+    // Scratch above this is given back before the next step allocates what stays with the plan.
+    static constexpr size_t kKept = 256u << 20;
+    char *base = nullptr;
+    size_t bytes = 0, used = 0;
+    ~PlanScratch() { cudaFree(base); }
+    int make(size_t n) {
+        DRONE_CUDA(cudaMalloc(&base, n));
+        bytes = n;
+        return DRONE_OK;
+    }
+    void give_back() {
+        cudaFree(base);
+        base = nullptr;
+        bytes = 0;
+    }
+};
+struct StepScratch {
+    explicit StepScratch(PlanScratch &p) : plan(p) {}
+    ~StepScratch() {
+        if (block.base) block.release();
+        else plan.used -= taken;
+    }
+    int make() {
+        if (plan.used + block.size() <= plan.bytes) {
+            block.place(plan.base + plan.used);
+            taken = block.size();
+            plan.used += taken;
+            return DRONE_OK;
+        }
+        DRONE_CUDA(block.make());
+        return DRONE_OK;
+    }
+    template <typename T> void add(T **array, size_t n) { block.add(array, n); }
+    PlanScratch &plan;
+    DeviceBlock block;
+    size_t taken = 0;
+};
+
+// Counts x4, offsets x4 and scratch x2 of build_work_lists, and the scan's own.
+static int list_scratch_bytes(int n, size_t *arrays, size_t *scan, cudaStream_t st) {
+    *arrays = sizeof(int) * (size_t)(n + 1) * 10;
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, *scan, (int *)nullptr, (int *)nullptr, n + 1, st));
+    return DRONE_OK;
+}
+
 static void free_side(Side &s) {
     cudaFree(s.hot_ids);
     cudaFree(s.col_plain);
@@ -344,8 +394,11 @@ static void free_side(Side &s) {
     s = Side();
 }
 
-// Build side[DRONE_OP_AT] from side[DRONE_OP_A] (arrays of A must be on the device).
-static int build_transpose(drone_plan *p, cudaStream_t st) {
+// Build side[DRONE_OP_AT] from side[DRONE_OP_A], whose rows and columns must be on the device; fill_values() puts its values
+// there.  Of the sort's four arrays only one is scratch: the keys lie in what becomes the columns, and until it is filled in
+// A's value array, and half of the edge ids lie in what becomes the values.
+template <typename Fill>
+static int build_transpose(drone_plan *p, PlanScratch &plan_scratch, cudaStream_t st, Fill fill_values) {
     const Side &a = p->side[DRONE_OP_A];
     Side &t = p->side[DRONE_OP_AT];
     const int n = p->n_rows, nnz = p->nnz;
@@ -355,25 +408,23 @@ static int build_transpose(drone_plan *p, cudaStream_t st) {
 
     int end_bit = 1;
     while (end_bit < 31 && (1LL << end_bit) < (long long)n) ++end_bit;
-    // scratch, one allocation; the sort's keys lie in what becomes the column array
-    struct Temp {
-        DeviceBlock block;
-        ~Temp() { block.release(); }
-    } scratch;
-    int *counts = nullptr, *src = nullptr, *keys_alt = nullptr, *perm = nullptr, *perm_alt = nullptr;
+    StepScratch scratch(plan_scratch);
+    int *counts = nullptr, *src = nullptr, *perm = nullptr;
     void *tmp = nullptr;
     const size_t words = sizeof(int) * (size_t)nnz;
-    scratch.block.add(&counts, sizeof(int) * (size_t)(n + 1));
-    scratch.block.add(&src, words);
-    scratch.block.add(&keys_alt, words);
-    scratch.block.add(&perm, words);
-    scratch.block.add(&perm_alt, words);
+    scratch.add(&counts, sizeof(int) * (size_t)(n + 1));
+    scratch.add(&src, words);
+    scratch.add(&perm, words);
     cub::DoubleBuffer<int> keys(t.col, nullptr), edges(nullptr, nullptr);
     size_t scan_bytes = 0, sort_bytes = 0;
     DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, counts, t.rowptr, n + 1, st));
     if (nnz > 0) DRONE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, edges, nnz, 0, end_bit, st));
-    scratch.block.add(&tmp, std::max(scan_bytes, sort_bytes));
-    DRONE_CUDA(scratch.block.make());
+    scratch.add(&tmp, std::max(scan_bytes, sort_bytes));
+    size_t list_arrays = 0, list_scan = 0;
+    int rc;
+    if ((rc = list_scratch_bytes(n, &list_arrays, &list_scan, st))) return rc;
+    if ((rc = plan_scratch.make(std::max(scratch.block.size(), list_arrays + list_scan + 512)))) return rc;
+    if ((rc = scratch.make())) return rc;
 
     // row pointer of the transpose: histogram of destinations, then exclusive scan
     DRONE_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)(n + 1), st));
@@ -390,10 +441,11 @@ static int build_transpose(drone_plan *p, cudaStream_t st) {
         iota_kernel<<<grid_for(nnz), 256, 0, st>>>(perm, nnz);
         DRONE_LAUNCH_CHECK("iota_kernel");
         DRONE_CUDA(cudaMemcpyAsync(t.col, a.col, words, cudaMemcpyDeviceToDevice, st));
-        keys = cub::DoubleBuffer<int>(t.col, keys_alt);
-        edges = cub::DoubleBuffer<int>(perm, perm_alt);
+        keys = cub::DoubleBuffer<int>(t.col, reinterpret_cast<int *>(a.val));
+        edges = cub::DoubleBuffer<int>(perm, reinterpret_cast<int *>(t.val));
         DRONE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, keys, edges, nnz, 0, end_bit, st));
         count_launch();
+        if ((rc = fill_values())) return rc;
         gather_transposed_kernel<<<grid_for(nnz), 256, 0, st>>>(edges.Current(), src, a.val, nnz, t.col, t.val);
         DRONE_LAUNCH_CHECK("gather_transposed_kernel");
     }
@@ -469,30 +521,25 @@ static int cut_ranges(const Side &s, const Ranges &out, int range_nnz, int K, co
 }
 
 // Work lists of one orientation: chunks and split rows of the long rows, the flagged stream of the short rows.
-static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
+static int build_work_lists(drone_plan *p, Side &s, PlanScratch &plan_scratch, cudaStream_t st) {
     const int n = p->n_rows;
     const int K = p->n_classes;
-    struct Temp {        // freed on every way out
-        int *buf = nullptr;
-        void *scan = nullptr;
-        DeviceBlock block;
-        ~Temp() { block.release(); }
-    } t;
+    StepScratch t(plan_scratch);
     const size_t stride = (size_t)(n + 1);
-    size_t tmp_bytes = 0;
-    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, t.buf, t.buf, n + 1, st));
-    t.block.add(&t.buf, sizeof(int) * stride * 10);  // 10 arrays of n+1 ints: counts x4, offsets x4, scratch x2
-    t.block.add(&t.scan, tmp_bytes);
-    DRONE_CUDA(t.block.make());
-    int *buf = t.buf;
+    size_t array_bytes = 0, tmp_bytes = 0;
+    int *buf = nullptr;
+    void *tmp = nullptr;
+    int rc;
+    if ((rc = list_scratch_bytes(n, &array_bytes, &tmp_bytes, st))) return rc;
+    t.add(&buf, array_bytes);
+    t.add(&tmp, tmp_bytes);
+    if ((rc = t.make())) return rc;
     int *cnt[4] = {buf, buf + stride, buf + 2 * stride, buf + 3 * stride};
     int *off[4] = {buf + 4 * stride, buf + 5 * stride, buf + 6 * stride, buf + 7 * stride};
     int *scratch = buf + 8 * stride;
     count_chunks_kernel<<<grid_for(n + 1), 256, 0, st>>>(s.rowptr, n, p->short_row_limit, p->chunk_nnz,
                                                         cnt[0], cnt[1], cnt[2], cnt[3]);
     DRONE_LAUNCH_CHECK("count_chunks_kernel");
-    void *tmp = t.scan;
-    int rc;
     int slot_start[kMaxRowClasses + 1], long_start[kMaxRowClasses + 1];
     if ((rc = class_major_scan(p, cnt[0], off[0], scratch, tmp, tmp_bytes, s.chunk_start, st))) return rc;
     if ((rc = class_major_scan(p, cnt[1], off[1], scratch, tmp, tmp_bytes, slot_start, st))) return rc;
@@ -559,30 +606,27 @@ static int build_work_lists(drone_plan *p, Side &s, cudaStream_t st) {
         const char *order = getenv("DRONE_CHUNK_ORDER");
         const bool by_column = order && order[0] == 'c' ? true : order && order[0] == 'r' ? false : s.hot_ids == nullptr;
         if (by_column && K == 1 && s.n_chunks > 1) {
-            struct Sort {
-                int *key = nullptr, *idx = nullptr, *key2 = nullptr, *idx2 = nullptr;
-                Chunk *sorted = nullptr;
-                void *tmp = nullptr;
-                DeviceBlock block;
-                ~Sort() { block.release(); }
-            } o;
+            StepScratch sort(plan_scratch);
+            int *key = nullptr, *idx = nullptr, *key2 = nullptr, *idx2 = nullptr;
+            Chunk *sorted = nullptr;
+            void *sort_tmp = nullptr;
             const size_t nb = sizeof(int) * (size_t)s.n_chunks;
             size_t sort_bytes = 0;
-            DRONE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, o.key, o.key2, o.idx, o.idx2, s.n_chunks, 0, 30, st));
-            o.block.add(&o.key, nb);
-            o.block.add(&o.idx, nb);
-            o.block.add(&o.key2, nb);
-            o.block.add(&o.idx2, nb);
-            o.block.add(&o.sorted, sizeof(Chunk) * (size_t)s.n_chunks);
-            o.block.add(&o.tmp, sort_bytes);
-            DRONE_CUDA(o.block.make());
-            chunk_first_column_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, s.n_chunks, s.col, o.key, o.idx);
+            DRONE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, key, key2, idx, idx2, s.n_chunks, 0, 30, st));
+            sort.add(&key, nb);
+            sort.add(&idx, nb);
+            sort.add(&key2, nb);
+            sort.add(&idx2, nb);
+            sort.add(&sorted, sizeof(Chunk) * (size_t)s.n_chunks);
+            sort.add(&sort_tmp, sort_bytes);
+            if ((rc = sort.make())) return rc;
+            chunk_first_column_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, s.n_chunks, s.col, key, idx);
             DRONE_LAUNCH_CHECK("chunk_first_column_kernel");
-            DRONE_CUDA(cub::DeviceRadixSort::SortPairs(o.tmp, sort_bytes, o.key, o.key2, o.idx, o.idx2, s.n_chunks, 0, 30, st));
+            DRONE_CUDA(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, key, key2, idx, idx2, s.n_chunks, 0, 30, st));
             count_launch();
-            permute_chunks_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, o.idx2, s.n_chunks, o.sorted);
+            permute_chunks_kernel<<<grid_for(s.n_chunks), 256, 0, st>>>(s.chunks, idx2, s.n_chunks, sorted);
             DRONE_LAUNCH_CHECK("permute_chunks_kernel");
-            DRONE_CUDA(cudaMemcpyAsync(s.chunks, o.sorted, sizeof(Chunk) * (size_t)s.n_chunks, cudaMemcpyDeviceToDevice, st));
+            DRONE_CUDA(cudaMemcpyAsync(s.chunks, sorted, sizeof(Chunk) * (size_t)s.n_chunks, cudaMemcpyDeviceToDevice, st));
             DRONE_CUDA(cudaStreamSynchronize(st));
         }
     }
@@ -709,8 +753,8 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
     DRONE_CUDA(cudaMalloc(&a.col, sizeof(int) * nnz_alloc));
     DRONE_CUDA(cudaMalloc(&a.val, sizeof(float) * nnz_alloc));
     DRONE_CUDA(cudaMemcpyAsync(a.rowptr, d_index, sizeof(int) * (size_t)(n_rows + 1), cudaMemcpyDeviceToDevice, st));
-    if (nnz > 0) {
-        DRONE_CUDA(cudaMemcpyAsync(a.col, d_dst, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToDevice, st));
+    if (nnz > 0) DRONE_CUDA(cudaMemcpyAsync(a.col, d_dst, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToDevice, st));
+    const auto fill_values = [&]() -> int {
         if (d_values) {
             DRONE_CUDA(cudaMemcpyAsync(a.val, d_values, sizeof(float) * (size_t)nnz, cudaMemcpyDeviceToDevice, st));
         } else {
@@ -718,8 +762,8 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
                                                                               d_out_degree, n_rows, a.val);
             DRONE_LAUNCH_CHECK("csr_values_kernel");
         }
-    }
-    DRONE_CUDA(cudaStreamSynchronize(st));
+        return DRONE_OK;
+    };
 
     const char *overlap = getenv("DRONE_SPMM_OVERLAP");   // "0" keeps every kernel of a call on the caller's stream
     if (!(overlap && overlap[0] == '0')) {
@@ -729,9 +773,15 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
     }
     DRONE_CUDA(cudaMalloc(&p->counter, sizeof(unsigned)));
     p->chunk_blocks_per_sm = env_int("DRONE_CHUNK_BLOCKS_PER_SM", 0);
+    PlanScratch scratch;
     if (orientations & DRONE_PLAN_AT) {
-        const int rc = build_transpose(p, st);
+        const int rc = build_transpose(p, scratch, st, fill_values);
         if (rc) return rc;
+        if (scratch.bytes > PlanScratch::kKept) scratch.give_back();
+    } else {
+        const int rc = nnz > 0 ? fill_values() : DRONE_OK;
+        if (rc) return rc;
+        DRONE_CUDA(cudaStreamSynchronize(st));
     }
     // Table of hot rows: only for graphs whose dense operand is far larger than L2 at the usual widths (at least
     // DRONE_HOT_MIN_ROWS rows, default 2^23: measured on R-MAT graphs with 32 features, the table gains 10 % at 2^26
@@ -756,11 +806,11 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
         }
     }
     if (orientations & DRONE_PLAN_AT) {
-        const int rc = build_work_lists(p, p->side[DRONE_OP_AT], st);
+        const int rc = build_work_lists(p, p->side[DRONE_OP_AT], scratch, st);
         if (rc) return rc;
     }
     if (orientations & DRONE_PLAN_A) {
-        int rc = build_work_lists(p, a, st);
+        int rc = build_work_lists(p, a, scratch, st);
         if (rc) return rc;
     } else {
         free_side(a);
@@ -978,7 +1028,8 @@ int drone_plan_set_row_classes(drone_plan *p, const int *d_row_class, int n_clas
         Side &s = p->side[o];
         if (!s.rowptr) continue;
         free_lists(s);
-        rc = build_work_lists(p, s, st);
+        PlanScratch none;
+        rc = build_work_lists(p, s, none, st);
     }
     return rc;
 }
