@@ -83,7 +83,8 @@ static long long padded_stride(int n_rows, int F) {
 }
 
 // The copies' buffers.  drone_plan_reserve makes them ahead of time; otherwise the first call that wants them does, unless
-// that call must not allocate, or they would take more than kPadBytes nobody asked for.
+// that call must not allocate (its width was reserved without them, the stream is being captured), or they would take more
+// than kPadBytes nobody asked for.
 constexpr size_t kPadBytes = (size_t)4 << 30;
 
 static int ensure_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
@@ -198,7 +199,7 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         const long long stride = padded_stride(p->n_rows, F);
         const size_t x_floats = (size_t)stride * (size_t)p->n_rows, y_floats = (size_t)Fp * (size_t)p->n_rows;
         vec4 = x_floats <= p->pad_x_floats && y_floats <= p->pad_y_floats;
-        if (!vec4 && !opt.no_allocation && sizeof(float) * (x_floats + y_floats) <= kPadBytes && may_allocate(st)) {
+        if (!vec4 && !opt.no_allocation && caller_F > p->reserved_features && sizeof(float) * (x_floats + y_floats) <= kPadBytes && may_allocate(st)) {
             vec4 = ensure_padding(p, x_floats, y_floats) == DRONE_OK;
             if (!vec4) cudaGetLastError();      // no memory for the copies: the rows are accessed float by float
         }
@@ -457,10 +458,11 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
     DeviceGuard guard;
     int rc = guard.enter(p->device);
     if (rc) return rc;
-    const size_t slots = (size_t)std::max(p->side[0].n_partials, p->side[1].n_partials);
-    if (slots > 0 && (rc = ensure_scratch(p, sizeof(float) * slots * (size_t)max_features))) return rc;
     DRONE_REQUIRE((what & ~(DRONE_RESERVE_HOST_OPERANDS | DRONE_RESERVE_PADDED_ROWS)) == 0,
                   "drone_plan_reserve: what=%d is not a combination of DRONE_RESERVE_* flags", what);
+    const size_t slots = (size_t)std::max(p->side[0].n_partials, p->side[1].n_partials);
+    const int copied_features = (max_features + 3) & ~3;      // the width of a call on padded copies
+    if (slots > 0 && (rc = ensure_scratch(p, sizeof(float) * slots * (size_t)copied_features))) return rc;
     if (what & DRONE_RESERVE_HOST_OPERANDS) {
         if ((rc = ensure_staging(p, sizeof(float) * (size_t)p->n_rows * (size_t)max_features))) return rc;
         if (!p->own_stream) DRONE_CUDA(cudaStreamCreateWithFlags(&p->own_stream, cudaStreamNonBlocking));
@@ -468,8 +470,10 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
     if ((what & DRONE_RESERVE_PADDED_ROWS) && p->n_rows > 0) {
         long long stride = 0;      // of the widths up to max_features, the one whose copy is largest
         for (int f = 9; f <= max_features; ++f) stride = std::max(stride, padded_stride(p->n_rows, f));
-        return ensure_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)((max_features + 3) & ~3) * (size_t)p->n_rows);
+        rc = ensure_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)copied_features * (size_t)p->n_rows);
+        if (rc) return rc;
     }
+    p->reserved_features = std::max(p->reserved_features, max_features);
     return DRONE_OK;
 }
 

@@ -105,8 +105,9 @@ class AggregationPlan:
 
     def reserve(self, max_features, host_operands=False, padded_rows=False):
         """Allocate now what calls with F <= max_features would allocate on first use (partial sums of split rows;
-        with host_operands the device staging of spmm_host; with padded_rows the copy through which widths that are
-        not multiples of 4 run on the float4 kernels)."""
+        with host_operands the device staging of spmm_host; with padded_rows the copies through which widths that are
+        not multiples of 4 run on the float4 kernels where that pays).  Such calls then allocate nothing: without
+        padded_rows they do without the copies."""
         with torch.cuda.device(self.device):
             check(_lib.lib().drone_plan_reserve(self._h, int(max_features),
                                                 (1 if host_operands else 0) | (2 if padded_rows else 0)))

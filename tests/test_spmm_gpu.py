@@ -657,3 +657,31 @@ def test_both_sides_of_the_copy_rule(cuda_device, n, per_row, f, copied):
         assert rc == 0, lib.drone_last_error()
         assert torch.equal(uncopied, y)
     assert copied == (torch.cuda.mem_get_info(cuda_device)[0] < free)
+
+
+def test_reserved_widths_allocate_nothing_for_copies(cuda_device):
+    """drone_plan_reserve on a graph whose odd widths are worth a padded copy.  Reserved without the copies: a call up to that
+    width takes no memory and reads the rows float by float.  Reserved with them: partial sums and copies are there for the
+    width the copied call runs at.  Not reserved: the call makes the copies.  The same bits every time."""
+    n, u, v = gg.rmat_graph(15, 64, seed=72, device=cuda_device, symmetrise=False, self_loops="add")
+    index, dst = gg.csr_by_source(u, v, n)
+    in_deg, out_deg = gg.degrees(u, v, n)
+    x = torch.randn((n, 41), device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(3))
+    wide = torch.zeros((n, 44), device=cuda_device)
+    results = []
+    for how in ("float by float", "copied", "unreserved"):
+        plan = db.AggregationPlan(index, dst, in_degree=in_deg, out_degree=out_deg)
+        assert plan.nnz >= 33 * n and plan.stats().n_partials[db.OP_AT] > 0
+        if how == "unreserved":
+            plan.spmm(db.OP_AT, wide)                     # makes the partial sums, and needs no copies
+        else:
+            plan.reserve(64 if how == "float by float" else 41, padded_rows=how == "copied")
+        out = torch.empty_like(x)
+        torch.cuda.synchronize()
+        held, free = plan.stats().scratch_bytes, torch.cuda.mem_get_info(cuda_device)[0]
+        plan.spmm(db.OP_AT, x, out=out)
+        torch.cuda.synchronize()
+        taken = free - torch.cuda.mem_get_info(cuda_device)[0]
+        assert (taken > 0) == (how == "unreserved") and plan.stats().scratch_bytes == held
+        results.append(out)
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
