@@ -20,6 +20,7 @@ int set_error(int code, const char *fmt, ...) {
     va_start(ap, fmt);
     vsnprintf(t_error, sizeof(t_error), fmt, ap);
     va_end(ap);
+    if (code == DRONE_E_CUDA) cudaGetLastError();      // reported now: the check after the next launch must not find it
     return code;
 }
 

@@ -142,6 +142,7 @@ struct drone_plan {
     // call.  X is copied into pad_x before the kernels, the result out of pad_y after them.
     float *pad_x = nullptr, *pad_y = nullptr;
     size_t pad_x_floats = 0, pad_y_floats = 0;
+    size_t pad_refused_bytes = ~(size_t)0;   // a call that needs this much new room for copies does without: so much did not fit
     int reserved_features = 0;     // drone_plan_reserve: calls up to this width allocate nothing
     int chunk_blocks_per_sm = 0;   // cap on resident blocks of the chunk kernel per SM (0: as many as fit)
     cudaStream_t own_stream = nullptr;

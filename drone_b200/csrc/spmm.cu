@@ -83,24 +83,58 @@ static long long padded_stride(int n_rows, int F) {
 }
 
 // The copies' buffers.  drone_plan_reserve makes them ahead of time; otherwise the first call that wants them does, unless
-// that call must not allocate (its width was reserved without them, the stream is being captured), or they would take more
-// than kPadBytes nobody asked for.
+// that call must not allocate (its width was reserved without them, the stream is being captured), they would take more
+// than kPadBytes nobody asked for, or so much did not fit before: the next drone_plan_reserve tries again.
 constexpr size_t kPadBytes = (size_t)4 << 30;
 
+// Floats of new memory that buffers of these sizes (0: not needed) take.
+static size_t padding_to_make(const drone_plan *p, size_t x_floats, size_t y_floats) {
+    return (x_floats > p->pad_x_floats ? x_floats : 0) + (y_floats > p->pad_y_floats ? y_floats : 0);
+}
+
+// What is there stays until its replacement exists, so that a failure costs nothing that was reserved before.
 static int ensure_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
-    if (x_floats <= p->pad_x_floats && y_floats <= p->pad_y_floats) return DRONE_OK;
-    DRONE_CUDA(cudaDeviceSynchronize());      // calls in flight use the buffers about to be replaced
+    const bool new_x = x_floats > p->pad_x_floats, new_y = y_floats > p->pad_y_floats;
+    if (!new_x && !new_y) return DRONE_OK;
+    float *x = nullptr, *y = nullptr;
+    cudaError_t e = new_x ? cudaMalloc(&x, sizeof(float) * x_floats) : cudaSuccess;
+    if (e == cudaSuccess && new_y) e = cudaMalloc(&y, sizeof(float) * y_floats);
+    if (e != cudaSuccess) {
+        cudaFree(x);
+        return set_error(DRONE_E_CUDA, "no memory for copies with padded rows (%zu bytes): %s",
+                         sizeof(float) * padding_to_make(p, x_floats, y_floats), cudaGetErrorString(e));
+    }
+    if ((new_x && p->pad_x) || (new_y && p->pad_y)) cudaDeviceSynchronize();      // calls in flight use what is replaced
+    if (new_x) {
+        cudaFree(p->pad_x);
+        p->pad_x = x;
+        p->pad_x_floats = x_floats;
+    }
+    if (new_y) {
+        cudaFree(p->pad_y);
+        p->pad_y = y;
+        p->pad_y_floats = y_floats;
+    }
+    return DRONE_OK;
+}
+
+// drone_plan_reserve's form: where old and new buffers do not fit together the old ones go first, and come back if the
+// new ones do not fit alone either.
+static int replace_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
+    p->pad_refused_bytes = ~(size_t)0;
+    if (ensure_padding(p, x_floats, y_floats) == DRONE_OK) return DRONE_OK;
+    const size_t old_x = p->pad_x_floats, old_y = p->pad_y_floats;
+    if (old_x + old_y == 0) return DRONE_E_CUDA;
+    DRONE_CUDA(cudaDeviceSynchronize());
     cudaFree(p->pad_x);
     cudaFree(p->pad_y);
     p->pad_x = p->pad_y = nullptr;
-    x_floats = std::max(x_floats, p->pad_x_floats);
-    y_floats = std::max(y_floats, p->pad_y_floats);
     p->pad_x_floats = p->pad_y_floats = 0;
-    DRONE_CUDA(cudaMalloc(&p->pad_x, sizeof(float) * x_floats));
-    DRONE_CUDA(cudaMalloc(&p->pad_y, sizeof(float) * y_floats));
-    p->pad_x_floats = x_floats;
-    p->pad_y_floats = y_floats;
-    return DRONE_OK;
+    if (ensure_padding(p, std::max(x_floats, old_x), std::max(y_floats, old_y)) == DRONE_OK) return DRONE_OK;
+    char message[512];
+    snprintf(message, sizeof(message), "%s", last_error_buffer());
+    ensure_padding(p, old_x, old_y);
+    return set_error(DRONE_E_CUDA, "%s", message);
 }
 
 // The copies are passes over [n, F]; what they save is in the gathers, so the line lies at a number of nonzeros per row, and
@@ -197,11 +231,13 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     if (!vec4 && F > 8 && worth_copying(p, F)) {
         const int Fp = (F + 3) & ~3;
         const long long stride = padded_stride(p->n_rows, F);
-        const size_t x_floats = (size_t)stride * (size_t)p->n_rows, y_floats = (size_t)Fp * (size_t)p->n_rows;
-        vec4 = x_floats <= p->pad_x_floats && y_floats <= p->pad_y_floats;
-        if (!vec4 && !opt.no_allocation && caller_F > p->reserved_features && sizeof(float) * (x_floats + y_floats) <= kPadBytes && may_allocate(st)) {
+        const size_t x_floats = copy_x ? (size_t)stride * (size_t)p->n_rows : 0, y_floats = copy_y ? (size_t)Fp * (size_t)p->n_rows : 0;
+        const size_t missing = sizeof(float) * padding_to_make(p, x_floats, y_floats);
+        vec4 = missing == 0;
+        if (!vec4 && !opt.no_allocation && caller_F > p->reserved_features && missing < p->pad_refused_bytes &&
+            sizeof(float) * (std::max(x_floats, p->pad_x_floats) + std::max(y_floats, p->pad_y_floats)) <= kPadBytes && may_allocate(st)) {
             vec4 = ensure_padding(p, x_floats, y_floats) == DRONE_OK;
-            if (!vec4) cudaGetLastError();      // no memory for the copies: the rows are accessed float by float
+            if (!vec4) p->pad_refused_bytes = missing;      // rows are accessed float by float, from now on without asking again
         }
         if (vec4) {
             if (copy_x) {
@@ -470,7 +506,7 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
     if ((what & DRONE_RESERVE_PADDED_ROWS) && p->n_rows > 0) {
         long long stride = 0;      // of the widths up to max_features, the one whose copy is largest
         for (int f = 9; f <= max_features; ++f) stride = std::max(stride, padded_stride(p->n_rows, f));
-        rc = ensure_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)copied_features * (size_t)p->n_rows);
+        rc = replace_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)copied_features * (size_t)p->n_rows);
         if (rc) return rc;
     }
     p->reserved_features = std::max(p->reserved_features, max_features);

@@ -200,7 +200,8 @@ int drone_spmm_rows(drone_plan *plan, int orientation, int row_class, int F,
  *                                has enough nonzeros per row, calls of more than 8 columns on such operands copy X, run
  *                                the float4 kernels and copy the result out: two extra passes over [n_rows, F], made up
  *                                for in the gathers.  On a plan that was not reserved for its width the first such call
- *                                makes the room itself, unless it takes more than 4 GB or the stream is being captured.
+ *                                makes the room itself, unless it takes more than 4 GB, so much did not fit before, or
+ *                                the stream is being captured.
  *                                Everywhere else such rows are accessed float by float; either way adds in the same
  *                                order.
  * After it, drone_spmm / drone_spmm_rows / drone_spmm_host with F <= max_features reach neither cudaMalloc nor a

@@ -685,3 +685,48 @@ def test_reserved_widths_allocate_nothing_for_copies(cuda_device):
         assert (taken > 0) == (how == "unreserved") and plan.stats().scratch_bytes == held
         results.append(out)
     assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+
+
+def test_copies_that_do_not_fit(cuda_device):
+    """A call whose padded copies do not fit into what memory is left reads its rows float by float: what had been reserved
+    for narrower calls stays, nothing half made is left behind, the allocation is not tried again by the next call, and a
+    reservation makes up for it.  The same bits by both routes."""
+    n, per_row, f = 200000, 70, 1001
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(5)
+    h = torch.unique(torch.randint(0, n * n, (n * per_row,), device=cuda_device, generator=gen))
+    u, v = (h // n).to(torch.int32), (h % n).to(torch.int32)
+    index, dst = gg.csr_by_source(u, v, n)
+    in_deg, out_deg = (d.clamp_(min=1) for d in gg.degrees(u, v, n))
+    del h
+    plan = db.AggregationPlan(index, dst, in_degree=in_deg, out_degree=out_deg)
+    plan.reserve(41, padded_rows=True)
+    x, out = torch.randn((n, f), device=cuda_device, generator=gen), torch.empty((n, f), device=cuda_device)
+    narrow, narrow_out = torch.randn((n, 41), device=cuda_device, generator=gen), torch.empty((n, 41), device=cuda_device)
+    wide = torch.zeros((n, f + 3), device=cuda_device)
+    plan.spmm(db.OP_AT, wide, out=torch.empty_like(wide))          # makes the partial sums of a call this wide
+    del wide
+    torch.cuda.empty_cache()
+
+    def call(a, b):
+        """(launches of the call, device memory it took)"""
+        torch.cuda.synchronize()
+        before, free = db.lib().drone_kernel_launch_count(), torch.cuda.mem_get_info(cuda_device)[0]
+        plan.spmm(db.OP_AT, a, out=b)
+        torch.cuda.synchronize()
+        return db.lib().drone_kernel_launch_count() - before, free - torch.cuda.mem_get_info(cuda_device)[0]
+
+    copied = call(narrow, narrow_out)
+    assert copied[1] == 0
+    # room for the copy of X (0.8 GB) and not for that of Y as well
+    ballast = torch.empty(torch.cuda.mem_get_info(cuda_device)[0] - (1 << 30) - (100 << 20), dtype=torch.uint8, device=cuda_device)
+    uncopied = call(x, out)
+    assert uncopied[1] == 0
+    first = out.cpu()
+    assert call(narrow, narrow_out) == copied
+    del ballast
+    torch.cuda.empty_cache()
+    assert call(x, out) == uncopied
+    plan.reserve(f, padded_rows=True)
+    assert call(x, out) == (uncopied[0] + 2, 0)
+    assert torch.equal(out.cpu(), first)
