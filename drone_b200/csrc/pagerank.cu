@@ -54,12 +54,11 @@ struct drone_pr {
     void *send = nullptr, *recv = nullptr;   // real2[max(up, down)]
     int *counters = nullptr;          // [0..3] exchange counts, [4] active count
     // parts held by one process: {part, row} of every contribution a master row takes, in m_pos order, {place, out
-    // degree} of that row in its part, and the plans they were made for
+    // degree} of that row in its part, and the plans these were filled in for
     int2 *pairs = nullptr, *targets = nullptr;
     std::vector<unsigned long long> pairs_for;
     unsigned char *shared = nullptr;  // [n_local] 1 for rows that other parts hold too
     char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
-    size_t control_bytes = 0;
     drone::DeviceBlock block;                // what the arrays made at creation are pieces of
     int sms = 0;
     unsigned barrier_start = 0, barrier_polls = 0;   // what the grid barrier's count starts at, and when its waits run out
@@ -1238,13 +1237,10 @@ static int prepare_pairs(std::vector<drone_pr *> &parts, cudaStream_t st) {
         }
         const int n = (int)x->m_pos.size();
         if (n > 0) {
-            if (!me->pairs) DRONE_CUDA(cudaMalloc(&me->pairs, sizeof(int2) * (size_t)n));
-            if (!me->targets) DRONE_CUDA(cudaMalloc(&me->targets, sizeof(int2) * (size_t)n));
             pr_pairs_kernel<<<grid1d(n), 256, 0, st>>>(x->d_m_pos, n, lists, P, me->pairs, me->targets);
             DRONE_LAUNCH_CHECK("pr_pairs_kernel");
         }
         if (me->n_local > 0) {
-            if (!me->shared) DRONE_CUDA(cudaMalloc(&me->shared, (size_t)me->n_local));
             DRONE_CUDA(cudaMemsetAsync(me->shared, 0, (size_t)me->n_local, st));
             const int up = (int)x->up_rows.size(), masters = (int)x->m_rows.size();
             if (up > 0) {
@@ -1331,16 +1327,7 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
 }
 
 static int run_local(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaStream_t st) {
-    drone_pr *lead = parts[0];
-    const size_t need = sizeof(RunControl) + sizeof(int) * 4 * parts.size() * kHistorySteps;
-    if (need > lead->control_bytes) {      // handles of one part get theirs at creation
-        DRONE_CUDA(cudaStreamSynchronize(st));
-        cudaFree(lead->control);
-        lead->control = nullptr;
-        lead->control_bytes = 0;
-        DRONE_CUDA(cudaMalloc(&lead->control, need));
-        lead->control_bytes = need;
-    }
+    const drone_pr *lead = parts[0];
     const int rc = prepare_pairs(parts, st);
     if (rc) return rc;
     const bool few = parts.size() <= 8;
@@ -1478,10 +1465,15 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         p->block.add(&p->recv, 2 * rs * nb);
         p->block.add(&p->counters, sizeof(int) * 8);
         p->block.add(&p->unfinished, sizeof(unsigned));
+        if (xplan->nranks > 1 && xplan->nranks <= kMaxLocalParts) {      // for runs over all parts in one process
+            p->block.add(&p->pairs, sizeof(int2) * xplan->m_pos.size());
+            p->block.add(&p->targets, sizeof(int2) * xplan->m_pos.size());
+            p->block.add(&p->shared, n1);
+        }
+        const size_t control_bytes = sizeof(RunControl) + sizeof(int) * 4 * (size_t)xplan->nranks * kHistorySteps;
+        p->block.add(&p->control, control_bytes);
         if (e == cudaSuccess) e = p->block.make();
-        p->control_bytes = sizeof(RunControl) + sizeof(int) * 4 * (size_t)xplan->nranks * kHistorySteps;
-        if (e == cudaSuccess) e = cudaMalloc(&p->control, p->control_bytes);
-        if (e == cudaSuccess) e = cudaMemset(p->control, 0, p->control_bytes);
+        if (e == cudaSuccess) e = cudaMemset(p->control, 0, control_bytes);
         if (e == cudaSuccess) e = cudaMemset(p->unfinished, 0, sizeof(unsigned));
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
         if (e == cudaSuccess && side.n_split_rows > 0) {
@@ -1513,8 +1505,6 @@ int drone_pr_destroy(drone_pr *p) {
     drone_plan_destroy(p->plan);
     cudaFree(p->place);
     p->block.release();
-    cudaFree(p->pairs); cudaFree(p->targets); cudaFree(p->shared);
-    cudaFree(p->control);
     if (prev >= 0) cudaSetDevice(prev);
     delete p;
     return DRONE_OK;

@@ -272,3 +272,18 @@ def test_a_wait_that_runs_out_is_reported(cuda_device, oracle, monkeypatch, part
     got = prk.gather_global(prs, graphs, n)
     touched = part.replicas > 0
     assert np.max(np.abs(got[touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
+
+
+def test_handles_allocate_when_they_are_made(cuda_device):
+    """drone_pr_create makes everything a handle needs: the first job and the first power iteration over several parts take no
+    device memory (the exchange plans' own copies, made on their first use, are there already)."""
+    n, u, v, out_deg, part = pr_case(scale=19, seed=73, parts=3)
+    graphs, prs = build_parts(part, n, u, v, cuda_device, True, 1e-6)
+    prk.step_local(prs, True)
+    fresh = [prk.PageRank(g, n, use_double=True, eps=1e-6) for g in graphs]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info(cuda_device)[0]
+    prk.step_local(fresh, True)
+    prk.power_iterate_local(fresh, 2, 0.85)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info(cuda_device)[0] == free
