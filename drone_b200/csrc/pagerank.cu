@@ -61,6 +61,7 @@ struct drone_pr {
     char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
     drone::DeviceBlock block;                // what the arrays made at creation are pieces of
     int sms = 0;
+    bool separate_steps = false;      // parts in one process take the kernels of one process per GPU (local_parts_run_separately)
     unsigned barrier_start = 0, barrier_polls = 0;   // what the grid barrier's count starts at, and when its waits run out
     unsigned run = 0;                 // number (in the process) of the launch that made the values; 0: the separate kernels did
     unsigned *unfinished = nullptr;   // device: number of the last launch that gave up
@@ -1047,14 +1048,24 @@ static int pull(drone_pr *p, cudaStream_t st) {
     return DRONE_OK;
 }
 
-// Moves the packed boundary entries of one process per GPU: up == true sends my `up` slices and receives `down` slices.
-struct NcclTransport {
-    virtual int move(drone_pr *p, bool up, size_t pair_bytes, bool dbl, cudaStream_t st) {
+// Moves the packed boundary entries of the parts this process steps (one, with one process per GPU): up == true sends their
+// `up` slices and receives `down` slices.
+struct Transport {
+    virtual int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, cudaStream_t st) = 0;
+    // where the entries sent to part p lie after move(): its receive buffer unless the transport delivers elsewhere
+    virtual const void *received(drone_pr *p) { return p->recv; }
+    virtual int allreduce(std::vector<drone_pr *> &parts, int slot, cudaStream_t st) = 0;
+    virtual ~Transport() {}
+};
+
+struct NcclTransport : Transport {
+    int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, cudaStream_t st) override {
+        drone_pr *p = parts[0];
         const drone_xplan *x = p->xplan;
         if (x->nranks == 1) return DRONE_OK;
         const std::vector<int> &s_off = up ? x->up_off : x->down_off;
         const std::vector<int> &r_off = up ? x->down_off : x->up_off;
-        const ncclDataType_t ty = dbl ? ncclDouble : ncclFloat;
+        const ncclDataType_t ty = p->dbl ? ncclDouble : ncclFloat;
         DRONE_NCCL(ncclGroupStart());
         for (int q = 0; q < x->nranks; ++q) {
             if (q == x->rank) continue;
@@ -1065,26 +1076,66 @@ struct NcclTransport {
         DRONE_NCCL(ncclGroupEnd());
         return DRONE_OK;
     }
-    // where the entries sent to part p lie after move(): its receive buffer unless the transport delivers elsewhere
-    virtual const void *received(drone_pr *p) { return p->recv; }
-    int allreduce(drone_pr *p, int slot, bool dbl, cudaStream_t st) {
+    int allreduce(std::vector<drone_pr *> &parts, int slot, cudaStream_t st) override {
+        drone_pr *p = parts[0];
         if (!p->comm || p->comm->nranks == 1) return DRONE_OK;
-        char *ptr = (char *)p->scalars + (size_t)slot * (dbl ? 8 : 4);
-        DRONE_NCCL(ncclAllReduce(ptr, ptr, 1, dbl ? ncclDouble : ncclFloat, ncclSum, p->comm->comm, st));
+        char *ptr = (char *)p->scalars + (size_t)slot * (p->dbl ? 8 : 4);
+        DRONE_NCCL(ncclAllReduce(ptr, ptr, 1, p->dbl ? ncclDouble : ncclFloat, ncclSum, p->comm->comm, st));
         return DRONE_OK;
     }
-    virtual ~NcclTransport() {}
 };
 
 // One process per GPU on one NVLink domain: entries are stored straight into the receiver's memory
 // (the exchange plan's peer-memory transport, exchange_p2p.cu); the scalar sums stay on NCCL.
 struct PeerTransport : NcclTransport {
     const void *landed = nullptr;
-    int move(drone_pr *p, bool up, size_t pair_bytes, bool, cudaStream_t st) override {
+    int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, cudaStream_t st) override {
+        drone_pr *p = parts[0];
         if (p->xplan->nranks == 1) return DRONE_OK;
         return p2p_move_elements(p->xplan, p->send, pair_bytes, up, st, &landed);
     }
     const void *received(drone_pr *p) override { return p->xplan->nranks == 1 ? p->recv : landed; }
+};
+
+// All parts in one process: device-to-device copies, and a kernel that adds the parts' scalars in rank order.
+struct ScalarLists {
+    void *of[kMaxLocalParts];
+};
+
+template <typename R>
+__global__ void pr_sum_scalars_kernel(const __grid_constant__ ScalarLists scalars, int n_parts, int slot) {
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    R s = 0;
+    for (int p = 0; p < n_parts; ++p) s += ((R *)scalars.of[p])[slot];
+    for (int p = 0; p < n_parts; ++p) ((R *)scalars.of[p])[slot] = s;
+}
+
+struct LocalTransport : Transport {
+    int move(std::vector<drone_pr *> &parts, bool up, size_t pair_bytes, cudaStream_t st) override {
+        const int P = (int)parts.size();
+        for (int p = 0; p < P; ++p)
+            for (int q = 0; q < P; ++q) {
+                if (p == q) continue;
+                const std::vector<int> &s_off = up ? parts[p]->xplan->up_off : parts[p]->xplan->down_off;
+                const std::vector<int> &r_off = up ? parts[q]->xplan->down_off : parts[q]->xplan->up_off;
+                const size_t ns = (size_t)(s_off[q + 1] - s_off[q]), nr = (size_t)(r_off[p + 1] - r_off[p]);
+                if (ns != nr)
+                    return set_error(DRONE_E_STATE, "exchange plans disagree between parts %d and %d (%zu vs %zu rows)", p, q, ns, nr);
+                if (ns)
+                    DRONE_CUDA(cudaMemcpyAsync((char *)parts[q]->recv + (size_t)r_off[p] * pair_bytes,
+                                               (char *)parts[p]->send + (size_t)s_off[q] * pair_bytes, ns * pair_bytes,
+                                               cudaMemcpyDeviceToDevice, st));
+            }
+        return DRONE_OK;
+    }
+    int allreduce(std::vector<drone_pr *> &parts, int slot, cudaStream_t st) override {
+        ScalarLists lists;
+        for (size_t p = 0; p < parts.size(); ++p) lists.of[p] = parts[p]->scalars;
+        if (parts[0]->dbl) pr_sum_scalars_kernel<double><<<1, 32, 0, st>>>(lists, (int)parts.size(), slot);
+        else pr_sum_scalars_kernel<float><<<1, 32, 0, st>>>(lists, (int)parts.size(), slot);
+        DRONE_LAUNCH_CHECK("pr_sum_scalars_kernel");
+        return DRONE_OK;
+    }
 };
 
 // The transport of a job that runs as one process per GPU: peer memory when the exchange plan has it enabled and its
@@ -1095,110 +1146,133 @@ static bool use_peer_transport(const drone_pr *p) {
 
 // mirror -> master (add), master -> mirror (assign)
 template <typename R>
-static int exchange(drone_pr *p, NcclTransport &tr, cudaStream_t st) {
+static int exchange(std::vector<drone_pr *> &parts, Transport &tr, cudaStream_t st) {
     int rc;
-    const drone_xplan *x = p->xplan;
-    const int n_up = (int)x->up_rows.size(), n_m = (int)x->m_rows.size(), n_down = (int)x->down_rows.size();
-    if (n_up) {
-        pr_pack_up_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const R *)p->diff, p->active,
-                                                          (Pair<R> *)p->send, p->counters);
-        DRONE_LAUNCH_CHECK("pr_pack_up_kernel");
+    for (drone_pr *p : parts) {
+        const drone_xplan *x = p->xplan;
+        const int n_up = (int)x->up_rows.size();
+        if (n_up) {
+            pr_pack_up_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const R *)p->diff, p->active,
+                                                              (Pair<R> *)p->send, p->counters);
+            DRONE_LAUNCH_CHECK("pr_pack_up_kernel");
+        }
     }
-    if ((rc = tr.move(p, true, sizeof(Pair<R>), sizeof(R) == 8, st))) return rc;
-    if (n_m) {
-        pr_apply_up_kernel<R><<<grid1d(n_m), 256, 0, st>>>(x->d_m_rows, x->d_m_off, x->d_m_pos, n_m,
-                                                          (const Pair<R> *)tr.received(p), (R *)p->diff, p->ubm, p->counters);
-        DRONE_LAUNCH_CHECK("pr_apply_up_kernel");
+    if ((rc = tr.move(parts, true, sizeof(Pair<R>), st))) return rc;
+    for (drone_pr *p : parts) {
+        const drone_xplan *x = p->xplan;
+        const int n_m = (int)x->m_rows.size(), n_down = (int)x->down_rows.size();
+        if (n_m) {
+            pr_apply_up_kernel<R><<<grid1d(n_m), 256, 0, st>>>(x->d_m_rows, x->d_m_off, x->d_m_pos, n_m,
+                                                              (const Pair<R> *)tr.received(p), (R *)p->diff, p->ubm, p->counters);
+            DRONE_LAUNCH_CHECK("pr_apply_up_kernel");
+        }
+        if (n_down) {
+            pr_pack_down_kernel<R><<<grid1d(n_down), 256, 0, st>>>(x->d_down_rows, n_down, (const R *)p->diff, p->active,
+                                                                  p->ubm, (Pair<R> *)p->send, p->counters);
+            DRONE_LAUNCH_CHECK("pr_pack_down_kernel");
+        }
     }
-    if (n_down) {
-        pr_pack_down_kernel<R><<<grid1d(n_down), 256, 0, st>>>(x->d_down_rows, n_down, (const R *)p->diff, p->active,
-                                                              p->ubm, (Pair<R> *)p->send, p->counters);
-        DRONE_LAUNCH_CHECK("pr_pack_down_kernel");
-    }
-    if ((rc = tr.move(p, false, sizeof(Pair<R>), sizeof(R) == 8, st))) return rc;
-    if (n_up) {
-        pr_apply_down_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const Pair<R> *)tr.received(p), (R *)p->diff,
-                                                             p->ubm, p->counters);
-        DRONE_LAUNCH_CHECK("pr_apply_down_kernel");
+    if ((rc = tr.move(parts, false, sizeof(Pair<R>), st))) return rc;
+    for (drone_pr *p : parts) {
+        const drone_xplan *x = p->xplan;
+        const int n_up = (int)x->up_rows.size();
+        if (n_up) {
+            pr_apply_down_kernel<R><<<grid1d(n_up), 256, 0, st>>>(x->d_up_rows, n_up, (const Pair<R> *)tr.received(p), (R *)p->diff,
+                                                                 p->ubm, p->counters);
+            DRONE_LAUNCH_CHECK("pr_apply_down_kernel");
+        }
     }
     return DRONE_OK;
 }
 
-// One superstep of the job on a rank whose boundary entries travel between GPUs.
+// One superstep of the job, its steps as kernels of their own: the part of a rank whose boundary entries travel between GPUs.
 template <typename R>
-static int delta_step(drone_pr *p, bool peval, NcclTransport &tr, drone_pr_response *res, cudaStream_t st) {
+static int delta_step(std::vector<drone_pr *> &parts, bool peval, Transport &tr, drone_pr_response *res, cudaStream_t st) {
     using clock = std::chrono::steady_clock;
     const auto t0 = clock::now();
     int rc;
-    DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 8, st));
-    p->run = 0;
-    const PartView<R> v = part_view<R>(p, p->sms);
-    const int grid = grid1d(p->n_local, kReduceBlocks);
-    if (peval) {
-        DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
-        pr_init_kernel<R><<<grid, 256, 0, st>>>(v, (R)1, 0, (R *)p->block_sums);
-        DRONE_LAUNCH_CHECK("pr_init_kernel");
-    } else {
-        pr_roll_scalars_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars);
-        DRONE_LAUNCH_CHECK("pr_roll_scalars_kernel");
-        pr_increment_kernel<R><<<grid, 256, 0, st>>>(v, (R)p->eps, (R *)p->block_sums);
-        DRONE_LAUNCH_CHECK("pr_increment_kernel");
+    for (drone_pr *p : parts) {
+        DRONE_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 8, st));
+        p->run = 0;
+        const PartView<R> v = part_view<R>(p, p->sms);
+        const int grid = grid1d(p->n_local, kReduceBlocks);
+        if (peval) {
+            DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
+            pr_init_kernel<R><<<grid, 256, 0, st>>>(v, (R)1, 0, (R *)p->block_sums);
+            DRONE_LAUNCH_CHECK("pr_init_kernel");
+        } else {
+            pr_roll_scalars_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars);
+            DRONE_LAUNCH_CHECK("pr_roll_scalars_kernel");
+            pr_increment_kernel<R><<<grid, 256, 0, st>>>(v, (R)p->eps, (R *)p->block_sums);
+            DRONE_LAUNCH_CHECK("pr_increment_kernel");
+        }
+        pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 0);
+        DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
+        if ((rc = pull<R, true>(p, st))) return rc;
+        p->started = true;
     }
-    pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 0);
-    DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
-    if ((rc = pull<R, true>(p, st))) return rc;
-    p->started = true;
     DRONE_CUDA(cudaStreamSynchronize(st));
     const auto t1 = clock::now();
-    if ((rc = exchange<R>(p, tr, st))) return rc;
-    if ((rc = tr.allreduce(p, 0, sizeof(R) == 8, st))) return rc;
-    if (p->n_local > 0) {
-        pr_count_active_kernel<<<grid1d(p->n_local), 256, 0, st>>>(p->active, p->n_local, p->counters);
-        DRONE_LAUNCH_CHECK("pr_count_active_kernel");
+    if ((rc = exchange<R>(parts, tr, st))) return rc;
+    if ((rc = tr.allreduce(parts, 0, st))) return rc;
+    std::vector<int> h(8 * parts.size());
+    for (size_t i = 0; i < parts.size(); ++i) {
+        drone_pr *p = parts[i];
+        if (p->n_local > 0) {
+            pr_count_active_kernel<<<grid1d(p->n_local), 256, 0, st>>>(p->active, p->n_local, p->counters);
+            DRONE_LAUNCH_CHECK("pr_count_active_kernel");
+        }
+        DRONE_CUDA(cudaMemcpyAsync(h.data() + 8 * i, p->counters, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
     }
-    int h[8];
-    DRONE_CUDA(cudaMemcpyAsync(h, p->counters, sizeof(h), cudaMemcpyDeviceToHost, st));
     DRONE_CUDA(cudaStreamSynchronize(st));
     const auto t2 = clock::now();
-    res->Mirror2MasterSendSize = h[0];
-    res->Mirror2MasterRecvSize = h[1];
-    res->Master2MirrorSendSize = h[2];
-    res->Master2MirrorRecvSize = h[3];
-    res->VisitedSize = h[4];
-    res->LocalVertexSize = p->n_local;
-    res->CalTime = std::chrono::duration<float>(t1 - t0).count();
-    res->SendTime = std::chrono::duration<float>(t2 - t1).count();
+    for (size_t i = 0; i < parts.size(); ++i) {
+        drone_pr_response &r = res[i];
+        r.Mirror2MasterSendSize = h[8 * i + 0];
+        r.Mirror2MasterRecvSize = h[8 * i + 1];
+        r.Master2MirrorSendSize = h[8 * i + 2];
+        r.Master2MirrorRecvSize = h[8 * i + 3];
+        r.VisitedSize = h[8 * i + 4];
+        r.LocalVertexSize = parts[i]->n_local;
+        r.CalTime = std::chrono::duration<float>(t1 - t0).count();
+        r.SendTime = std::chrono::duration<float>(t2 - t1).count();
+    }
     return DRONE_OK;
 }
 
 template <typename R>
-static int power_iterations(drone_pr *p, int iterations, double damping, NcclTransport &tr, cudaStream_t st) {
+static int power_iterations(std::vector<drone_pr *> &parts, int iterations, double damping, Transport &tr, cudaStream_t st) {
     int rc;
-    const PartView<R> v = part_view<R>(p, p->sms);
-    p->run = 0;
-    const int grid = grid1d(p->n_local, kReduceBlocks);
-    const R start = (R)1 / (R)p->global_v;
-    DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
-    pr_init_kernel<R><<<grid, 256, 0, st>>>(v, start, 1, (R *)p->block_sums);
-    DRONE_LAUNCH_CHECK("pr_init_kernel");
-    pr_set_scalar_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, 3, start);
-    DRONE_LAUNCH_CHECK("pr_set_scalar_kernel");
-    p->started = false;
+    for (drone_pr *p : parts) {
+        const R start = (R)1 / (R)p->global_v;
+        DRONE_CUDA(cudaMemsetAsync(p->scalars, 0, sizeof(R) * 4, st));
+        pr_init_kernel<R><<<grid1d(p->n_local, kReduceBlocks), 256, 0, st>>>(part_view<R>(p, p->sms), start, 1, (R *)p->block_sums);
+        DRONE_LAUNCH_CHECK("pr_init_kernel");
+        pr_set_scalar_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, 3, start);
+        DRONE_LAUNCH_CHECK("pr_set_scalar_kernel");
+        p->started = false;
+        p->run = 0;
+    }
     for (int it = 0; it < iterations; ++it) {
-        DRONE_CUDA(cudaMemsetAsync((char *)p->scalars + 2 * sizeof(R), 0, sizeof(R), st));
-        pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid, (R *)p->scalars, 2);
-        DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
-        if (p->xplan->rank == 0 && p->n_isolated > 0) {
-            pr_power_isolated_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, p->n_isolated);
-            DRONE_LAUNCH_CHECK("pr_power_isolated_kernel");
+        for (drone_pr *p : parts) {
+            DRONE_CUDA(cudaMemsetAsync((char *)p->scalars + 2 * sizeof(R), 0, sizeof(R), st));
+            pr_fold_block_sums_kernel<R><<<1, 32, 0, st>>>((const R *)p->block_sums, grid1d(p->n_local, kReduceBlocks), (R *)p->scalars, 2);
+            DRONE_LAUNCH_CHECK("pr_fold_block_sums_kernel");
+            if (p->xplan->rank == 0 && p->n_isolated > 0) {
+                pr_power_isolated_kernel<R><<<1, 32, 0, st>>>((R *)p->scalars, p->n_isolated);
+                DRONE_LAUNCH_CHECK("pr_power_isolated_kernel");
+            }
+            // with flags: the exchange's pack kernels send the rows that have some in-neighbour
+            if ((rc = pull<R, true>(p, st))) return rc;
         }
-        // with flags: the exchange's pack kernels send the rows that have some in-neighbour
-        if ((rc = pull<R, true>(p, st))) return rc;
-        if ((rc = exchange<R>(p, tr, st))) return rc;
-        if ((rc = tr.allreduce(p, 2, sizeof(R) == 8, st))) return rc;
-        // new values, and what they publish for the next iteration, in one pass
-        pr_power_apply_kernel<R><<<grid, 256, 0, st>>>(v, (R)damping, it + 1 == iterations, (R *)p->block_sums);
-        DRONE_LAUNCH_CHECK("pr_power_apply_kernel");
+        if ((rc = exchange<R>(parts, tr, st))) return rc;
+        if ((rc = tr.allreduce(parts, 2, st))) return rc;
+        for (drone_pr *p : parts) {
+            // new values, and what they publish for the next iteration, in one pass
+            pr_power_apply_kernel<R><<<grid1d(p->n_local, kReduceBlocks), 256, 0, st>>>(part_view<R>(p, p->sms), (R)damping,
+                                                                                       it + 1 == iterations, (R *)p->block_sums);
+            DRONE_LAUNCH_CHECK("pr_power_apply_kernel");
+        }
     }
     return DRONE_OK;
 }
@@ -1354,10 +1428,22 @@ static int read_control(std::vector<drone_pr *> &parts, int steps, RunControl *c
     return set_error(DRONE_E_STATE, "PageRank: a wait between the blocks of a superstep ran out");
 }
 
+// Parts in one process usually run in the persistent kernel.  Handles made with DRONE_PR_SEPARATE_STEPS=1 take the kernels and
+// the order of one process per GPU instead, with copies for messages: so that those can be tested on one GPU.
+static bool local_parts_run_separately(const std::vector<drone_pr *> &parts) {
+    for (const drone_pr *p : parts)
+        if (!p->separate_steps) return false;
+    return true;
+}
+
 // One superstep of all given parts.
 static int step_parts(std::vector<drone_pr *> &parts, bool peval, drone_pr_response *res, cudaStream_t st) {
     for (drone_pr *p : parts)
         if (!peval && !p->started) return set_error(DRONE_E_STATE, "PR_IncEVal called before PR_PEVal");
+    if (local_parts_run_separately(parts)) {
+        LocalTransport copies;
+        return parts[0]->dbl ? delta_step<double>(parts, peval, copies, res, st) : delta_step<float>(parts, peval, copies, res, st);
+    }
     RunRequest rq;
     rq.job = true;
     rq.peval = peval;
@@ -1427,6 +1513,8 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
     p->comm = comm;
     p->barrier_start = barrier_start();
     p->barrier_polls = barrier_polls();
+    const char *separate = getenv("DRONE_PR_SEPARATE_STEPS");
+    p->separate_steps = separate && separate[0] == '1';
     cudaGetDevice(&p->device);
     const size_t rs = p->dbl ? 8 : 4;
     const size_t n1 = (size_t)(n_local > 0 ? n_local : 1);
@@ -1522,7 +1610,7 @@ static int run_step(drone_pr *p, bool peval, drone_pr_response *res, void *strea
     PeerTransport peer;
     NcclTransport nccl;
     NcclTransport &tr = use_peer_transport(p) ? peer : nccl;
-    return p->dbl ? delta_step<double>(p, peval, tr, res, st) : delta_step<float>(p, peval, tr, res, st);
+    return p->dbl ? delta_step<double>(parts, peval, tr, res, st) : delta_step<float>(parts, peval, tr, res, st);
 }
 
 int drone_pr_peval(drone_pr *p, drone_pr_response *res, void *stream) {
@@ -1570,6 +1658,21 @@ int drone_pr_job_local(int n_parts, drone_pr **prs, int max_steps, int *n_steps,
     rq.job = true;
     std::vector<int> h((size_t)kHistorySteps * n_parts * 4);
     int total = 0;
+    if (local_parts_run_separately(parts)) {
+        std::vector<drone_pr_response> res((size_t)n_parts);
+        for (bool sent = true; sent && total < max_steps; ++total) {
+            if ((rc = step_parts(parts, total == 0, res.data(), (cudaStream_t)stream))) return rc;
+            sent = false;
+            for (int i = 0; i < n_parts; ++i) {
+                const int four[4] = {res[i].Mirror2MasterSendSize, res[i].Mirror2MasterRecvSize, res[i].Master2MirrorSendSize,
+                                     res[i].Master2MirrorRecvSize};
+                for (int k = 0; k < 4; ++k) sent = sent || four[k] != 0;
+                if (sizes) memcpy(sizes + ((size_t)total * n_parts + i) * 4, four, sizeof(four));
+            }
+        }
+        *n_steps = total;
+        return DRONE_OK;
+    }
     for (RunControl c{}; !c.done && total < max_steps; total += c.steps) {
         rq.peval = total == 0;
         rq.max_steps = std::min(kHistorySteps, max_steps - total);
@@ -1582,6 +1685,11 @@ int drone_pr_job_local(int n_parts, drone_pr **prs, int max_steps, int *n_steps,
 }
 
 static int run_power(std::vector<drone_pr *> &parts, int iterations, double damping, cudaStream_t st) {
+    if (local_parts_run_separately(parts)) {
+        LocalTransport copies;
+        return parts[0]->dbl ? power_iterations<double>(parts, iterations, damping, copies, st)
+                             : power_iterations<float>(parts, iterations, damping, copies, st);
+    }
     RunRequest rq;
     rq.iterations = iterations;
     rq.damping = damping;
@@ -1603,7 +1711,8 @@ int drone_pr_power_iterate(drone_pr *p, int iterations, double damping, void *st
     PeerTransport peer;
     NcclTransport nccl;
     NcclTransport &tr = use_peer_transport(p) ? peer : nccl;
-    return p->dbl ? power_iterations<double>(p, iterations, damping, tr, st) : power_iterations<float>(p, iterations, damping, tr, st);
+    return p->dbl ? power_iterations<double>(parts, iterations, damping, tr, st)
+                  : power_iterations<float>(parts, iterations, damping, tr, st);
 }
 
 int drone_pr_power_iterate_local(int n_parts, drone_pr **prs, int iterations, double damping, void *stream) {

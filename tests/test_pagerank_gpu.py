@@ -287,3 +287,40 @@ def test_handles_allocate_when_they_are_made(cuda_device):
     prk.power_iterate_local(fresh, 2, 0.85)
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info(cuda_device)[0] == free
+
+
+@pytest.mark.parametrize("scale,parts,use_double", [(5, 2, True), (13, 1, False), (13, 3, True), (15, 4, True), (16, 2, False),
+                                                    (12, 12, False)])
+def test_separate_steps_of_one_process_per_gpu(cuda_device, oracle, monkeypatch, scale, parts, use_double):
+    """The kernels and the order of steps that a job takes with one process per GPU (pull, pack and apply of both directions,
+    dangling mass, isolated vertices), here with all parts in one process and copies for messages: against the double oracle
+    of both schedules, and against the persistent kernel in supersteps, exchange sizes, visited vertices and values."""
+    n, u, v, out_deg, part = pr_case(scale=scale, seed=80 + scale, parts=parts)
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want_power = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
+    touched = part.replicas > 0
+    tol = PR_TOL if use_double else 1e-4
+    results = []
+    for separate in ("0", "1"):
+        monkeypatch.setenv("DRONE_PR_SEPARATE_STEPS", separate)
+        graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+        before = db.lib().drone_kernel_launch_count()
+        steps, sizes = prk.run_job_local(prs)
+        delta = prk.gather_global(prs, graphs, n)
+        visited = [[r.VisitedSize for r in prk.step_local(prs, first)] for first in (True, False)]
+        prk.power_iterate_local(prs, 20, 0.85)
+        launches = db.lib().drone_kernel_launch_count() - before
+        assert (launches > 20 * parts) == (separate == "1")
+        power = prk.gather_global(prs, graphs, n)
+        assert np.max(np.abs(power[touched] - want_power[touched]) / want_power[touched]) < tol
+        # every replica of a vertex ends with its master's value, bit for bit
+        for p, g in zip(prs, graphs):
+            assert np.array_equal(p.values(), power[g.host.l2g])
+        results.append((steps, sizes, visited, delta))
+    if use_double:
+        want, want_steps, want_sizes = oracle.pr_drone_cuda(n, part.part_u, part.part_v, out_deg, part.owner, eps=1e-6, dtype=np.float64)
+        assert results[1][0] == want_steps
+        assert np.array_equal(np.array([[sum(s[i] for s in step) for i in range(4)] for step in results[1][1]]), want_sizes)
+        assert np.max(np.abs(results[1][3][touched] - want[touched]) / np.abs(want[touched])) < PR_TOL
+        assert results[0][:3] == results[1][:3]
+    assert np.max(np.abs(results[0][3][touched] - results[1][3][touched]) / np.abs(results[0][3][touched])) < (PR_TOL if use_double else 2e-4)
