@@ -103,3 +103,19 @@ struct RowColumn {
     do {                                                               \
         if (!(cond)) return drone::set_error(DRONE_E_INVALID, __VA_ARGS__); \
     } while (0)
+
+namespace drone {
+
+// A handle's device for the duration of a call: the caller's comes back on every way out.
+struct OnDevice {
+    int prev = -1, mine = -1;
+    int enter(int device) {
+        mine = device;
+        DRONE_CUDA(cudaGetDevice(&prev));
+        if (prev != mine) DRONE_CUDA(cudaSetDevice(mine));
+        return DRONE_OK;
+    }
+    ~OnDevice() { if (prev >= 0 && prev != mine) cudaSetDevice(prev); }
+};
+
+}  // namespace drone

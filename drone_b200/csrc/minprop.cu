@@ -692,14 +692,10 @@ int drone_mp_destroy(drone_mp *p) {
 static int mp_run(std::vector<drone_mp *> &parts, bool peval, int source_global, bool local, drone_pr_response *res,
                   void *stream) {
     DRONE_REQUIRE(res != nullptr, "Response pointer is NULL");
-    int prev = -1;
-    DRONE_CUDA(cudaGetDevice(&prev));
-    const int dev = parts[0]->device;
-    if (prev != dev) DRONE_CUDA(cudaSetDevice(dev));     // calls may arrive on any host thread
-    int rc = mp_prepare(parts);
-    if (rc == DRONE_OK) rc = mp_step(parts, peval, source_global, local, res, (cudaStream_t)stream);
-    if (prev != dev) cudaSetDevice(prev);
-    return rc;
+    OnDevice dev;
+    int rc = dev.enter(parts[0]->device);      // calls may arrive on any host thread
+    if (rc || (rc = mp_prepare(parts))) return rc;
+    return mp_step(parts, peval, source_global, local, res, (cudaStream_t)stream);
 }
 
 int drone_mp_peval(drone_mp *p, int source_global_id, drone_pr_response *res, void *stream) {
@@ -742,12 +738,11 @@ int drone_mp_device_arrays(drone_mp *p, void **d_value, int **d_active, int **d_
 int drone_mp_values(drone_mp *p, void *h_out, void *stream) {
     DRONE_REQUIRE(p != nullptr && h_out != nullptr, "drone_mp_values: NULL argument");
     if (p->n_local == 0) return DRONE_OK;
-    int prev = -1;
-    DRONE_CUDA(cudaGetDevice(&prev));
-    if (prev != p->device) DRONE_CUDA(cudaSetDevice(p->device));
+    OnDevice dev;
+    const int rc = dev.enter(p->device);
+    if (rc) return rc;
     DRONE_CUDA(cudaMemcpyAsync(h_out, p->value, sizeof(unsigned) * (size_t)p->n_local, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     DRONE_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    if (prev != p->device) cudaSetDevice(prev);
     return DRONE_OK;
 }
 

@@ -940,12 +940,6 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
     if (blockIdx.x == 0 && threadIdx.x == 0) a.control->t_end = now_ns();
 }
 
-// slot_split[slot] = index of the split row the slot belongs to
-__global__ void pr_slot_split_kernel(const SplitRow *__restrict__ split, int n_split, int *slot_split) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_split; i += gridDim.x * blockDim.x)
-        for (int k = 0; k < split[i].nslots; ++k) slot_split[split[i].slot0 + k] = i;
-}
-
 // pairs[k] = {part, row} (and targets[k] = {place, out degree} of that row) behind position m_pos[k] of part q's receive
 // buffer: peer p's entries start at down_off[p] there and are, in the same order, peer p's up list for q.
 struct PeerLists {
@@ -1468,17 +1462,6 @@ static int step_parts(std::vector<drone_pr *> &parts, bool peval, drone_pr_respo
     return DRONE_OK;
 }
 
-struct OnDevice {      // the handle's device for the duration of a call
-    int prev = -1, mine = -1;
-    int enter(int device) {
-        mine = device;
-        DRONE_CUDA(cudaGetDevice(&prev));
-        if (prev != mine) DRONE_CUDA(cudaSetDevice(mine));
-        return DRONE_OK;
-    }
-    ~OnDevice() { if (prev >= 0 && prev != mine) cudaSetDevice(prev); }
-};
-
 }  // namespace drone
 
 using namespace drone;
@@ -1566,9 +1549,7 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
         if (e == cudaSuccess && side.n_split_rows > 0) {
             e = cudaMemset(p->arrived, 0, sizeof(int) * (size_t)side.n_split_rows);
-            pr_slot_split_kernel<<<grid1d(side.n_split_rows), 256>>>(side.split, side.n_split_rows, p->slot_split);
-            if (e == cudaSuccess) e = cudaGetLastError();
-            count_launch();
+            if (e == cudaSuccess && (rc = fill_slot_split(side, p->slot_split, nullptr))) break;
         }
         if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: cudaMalloc failed: %s", cudaGetErrorString(e)); break; }
         if (n_local > 0) {

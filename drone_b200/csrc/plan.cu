@@ -325,6 +325,12 @@ static inline int grid_for(long long n, int block = 256, int cap = 148 * 32) {
 // host
 // ---------------------------------------------------------------------------
 
+int fill_slot_split(const Side &s, int *slot_split, cudaStream_t st) {
+    fill_slot_split_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, slot_split);
+    DRONE_LAUNCH_CHECK("fill_slot_split_kernel");
+    return DRONE_OK;
+}
+
 static int env_int(const char *name, int dflt) {
     const char *s = getenv(name);
     if (!s || !*s) return dflt;
@@ -568,8 +574,7 @@ static int build_work_lists(drone_plan *p, Side &s, PlanScratch &plan_scratch, c
         DRONE_LAUNCH_CHECK("fill_chunks_kernel");
         if (s.small && s.n_split_rows > 0) {
             DRONE_CUDA(cudaMemsetAsync(s.arrived, 0, sizeof(int) * (size_t)s.n_split_rows, st));
-            fill_slot_split_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, s.slot_split);
-            DRONE_LAUNCH_CHECK("fill_slot_split_kernel");
+            if ((rc = fill_slot_split(s, s.slot_split, st))) return rc;
         }
         if (s.n_split_rows > 0 && (!s.small || p->nnz > kSmallNnzMostFloats)) {   // for the separate kernels
             int *d_max = scratch, *d_count = scratch + 1;
@@ -732,6 +737,7 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
                             const float *d_values, const int *d_in_degree, const int *d_out_degree,
                             int orientations, cudaStream_t st, bool for_spmm) {
     DRONE_CUDA(cudaGetDevice(&p->device));
+    DRONE_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device));
     {
         const int rc = validate_csr("drone_plan_create", d_index, d_dst, n_rows, n_rows, nnz, st);
         if (rc) return rc;
@@ -969,19 +975,15 @@ int drone_plan_set_row_classes(drone_plan *p, const int *d_row_class, int n_clas
     DRONE_REQUIRE(n_classes >= 1 && n_classes <= kMaxRowClasses, "drone_plan_set_row_classes: n_classes=%d outside 1..%d",
                   n_classes, kMaxRowClasses);
     DRONE_REQUIRE(n_classes == 1 || d_row_class != nullptr, "drone_plan_set_row_classes: d_row_class is NULL");
-    struct Restore {      // the caller's device comes back on every way out
-        int prev = -1, mine = -1;
-        ~Restore() { if (prev >= 0 && prev != mine) cudaSetDevice(prev); }
-    } dev;
+    OnDevice dev;
+    int rc = dev.enter(p->device);
+    if (rc) return rc;
     struct Temp {         // scratch of this call
         int *keys_out = nullptr, *rows = nullptr, *counts = nullptr, *order = nullptr;
         void *sort = nullptr;
         ~Temp() { cudaFree(keys_out); cudaFree(rows); cudaFree(counts); cudaFree(order); cudaFree(sort); }
     } t;
     cudaStream_t st = (cudaStream_t)stream;
-    DRONE_CUDA(cudaGetDevice(&dev.prev));
-    dev.mine = p->device;
-    if (dev.prev != p->device) DRONE_CUDA(cudaSetDevice(p->device));
     const int n = p->n_rows;
     int h_counts[kMaxRowClasses] = {0};
     const bool classes = n_classes > 1 && n > 0;
@@ -1024,7 +1026,6 @@ int drone_plan_set_row_classes(drone_plan *p, const int *d_row_class, int n_clas
         p->n_classes = n_classes;
         for (int c = 0; c < n_classes; ++c) p->class_start[c + 1] = p->class_start[c] + h_counts[c];
     }
-    int rc = DRONE_OK;
     for (int o = 0; o < 2 && rc == DRONE_OK; ++o) {
         Side &s = p->side[o];
         if (!s.rowptr) continue;

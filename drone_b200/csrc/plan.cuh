@@ -6,8 +6,10 @@
 namespace drone {
 
 // Plans with at most this many nonzeros run a call as one launch: up to here the launches of the separate kernels take
-// longer than what handing chunks out dynamically, and overlapping the two kinds of rows, gains (R-MAT directed + I, one
-// launch / separate kernels, us at F = 16 | 64: 4.3 M nonzeros 49 / 89 | 133 / 160, 8.5 M 88 / 110 | 246 / 192).
+// longer than what handing chunks out dynamically, and overlapping the two kinds of rows, gains.  The two cross between 6 and
+// 8.5 M nonzeros at every width of 8 and more (time of one launch over time of the separate kernels, R-MAT and power law, at 4.2 |
+// 6.4 | 7.9 | 8.5 | 12.6 M nonzeros: F = 16 0.74 | 0.96 | 0.95 | 1.07 | 1.16, F = 64 0.81 | 0.97 | 1.00 | 1.08 | 1.05, F = 256
+// 0.71 | 1.01 | 0.93 | 0.88 | 1.02; F = 4 still 0.91 at 12.6 M).
 constexpr int kSmallNnz = 6 << 20;
 constexpr int kSmallNnzManyFloats = 1 << 20, kSmallNnzMostFloats = 1 << 15;   // the same with 8 or 16 floats of a row per lane
 constexpr int kWideSlots = 64;              // split rows above this many partial slots are reduced by a whole block
@@ -101,6 +103,8 @@ struct Side {
 
 struct drone_plan;
 namespace drone {
+// slot_split[slot] = the slot's entry of s.split, for all partial slots of the side.
+int fill_slot_split(const Side &s, int *slot_split, cudaStream_t st);
 // drone_plan_create for users inside the library that read the plan's lists with kernels of their own (the
 // PageRank pull): never tags columns.
 int plan_create_untagged(drone_plan **out, int n_rows, int nnz, const int *d_index, const int *d_dst, const float *d_values,
@@ -114,6 +118,7 @@ int plan_order_columns_by_frequency(drone_plan *p, int orientation, const int *d
 
 struct drone_plan {
     int device = 0;
+    int sms = 0;               // multiprocessors of the device
     int n_rows = 0;
     int nnz = 0;
     bool for_spmm = true;      // false: a plan whose lists other kernels of the library read (plan_create_untagged)

@@ -9,18 +9,6 @@
 
 namespace drone {
 
-// Puts the caller's device back on every way out of an entry point that had to switch to the plan's device.
-struct DeviceGuard {
-    int prev = -1, mine = -1;
-    int enter(int device) {
-        mine = device;
-        DRONE_CUDA(cudaGetDevice(&prev));
-        if (prev != mine) DRONE_CUDA(cudaSetDevice(mine));
-        return DRONE_OK;
-    }
-    ~DeviceGuard() { if (prev >= 0 && prev != mine) cudaSetDevice(prev); }
-};
-
 // in_scale[i] = 1/sqrt(inDegree[i]), out_scale[i] = 1/sqrt(outDegree[i]) (0 for a degree of 0): the two factors of the
 // reference's edge coefficient 1/sqrt(outDegree[u] * inDegree[v]).
 __global__ void degree_scales_kernel(const int *__restrict__ in_deg, const int *__restrict__ out_deg, int n,
@@ -278,6 +266,7 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     a.side = &s;
     a.n_rows = p->n_rows;
     a.nnz = p->nnz;
+    a.sms = p->sms;
     a.ldy = ldy;
     a.partials = p->scratch;
     a.counter = p->counter;
@@ -340,12 +329,10 @@ int drone_spmm(drone_plan *p, int orientation, int F, const float *d_X, int ldx,
     if (p->n_rows == 0) return DRONE_OK;
     DRONE_REQUIRE(d_X && d_Y, "drone_spmm: NULL operand");
     DRONE_REQUIRE(d_X != d_Y, "drone_spmm: X and Y must not alias");
-    int dev = -1;
-    DRONE_CUDA(cudaGetDevice(&dev));
-    if (dev != p->device) DRONE_CUDA(cudaSetDevice(p->device));
-    const int rc = spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream);
-    if (dev != p->device) cudaSetDevice(dev);
-    return rc;
+    OnDevice guard;
+    const int rc = guard.enter(p->device);
+    if (rc) return rc;
+    return spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream);
 }
 
 int drone_spmm_ex(drone_plan *p, int orientation, int F, const float *d_X, int ldx, float *d_Y, int ldy,
@@ -382,7 +369,7 @@ int drone_spmm_ex(drone_plan *p, int orientation, int F, const float *d_X, int l
     }
     DRONE_REQUIRE(d_X && d_Y, "drone_spmm_ex: NULL operand");
     DRONE_REQUIRE(d_X != d_Y, "drone_spmm_ex: X and Y must not alias");
-    DeviceGuard guard;
+    OnDevice guard;
     int rc = guard.enter(p->device);
     if (rc) return rc;
     return spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream, opt);
@@ -412,14 +399,12 @@ int drone_spmm_rows(drone_plan *p, int orientation, int row_class, int F, const 
     if (p->n_rows == 0) return DRONE_OK;
     DRONE_REQUIRE(d_X && d_Y, "drone_spmm_rows: NULL operand");
     DRONE_REQUIRE(d_X != d_Y, "drone_spmm_rows: X and Y must not alias");
-    int dev = -1;
-    DRONE_CUDA(cudaGetDevice(&dev));
-    if (dev != p->device) DRONE_CUDA(cudaSetDevice(p->device));
+    OnDevice guard;
+    const int rc = guard.enter(p->device);
+    if (rc) return rc;
     CallOptions opt;
     opt.row_class = row_class;
-    const int rc = spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream, opt);
-    if (dev != p->device) cudaSetDevice(dev);
-    return rc;
+    return spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream, opt);
 }
 
 static int ensure_staging(drone_plan *p, size_t bytes) {
@@ -491,7 +476,7 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
     DRONE_REQUIRE(p != nullptr, "drone_plan_reserve: plan is NULL");
     DRONE_REQUIRE(max_features >= 1 && max_features <= 1024, "drone_plan_reserve: max_features=%d outside 1..1024",
                   max_features);
-    DeviceGuard guard;
+    OnDevice guard;
     int rc = guard.enter(p->device);
     if (rc) return rc;
     DRONE_REQUIRE((what & ~(DRONE_RESERVE_HOST_OPERANDS | DRONE_RESERVE_PADDED_ROWS)) == 0,
@@ -521,7 +506,7 @@ int drone_spmm_host(drone_plan *p, int orientation, int F, const float *h_X, flo
     DRONE_REQUIRE(F >= 1 && F <= 1024, "drone_spmm_host: feature width F=%d outside 1..1024", F);
     if (p->n_rows == 0) return DRONE_OK;
     DRONE_REQUIRE(h_X && h_Y, "drone_spmm_host: NULL operand");
-    DeviceGuard guard;
+    OnDevice guard;
     int rc = guard.enter(p->device);
     if (rc) return rc;
     const size_t bytes = sizeof(float) * (size_t)p->n_rows * (size_t)F;
@@ -569,7 +554,7 @@ int drone_spmm_host_submit(drone_plan *p, int orientation, int F, const float *h
     DRONE_REQUIRE(F >= 1 && F <= 1024, "drone_spmm_host_submit: feature width F=%d outside 1..1024", F);
     DRONE_REQUIRE(ticket != nullptr, "drone_spmm_host_submit: ticket is NULL");
     DRONE_REQUIRE(p->n_rows == 0 || (h_X && h_Y), "drone_spmm_host_submit: NULL operand");
-    DeviceGuard guard;
+    OnDevice guard;
     int rc = guard.enter(p->device);
     if (rc) return rc;
     const long long k = p->submitted;
@@ -598,7 +583,7 @@ int drone_spmm_host_wait(drone_plan *p, long long ticket) {
     DRONE_REQUIRE(ticket >= 0 && ticket < p->submitted, "drone_spmm_host_wait: ticket %lld was not issued (%lld calls so far)",
                   ticket, p->submitted);
     if (p->n_rows == 0 || ticket + 2 < p->submitted) return DRONE_OK;     // a later submit on the slot waited for it
-    DeviceGuard guard;
+    OnDevice guard;
     const int rc = guard.enter(p->device);
     if (rc) return rc;
     DRONE_CUDA(cudaEventSynchronize(p->queue_out[ticket & 1]));
@@ -668,11 +653,11 @@ extern "C" int drone_spmm_static_scratch(drone_plan *p, int orientation, int F, 
                                 "drone_spmm_static_scratch: this plan needs %zu bytes of partial sums at F=%d, the built-in "
                                 "scratch holds %zu; use drone_spmm",
                                 need * sizeof(float), F, (size_t)DRONE_STATIC_SCRATCH_BYTES);
-    int dev = -1;
-    DRONE_CUDA(cudaGetDevice(&dev));
-    if (dev != p->device) DRONE_CUDA(cudaSetDevice(p->device));
+    drone::OnDevice guard;
+    int rc = guard.enter(p->device);
+    if (rc) return rc;
     float *partials = nullptr;
-    int rc = drone::static_partials_address(p->device, &partials);
+    rc = drone::static_partials_address(p->device, &partials);
     if (rc == DRONE_OK) {
         // same route as drone_spmm (a padded copy where the plan already has room for it, no column slices), with the
         // partial sums in the built-in array: the plan's own scratch pointer is swapped for the duration of the call
@@ -689,6 +674,5 @@ extern "C" int drone_spmm_static_scratch(drone_plan *p, int orientation, int F, 
         p->scratch_bytes = plan_scratch_bytes;
         p->slice_forced = plan_slices;
     }
-    if (dev != p->device) cudaSetDevice(dev);
     return rc;
 }

@@ -785,6 +785,7 @@ struct SpmmArgs {
     const Side *side;
     int n_rows;
     int nnz;
+    int sms;         // multiprocessors of the device
     int nvec;
     Gather gather;
     float *Y;
@@ -851,7 +852,7 @@ static int launch_all(const SpmmArgs &a) {
         // 120,000 rows of 5, F = 64, one wave: 22 / 25).
         auto kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0>;
         if constexpr (VEC == 4 && VPL == 1 && G >= 4 && EXACT) {
-            if (short_blocks > 148 * 4 && s.n_short_entries >= a.nnz / 2) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 5>;
+            if (short_blocks > a.sms * 4 && s.n_short_entries >= a.nnz / 2) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 5>;
         }
         DRONE_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const Chunk *)s.chunks + chunk_lo, n_chunks,
                                       chunk_blocks, (const int *)s.col, (const float *)s.val, (const SplitRow *)s.split,
@@ -887,7 +888,7 @@ static int launch_all(const SpmmArgs &a) {
         static int resident_all = 0;
         if (resident_all == 0) resident_all = resident_grid(kernel, 0);
         int resident = resident_all;
-        if (a.resident_per_sm > 0) resident = std::min(resident, a.resident_per_sm * 148);
+        if (a.resident_per_sm > 0) resident = std::min(resident, a.resident_per_sm * a.sms);
         int grid = ceil_div(ceil_div(n_chunks, kChunkGroup), 8);
         if (resident > 0 && grid > resident) grid = resident;
         DRONE_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), a.st));

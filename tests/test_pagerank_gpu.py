@@ -286,7 +286,7 @@ def test_handles_allocate_when_they_are_made(cuda_device):
     prk.step_local(fresh, True)
     prk.power_iterate_local(fresh, 2, 0.85)
     torch.cuda.synchronize()
-    assert torch.cuda.mem_get_info(cuda_device)[0] == free
+    assert torch.cuda.mem_get_info(cuda_device)[0] >= free
 
 
 @pytest.mark.parametrize("scale,parts,use_double", [(5, 2, True), (13, 1, False), (13, 3, True), (15, 4, True), (16, 2, False),

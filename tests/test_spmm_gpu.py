@@ -1,5 +1,6 @@
 """Parity of the CUDA aggregation (through the C ABI) with the double-precision oracle, the
 committed golden vectors, and cuSPARSE called as the reference calls it."""
+import gc
 import os
 
 import numpy as np
@@ -709,24 +710,24 @@ def test_copies_that_do_not_fit(cuda_device):
     torch.cuda.empty_cache()
 
     def call(a, b):
-        """(launches of the call, device memory it took)"""
+        """Launches of the call, which takes no device memory (a failing allocation may make the driver give some back)."""
         torch.cuda.synchronize()
         before, free = db.lib().drone_kernel_launch_count(), torch.cuda.mem_get_info(cuda_device)[0]
         plan.spmm(db.OP_AT, a, out=b)
         torch.cuda.synchronize()
-        return db.lib().drone_kernel_launch_count() - before, free - torch.cuda.mem_get_info(cuda_device)[0]
+        assert torch.cuda.mem_get_info(cuda_device)[0] >= free
+        return db.lib().drone_kernel_launch_count() - before
 
+    gc.collect()
     copied = call(narrow, narrow_out)
-    assert copied[1] == 0
     # room for the copy of X (0.8 GB) and not for that of Y as well
     ballast = torch.empty(torch.cuda.mem_get_info(cuda_device)[0] - (1 << 30) - (100 << 20), dtype=torch.uint8, device=cuda_device)
     uncopied = call(x, out)
-    assert uncopied[1] == 0
     first = out.cpu()
     assert call(narrow, narrow_out) == copied
     del ballast
     torch.cuda.empty_cache()
     assert call(x, out) == uncopied
     plan.reserve(f, padded_rows=True)
-    assert call(x, out) == (uncopied[0] + 2, 0)
+    assert call(x, out) == uncopied + 2
     assert torch.equal(out.cpu(), first)
