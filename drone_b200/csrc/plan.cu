@@ -576,7 +576,7 @@ static int build_work_lists(drone_plan *p, Side &s, PlanScratch &plan_scratch, c
             DRONE_CUDA(cudaMemsetAsync(s.arrived, 0, sizeof(int) * (size_t)s.n_split_rows, st));
             if ((rc = fill_slot_split(s, s.slot_split, st))) return rc;
         }
-        if (s.n_split_rows > 0 && (!s.small || p->nnz > kSmallNnzMostFloats)) {   // for the separate kernels
+        if (s.n_split_rows > 0 && (!s.small || p->nnz > small_nnz_floats(32))) {   // for the separate kernels
             int *d_max = scratch, *d_count = scratch + 1;
             DRONE_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(int), st));
             max_nslots_kernel<<<grid_for(s.n_split_rows), 256, 0, st>>>(s.split, s.n_split_rows, d_max);

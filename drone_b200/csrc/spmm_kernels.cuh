@@ -417,9 +417,10 @@ spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, cons
 // ---------------------------------------------------------------------------
 constexpr int kChunkGroup = 4;
 
+// SURE: how many of a lane's vectors need no test against the width.
 // Sum of one chunk: nonzeros [k0, k0 + len), taken in interleaved order by the warp's lane groups; (c, v) hold the
 // lane's entry of the first 32.  Every lane group ends with the same totals in acc.
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT, bool EARLY>
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT, bool EARLY, int SURE>
 __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const int *__restrict__ col,
                                           const float *__restrict__ val, const Gather &g, int k0, int len, int c, float v,
                                           int nvec, unsigned long long pol_keep, unsigned long long pol_stream) {
@@ -427,7 +428,6 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
     constexpr int RPW = 32 / G;
     constexpr int UU = MinOf<U, G>::value;
     constexpr bool BRANCH = VEC == 1 && VPL == 32 && !EARLY;
-    constexpr int SURE = VPL == 4 && EARLY ? 0 : sure_vectors(G, VPL, VEC);      // F = 95, 10,000 rows of 81: 37 / 39 us with it
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gi = lane / G;
@@ -554,7 +554,7 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
             }
 
             V acc[VPL];
-            sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT, false>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
+            sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT, false, sure_vectors(G, VPL, VEC)>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
 
             if (gi == 0) {
                 if (slot < 0) {
@@ -691,7 +691,7 @@ __device__ __forceinline__ void store_vector(const RowDestination<VEC> &dest, in
     else st_stream(dest.ptr + vi, v, pol);
 }
 
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, int BLOCKS_PER_SM>
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, int BLOCKS_PER_SM, int SURE = sure_vectors(G, VPL, VEC)>
 __global__ void __launch_bounds__(256, BLOCKS_PER_SM)
 spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_blocks, const int *__restrict__ col,
                   const float *__restrict__ val, const SplitRow *__restrict__ split, const int *__restrict__ slot_split,
@@ -724,7 +724,7 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
     const int4 sr = ch.w >= 0 ? __ldg(reinterpret_cast<const int4 *>(split) + which) : ch;      // row, first slot, slots
     V acc[VPL];
     wait_for_operands();
-    sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false, true>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
+    sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false, true, SURE>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
     int row = ch.x;
     if (ch.w >= 0) {
         if (gi == 0) {
@@ -830,10 +830,10 @@ static int launch_all(const SpmmArgs &a) {
     class_range(a.row_class, s.n_classes, s.chunk_start, &chunk_lo, &n_chunks);
     class_range(a.row_class, s.n_classes, s.split_start, &split_lo, &n_split);
     class_range(a.row_class, s.n_classes, s.wide_start, &wide_lo, &n_wide);
-    // Lanes with many single floats of a row (odd widths above 128) keep few warps resident, so that one launch covers less
-    // (power-law graphs, one launch / separate kernels, us: F = 201 0.7 M nonzeros 75 / 107, 1.3 M 184 / 153; F = 401
-    // 0.02 M 14 / 31, 0.05 M 41 / 38).
-    const bool one_launch = s.small && (VEC == 4 || VPL < 8 || a.nnz <= (VPL < 16 ? kSmallNnzManyFloats : kSmallNnzMostFloats));
+    // Odd widths above 128, one launch / separate kernels, us, power law: F = 131 30,000 rows of 41 89 / 136, 130,000 of 25 261 / 305,
+    // of 41 394 / 374; F = 301 60,000 of 41 308 / 336, 130,000 of 25 624 / 606; F = 401 10,000 of 13 39 / 42, 30,000 of 13 87 / 80; F = 601
+    // 3,000 of 13 32 / 47, 30,000 of 13 224 / 210.
+    const bool one_launch = s.small && (VEC == 4 || a.nnz <= small_nnz_floats(VPL));
     if (!HOT && one_launch) {
         const int chunk_blocks = ceil_div(n_chunks, 8), short_blocks = ceil_div(n_ranges, 8 * RPW);
         if (chunk_blocks + short_blocks == 0) return DRONE_OK;
@@ -853,6 +853,11 @@ static int launch_all(const SpmmArgs &a) {
         auto kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0>;
         if constexpr (VEC == 4 && VPL == 1 && G >= 4 && EXACT) {
             if (short_blocks > a.sms * 4 && s.n_short_entries >= a.nnz / 2) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 5>;
+        }
+        // On the smallest plans the chunks of F = 65 to 128 are quicker with a test per vector (without / with, us, F = 95: 10,000
+        // rows of 81 39 / 37, 30,000 rows of 41 53 / 60, 250,000 of 7 130 / 153).
+        if constexpr (VEC == 1 && VPL == 4 && sure_vectors(G, VPL, VEC) > 0) {
+            if (a.nnz < 1 << 20) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0, 0>;
         }
         DRONE_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const Chunk *)s.chunks + chunk_lo, n_chunks,
                                       chunk_blocks, (const int *)s.col, (const float *)s.val, (const SplitRow *)s.split,
