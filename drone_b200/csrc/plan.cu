@@ -49,18 +49,22 @@ __global__ void csr_values_kernel(const int *__restrict__ index, const int *__re
     }
 }
 
-// src[k] = row that owns nonzero k (upper bound search in rowptr).
+// The row that owns nonzero k: the last one with rowptr[row] <= k.
+__device__ __forceinline__ int row_of(const int *__restrict__ rowptr, int n_rows, int k) {
+    int lo = 0, hi = n_rows;
+    while (hi - lo > 1) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if (__ldg(rowptr + mid) <= k) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// src[k] = row that owns nonzero k
 __global__ void expand_rows_kernel(const int *__restrict__ rowptr, int n_rows, int nnz,
                                    int *__restrict__ src) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nnz;
-         k += (long long)gridDim.x * blockDim.x) {
-        int lo = 0, hi = n_rows;  // find the last row with rowptr[row] <= k
-        while (hi - lo > 1) {
-            const int mid = lo + ((hi - lo) >> 1);
-            if (rowptr[mid] <= (int)k) lo = mid; else hi = mid;
-        }
-        src[k] = lo;
-    }
+         k += (long long)gridDim.x * blockDim.x)
+        src[k] = row_of(rowptr, n_rows, (int)k);
 }
 
 __global__ void histogram_kernel(const int *__restrict__ keys, int n, int *__restrict__ counts) {
@@ -69,13 +73,14 @@ __global__ void histogram_kernel(const int *__restrict__ keys, int n, int *__res
         atomicAdd(counts + keys[k], 1);
 }
 
-// colT[i] = src[perm[i]], valT[i] = val[perm[i]]; perm may lie in valT's memory (entry i is read before it is written)
-__global__ void gather_transposed_kernel(const int *perm, const int *__restrict__ src, const float *__restrict__ val, int nnz,
-                                         int *__restrict__ col_t, float *val_t) {
+// colT[i] = row of nonzero perm[i] (src[perm[i]], or looked up without src), valT[i] = val[perm[i]]; perm may lie in valT's
+// memory (entry i is read before it is written)
+__global__ void gather_transposed_kernel(const int *perm, const int *__restrict__ src, const int *__restrict__ rowptr, int n_rows,
+                                         const float *__restrict__ val, int nnz, int *__restrict__ col_t, float *val_t) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nnz;
          i += (long long)gridDim.x * blockDim.x) {
         const int p = perm[i];
-        col_t[i] = src[p];
+        col_t[i] = src ? src[p] : row_of(rowptr, n_rows, p);
         val_t[i] = val[p];
     }
 }
@@ -340,8 +345,8 @@ static int env_int(const char *name, int dflt) {
 
 // Scratch of making a plan, one allocation for all of its steps: cudaMalloc of a few hundred kilobytes takes 3 us where the
 // driver has room in a mapping, and 300 us, and as much again to free, where it has to map some.  Kept to the end, it also holds
-// the mapping that the lists then find room in (ms to make a plan, an allocation per step / one for all; R-MAT-12 sym 2.65 / 2.2,
-// with other plans alive 1.8 / 1.1 to 1.5; R-MAT-14 3.25 / 2.65, -16 5.7 / 4.45, -18 7.9 / 5.4, -20 10.8 / 7.8).  Steps take
+// the mapping that the lists then find room in (ms to make a plan, an allocation per step / one for all; R-MAT-12 sym 2.6 / 2.1,
+// with other plans alive 1.8 / 0.8; R-MAT-14 3.25 / 2.75, -16 5.7 / 4.4, -18 7.9 / 5.4, -20 10.7 / 8.0).  Steps take
 // their pieces from it like from a stack; what does not fit gets an allocation of its own.
 struct PlanScratch {
     // Scratch above this is given back before the next step allocates what stays with the plan.
@@ -403,7 +408,8 @@ static void free_side(Side &s) {
 
 // Build side[DRONE_OP_AT] from side[DRONE_OP_A], whose rows and columns must be on the device; fill_values() puts its values
 // there.  Of the sort's four arrays only one is scratch: the keys lie in what becomes the columns, and until it is filled in
-// A's value array, and half of the edge ids lie in what becomes the values.
+// A's value array, and half of the edge ids lie in what becomes the values.  Up to a million nonzeros the rows are looked up
+// when they are needed instead of being written down, which leaves 4 bytes of scratch a nonzero.
 template <typename Fill>
 static int build_transpose(drone_plan *p, PlanScratch &plan_scratch, cudaStream_t st, Fill fill_values) {
     const Side &a = p->side[DRONE_OP_A];
@@ -420,7 +426,7 @@ static int build_transpose(drone_plan *p, PlanScratch &plan_scratch, cudaStream_
     void *tmp = nullptr;
     const size_t words = sizeof(int) * (size_t)nnz;
     scratch.add(&counts, sizeof(int) * (size_t)(n + 1));
-    scratch.add(&src, words);
+    if (nnz > 1 << 20) scratch.add(&src, words);
     scratch.add(&perm, words);
     cub::DoubleBuffer<int> keys(t.col, nullptr), edges(nullptr, nullptr);
     size_t scan_bytes = 0, sort_bytes = 0;
@@ -443,8 +449,10 @@ static int build_transpose(drone_plan *p, PlanScratch &plan_scratch, cudaStream_
     count_launch();
     if (nnz > 0) {
         // stable sort of edge ids by destination: sources stay ascending inside a row
-        expand_rows_kernel<<<grid_for(nnz), 256, 0, st>>>(a.rowptr, n, nnz, src);
-        DRONE_LAUNCH_CHECK("expand_rows_kernel");
+        if (src) {
+            expand_rows_kernel<<<grid_for(nnz), 256, 0, st>>>(a.rowptr, n, nnz, src);
+            DRONE_LAUNCH_CHECK("expand_rows_kernel");
+        }
         iota_kernel<<<grid_for(nnz), 256, 0, st>>>(perm, nnz);
         DRONE_LAUNCH_CHECK("iota_kernel");
         DRONE_CUDA(cudaMemcpyAsync(t.col, a.col, words, cudaMemcpyDeviceToDevice, st));
@@ -453,7 +461,7 @@ static int build_transpose(drone_plan *p, PlanScratch &plan_scratch, cudaStream_
         DRONE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, keys, edges, nnz, 0, end_bit, st));
         count_launch();
         if ((rc = fill_values())) return rc;
-        gather_transposed_kernel<<<grid_for(nnz), 256, 0, st>>>(edges.Current(), src, a.val, nnz, t.col, t.val);
+        gather_transposed_kernel<<<grid_for(nnz), 256, 0, st>>>(edges.Current(), src, a.rowptr, n, a.val, nnz, t.col, t.val);
         DRONE_LAUNCH_CHECK("gather_transposed_kernel");
     }
     DRONE_CUDA(cudaStreamSynchronize(st));
