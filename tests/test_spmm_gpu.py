@@ -301,8 +301,8 @@ def test_table_of_hot_rows(cuda_device, oracle, f):
 @pytest.mark.parametrize("f,lead,shift", [(41, 41, 0), (47, 47, 0), (33, 36, 0), (32, 40, 1), (64, 72, 3), (125, 125, 0), (9, 11, 2)])
 def test_rows_that_do_not_start_on_16_bytes(cuda_device, oracle, f, lead, shift):
     """Operands whose rows cannot be read 16 bytes at a time (odd widths, odd leading dimensions, a view that starts
-    inside a row), without and with the padded staging of drone_plan_reserve: both against the double oracle, each
-    repeatable bit for bit, nothing written outside the result's rows, and a row that is never gathered may hold NaN
+    inside a row), without and with the reservation of padded copies (which a graph this small does not use:
+    test_copied_rows_in_place_and_in_classes has one that does): both against the double oracle, each repeatable bit for bit, nothing written outside the result's rows, and a row that is never gathered may hold NaN
     without leaking into the result."""
     n, u, v = gg.rmat_graph(11, 16, seed=42, symmetrise=False, self_loops="drop")
     u, v = u.numpy(), v.numpy()
@@ -341,7 +341,7 @@ def test_rows_that_do_not_start_on_16_bytes(cuda_device, oracle, f, lead, shift)
 
 
 def test_padded_rows_with_row_classes(cuda_device, oracle):
-    """The padded route computes one row class at a time like the plain one: other rows of Y stay as they are."""
+    """With padded copies reserved, one row class at a time is computed like the whole: other rows of Y stay as they are."""
     n, u, v = gg.rmat_graph(11, 16, seed=43, symmetrise=False, self_loops="add")
     index, dst, in_deg, out_deg, val = graph_case(gg, oracle, n, u.numpy(), v.numpy())
     plan = make_plan(cuda_device, index, dst, in_deg, out_deg)
@@ -584,9 +584,9 @@ def test_one_launch_and_separate_kernels(cuda_device, oracle, f):
 
 @pytest.mark.parametrize("f", [5, 13, 41, 62, 100, 127, 255, 383, 511, 1021])
 def test_copied_and_uncopied_rows_have_the_same_bits(cuda_device, oracle, f):
-    """Rows that cannot be read 16 bytes at a time, through the padded copy (drone_spmm on a plan that is not small) and
-    float by float (a small plan; the entry point that may not allocate, on a plan that has no copy yet): one order of
-    additions, so the same bits."""
+    """Rows that cannot be read 16 bytes at a time, by the route drone_spmm takes (a padded copy at the widths above 384, float
+    by float otherwise) and by the entry point that may not allocate, on a plan that has no copy yet: one order of additions,
+    so the same bits, in one launch and in separate kernels."""
     import ctypes as C
     n, u, v = gg.rmat_graph(10, 16, seed=62, symmetrise=False, self_loops="add")
     index, dst, in_deg, out_deg, val = graph_case(gg, oracle, n, u.numpy(), v.numpy())
@@ -732,3 +732,55 @@ def test_copies_that_do_not_fit(cuda_device):
     plan.reserve(f, padded_rows=True)
     assert call(x, out) == uncopied + 2
     assert torch.equal(out.cpu(), first)
+
+
+@pytest.mark.parametrize("f,lead,shift", [(41, 41, 0), (47, 52, 0), (64, 72, 3), (30, 31, 0), (44, 45, 0)])
+def test_copied_rows_in_place_and_in_classes(cuda_device, f, lead, shift):
+    """The padded copies on a graph that uses them: odd widths, odd leading dimensions, views that start inside a row, only one
+    of the operands unaligned; whole and one row class at a time.  Bit for bit what the same call on aligned operands, or
+    float by float, gives; nothing outside the result's rows is written, and a row that nobody gathers may hold NaN."""
+    n = 30000
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(90 + f)
+    h = torch.unique(torch.randint(0, n * n, (n * 40,), device=cuda_device, generator=gen))
+    u, v = (h // n).to(torch.int32), (h % n).to(torch.int32)
+    u, v = u[u != 7], v[u != 7]                           # nobody gathers X[7]
+    index, dst = gg.csr_by_source(u, v, n)
+    in_deg, out_deg = (d.clamp_(min=1) for d in gg.degrees(u, v, n))
+
+    def plan_of():
+        return db.AggregationPlan(index, dst, in_degree=in_deg, out_degree=out_deg)
+
+    def unaligned(fill):
+        return torch.full((n + 1, lead + shift), fill, device=cuda_device)[:n, shift:shift + f]
+
+    x = unaligned(0.0)
+    x.copy_(torch.randn((n, f), device=cuda_device, generator=gen))
+    x[7] = float("nan")
+    bare = plan_of()
+    bare.reserve(1024)                                    # reserved without the copies: float by float
+    want = torch.empty((n, f), device=cuda_device)
+    bare.spmm(db.OP_AT, x, out=want)
+    assert torch.isfinite(want).all()
+    plan = plan_of()
+    aligned_x = torch.zeros((n, (f + 3 & ~3) + 4), device=cuda_device)[:, :f]
+    aligned_x.copy_(x)
+    aligned_y = torch.empty_like(aligned_x)
+    # f = 44 and 64 have aligned rows of their own width: only the leading dimension or the start is odd
+    for xs, ys in ((x, unaligned(3.0)), (aligned_x, unaligned(3.0)), (x, aligned_y)):
+        plan.spmm(db.OP_AT, xs, out=ys)
+        assert torch.equal(ys, want)
+        if ys is not aligned_y:
+            whole = ys._base if ys._base is not None else ys
+            whole = whole.clone()
+            whole[:n, shift:shift + f] = 3.0
+            assert (whole == 3.0).all()
+    assert torch.equal(plan.spmm(db.OP_AT, x, relu=True), torch.clamp_min(want, 0.0))
+    cls = (torch.arange(n, device=cuda_device) % 3).to(torch.int32)
+    plan.set_row_classes(cls, 3)
+    y = unaligned(9.0)
+    plan.spmm(db.OP_AT, x, out=y, row_class=1)
+    assert torch.equal(y[cls == 1], want[cls == 1]) and (y[cls != 1] == 9.0).all()
+    for c in (0, 2):
+        plan.spmm(db.OP_AT, x, out=y, row_class=c)
+    assert torch.equal(y, want)
