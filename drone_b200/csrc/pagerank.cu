@@ -241,7 +241,7 @@ __device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R d
 // Bound: one scattered gather per edge.  A load of 32 scattered words from L2 costs the LSU 32 wavefronts whatever
 // its hit rate, which caps the whole part at about 2.9e11 gathers per second; a shared-memory load of 32 scattered
 // words costs 3 to 4.  So every block first copies the most gathered part of the array (a prefix, see `place`) into
-// shared memory and gathers from global memory only what lies behind it (R-MAT-22: 59 % of the gathers hit 51,200
+// shared memory and gathers from global memory only what lies behind it (R-MAT-22: 56 % of the gathers hit 40,960
 // floats).  Measured, R-MAT-22 float: 0.323 -> 0.256 ms per power iteration.
 //
 // `table`: the first p.table_n published values, in shared memory.  `warp` of `n_warps`: this warp's share of the work.
@@ -294,8 +294,8 @@ __device__ __forceinline__ void load_table(const PartView<R> &p, R *table) {
 }
 
 // Split rows: the warps note the slots they filled and, 32 chunks at a time, make them visible with one fence and count
-// them in; the warp that counts in a row's last slot adds the row's slots, in slot order.  (A fence per chunk was 11 %
-// of the stall cycles of the whole kernel.)  `slot`: lane l's l-th noted slot, -1 for none.
+// them in; the warp that counts in a row's last slot adds the row's slots, in slot order.  (Waiting at fences is 1.4 %
+// of the stall cycles this way; with a fence per chunk it was 11 %.)  `slot`: lane l's l-th noted slot, -1 for none.
 template <typename R, bool FLAGS>
 __device__ __forceinline__ void close_slots(const PartView<R> &p, int slot) {
     const int lane = threadIdx.x & 31;

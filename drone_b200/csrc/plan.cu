@@ -799,14 +799,14 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
         DRONE_CUDA(cudaStreamSynchronize(st));
     }
     // Table of hot rows: only for graphs whose dense operand is far larger than L2 at the usual widths (at least
-    // DRONE_HOT_MIN_ROWS rows, default 2^23: measured on R-MAT graphs with 32 features, the table gains 10 % at 2^26
-    // rows and loses 10 % at 2^22, where most gathers hit L2 anyway).  Its size is DRONE_HOT_TABLE_MB (default 64;
-    // 0 switches it off); a position is tagged for as many rows as fit at a width of 32 floats, calls with wider rows
-    // use a prefix of the positions.
+    // DRONE_HOT_MIN_ROWS rows, default 2^24; ms a call without / with it, R-MAT directed + I, F = 32, plain and value-free: 2^22 rows
+    // 0.85 / 0.95 and 0.85 / 0.99, 2^23 1.91 / 2.05 and 1.86 / 2.06, 2^24 4.35 / 4.26 and 4.14 / 4.26, 2^26 plain 10 % less with it).
+    // Its size is DRONE_HOT_TABLE_MB (default 64; 0 switches it off); a position is tagged for as many rows as fit at a width of 32
+    // floats, calls with wider rows use a prefix of the positions.
     {
         const char *mb = getenv("DRONE_HOT_TABLE_MB");
         const long long table_mb = (mb && *mb) ? atoll(mb) : 64;
-        const int min_rows = env_int("DRONE_HOT_MIN_ROWS", 1 << 23);
+        const int min_rows = env_int("DRONE_HOT_MIN_ROWS", 1 << 24);
         long long n_hot = table_mb * (1LL << 20) / 128;
         if (n_hot > n_rows / 4) n_hot = n_rows / 4;
         if (for_spmm && table_mb > 0 && n_rows >= min_rows && n_rows < (1 << 29) && nnz > 0 && n_hot > 0) {
