@@ -11,8 +11,10 @@ namespace drone {
 // 6.4 | 7.9 | 8.5 | 12.6 M nonzeros: F = 16 0.74 | 0.96 | 0.95 | 1.07 | 1.16, F = 64 0.81 | 0.97 | 1.00 | 1.08 | 1.05, F = 256
 // 0.71 | 1.01 | 0.93 | 0.88 | 1.02; F = 4 still 0.91 at 12.6 M).
 constexpr int kSmallNnz = 6 << 20;
-// Of those, lanes with 8 or 12, 16, and 32 single floats of a row keep few warps resident, so that one launch covers less.
-constexpr int small_nnz_floats(int VPL) { return VPL < 8 ? 0x7fffffff : VPL < 16 ? 3 << 20 : VPL < 32 ? 1 << 17 : 1 << 15; }
+// Of those, lanes with 8, 12, 16, and 32 single floats of a row keep few warps resident, so that one launch covers less.
+constexpr int small_nnz_floats(int VPL) {
+    return VPL < 8 ? 0x7fffffff : VPL == 8 ? 5 << 20 : VPL < 16 ? 3 << 20 : VPL < 32 ? 1 << 17 : 1 << 15;
+}
 constexpr int kWideSlots = 64;              // split rows above this many partial slots are reduced by a whole block
 constexpr int kShortRangeNnz = 64;          // stream entries per lane group (plus at most one more row) ...
 // ... and in small plans, where one group's walk is the length of the call, as long as the stream's entries times the lanes of

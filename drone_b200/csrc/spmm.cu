@@ -130,8 +130,8 @@ static int replace_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
 //   F = 13, 270,000 rows of 9, 17, 33: 57 / 52, 94 / 76, 139 / 113; F = 63, rows of 33: 40,000 52 / 52, 250,000 266 / 239;
 //   Reddit-shaped (491 a row), F = 41: 2410 / 1512; R-MAT-22 (17 a row), F = 41: 1710 / 2175.
 //   F = 95 and 127, rows of 33: 90,000 122 / 149 and 130 / 159, 250,000 (above kSmallNnz) 440 / 408 and 543 / 493.
-//   F = 131 and 255: in one launch 40,000 rows of 13 52 / 66 and 58 / 82, 30,000 rows of 41 89 / 111 and 99 / 115; in separate kernels
-//   60,000 rows of 61 252 / 304 and 326 / 310; above kSmallNnz (130,000 rows of 61) 514 / 482 and 952 / 824.
+//   F = 131 and 255: in one launch 40,000 rows of 13 52 / 66 and 58 / 82, 30,000 rows of 41 89 / 111 and 99 / 115,
+//   60,000 rows of 61 252 / 304 and 308 / 310; above kSmallNnz (130,000 rows of 61) 514 / 482 and 952 / 824.
 //   F = 301, rows of 81: 10,000 (one launch) 82 / 101, 60,000 561 / 534.  F = 401, 10,000 rows of 13 (one launch) and 19: 39 / 47
 //   and 79 / 54.  F = 511, 60,000 rows of 41 and 81: 531 / 486 and 1050 / 755.  F = 601, rows of 81: 60,000 3301 / 4111, 90,000
 //   4961 / 2536.
@@ -142,10 +142,11 @@ static bool worth_copying(const drone_plan *p, int F) {
     if (F <= 64) return p->nnz >= 1 << 20 && per_row >= (F <= 32 ? 16 : 32);
     if (F <= 128) return many && per_row >= 32;
     const bool whole_steps = ((F + 3) & ~3) % 128 == 0;
-    if (F <= 384 && p->nnz <= small_nnz_floats(8)) return whole_steps && F <= 256 && per_row >= 60;
+    if (F <= 256 && !many) return whole_steps && per_row >= 60;
+    if (F <= 384 && p->nnz <= small_nnz_floats(12)) return false;
     if (F <= 512 && p->nnz <= small_nnz_floats(16)) return false;
     if (whole_steps && per_row >= 60) return true;
-    if (per_row >= 64) return many || bytes <= 30e6 || (F > 256 && (F <= 512 || bytes <= 100e6));
+    if (per_row >= 64) return many || F <= 512 || bytes <= 100e6;
     return F > 384 && per_row >= 12 && bytes <= 40e6;
 }
 

@@ -824,16 +824,19 @@ static int launch_all(const SpmmArgs &a) {
     constexpr int RPW = 32 / G;
     const Side &s = *a.side;
     int range_lo, n_ranges, chunk_lo, n_chunks, split_lo, n_split, wide_lo, n_wide;
-    const bool fine = s.fine.row != nullptr && (G <= 2 || (long long)s.n_short_entries * G < kFineRangeLanes);
+    // Odd widths above 128, one launch / separate kernels, us, power law: F = 131 30,000 rows of 41 89 / 136, 130,000 of 25 261 / 305,
+    // of 41 394 / 374, 60,000 of 61 252 / 253; F = 301 60,000 of 41 308 / 336, 130,000 of 25 624 / 606; F = 401 10,000 of 13 39 / 42,
+    // 30,000 of 13 87 / 80; F = 601 3,000 of 13 32 / 47, 30,000 of 13 224 / 210.
+    const bool one_launch = s.small && (VEC == 4 || a.nnz <= small_nnz_floats(VPL));
+    // (Above 512 single floats the line of the separate kernels lies lower; ranges of 16 / 64, us, F = 601: 28,000 rows of 4 62 / 65,
+    // 20,000 rows of 7 81 / 74.)
+    const long long fine_lanes = one_launch || VPL < 32 ? kFineRangeLanes : 4LL << 20;
+    const bool fine = s.fine.row != nullptr && (G <= 2 || (long long)s.n_short_entries * G < fine_lanes);
     const Ranges &ranges = fine ? s.fine : s.ranges;
     class_range(a.row_class, s.n_classes, ranges.start, &range_lo, &n_ranges);
     class_range(a.row_class, s.n_classes, s.chunk_start, &chunk_lo, &n_chunks);
     class_range(a.row_class, s.n_classes, s.split_start, &split_lo, &n_split);
     class_range(a.row_class, s.n_classes, s.wide_start, &wide_lo, &n_wide);
-    // Odd widths above 128, one launch / separate kernels, us, power law: F = 131 30,000 rows of 41 89 / 136, 130,000 of 25 261 / 305,
-    // of 41 394 / 374; F = 301 60,000 of 41 308 / 336, 130,000 of 25 624 / 606; F = 401 10,000 of 13 39 / 42, 30,000 of 13 87 / 80; F = 601
-    // 3,000 of 13 32 / 47, 30,000 of 13 224 / 210.
-    const bool one_launch = s.small && (VEC == 4 || a.nnz <= small_nnz_floats(VPL));
     if (!HOT && one_launch) {
         const int chunk_blocks = ceil_div(n_chunks, 8), short_blocks = ceil_div(n_ranges, 8 * RPW);
         if (chunk_blocks + short_blocks == 0) return DRONE_OK;

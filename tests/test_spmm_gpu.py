@@ -629,7 +629,7 @@ def test_larger_one_launch_plans(cuda_device, oracle, n, per_row, f):
 
 
 @pytest.mark.parametrize("n,per_row,f,copied", [(40000, 12, 131, False), (30000, 40, 131, False), (40000, 70, 255, True), (40000, 70, 383, False),
-                                                (40000, 80, 129, True), (45000, 80, 257, True), (50000, 75, 161, False),
+                                                (40000, 80, 129, False), (80000, 80, 129, True), (45000, 80, 257, True), (50000, 75, 161, False),
                                                 (60000, 62, 253, True), (50000, 70, 253, True), (40000, 33, 95, False),
                                                 (40000, 33, 63, True), (10000, 20, 383, False), (10000, 20, 401, True), (6000, 20, 401, False),
                                                 (9000, 10, 513, False), (210000, 33, 65, True), (210000, 31, 129, False)])
