@@ -41,6 +41,7 @@ struct drone_pr {
     drone_comm *comm = nullptr;       // borrowed (may be NULL for a single part)
     int *out_degree = nullptr, *mirror2worker = nullptr;
     void *pr = nullptr, *acc = nullptr, *diff = nullptr, *push = nullptr;   // real[n] each
+    void *push2 = nullptr;            // real[n] sums of a stream's rows
     // Where vertex i publishes its delta.  The deltas lie in the order of how often they are gathered (most gathered
     // first) and the pull lists' columns are renumbered to match, so that a prefix of the array, small enough for
     // shared memory, serves most gathers.  NULL (few vertices): delta i lies at i.
@@ -59,7 +60,11 @@ struct drone_pr {
     std::vector<unsigned long long> pairs_for;
     unsigned char *shared = nullptr;  // [n_local] 1 for rows that other parts hold too
     char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
-    drone::DeviceBlock block;                // what the arrays made at creation are pieces of
+    drone::RowStream stream;                 // one part too large for slices: its rows in the order of place
+    int *stream_od = nullptr;
+    void *stream_tails = nullptr;
+    drone::DeviceBlock stream_block;         // what the stream's arrays are pieces of
+    drone::DeviceBlock block;                // what the other arrays made at creation are pieces of
     int sms = 0;
     bool separate_steps = false;      // parts in one process take the kernels of one process per GPU (local_parts_run_separately)
     unsigned barrier_start = 0, barrier_polls = 0;   // what the grid barrier's count starts at, and when its waits run out
@@ -940,6 +945,12 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
     if (blockIdx.x == 0 && threadIdx.x == 0) a.control->t_end = now_ns();
 }
 
+}  // namespace drone
+
+#include "pagerank_stream.cuh"
+
+namespace drone {
+
 // pairs[k] = {part, row} (and targets[k] = {place, out degree} of that row) behind position m_pos[k] of part q's receive
 // buffer: peer p's entries start at down_off[p] there and are, in the same order, peer p's up list for q.
 struct PeerLists {
@@ -976,6 +987,7 @@ static inline int grid1d(long long n, int cap = 148 * 16) {
 // Fewer vertices than this lie in local-id order: all their published values fit the table in either type, so ordering
 // them by how often they are gathered (a sort at creation) would gain nothing.
 constexpr long long kOrderMinRows = 16 << 10;
+constexpr long long kStreamEdges = 20000;      // edges per SM from which a part's power iterations take the stream
 constexpr int kTableBytes = 160 * 1024;        // shared memory for the table; the rest of the SM serves as L1, whose lines are
                                                // what gathers in flight wait in (R-MAT-22: 5.3 ms with 64 to 160 KB, 7.0 with 200)
 
@@ -1325,6 +1337,15 @@ static int prepare_pairs(std::vector<drone_pr *> &parts, cudaStream_t st) {
     return DRONE_OK;
 }
 
+// Number of a launch in the process, never 0.
+static unsigned next_run() {
+    static std::atomic<unsigned> runs{0};
+    unsigned run;
+    do run = ++runs;
+    while (run == 0);
+    return run;
+}
+
 // What one persistent launch is asked to do.
 struct RunRequest {
     bool job = false;              // supersteps of the job; otherwise the power iteration
@@ -1365,9 +1386,7 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     }
     a.block_sums = (R *)lead->block_sums;
     a.control = (RunControl *)lead->control;
-    static std::atomic<unsigned> runs{0};
-    do a.run = ++runs;
-    while (a.run == 0);
+    a.run = next_run();
     a.barrier_start = lead->barrier_start;
     a.barrier_polls = lead->barrier_polls;
     a.history = (int *)(lead->control + sizeof(RunControl));
@@ -1394,11 +1413,42 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     return DRONE_OK;
 }
 
+template <typename R>
+static int launch_stream(drone_pr *p, const RunRequest &rq, cudaStream_t st) {
+    StreamArgs<R> a;
+    a.part = part_view<R>(p, p->sms);
+    a.part.table_n = std::min<int>(a.part.table_n, kStreamTableBytes / (int)sizeof(R));
+    a.rows = p->stream;
+    a.od = p->stream_od;
+    a.sum = (R *)p->push2;
+    a.tails = (R *)p->stream_tails;
+    a.block_sums = (R *)p->block_sums;
+    a.control = (RunControl *)p->control;
+    a.barrier_start = p->barrier_start;
+    a.barrier_polls = p->barrier_polls;
+    a.run = p->run = next_run();
+    a.damping = (R)rq.damping;
+    a.iterations = rq.iterations;
+    a.n_isolated = p->n_isolated;
+    p->started = false;
+    DRONE_CUDA(cudaMemsetAsync(p->control, 0, sizeof(RunControl), st));
+    if (p->barrier_start != 0)
+        DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &p->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
+    const int rc = allow_table(pr_stream_kernel<R>);
+    if (rc) return rc;
+    void *args[] = {&a};
+    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)pr_stream_kernel<R>, dim3(p->sms), dim3(stream_threads<R>()), args,
+                                           (size_t)a.part.table_n * sizeof(R), st));
+    count_launch();
+    return DRONE_OK;
+}
+
 static int run_local(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaStream_t st) {
     const drone_pr *lead = parts[0];
     const int rc = prepare_pairs(parts, st);
     if (rc) return rc;
     const bool few = parts.size() <= 8;
+    if (!rq.job && lead->stream.col) return lead->dbl ? launch_stream<double>(parts[0], rq, st) : launch_stream<float>(parts[0], rq, st);
     if (lead->dbl) {
         if (rq.job) return few ? launch_run<double, 8, true>(parts, rq, st) : launch_run<double, kMaxLocalParts, true>(parts, rq, st);
         if (parts.size() == 1) return launch_run<double, 1, false>(parts, rq, st);
@@ -1523,6 +1573,7 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         p->block.add(&p->acc, rs * n1);
         p->block.add(&p->diff, rs * n1);
         p->block.add(&p->push, rs * n1);
+        p->block.add(&p->push2, rs * n1);
         p->block.add(&p->active, sizeof(int) * n1);
         p->block.add(&p->ubm, sizeof(int) * n1);
         p->block.add(&p->scalars, 8 * 4);
@@ -1557,6 +1608,16 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
             if (e == cudaSuccess) e = cudaMemcpy(p->mirror2worker, d_mirror2worker, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
             if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: copy failed: %s", cudaGetErrorString(e)); break; }
         }
+        // one part of many edges: as one stream
+        if (xplan->nranks == 1 && p->place && nnz > 0 && (long long)nnz > (long long)p->sms * kStreamEdges) {
+            p->stream_block.add(&p->stream_od, sizeof(int) * n1);
+            const int warps = p->sms * (p->dbl ? stream_threads<double>() : stream_threads<float>()) / 32;
+            p->stream_block.add(&p->stream_tails, rs * 4 * (size_t)warps);      // a piece each
+            if ((rc = plan_rows_in_order(p->plan, DRONE_OP_AT, p->place, warps, &p->stream, &p->stream_block, nullptr))) break;
+            pr_stream_degrees_kernel<<<grid1d(n_local), 256>>>(p->stream.row_of, p->out_degree, p->mirror2worker, n_local, p->stream_od);
+            count_launch();
+            if ((e = cudaDeviceSynchronize()) != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: %s", cudaGetErrorString(e)); break; }
+        }
     } while (0);
     if (rc) {
         drone_pr_destroy(p);
@@ -1574,6 +1635,7 @@ int drone_pr_destroy(drone_pr *p) {
     drone_plan_destroy(p->plan);
     cudaFree(p->place);
     p->block.release();
+    p->stream_block.release();
     if (prev >= 0) cudaSetDevice(prev);
     delete p;
     return DRONE_OK;

@@ -878,6 +878,88 @@ int plan_order_columns_by_frequency(drone_plan *p, int orientation, const int *d
     t.place = nullptr;
     return DRONE_OK;
 }
+
+// lengths[i] = edges of the row at position i, filled[i] = 1 where there are any (both 0 at i = n)
+__global__ void ordered_lengths_kernel(const int *__restrict__ rowptr, const int *__restrict__ row_of, int n, int *lengths, int *filled) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+        const int r = i < n ? row_of[i] : 0, d = i < n ? rowptr[r + 1] - rowptr[r] : 0;
+        lengths[i] = d;
+        filled[i] = d > 0;
+    }
+}
+
+// at[i], from the number of rows with edges before position i
+__global__ void ordered_at_kernel(const RowStream s, const int *__restrict__ filled_before, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int b = s.ptr[i], e = s.ptr[i + 1];
+        s.at[i] = e == b ? -1 : filled_before[i] | (s.piece_of(b) != s.piece_of(e - 1) ? kSpansPieces : 0);
+    }
+}
+
+// A warp copies one row after the other, the last column marked.
+__global__ void ordered_columns_kernel(const int *__restrict__ rowptr, const int *__restrict__ col, const int *__restrict__ row_of,
+                                       const int *__restrict__ ptr, int n, unsigned *__restrict__ out) {
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const int from = rowptr[row_of[i]], to = ptr[i], len = ptr[i + 1] - to;
+        for (int k = lane; k < len; k += 32) out[to + k] = (unsigned)col[from + k] | (k + 1 == len ? kRowEnd : 0u);
+    }
+}
+
+// first[q] = which of the rows with edges the first edge of piece q belongs to
+__global__ void piece_first_kernel(const RowStream s, const int *__restrict__ filled_before, int n) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < s.n_pieces; q += gridDim.x * blockDim.x)
+        s.first[q] = filled_before[row_of(s.ptr, n, s.first_tile(q) * kTileEdges)];
+}
+
+int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place, int warps, RowStream *out, DeviceBlock *block, cudaStream_t st) {
+    const Side &s = p->side[orientation];
+    const int n = p->n_rows, nnz = p->nnz;
+    if (!s.ready || s.hot_ids || nnz == 0) return set_error(DRONE_E_STATE, "plan_rows_in_order: orientation not prepared, tagged, or without edges");
+    RowStream r;
+    r.n_tiles = ceil_div(nnz, kTileEdges);
+    // Equal shares for all warps, of up to four pieces from different parts of the stream: long rows, which come first, are
+    // quicker than short ones (pieces of a fixed 16 tiles left the slowest warp 13 us behind from R-MAT-19 to R-MAT-22).
+    r.n_pieces = std::min(r.n_tiles, warps * std::max(1, std::min(4, r.n_tiles / warps / 16)));
+    const size_t words = sizeof(int) * (size_t)(n + 1), edges = sizeof(int) * (size_t)r.n_tiles * kTileEdges;
+    block->add(&r.ptr, words);
+    block->add(&r.at, words);
+    block->add(&r.row_of, words);
+    block->add(&r.first, sizeof(int) * (size_t)r.n_pieces);
+    block->add(&r.col, edges);
+    DRONE_CUDA(block->make());
+    struct Temp {
+        int *lengths = nullptr, *filled = nullptr, *before = nullptr;
+        void *scan = nullptr;
+        DeviceBlock block;
+        ~Temp() { block.release(); }
+    } t;
+    size_t scan_bytes = 0;
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, t.lengths, r.ptr, n + 1, st));
+    t.block.add(&t.lengths, words);
+    t.block.add(&t.filled, words);
+    t.block.add(&t.before, words);
+    t.block.add(&t.scan, scan_bytes);
+    DRONE_CUDA(t.block.make());
+    scatter_positions_kernel<<<grid_for(n), 256, 0, st>>>(d_place, n, r.row_of);
+    DRONE_LAUNCH_CHECK("scatter_positions_kernel");
+    ordered_lengths_kernel<<<grid_for(n + 1), 256, 0, st>>>(s.rowptr, r.row_of, n, t.lengths, t.filled);
+    DRONE_LAUNCH_CHECK("ordered_lengths_kernel");
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(t.scan, scan_bytes, t.lengths, r.ptr, n + 1, st));
+    DRONE_CUDA(cub::DeviceScan::ExclusiveSum(t.scan, scan_bytes, t.filled, t.before, n + 1, st));
+    count_launch();
+    count_launch();
+    ordered_at_kernel<<<grid_for(n), 256, 0, st>>>(r, t.before, n);
+    DRONE_LAUNCH_CHECK("ordered_at_kernel");
+    piece_first_kernel<<<grid_for(r.n_pieces), 256, 0, st>>>(r, t.before, n);
+    DRONE_LAUNCH_CHECK("piece_first_kernel");
+    DRONE_CUDA(cudaMemsetAsync(r.col + (size_t)(r.n_tiles - 1) * kTileEdges, 0, sizeof(int) * kTileEdges, st));
+    ordered_columns_kernel<<<grid_for((long long)n * 32), 256, 0, st>>>(s.rowptr, s.col, r.row_of, r.ptr, n, r.col);
+    DRONE_LAUNCH_CHECK("ordered_columns_kernel");
+    DRONE_CUDA(cudaStreamSynchronize(st));
+    *out = r;
+    return DRONE_OK;
+}
 }  // namespace drone
 
 using namespace drone;

@@ -117,6 +117,29 @@ int plan_create_untagged(drone_plan **out, int n_rows, int nnz, const int *d_ind
 // the plan's lists means position (*d_place_out)[c], a device array of n_rows ints the caller owns.  For users inside
 // the library whose gathered operand is their own array and can be laid out in that order (the PageRank pull).
 int plan_order_columns_by_frequency(drone_plan *p, int orientation, const int *d_other_rowptr, int **d_place_out, void *stream);
+
+// The rows of one orientation of such a plan in the order of `place` as well, their edges as one stream.  Pieces of it are what
+// warps work on (power iterations on R-MAT-22: see pagerank_stream.cuh).
+constexpr int kTileEdges = 256;                  // what a warp takes at a time
+constexpr unsigned kRowEnd = 0x80000000u;        // flag on a column: last edge of its row
+constexpr int kSpansPieces = 0x40000000;         // flag on `at`: the row begins in an earlier piece than it ends in
+struct RowStream {
+    int *ptr = nullptr;        // [n + 1] first edge of the row at position i
+    int *at = nullptr;         // [n] which of the rows with edges it is, | kSpansPieces; -1: it has none
+    int *row_of = nullptr;     // [n] the row at position i
+    int *first = nullptr;      // [n_pieces] which of the rows with edges a piece's first edge belongs to
+    unsigned *col = nullptr;   // [n_tiles * kTileEdges] columns | kRowEnd; 0 beyond the last edge
+    int n_pieces = 0, n_tiles = 0;
+#ifdef __CUDACC__
+    // Piece q is tiles [first_tile(q), first_tile(q + 1)), one more or less than any other piece; none is empty.
+    __host__ __device__ int first_tile(int q) const { return (int)((long long)n_tiles * q / n_pieces); }
+    __host__ __device__ int piece_of(int edge) const {
+        return (int)(((long long)(edge / kTileEdges + 1) * n_pieces - 1) / n_tiles);
+    }
+#endif
+};
+// Fills in what `out` points to: `block` is made with its arrays.  `warps`: how many will share the pieces.
+int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place, int warps, RowStream *out, DeviceBlock *block, cudaStream_t st);
 }  // namespace drone
 
 struct drone_plan {

@@ -324,3 +324,25 @@ def test_separate_steps_of_one_process_per_gpu(cuda_device, oracle, monkeypatch,
         assert np.max(np.abs(results[1][3][touched] - want[touched]) / np.abs(want[touched])) < PR_TOL
         assert results[0][:3] == results[1][:3]
     assert np.max(np.abs(results[0][3][touched] - results[1][3][touched]) / np.abs(results[0][3][touched])) < (PR_TOL if use_double else 2e-4)
+
+
+@pytest.mark.parametrize("use_double", [False, True])
+@pytest.mark.parametrize("scale,edge_factor", [(18, 24), (18, 96), (20, 8)])
+def test_power_iterations_over_a_stream_of_edges(cuda_device, oracle, scale, edge_factor, use_double):
+    """One part of many edges: rows that several pieces of the stream share, rows without edges, vertices without out-edges;
+    the same bits every time."""
+    n, u, v = gg.rmat_graph(scale, edge_factor, seed=90 + edge_factor, symmetrise=False, self_loops="drop")
+    u, v = u.numpy(), v.numpy()
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 5, 0.85)
+    part = pt.ebv_partition(n, u, v, 1, keep_self_loops=False)
+    graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 0.0)
+    touched = part.replicas > 0
+    runs = []
+    for _ in range(2):
+        prk.power_iterate_local(prs, 5, 0.85)
+        runs.append(prk.gather_global(prs, graphs, n))
+    assert np.max(np.abs(runs[0][touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
+    assert np.array_equal(runs[0], runs[1])
+    prk.power_iterate_local(prs, 0, 0.85)
+    assert np.ptp(prk.gather_global(prs, graphs, n)[touched]) == 0
