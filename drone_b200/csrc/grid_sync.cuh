@@ -28,16 +28,18 @@ inline unsigned barrier_start() {
     return v && *v ? (unsigned)strtoul(v, nullptr, 10) : 0u;
 }
 
-// Every thread of the grid arrives; false when a wait ran out (in some block), then everybody returns.  `phase`: what
-// `arrived` has to reach, at first its start.  The count only grows, so that a barrier is one atomic and one comparison
-// modulo 2^32 (the blocks of a grid are far closer together than 2^31); a count of 64 bits took 0.2 us more per barrier.
-__device__ inline bool grid_barrier(GridBarrier *b, unsigned &phase, unsigned poll_limit) {
+// The two halves of a barrier, for a block with work between them.  One thread of every block arrives, after a block-wide
+// barrier behind what the others are to see; then every thread of the block waits, which is false when a wait ran out (in some
+// block): then everybody returns.  `phase`: what `arrived` has to reach, at first its start.  The count only grows, so that a
+// barrier is one atomic and one comparison modulo 2^32 (the blocks of a grid are far closer together than 2^31); a count of 64
+// bits took 0.2 us more per barrier.
+__device__ inline void grid_arrive(GridBarrier *b) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(&b->arrived) : "memory");
+}
+__device__ inline bool grid_wait(GridBarrier *b, unsigned &phase, unsigned poll_limit) {
     __shared__ int ok;
     phase += gridDim.x;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&b->arrived, 1u);
         int failed = 0;
         for (unsigned polls = 0;; ) {
             unsigned seen;
@@ -50,11 +52,17 @@ __device__ inline bool grid_barrier(GridBarrier *b, unsigned &phase, unsigned po
             if ((int)(seen - phase) >= 0) break;
             if ((++polls & 255u) == 0 && (failed = *(volatile int *)&b->failed) != 0) break;
         }
-        __threadfence();
         ok = failed ? 0 : 1;
     }
     __syncthreads();
     return ok != 0;
+}
+
+// Both at once.
+__device__ inline bool grid_barrier(GridBarrier *b, unsigned &phase, unsigned poll_limit) {
+    __syncthreads();
+    if (threadIdx.x == 0) grid_arrive(b);
+    return grid_wait(b, phase, poll_limit);
 }
 
 }  // namespace drone

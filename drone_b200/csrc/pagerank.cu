@@ -21,6 +21,7 @@
 #include "grid_sync.cuh"
 #include "plan.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstdlib>
@@ -41,7 +42,7 @@ struct drone_pr {
     drone_comm *comm = nullptr;       // borrowed (may be NULL for a single part)
     int *out_degree = nullptr, *mirror2worker = nullptr;
     void *pr = nullptr, *acc = nullptr, *diff = nullptr, *push = nullptr;   // real[n] each
-    void *push2 = nullptr;            // real[n] sums of a stream's rows
+    void *push2 = nullptr;            // real[n] second buffer of the published values (pr_resident_kernel)
     // Where vertex i publishes its delta.  The deltas lie in the order of how often they are gathered (most gathered
     // first) and the pull lists' columns are renumbered to match, so that a prefix of the array, small enough for
     // shared memory, serves most gathers.  NULL (few vertices): delta i lies at i.
@@ -58,7 +59,9 @@ struct drone_pr {
     // degree} of that row in its part, and the plans these were filled in for
     int2 *pairs = nullptr, *targets = nullptr;
     std::vector<unsigned long long> pairs_for;
-    unsigned char *shared = nullptr;  // [n_local] 1 for rows that other parts hold too
+    int *role = nullptr;              // [n_local] kOwnRow, kMirrorRow, or the number of the master row
+    // [b - 1]: {rows, edges} of the largest slice when this part's rows are dealt to b blocks; empty: too large for that
+    std::vector<int2> slices;
     char *control = nullptr;          // RunControl + superstep counts of the persistent kernel (part 0 of a run)
     drone::RowStream stream;                 // one part too large for slices: its rows in the order of place
     int *stream_od = nullptr;
@@ -94,6 +97,8 @@ __device__ __forceinline__ bool is_pushed(float v) { return __float_as_uint(v) !
 __device__ __forceinline__ bool is_pushed(double v) { return __double_as_longlong(v) != (long long)0x8000000000000000ULL; }
 template <typename R> __device__ __forceinline__ R not_pushed() { return (R)-0.0; }
 
+constexpr int kOwnRow = -1, kMirrorRow = -2;      // roles of a row that no other part holds, and of one whose master is elsewhere
+
 // Device view of one part.
 template <typename R>
 struct PartView {
@@ -110,7 +115,9 @@ struct PartView {
     const int *m_rows, *m_off;
     const int2 *pairs, *targets;
     unsigned *unfinished;
-    const unsigned char *shared;           // power iteration over several parts: 1 where the vertex is on others too
+    const int *rowptr;
+    R *push2;
+    const int *role;                       // runs over several parts: kOwnRow, kMirrorRow, or the number of the master row
 };
 
 // Sum of v over the block in a fixed order (tree over warps), result in thread 0.
@@ -207,7 +214,7 @@ __device__ __forceinline__ R increment_vertices(const PartView<R> &p, R eps, R g
 
 // pr' = (1-d)/V + d * (sum over in-edges + dangling/V), published as pr'/outDegree for the next iteration; after the
 // last one (`last`) the value itself is stored instead: before that nobody can see it.  Leaves out the vertices that
-// p.shared marks (SHARED).
+// other parts hold too (SHARED).
 template <typename R, bool SHARED>
 __device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R dang, bool last, int first, int stride) {
     const R base = ((R)1 - damping) / p.global_v;
@@ -220,7 +227,7 @@ __device__ __forceinline__ R power_vertices(const PartView<R> &p, R damping, R d
 #pragma unroll
         for (int b = 0; b < kVertexBatch; ++b) {
             const int i = i0 + b * stride;
-            skip[b] = i >= p.n ? 1 : SHARED ? (int)__ldg(p.shared + i) : 0;
+            skip[b] = i >= p.n ? 1 : SHARED && p.role ? __ldg(p.role + i) != kOwnRow : 0;
             d[b] = i < p.n ? p.diff[i] : (R)0;
             od[b] = i < p.n && !last ? __ldg(p.out_degree + i) : 1;
             at[b] = i < p.n && !last && p.place ? __ldg(p.place + i) : i;
@@ -711,7 +718,7 @@ __device__ __forceinline__ void note_moved(unsigned *moved, int *counts, int q, 
 // The other parts' arrays, by part.
 template <typename R, int MAXP>
 struct PartArrays {
-    R *diff[MAXP], *push[MAXP], *pr[MAXP];
+    R *diff[MAXP], *push[MAXP], *pr[MAXP], *acc[MAXP];
     int *active[MAXP], *ubm[MAXP];
 };
 
@@ -947,6 +954,7 @@ __global__ void __launch_bounds__(THREADS, 1) pr_run_kernel(const __grid_constan
 
 }  // namespace drone
 
+#include "pagerank_resident.cuh"
 #include "pagerank_stream.cuh"
 
 namespace drone {
@@ -971,8 +979,9 @@ __global__ void pr_pairs_kernel(const int *__restrict__ m_pos, int n, const __gr
     }
 }
 
-__global__ void pr_mark_rows_kernel(const int *__restrict__ rows, int n, unsigned char *mark) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) mark[rows[i]] = 1;
+// role[rows[i]]: that of a mirror, or the row's number in the list of masters.
+__global__ void pr_roles_kernel(const int *__restrict__ rows, int n, bool masters, int *role) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) role[rows[i]] = masters ? i : kMirrorRow;
 }
 
 // ---- host side ----
@@ -987,7 +996,6 @@ static inline int grid1d(long long n, int cap = 148 * 16) {
 // Fewer vertices than this lie in local-id order: all their published values fit the table in either type, so ordering
 // them by how often they are gathered (a sort at creation) would gain nothing.
 constexpr long long kOrderMinRows = 16 << 10;
-constexpr long long kStreamEdges = 20000;      // edges per SM from which a part's power iterations take the stream
 constexpr int kTableBytes = 160 * 1024;        // shared memory for the table; the rest of the SM serves as L1, whose lines are
                                                // what gathers in flight wait in (R-MAT-22: 5.3 ms with 64 to 160 KB, 7.0 with 200)
 
@@ -1029,7 +1037,9 @@ static PartView<R> part_view(const drone_pr *p, int blocks) {
     v.pairs = p->pairs;
     v.targets = p->targets;
     v.unfinished = p->unfinished;
-    v.shared = nullptr;
+    v.rowptr = s.rowptr;
+    v.push2 = (R *)p->push2;
+    v.role = p->role;
     const long long capacity = kTableBytes / (long long)sizeof(R);
     long long t = std::min<long long>(capacity, p->n_local);
     if (!p->place && p->n_local > capacity) t = 0;
@@ -1321,15 +1331,15 @@ static int prepare_pairs(std::vector<drone_pr *> &parts, cudaStream_t st) {
             DRONE_LAUNCH_CHECK("pr_pairs_kernel");
         }
         if (me->n_local > 0) {
-            DRONE_CUDA(cudaMemsetAsync(me->shared, 0, (size_t)me->n_local, st));
+            DRONE_CUDA(cudaMemsetAsync(me->role, 0xff, sizeof(int) * (size_t)me->n_local, st));      // kOwnRow
             const int up = (int)x->up_rows.size(), masters = (int)x->m_rows.size();
             if (up > 0) {
-                pr_mark_rows_kernel<<<grid1d(up), 256, 0, st>>>(x->d_up_rows, up, me->shared);
-                DRONE_LAUNCH_CHECK("pr_mark_rows_kernel");
+                pr_roles_kernel<<<grid1d(up), 256, 0, st>>>(x->d_up_rows, up, false, me->role);
+                DRONE_LAUNCH_CHECK("pr_roles_kernel");
             }
             if (masters > 0) {
-                pr_mark_rows_kernel<<<grid1d(masters), 256, 0, st>>>(x->d_m_rows, masters, me->shared);
-                DRONE_LAUNCH_CHECK("pr_mark_rows_kernel");
+                pr_roles_kernel<<<grid1d(masters), 256, 0, st>>>(x->d_m_rows, masters, true, me->role);
+                DRONE_LAUNCH_CHECK("pr_roles_kernel");
             }
         }
         me->pairs_for = key;
@@ -1355,14 +1365,56 @@ struct RunRequest {
     double damping = 0;
 };
 
+// Whether the parts' edges and rows fit the shared memory of the blocks they are dealt to, and how that is divided.  The table
+// takes what is left, up to a value for every 8 bytes of which a block has an edge; with less than a quarter of that the kernel
+// that leaves the columns in global memory has the better table.
+constexpr size_t kSliceBytes = 216 * 1024;
+constexpr long long kSliceEdges = kSliceBytes / sizeof(unsigned);      // more edges per SM than this never fit
+
+static bool all_values_or_order(const drone_pr *p, size_t value) { return p->place || p->n_local <= kTableBytes / (int)value; }
+
+static bool slices_fit(int n_parts, drone_pr *const *parts, const int *first_block, size_t value, bool job, SliceRoom *room, size_t *bytes) {
+    *room = SliceRoom{0, 0, 0};
+    long long table = 0;
+    for (int q = 0; q < n_parts; ++q) {
+        const drone_pr *p = parts[q];
+        const int blocks = first_block[q + 1] - first_block[q];
+        if (p->n_local == 0 || blocks > (int)p->slices.size()) return false;
+        const int2 most = p->slices[blocks - 1];
+        room->rows = std::max(room->rows, (most.x + 3) & ~3);
+        room->edges = std::max(room->edges, most.y);
+        if (!all_values_or_order(p, value)) continue;
+        const long long worth = (long long)p->nnz / blocks * 8 / (long long)value;
+        table = std::max(table, std::min<long long>(worth, std::min<long long>(kTableBytes / (long long)value, p->n_local)));
+    }
+    const size_t used = slice_row_bytes(value, job, n_parts > 1) * (size_t)room->rows + sizeof(unsigned) * (size_t)room->edges;
+    if (used > kSliceBytes) return false;
+    const long long left = (long long)((kSliceBytes - used) / value) & ~3LL;
+    if (left < table / 4) return false;
+    room->table = (int)std::min<long long>((table + 3) & ~3LL, left);
+    *bytes = used + value * (size_t)room->table;
+    return true;
+}
+
+// A block has at least about 1024 edges and vertices to work through; more blocks only make the barriers longer.
+static int run_blocks(long long edges, int n_parts, int sms) {
+    return std::max(n_parts, (int)std::min<long long>(sms, (edges + 1023) / 1024));
+}
+
+static bool slices_fit_alone(drone_pr *p) {
+    const int first_block[2] = {0, run_blocks((long long)p->nnz + p->n_local, 1, p->sms)};
+    SliceRoom room;
+    size_t bytes = 0;
+    return slices_fit(1, &p, first_block, p->dbl ? 8 : 4, false, &room, &bytes);
+}
+
 template <typename R, int MAXP, bool JOB>
 static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaStream_t st) {
     const int P = (int)parts.size();
     drone_pr *lead = parts[0];
     long long edges = 0;
     for (drone_pr *p : parts) edges += (long long)p->nnz + p->n_local;
-    // A block has at least about 2048 edges and vertices to work through; more blocks only make the barriers longer.
-    const int grid = std::max(P, (int)std::min<long long>(lead->sms, (edges + 2047) / 2048));
+    const int grid = run_blocks(edges, P, lead->sms);
     // More warps hide more of a chunk's latencies (R-MAT-22: 6.5 ms with 512 threads, 5.3 with 768); fewer meet sooner at
     // a barrier and have the registers for more gathers each (R-MAT-16, two parts: 0.40 against 0.46 ms).
     const int threads = edges / grid > 32768 ? kPullThreads : 512;
@@ -1381,7 +1433,6 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     size_t table = 0;
     for (int q = 0; q < P; ++q) {
         a.part[q] = part_view<R>(parts[q], a.first_block[q + 1] - a.first_block[q]);
-        a.part[q].shared = parts[q]->shared;
         table = std::max(table, (size_t)a.part[q].table_n * sizeof(R));
     }
     a.block_sums = (R *)lead->block_sums;
@@ -1400,11 +1451,23 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
     DRONE_CUDA(cudaMemsetAsync(lead->control, 0, sizeof(RunControl) + (JOB ? sizeof(int) * 4 * (size_t)P * rq.max_steps : 0), st));
     if (lead->barrier_start != 0)
         DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &lead->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
-    auto kernel = threads == 512 ? pr_run_kernel<R, MAXP, JOB, 512> : pr_run_kernel<R, MAXP, JOB, kPullThreads>;
-    const int rc = allow_table(kernel);
-    if (rc) return rc;
-    void *args[] = {&a};
-    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(threads), args, table, st));
+    SliceRoom room;
+    size_t bytes = 0;
+    if (slices_fit(P, parts.data(), a.first_block, sizeof(R), JOB, &room, &bytes)) {
+        for (int q = 0; q < P; ++q) a.part[q].table_n = all_values_or_order(parts[q], sizeof(R)) ? std::min(room.table, parts[q]->n_local) : 0;
+        auto kernel = pr_resident_kernel<R, MAXP, JOB>;
+        DRONE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSliceBytes));
+        void *args[] = {&a, &room};
+        DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(kSliceThreads), args, bytes, st));
+    } else if constexpr (MAXP == 1) {
+        return launch_run<R, 8, JOB>(parts, rq, st);      // few vertices with very many edges, in no order (part_view)
+    } else {
+        auto kernel = threads == 512 ? pr_run_kernel<R, MAXP, JOB, 512> : pr_run_kernel<R, MAXP, JOB, kPullThreads>;
+        const int rc = allow_table(kernel);
+        if (rc) return rc;
+        void *args[] = {&a};
+        DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(threads), args, table, st));
+    }
     count_launch();
     for (drone_pr *p : parts) {
         p->started = JOB;
@@ -1590,7 +1653,7 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         if (xplan->nranks > 1 && xplan->nranks <= kMaxLocalParts) {      // for runs over all parts in one process
             p->block.add(&p->pairs, sizeof(int2) * xplan->m_pos.size());
             p->block.add(&p->targets, sizeof(int2) * xplan->m_pos.size());
-            p->block.add(&p->shared, n1);
+            p->block.add(&p->role, sizeof(int) * n1);
         }
         const size_t control_bytes = sizeof(RunControl) + sizeof(int) * 4 * (size_t)xplan->nranks * kHistorySteps;
         p->block.add(&p->control, control_bytes);
@@ -1603,13 +1666,22 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
             if (e == cudaSuccess && (rc = fill_slot_split(side, p->slot_split, nullptr))) break;
         }
         if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: cudaMalloc failed: %s", cudaGetErrorString(e)); break; }
+        // how large the blocks' slices would be, for the runs that keep them in shared memory (DRONE_PR_SLICES=0: none do)
+        const char *slices = getenv("DRONE_PR_SLICES");
+        if (e == cudaSuccess && n_local > 0 && !(slices && slices[0] == '0') && (xplan->nranks == 1 || !comm) && nnz <= (long long)p->sms * kSliceEdges && p->sms <= kBlockSums) {
+            pr_slice_sizes_kernel<<<p->sms, 256>>>(side.rowptr, n_local, (int2 *)p->block_sums);
+            count_launch();
+            p->slices.resize((size_t)p->sms);
+            e = cudaMemcpy(p->slices.data(), p->block_sums, sizeof(int2) * p->slices.size(), cudaMemcpyDeviceToHost);
+            if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: %s", cudaGetErrorString(e)); break; }
+        }
         if (n_local > 0) {
             e = cudaMemcpy(p->out_degree, d_out_degree, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(p->mirror2worker, d_mirror2worker, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
             if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: copy failed: %s", cudaGetErrorString(e)); break; }
         }
-        // one part of many edges: as one stream
-        if (xplan->nranks == 1 && p->place && nnz > 0 && (long long)nnz > (long long)p->sms * kStreamEdges) {
+        // one part whose slices do not fit: its edges as one stream
+        if (xplan->nranks == 1 && p->place && nnz > 0 && !slices_fit_alone(p)) {
             p->stream_block.add(&p->stream_od, sizeof(int) * n1);
             const int warps = p->sms * (p->dbl ? stream_threads<double>() : stream_threads<float>()) / 32;
             p->stream_block.add(&p->stream_tails, rs * 4 * (size_t)warps);      // a piece each

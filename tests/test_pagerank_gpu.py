@@ -1,13 +1,16 @@
 """PageRank on the device against the oracles: DRONE's GPU-job schedule in double (1e-9) and float,
 synchronous power iteration (the 20-iteration, damping 0.85 configuration), all parts on one GPU or
 one process per GPU over NCCL."""
+import ctypes as C
 import os
+import types
 
 import numpy as np
 import pytest
 import torch
 
 import drone_b200 as db
+from drone_b200._lib import check
 from helpers import run_ranks
 from drone_b200 import graphgen as gg
 from drone_b200 import graphsum as gs
@@ -346,3 +349,55 @@ def test_power_iterations_over_a_stream_of_edges(cuda_device, oracle, scale, edg
     assert np.array_equal(runs[0], runs[1])
     prk.power_iterate_local(prs, 0, 0.85)
     assert np.ptp(prk.gather_global(prs, graphs, n)[touched]) == 0
+
+
+@pytest.mark.parametrize("scale,parts,use_double", [(4, 1, True), (5, 2, False), (9, 3, True), (12, 12, True), (13, 1, False),
+                                                    (15, 9, True), (16, 1, True), (16, 4, True), (17, 2, False)])
+def test_slices_in_shared_memory(cuda_device, oracle, monkeypatch, scale, parts, use_double):
+    """Graphs whose edges fit the SMs' shared memory, against the kernels for larger ones: fewer rows than threads, rows that
+    many threads share, rows without edges, more than eight parts, masters with more than four mirrors; the job at once and
+    superstep by superstep, with everything a caller can see of its state."""
+    n, u, v, out_deg, part = pr_case(scale=scale, seed=110 + scale, parts=parts)
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
+    touched = part.replicas > 0
+    tol = PR_TOL if use_double else 1e-4
+    results = []
+    for slices in ("0", "1"):
+        monkeypatch.setenv("DRONE_PR_SLICES", slices)
+        graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+        steps, sizes = prk.run_job_local(prs)
+        delta = prk.gather_global(prs, graphs, n)
+        some = [[(r.Mirror2MasterSendSize, r.Master2MirrorRecvSize, r.VisitedSize) for r in prk.step_local(prs, first)]
+                for first in (True, False, False)]
+        prk.step_local(prs, True)
+        prk.step_local(prs, False)
+        state = [device_state(p) for p in prs]
+        prk.power_iterate_local(prs, 20, 0.85)
+        power = prk.gather_global(prs, graphs, n)
+        assert np.max(np.abs(power[touched] - want[touched]) / want[touched]) < tol
+        for p, g in zip(prs, graphs):
+            assert np.array_equal(p.values(), power[g.host.l2g])
+        results.append((steps, sizes, some, delta, state))
+    a, b = results
+    assert np.max(np.abs(a[3][touched] - b[3][touched]) / np.abs(a[3][touched])) < (PR_TOL if use_double else 2e-4)
+    if use_double:
+        assert a[:3] == b[:3]
+    for x, y in zip(a[4], b[4]):
+        for name in ("active", "ubm"):
+            assert np.array_equal(x[name], y[name])
+        for name in ("pr", "acc", "diff"):
+            # values start at 1, and so do the terms of a sum, whatever cancels in it: a float sum is off by a few 2^-24 of that
+            assert np.max(np.abs(x[name] - y[name]) / np.maximum(np.abs(x[name]), 1e-3 if use_double else 1.0)) < (PR_TOL if use_double else 1e-4), name
+
+
+def device_state(job):
+    """The arrays of drone_pr_device_arrays, copied."""
+    ptrs = [C.c_void_p(0) for _ in range(5)]
+    check(db.lib().drone_pr_device_arrays(job.handle, *[C.byref(p) for p in ptrs]))
+    kinds = ["<f8" if job.use_double else "<f4"] * 3 + ["<i4"] * 2
+    out = {}
+    for name, p, t in zip(("pr", "acc", "diff", "active", "ubm"), ptrs, kinds):
+        view = types.SimpleNamespace(__cuda_array_interface__={"shape": (job.n_local,), "typestr": t, "data": (p.value, False), "version": 2})
+        out[name] = torch.as_tensor(view, device="cuda").cpu().numpy()
+    return out
