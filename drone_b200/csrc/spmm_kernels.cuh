@@ -395,6 +395,86 @@ __device__ __forceinline__ void walk_short_range(long long range, const int *__r
     }
 }
 
+// The same for rows that one or two lanes hold: with an entry a lane their group would have one or two gathers in flight, so a
+// lane takes EPL entries of the stream at a time (the neighbours of the first come from L1).  us a call before / with it, and with
+// the chunks' batches below: F = 1 R-MAT-12 15 / 9, power law 60,000 rows of 21 30 / 16, 1 M rows of 21 358 / 149; F = 2 R-MAT-18
+// 69 / 46; F = 4 R-MAT-12 16 / 11, 300,000 rows of 8 34 / 24, R-MAT-21 472 / 334; F = 8 R-MAT-12 10.2 / 9.4, R-MAT-21 400 / 370.
+// Two lanes with four entries each were no better (R-MAT-20, F = 8: 123 / 141), nor were groups of four lanes with two.
+constexpr int short_entries_per_lane(int G, int VPL, int VEC) {
+    return VPL > 1 || G > 2 ? 1 : VEC == 1 ? 8 / G : 4 / G;
+}
+template <int G, int VEC, bool EXACT, bool UNIT, bool HOT, bool EARLY>
+__device__ __forceinline__ void walk_short_range_narrow(long long range, const int *__restrict__ s_range_row, int n_ranges,
+                                                        const int *__restrict__ s_rowptr, const int *__restrict__ s_rows,
+                                                        const int *__restrict__ s_col, const float *__restrict__ s_val,
+                                                        const Gather &g, float *__restrict__ Y, long long ldy, int nvec,
+                                                        const Epilogue &epi) {
+    using V = typename Vec<VEC>::type;
+    constexpr int EPL = short_entries_per_lane(G, 1, VEC), BATCH = G * EPL;
+    const int gl = threadIdx.x & (G - 1);
+    int ri = 0, k = 0, kend = 0;
+    if (range < n_ranges) {
+        ri = s_range_row[range];
+        const int ri_end = s_range_row[range + 1];
+        k = s_rowptr[ri];
+        kend = s_rowptr[ri_end];
+    }
+    int maxlen = kend - k;
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, o));
+    const unsigned long long pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
+    V acc = Vec<VEC>::zero();
+    unsigned c_next[EPL];
+    float v_next[EPL];
+    auto request = [&](int at) {      // entry e * G + gl of the batch at `at`
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+            const int i = at + e * G + gl;
+            c_next[e] = i < kend ? (unsigned)__ldg(s_col + i) : kPlaceholder;
+            v_next[e] = UNIT ? 1.f : i < kend ? __ldg(s_val + i) : 0.f;
+        }
+    };
+    request(k);
+    if (EARLY) wait_for_operands();
+    for (int base = 0; base < maxlen; base += BATCH) {
+        unsigned c[EPL];
+        float v[EPL];
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+            c[e] = (c_next[e] & ~kColMask) | resolve_column<HOT>(g, c_next[e] & kColMask);
+            v[e] = v_next[e];
+        }
+        request(k + base + BATCH);      // next batch, before this batch's gathers
+        unsigned cc[BATCH];
+        float vv[BATCH];
+        V x[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            cc[u] = __shfl_sync(0xffffffffu, c[u / G], u, G);      // lane numbers count modulo G
+            vv[u] = UNIT ? 1.f : __shfl_sync(0xffffffffu, v[u / G], u, G);
+            const bool live = !(cc[u] & kPlaceholder);
+            x[u] = ld_gathered_if<EARLY>(row_address<VEC, HOT>(g, live ? (cc[u] & kColMask) : 0u, gl, nvec), pol_keep,
+                                         live && (EXACT || gl < nvec));
+        }
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            Vec<VEC>::fma(acc, vv[u], x[u]);
+            if (cc[u] & kLastInRow) {
+                const int row = s_rows[ri];
+                const float scale = row_scale_of<EARLY>(epi, row);
+                const RowDestination<VEC> dest = row_destination<VEC>(epi, Y, ldy, row);
+                if (EXACT || gl < nvec) {
+                    const V out = finish_row<VEC>(acc, epi, scale);
+                    if (dest.remote) dest.ptr[gl] = out;
+                    else st_stream(dest.ptr + gl, out, pol_stream);
+                }
+                acc = Vec<VEC>::zero();
+                ++ri;
+            }
+        }
+    }
+}
+
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
 __global__ void __launch_bounds__(256, short_blocks_per_sm(G, VPL, VEC, EXACT))
 spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, const int *__restrict__ s_rowptr,
@@ -402,8 +482,12 @@ spmm_short_stream_kernel(const int *__restrict__ s_range_row, int n_ranges, cons
                          const float *__restrict__ s_val, Gather g, float *__restrict__ Y, long long ldy, int nvec,
                          Epilogue epi) {
     const long long range = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * (32 / G) + (threadIdx.x & 31) / G;
-    walk_short_range<G, VPL, VEC, U, EXACT, UNIT, HOT, false>(range, s_range_row, n_ranges, s_rowptr, s_rows, s_col, s_val, g, Y,
-                                                       ldy, nvec, epi);
+    if constexpr (short_entries_per_lane(G, VPL, VEC) > 1)
+        walk_short_range_narrow<G, VEC, EXACT, UNIT, HOT, false>(range, s_range_row, n_ranges, s_rowptr, s_rows, s_col, s_val, g, Y, ldy,
+                                                                 nvec, epi);
+    else
+        walk_short_range<G, VPL, VEC, U, EXACT, UNIT, HOT, false>(range, s_range_row, n_ranges, s_rowptr, s_rows, s_col, s_val, g, Y,
+                                                                  ldy, nvec, epi);
 }
 
 // ---------------------------------------------------------------------------
@@ -506,6 +590,59 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
         for (int p = 0; p < VPL; ++p) Vec<VEC>::add(acc[p], Vec<VEC>::shfl_xor(acc[p], o));
 }
 
+// Batches of 32 entries that a warp takes together: a batch of rows that one or two lanes hold is one or two gathers a lane.
+// Four, but two in the one launch of a small plan for pairs of lanes, where four cost registers that its short rows want (us, F = 8,
+// two / four: power law, 100,000 rows of 51 51 / 75; the separate kernels: R-MAT-18 70 / 60, R-MAT-20 129 / 123).
+constexpr int chunk_batches(int G, int VPL, int VEC, bool one_launch) {
+    return VPL > 1 || G > 2 ? 1 : G == 2 && VEC == 4 && one_launch ? 2 : 4;
+}
+
+// The lane's entries of the first NB batches of [k0, k0 + len).
+template <int NB, bool UNIT>
+__device__ __forceinline__ void first_batches(int (&c)[NB], float (&v)[NB], const int *__restrict__ col, const float *__restrict__ val,
+                                              int k0, int len, unsigned long long pol_stream) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const bool live = b * 32 + lane < len;
+        c[b] = live ? ld_stream(col + k0 + b * 32 + lane, pol_stream) : 0;
+        v[b] = UNIT ? 1.f : live ? ld_stream(val + k0 + b * 32 + lane, pol_stream) : 0.f;
+    }
+}
+
+// sum_chunk for such rows, the same sums in the same order.
+template <int G, int VEC, bool EXACT, bool UNIT, bool HOT, bool EARLY, int NB>
+__device__ __forceinline__ void sum_chunk_narrow(typename Vec<VEC>::type &acc, const int *__restrict__ col, const float *__restrict__ val,
+                                                 const Gather &g, int k0, int len, int (&c)[NB], float (&v)[NB], int nvec,
+                                                 unsigned long long pol_keep, unsigned long long pol_stream) {
+    using V = typename Vec<VEC>::type;
+    constexpr int RPW = 32 / G;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), gi = lane / G;
+    acc = Vec<VEC>::zero();
+    for (int base = 0; base < len; base += 32 * NB) {
+        int c_next[NB];
+        float v_next[NB], vv[NB * G];
+        V x[NB * G];
+        first_batches<NB, UNIT>(c_next, v_next, col, val, k0 + base + 32 * NB, len - base - 32 * NB, pol_stream);
+#pragma unroll
+        for (int i = 0; i < NB * G; ++i) {
+            const int e = (i % G) * RPW + gi, cc = __shfl_sync(0xffffffffu, c[i / G], e);
+            vv[i] = UNIT ? 1.f : __shfl_sync(0xffffffffu, v[i / G], e);
+            x[i] = ld_gathered_if<EARLY>(row_address<VEC, HOT>(g, (unsigned)cc, gl, nvec), pol_keep,
+                                         base + i / G * 32 + e < len && (EXACT || gl < nvec));
+        }
+#pragma unroll
+        for (int i = 0; i < NB * G; ++i) Vec<VEC>::fma(acc, vv[i], x[i]);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            c[b] = (int)resolve_column<HOT>(g, (unsigned)c_next[b]);
+            v[b] = v_next[b];
+        }
+    }
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) Vec<VEC>::add(acc, Vec<VEC>::shfl_xor(acc, o));
+}
+
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
 __global__ void __launch_bounds__(256, chunk_blocks_per_sm(G, VPL, VEC, EXACT))
 spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__restrict__ col,
@@ -529,9 +666,16 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
         if (lane == 0) next_group = atomicAdd(counter, (unsigned)kChunkGroup);   // needed only after this group
 
         // first batch of the group's first chunk
+        constexpr int NB = chunk_batches(G, VPL, VEC, false);
+        int cs[NB];      // the same of several batches (NB > 1)
+        float vs[NB];
         int c = 0;
         float v = UNIT ? 1.f : 0.f;
-        {
+        if constexpr (NB > 1) {
+            first_batches<NB, UNIT>(cs, vs, col, val, __shfl_sync(0xffffffffu, desc.y, 0), __shfl_sync(0xffffffffu, desc.z, 0), pol_stream);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) cs[b] = (int)resolve_column<HOT>(g, (unsigned)cs[b]);
+        } else {
             const int k0 = __shfl_sync(0xffffffffu, desc.y, 0), len = __shfl_sync(0xffffffffu, desc.z, 0);
             if (lane < len) {
                 c = ld_stream(col + k0 + lane, pol_stream);
@@ -543,9 +687,14 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
             const int row = __shfl_sync(0xffffffffu, desc.x, j), k0 = __shfl_sync(0xffffffffu, desc.y, j);
             const int len = __shfl_sync(0xffffffffu, desc.z, j), slot = __shfl_sync(0xffffffffu, desc.w, j);
             // first batch of the chunk after this one, requested now and used when this chunk is done
+            int cs_ahead[NB];
+            float vs_ahead[NB];
             int c_ahead = 0;
             float v_ahead = UNIT ? 1.f : 0.f;
-            if (j + 1 < in_group) {
+            if constexpr (NB > 1) {
+                const int nk0 = __shfl_sync(0xffffffffu, desc.y, j + 1), nlen = __shfl_sync(0xffffffffu, desc.z, j + 1);
+                first_batches<NB, UNIT>(cs_ahead, vs_ahead, col, val, nk0, j + 1 < in_group ? nlen : 0, pol_stream);
+            } else if (j + 1 < in_group) {
                 const int nk0 = __shfl_sync(0xffffffffu, desc.y, j + 1), nlen = __shfl_sync(0xffffffffu, desc.z, j + 1);
                 if (lane < nlen) {
                     c_ahead = ld_stream(col + nk0 + lane, pol_stream);
@@ -554,7 +703,10 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
             }
 
             V acc[VPL];
-            sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT, false, sure_vectors(G, VPL, VEC)>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
+            if constexpr (NB > 1)
+                sum_chunk_narrow<G, VEC, EXACT, UNIT, HOT, false, NB>(acc[0], col, val, g, k0, len, cs, vs, nvec, pol_keep, pol_stream);
+            else
+                sum_chunk<G, VPL, VEC, U, EXACT, UNIT, HOT, false, sure_vectors(G, VPL, VEC)>(acc, col, val, g, k0, len, c, v, nvec, pol_keep, pol_stream);
 
             if (gi == 0) {
                 if (slot < 0) {
@@ -576,8 +728,16 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
                         if (EXACT || gl + p * G < nvec) out[p * G] = acc[p];
                 }
             }
-            c = (int)resolve_column<HOT>(g, (unsigned)c_ahead);
-            v = v_ahead;
+            if constexpr (NB > 1) {
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    cs[b] = (int)resolve_column<HOT>(g, (unsigned)cs_ahead[b]);
+                    vs[b] = vs_ahead[b];
+                }
+            } else {
+                c = (int)resolve_column<HOT>(g, (unsigned)c_ahead);
+                v = v_ahead;
+            }
         }  // chunks of the group
         group = __shfl_sync(0xffffffffu, next_group, 0);
     }
@@ -706,17 +866,26 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
     let_next_kernel_start();
     if ((int)blockIdx.x >= chunk_blocks) {
         const long long warp = (((int)blockIdx.x - chunk_blocks) * (long long)blockDim.x + threadIdx.x) >> 5;
-        walk_short_range<G, VPL, VEC, U, EXACT, UNIT, false, true>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
-                                                             s_val, g, Y, ldy, nvec, epi);
+        if constexpr (short_entries_per_lane(G, VPL, VEC) > 1)
+            walk_short_range_narrow<G, VEC, EXACT, UNIT, false, true>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
+                                                                      s_val, g, Y, ldy, nvec, epi);
+        else
+            walk_short_range<G, VPL, VEC, U, EXACT, UNIT, false, true>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
+                                                                       s_val, g, Y, ldy, nvec, epi);
         return;
     }
     const int at = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (at >= n_chunks) return;
     const unsigned long long pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
     const int4 ch = __ldg(reinterpret_cast<const int4 *>(chunks) + at);      // row, first nonzero, length, slot
+    constexpr int NB = chunk_batches(G, VPL, VEC, true);
+    int cs[NB];
+    float vs[NB];
     int c = 0;
     float v = UNIT ? 1.f : 0.f;
-    if (lane < ch.z) {
+    if constexpr (NB > 1) {
+        first_batches<NB, UNIT>(cs, vs, col, val, ch.y, ch.z, pol_stream);
+    } else if (lane < ch.z) {
         c = ld_stream(col + ch.y + lane, pol_stream);
         if (!UNIT) v = ld_stream(val + ch.y + lane, pol_stream);
     }
@@ -724,7 +893,10 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
     const int4 sr = ch.w >= 0 ? __ldg(reinterpret_cast<const int4 *>(split) + which) : ch;      // row, first slot, slots
     V acc[VPL];
     wait_for_operands();
-    sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false, true, SURE>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
+    if constexpr (NB > 1)
+        sum_chunk_narrow<G, VEC, EXACT, UNIT, false, true, NB>(acc[0], col, val, g, ch.y, ch.z, cs, vs, nvec, pol_keep, pol_stream);
+    else
+        sum_chunk<G, VPL, VEC, 2 * U, EXACT, UNIT, false, true, SURE>(acc, col, val, g, ch.y, ch.z, c, v, nvec, pol_keep, pol_stream);
     int row = ch.x;
     if (ch.w >= 0) {
         if (gi == 0) {
