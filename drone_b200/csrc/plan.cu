@@ -741,6 +741,16 @@ int validate_csr(const char *who, const int *d_index, const int *d_col, int n_ro
     return DRONE_OK;
 }
 
+// Nonzeros per chunk, and of a row that the short-row stream still takes.  The serial work of one warp is most of a call that
+// does not fill the GPU, and wide rows have few gathers in flight: shorter chunks and streamed rows there (us, rows up to 32 in the
+// stream and chunks of 256 / rows up to 16 and chunks of 64: R-MAT-11 F = 16 8.2 / 7.5, F = 256 40 / 15; R-MAT-12 F = 64 12.3 /
+// 8.1, F = 256 41 / 18; power law, 8,000 rows of 16, F = 64 8.0 / 6.5; with 212,000 nonzeros (R-MAT-13) and chunks of 128 F = 16
+// 9.5 / 8.5, F = 256 45 / 27; from 600,000 on either costs 5 to 20 % at widths up to 32).  The lines lie where a plan's partial
+// sums, at most one for every half a chunk and a bit, still fit drone_spmm_static_scratch at every width, as they do with chunks of
+// 256.  Very large graphs take longer chunks so that the chunk list stays below 1 % of the CSR stream.
+static int chunk_nnz_for(int nnz) { return nnz <= 1 << 17 ? 64 : nnz <= 1 << 18 ? 128 : nnz <= 1 << 28 ? 256 : 1024; }
+static int short_row_limit_for(int nnz) { return nnz <= 1 << 18 ? 16 : 32; }
+
 static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_index, const int *d_dst,
                             const float *d_values, const int *d_in_degree, const int *d_out_degree,
                             int orientations, cudaStream_t st, bool for_spmm) {
@@ -753,11 +763,8 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
     p->for_spmm = for_spmm;
     p->n_rows = n_rows;
     p->nnz = nnz;
-    p->short_row_limit = env_int("DRONE_SHORT_ROW_LIMIT", 32);
-    // Chunks of 256 nonzeros keep the serial work of one warp near ten microseconds;
-    // very large graphs take longer chunks so that the chunk list stays below 1% of
-    // the CSR stream.
-    p->chunk_nnz = env_int("DRONE_CHUNK_NNZ", nnz > (1 << 28) ? 1024 : 256);
+    p->short_row_limit = env_int("DRONE_SHORT_ROW_LIMIT", for_spmm ? short_row_limit_for(nnz) : 32);
+    p->chunk_nnz = env_int("DRONE_CHUNK_NNZ", for_spmm ? chunk_nnz_for(nnz) : 256);
     if (p->chunk_nnz < p->short_row_limit) p->chunk_nnz = p->short_row_limit;
     const char *slice = getenv("DRONE_SLICE_WIDTH");       // read per plan, so that one process can hold plans of each kind
     p->slice_forced = (slice && *slice) ? atoi(slice) : -1;

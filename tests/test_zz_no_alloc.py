@@ -110,3 +110,25 @@ def test_static_scratch_refuses_what_does_not_fit(cuda_device):
     y8 = torch.empty((n, 8), device=cuda_device)
     assert call_static(plan, db.OP_A, x8, y8) == 0
     assert torch.equal(y8, plan.spmm(db.OP_A, x8))
+
+
+@pytest.mark.parametrize("nnz,length", [(1 << 17, 65), (1 << 17, 1 << 17), ((1 << 17) + 1, 65), (1 << 18, 129), ((1 << 18) + 1, 257)])
+def test_static_scratch_takes_small_plans_at_every_width(cuda_device, nnz, length):
+    """Plans on both sides of where chunks get longer, their rows of the lengths that need most partial sums: the widest call
+    still fits the built-in scratch, and gives what the allocating one gives."""
+    n = (nnz + length - 1) // length + 1
+    n = max(n, length)                           # no column twice in a row
+    degree = np.zeros(n, np.int64)
+    degree[:nnz // length] = length
+    degree[nnz // length] = nnz % length
+    index = torch.as_tensor(np.concatenate([[0], np.cumsum(degree)]).astype(np.int32))
+    dst = torch.as_tensor(np.concatenate([np.arange(d) for d in degree if d]).astype(np.int32))
+    values = torch.rand(nnz, generator=torch.Generator().manual_seed(nnz))
+    plan = db.AggregationPlan(index.to(cuda_device), dst.to(cuda_device), values=values.to(cuda_device), orientations=1)
+    x = torch.randn((n, 1024), device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(1))
+    y = torch.empty_like(x)
+    assert call_static(plan, db.OP_A, x, y) == 0
+    other = plan.spmm(db.OP_A, x)                # in column slices where X is large, which add in another order
+    assert (y - other).abs().max() <= 1e-5 * y.abs().max()
+    want = torch.sparse_csr_tensor(index.long(), dst.long(), values.double(), (n, n)) @ x[:, :8].double().cpu()
+    assert (y[:, :8].cpu() - want).abs().max() <= 1e-5 * want.abs().max()
