@@ -94,6 +94,8 @@ def _declare(lib):
         "drone_comm_bcast": (i, [vp, vp, C.c_size_t, i, vp]),
         "drone_comm_reduce_sum": (i, [vp, vp, C.c_size_t, i, vp]),
         "drone_clear_mirror_rows": (i, [vp, i, i, i, vp, vp]),
+        "drone_softmax_loss": (i, [i, i, vp, i, vp, vp, vp, i, vp, vp, vp]),
+        "drone_relu_mask": (i, [i, i, vp, i, vp, i, vp]),
         "drone_xplan_create": (i, [C.POINTER(vp), i, i, i, vp, vp, vp, vp, i]),
         "drone_xplan_destroy": (i, [vp]),
         "drone_xplan_enable_p2p": (i, [vp, vp, vp]),

@@ -1,8 +1,7 @@
 """Host-side mirror of the reference's GCN step around the aggregation path (CUDAGCN::forward / backward,
 cuda_gcn/src/cuda/cuda_gcn.cu:44-83,119-170), for any number of layers.  Only the GraphSum layers, the masking of
-mirror rows and the weight broadcast / gradient reduce are this library's kernels and NCCL calls; the dense layers
-either side stay on cuBLAS (torch.matmul) and cross-entropy on torch, as in the reference they stay on cuBLAS and
-small element-wise kernels.  Used to time an epoch and to check gradients end to end.
+mirror rows, the loss, the ReLU's gradient and the weight broadcast / gradient reduce are this library's kernels and NCCL
+calls; the dense layers either side stay on cuBLAS (torch.matmul).  Used to time an epoch and to check gradients end to end.
 
 Layer l = 1..L:  H_l = A_{l-1} · W_l  (Matmul)  ->  Z_l = Â^T-aggregation of H_l + mirror/master sync (GraphSum)
                  ->  A_l = ReLU(Z_l) for l < L, logits = Z_L.
@@ -10,7 +9,7 @@ The reference's module list is this with L = 2 (cuda_gcn.cu:44-83); its layer in
 """
 import torch
 
-from ._lib import OP_A, OP_AT
+from ._lib import OP_A, OP_AT, check, lib
 from .graphsum import aggregate_and_exchange, clear_mirror_rows, exchange_sum
 
 
@@ -40,6 +39,12 @@ class GCN:
         self.mirror2worker = graph.mirror2worker if worker_num > 1 else None
         self.labelled = truth >= 0
         self.safe_truth = truth.clamp(min=0).long()
+        # element-wise steps: one kernel each on the GPU, torch elsewhere
+        self._kernels = x.is_cuda and all(t.dtype == torch.float32 for t in (x, *self.weights))
+        if self._kernels:
+            if n > 0 and int(self.safe_truth.max()) >= dims[-1]:
+                raise ValueError("a label is outside 0..%d" % (dims[-1] - 1))
+            self._scratch = torch.empty(2368, dtype=torch.float64, device=dev)      # DRONE_LOSS_SCRATCH
         self.d_w = [None] * self.n_layers
         self.loss = None
 
@@ -99,8 +104,19 @@ class GCN:
             if relu and not fused:
                 self.z[l].clamp_(min=0)                                    # CUDAReLU::forward, in place
             a = self.z[l]
-        logits = self.z[last]
-        # CUDACrossEntropyLoss::forward: loss = mean over labelled rows; gradient not divided by the count
+        return self._softmax_loss(self.z[last])
+
+    def _softmax_loss(self, logits):
+        """CUDACrossEntropyLoss::forward: loss = mean over labelled rows; gradient not divided by the count."""
+        if self._kernels:
+            n, classes = logits.shape
+            self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), device=logits.device)
+            stream = torch._C._cuda_getCurrentRawStream(logits.device.index)
+            with torch.cuda.device(logits.device):
+                check(lib().drone_softmax_loss(n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
+                                               self.labelled.data_ptr(), self.d_logits.data_ptr(), classes, self.loss.data_ptr(),
+                                               self._scratch.data_ptr(), stream))
+            return self.loss
         zmax = logits.max(dim=1, keepdim=True).values
         e = torch.exp(logits - zmax)
         s = e.sum(dim=1, keepdim=True)
@@ -113,6 +129,15 @@ class GCN:
         self.d_logits.mul_(self.labelled.unsqueeze(1))
         return self.loss
 
+    def _relu_mask(self, grad, out):
+        if not self._kernels:
+            return grad.mul_(out > 0)
+        n, f = grad.shape
+        with torch.cuda.device(grad.device):
+            check(lib().drone_relu_mask(n, f, grad.data_ptr(), f, out.data_ptr(), f,
+                                        torch._C._cuda_getCurrentRawStream(grad.device.index)))
+        return grad
+
     def backward(self):
         g = self.d_logits
         for l in range(self.n_layers - 1, -1, -1):
@@ -124,7 +149,7 @@ class GCN:
                 clear_mirror_rows(self.d_h[l], self.mirror2worker)         # ... clear_mirror_grad (in place) ...
             self.d_w[l] = a_prev.t() @ self.d_h[l]                         # ... then dW
             if l > 0:
-                g = d_a.mul_(self.z[l - 1] > 0)                            # CUDAReLU::backward: the mask is (output > 0)
+                g = self._relu_mask(d_a, self.z[l - 1])                    # CUDAReLU::backward: the mask is (output > 0)
                 if l == 1:
                     self.d_z1 = g
         return tuple(self.d_w)

@@ -322,6 +322,17 @@ int drone_comm_reduce_sum(drone_comm *comm, float *d_buf, size_t count, int root
  */
 int drone_clear_mirror_rows(float *d_rows, int n_rows, int F, int ld, const int *d_mirror2worker, void *stream);
 
+/* Softmax cross-entropy over [n_rows, classes] logits with its gradient (CUDACrossEntropyLoss::forward,
+ * cuda_gcn/src/cuda/cuda_kernel.cu:326-370): *d_loss = mean over the rows with d_labelled[r] != 0 (0 where there are none),
+ * d_grad = (softmax - one-hot) * labelled, not divided by their number.  d_truth[r]: the row's class, 0..classes-1 (also
+ * where it is not labelled).  d_scratch: DRONE_LOSS_SCRATCH doubles, 16-byte aligned.  d_grad may be d_logits.  Asynchronous. */
+#define DRONE_LOSS_SCRATCH 2368
+int drone_softmax_loss(int n_rows, int classes, const float *d_logits, int ld, const long long *d_truth, const unsigned char *d_labelled,
+                       float *d_grad, int ld_grad, float *d_loss, double *d_scratch, void *stream);
+
+/* d_grad *= (d_out > 0), [n_rows, F] (CUDAReLU::backward, cuda_module.cu:513-523).  Asynchronous. */
+int drone_relu_mask(int n_rows, int F, float *d_grad, int ld_grad, const float *d_out, int ld_out, void *stream);
+
 /*
  * Routing plan of one rank, from the reference's routing tables (host arrays,
  * indexed by local vertex id):
