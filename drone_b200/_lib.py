@@ -96,6 +96,8 @@ def _declare(lib):
         "drone_clear_mirror_rows": (i, [vp, i, i, i, vp, vp]),
         "drone_softmax_loss": (i, [i, i, vp, i, vp, vp, vp, i, vp, vp, vp]),
         "drone_relu_mask": (i, [i, i, vp, i, vp, i, vp]),
+        "drone_weight_gradient_scratch": (i, [i, i, i, C.POINTER(ll)]),
+        "drone_weight_gradient": (i, [i, i, i, vp, i, vp, i, vp, vp, ll, vp]),
         "drone_xplan_create": (i, [C.POINTER(vp), i, i, i, vp, vp, vp, vp, i]),
         "drone_xplan_destroy": (i, [vp]),
         "drone_xplan_enable_p2p": (i, [vp, vp, vp]),

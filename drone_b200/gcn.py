@@ -1,12 +1,14 @@
 """Host-side mirror of the reference's GCN step around the aggregation path (CUDAGCN::forward / backward,
 cuda_gcn/src/cuda/cuda_gcn.cu:44-83,119-170), for any number of layers.  Only the GraphSum layers, the masking of
-mirror rows, the loss, the ReLU's gradient and the weight broadcast / gradient reduce are this library's kernels and NCCL
-calls; the dense layers either side stay on cuBLAS (torch.matmul).  Used to time an epoch and to check gradients end to end.
+mirror rows, the loss, the ReLU's gradient, the weight gradients and the weight broadcast / gradient reduce are this library's
+kernels and NCCL calls; the other products of the dense layers stay on cuBLAS (torch.matmul).  Used to time an epoch and to check gradients end to end.
 
 Layer l = 1..L:  H_l = A_{l-1} · W_l  (Matmul)  ->  Z_l = Â^T-aggregation of H_l + mirror/master sync (GraphSum)
                  ->  A_l = ReLU(Z_l) for l < L, logits = Z_L.
 The reference's module list is this with L = 2 (cuda_gcn.cu:44-83); its layer interface allows more.
 """
+import ctypes as C
+
 import torch
 
 from ._lib import OP_A, OP_AT, check, lib
@@ -45,6 +47,7 @@ class GCN:
             if n > 0 and int(self.safe_truth.max()) >= dims[-1]:
                 raise ValueError("a label is outside 0..%d" % (dims[-1] - 1))
             self._scratch = torch.empty(2368, dtype=torch.float64, device=dev)      # DRONE_LOSS_SCRATCH
+            self._shares = {}
         self.d_w = [None] * self.n_layers
         self.loss = None
 
@@ -106,16 +109,25 @@ class GCN:
             a = self.z[l]
         return self._softmax_loss(self.z[last])
 
+    def _stream(self):
+        return torch._C._cuda_getCurrentRawStream(self.x.device.index)
+
+    def _call(self, name, *args):
+        """A library call on the model's device."""
+        if torch.cuda.current_device() == self.x.device.index:
+            check(getattr(lib(), name)(*args))
+        else:
+            with torch.cuda.device(self.x.device):
+                check(getattr(lib(), name)(*args))
+
     def _softmax_loss(self, logits):
         """CUDACrossEntropyLoss::forward: loss = mean over labelled rows; gradient not divided by the count."""
         if self._kernels:
             n, classes = logits.shape
             self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), device=logits.device)
-            stream = torch._C._cuda_getCurrentRawStream(logits.device.index)
-            with torch.cuda.device(logits.device):
-                check(lib().drone_softmax_loss(n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
-                                               self.labelled.data_ptr(), self.d_logits.data_ptr(), classes, self.loss.data_ptr(),
-                                               self._scratch.data_ptr(), stream))
+            self._call("drone_softmax_loss", n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
+                       self.labelled.data_ptr(), self.d_logits.data_ptr(), classes, self.loss.data_ptr(), self._scratch.data_ptr(),
+                       self._stream())
             return self.loss
         zmax = logits.max(dim=1, keepdim=True).values
         e = torch.exp(logits - zmax)
@@ -133,10 +145,22 @@ class GCN:
         if not self._kernels:
             return grad.mul_(out > 0)
         n, f = grad.shape
-        with torch.cuda.device(grad.device):
-            check(lib().drone_relu_mask(n, f, grad.data_ptr(), f, out.data_ptr(), f,
-                                        torch._C._cuda_getCurrentRawStream(grad.device.index)))
+        self._call("drone_relu_mask", n, f, grad.data_ptr(), f, out.data_ptr(), f, self._stream())
         return grad
+
+    def _weight_gradient(self, a, g):
+        if not self._kernels or a.stride(1) != 1:
+            return a.t() @ g
+        (k, m), n = a.shape, g.shape[1]
+        floats = self._shares.get((k, m, n))
+        if floats is None:      # a property of the shape
+            size = C.c_longlong(0)
+            self._call("drone_weight_gradient_scratch", k, m, n, C.byref(size))
+            floats = self._shares[(k, m, n)] = size.value
+        out, parts = torch.empty((m, n), device=g.device), torch.empty(floats, device=g.device)
+        self._call("drone_weight_gradient", k, m, n, a.data_ptr(), max(m, a.stride(0)), g.data_ptr(), n, out.data_ptr(),
+                   parts.data_ptr(), floats, self._stream())
+        return out
 
     def backward(self):
         g = self.d_logits
@@ -147,7 +171,7 @@ class GCN:
                 d_a = torch.matmul(self.d_h[l], self.weights[l].t(), out=self.d_a[l - 1])   # CUDAMatmul::backward: dA first ...
             if self.mirror2worker is not None:
                 clear_mirror_rows(self.d_h[l], self.mirror2worker)         # ... clear_mirror_grad (in place) ...
-            self.d_w[l] = a_prev.t() @ self.d_h[l]                         # ... then dW
+            self.d_w[l] = self._weight_gradient(a_prev, self.d_h[l])       # ... then dW
             if l > 0:
                 g = self._relu_mask(d_a, self.z[l - 1])                    # CUDAReLU::backward: the mask is (output > 0)
                 if l == 1:

@@ -143,3 +143,19 @@ def test_labels_outside_the_classes_are_refused(cuda_device):
     with pytest.raises(ValueError, match="label"):
         gcn.GCN(None, torch.zeros((3, 4), device=cuda_device), torch.tensor([0, 5, -1], dtype=torch.int32, device=cuda_device),
                 [torch.zeros((4, 5), device=cuda_device)])
+
+
+@pytest.mark.parametrize("k,m,n", [(1, 1, 1), (15, 3, 5), (17, 64, 64), (63, 65, 7), (64, 128, 64), (65, 129, 65), (1000, 602, 128),
+                                   (3001, 100, 16), (9999, 33, 47), (20000, 128, 41), (300, 700, 300), (0, 5, 6)])
+def test_weight_gradient(cuda_device, k, m, n):
+    """Tiles and shares at their edges, odd widths and leading dimensions, against double; the same bits every time."""
+    gen = torch.Generator(cuda_device).manual_seed(k + m + n)
+    model = gcn.GCN(None, torch.zeros((1, 4), device=cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device),
+                    [torch.zeros((4, 5), device=cuda_device)], aggregate=lambda *a: None)
+    a = torch.randn((k, m + 3), device=cuda_device, generator=gen)[:, 1:m + 1]
+    g = torch.randn((k, n), device=cuda_device, generator=gen)
+    got, want = model._weight_gradient(a, g), a.double().t() @ g.double()
+    # a chain of k additions of terms of size 1: sqrt(k) roundings of a sum that has grown to sqrt(k), and some to spare
+    assert (got - want).abs().max() <= 6 * 2.0 ** -24 * (k + 30) if k else (got == 0).all()
+    assert torch.equal(got, model._weight_gradient(a, g))
+    assert torch.equal(model._weight_gradient(a.contiguous(), g), got)
