@@ -1685,7 +1685,11 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
             p->stream_block.add(&p->stream_od, sizeof(int) * n1);
             const int warps = p->sms * (p->dbl ? stream_threads<double>() : stream_threads<float>()) / 32;
             p->stream_block.add(&p->stream_tails, rs * 4 * (size_t)warps);      // a piece each
-            if ((rc = plan_rows_in_order(p->plan, DRONE_OP_AT, p->place, warps, &p->stream, &p->stream_block, nullptr))) break;
+            if (plan_rows_in_order(p->plan, DRONE_OP_AT, p->place, warps, &p->stream, &p->stream_block, nullptr)) {
+                p->stream_block.release();      // no room: power iterations do without (pr_run_kernel)
+                p->stream = RowStream();
+                break;
+            }
             pr_stream_degrees_kernel<<<grid1d(n_local), 256>>>(p->stream.row_of, p->out_degree, p->mirror2worker, n_local, p->stream_od);
             count_launch();
             if ((e = cudaDeviceSynchronize()) != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: %s", cudaGetErrorString(e)); break; }

@@ -122,7 +122,7 @@ class GCN:
 
     def _softmax_loss(self, logits):
         """CUDACrossEntropyLoss::forward: loss = mean over labelled rows; gradient not divided by the count."""
-        if self._kernels:
+        if self._kernels and self.labelled.dtype == torch.bool and self.safe_truth.dtype == torch.int64:
             n, classes = logits.shape
             self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), device=logits.device)
             self._call("drone_softmax_loss", n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
@@ -149,7 +149,7 @@ class GCN:
         return grad
 
     def _weight_gradient(self, a, g):
-        if not self._kernels or a.stride(1) != 1:
+        if not self._kernels or a.stride(1) != 1 or max(a.shape[1], g.shape[1]) > 1 << 15:
             return a.t() @ g
         (k, m), n = a.shape, g.shape[1]
         floats = self._shares.get((k, m, n))

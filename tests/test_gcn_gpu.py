@@ -102,60 +102,3 @@ def test_gcn_step_two_gpus():
     if torch.cuda.device_count() < 2:
         pytest.skip("needs two GPUs")
     run_ranks(_rank, 2, (29800 + os.getpid() % 2000,))
-
-
-@pytest.mark.parametrize("classes", [1, 7, 8, 9, 16, 17, 33, 41, 64, 65, 256, 257, 1000])
-@pytest.mark.parametrize("n,share", [(1, 1.0), (37, 0.0), (5003, 0.66), (200001, 0.66)])
-def test_loss_and_relu_mask(cuda_device, n, share, classes):
-    """The loss kernel at the edges of its lane groups, without labelled rows, and with rows of infinities, against the same
-    steps in double; the mask of the ReLU's gradient, where it is read as vectors and where not."""
-    if n * classes > 3e7:
-        pytest.skip("the shape is covered with fewer classes")
-    gen = torch.Generator(cuda_device).manual_seed(n + classes)
-    model = gcn.GCN(None, torch.zeros((n, 4), device=cuda_device),
-                    torch.randint(0, classes, (n,), device=cuda_device, generator=gen, dtype=torch.int32),
-                    [torch.zeros((4, classes), device=cuda_device)], aggregate=lambda *a: None)
-    model.labelled = torch.rand(n, device=cuda_device, generator=gen) < share
-    logits = torch.randn((n, classes), device=cuda_device, generator=gen) * 4
-    z, lab = logits.double(), model.labelled
-    p = torch.softmax(z, 1)
-    want_loss = -(torch.log_softmax(z, 1).gather(1, model.safe_truth[:, None])[:, 0] * lab).sum() / max(int(lab.sum()), 1)
-    want = (p - torch.nn.functional.one_hot(model.safe_truth, classes)) * lab[:, None]
-    loss = model._softmax_loss(logits)
-    # exponentials, a sum of `classes` terms and a quotient in float
-    assert (model.d_logits - want).abs().max() <= (8 + classes / 8) * 2.0 ** -24
-    assert abs(float(loss) - float(want_loss)) <= 1e-6 * max(1.0, float(want_loss))
-    assert torch.equal(model._softmax_loss(logits), loss)
-    if n > 30 and classes > 4:      # what torch makes of infinities and NaN, entry by entry
-        odd = logits.clone()
-        odd[3, 1], odd[5, 2], odd[7, 0], odd[9] = float("inf"), float("nan"), -float("inf"), -float("inf")
-        model._softmax_loss(odd)
-        want = (torch.softmax(odd, 1) - torch.nn.functional.one_hot(model.safe_truth, classes)) * lab[:, None]
-        assert torch.equal(model.d_logits.isnan(), want.isnan())
-        fine = ~want.isnan()
-        assert (model.d_logits - want)[fine].abs().max() <= (8 + classes / 8) * 2.0 ** -23
-    grad, out = torch.randn_like(logits), torch.randn_like(logits).clamp_(min=0)
-    want = grad * (out > 0)
-    assert torch.equal(model._relu_mask(grad, out), want)
-
-
-def test_labels_outside_the_classes_are_refused(cuda_device):
-    with pytest.raises(ValueError, match="label"):
-        gcn.GCN(None, torch.zeros((3, 4), device=cuda_device), torch.tensor([0, 5, -1], dtype=torch.int32, device=cuda_device),
-                [torch.zeros((4, 5), device=cuda_device)])
-
-
-@pytest.mark.parametrize("k,m,n", [(1, 1, 1), (15, 3, 5), (17, 64, 64), (63, 65, 7), (64, 128, 64), (65, 129, 65), (1000, 602, 128),
-                                   (3001, 100, 16), (9999, 33, 47), (20000, 128, 41), (300, 700, 300), (0, 5, 6)])
-def test_weight_gradient(cuda_device, k, m, n):
-    """Tiles and shares at their edges, odd widths and leading dimensions, against double; the same bits every time."""
-    gen = torch.Generator(cuda_device).manual_seed(k + m + n)
-    model = gcn.GCN(None, torch.zeros((1, 4), device=cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device),
-                    [torch.zeros((4, 5), device=cuda_device)], aggregate=lambda *a: None)
-    a = torch.randn((k, m + 3), device=cuda_device, generator=gen)[:, 1:m + 1]
-    g = torch.randn((k, n), device=cuda_device, generator=gen)
-    got, want = model._weight_gradient(a, g), a.double().t() @ g.double()
-    # a chain of k additions of terms of size 1: sqrt(k) roundings of a sum that has grown to sqrt(k), and some to spare
-    assert (got - want).abs().max() <= 6 * 2.0 ** -24 * (k + 30) if k else (got == 0).all()
-    assert torch.equal(got, model._weight_gradient(a, g))
-    assert torch.equal(model._weight_gradient(a.contiguous(), g), got)
