@@ -120,10 +120,15 @@ class GCN:
             with torch.cuda.device(self.x.device):
                 check(getattr(lib(), name)(*args))
 
+    def _per_row(self, t, dtype, n):
+        """Whether t is one value of this type a row, side by side on the model's device."""
+        return t.dtype == dtype and t.shape == (n,) and t.device == self.x.device and t.is_contiguous()
+
     def _softmax_loss(self, logits):
         """CUDACrossEntropyLoss::forward: loss = mean over labelled rows; gradient not divided by the count."""
-        if self._kernels and self.labelled.dtype == torch.bool and self.safe_truth.dtype == torch.int64:
-            n, classes = logits.shape
+        n, classes = logits.shape
+        if (self._kernels and logits.is_contiguous() and self._per_row(self.labelled, torch.bool, n)
+                and self._per_row(self.safe_truth, torch.int64, n)):
             self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), device=logits.device)
             self._call("drone_softmax_loss", n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
                        self.labelled.data_ptr(), self.d_logits.data_ptr(), classes, self.loss.data_ptr(), self._scratch.data_ptr(),
@@ -149,9 +154,11 @@ class GCN:
         return grad
 
     def _weight_gradient(self, a, g):
-        if not self._kernels or a.stride(1) != 1 or max(a.shape[1], g.shape[1]) > 1 << 15:
-            return a.t() @ g
         (k, m), n = a.shape, g.shape[1]
+        # rows one after the other: an expanded or overlapping input has none to step over
+        in_rows = a.stride(1) == 1 and (k <= 1 or m <= a.stride(0) < 1 << 31)
+        if not self._kernels or not in_rows or max(m, n) > 1 << 15:
+            return a.t() @ g
         floats = self._shares.get((k, m, n))
         if floats is None:      # a property of the shape
             size = C.c_longlong(0)

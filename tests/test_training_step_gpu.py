@@ -62,3 +62,25 @@ def test_weight_gradient(cuda_device, k, m, n):
     assert (got - want).abs().max() <= 6 * 2.0 ** -24 * (k + 30) if k else (got == 0).all()
     assert torch.equal(got, model._weight_gradient(a, g))
     assert torch.equal(model._weight_gradient(a.contiguous(), g), got)
+
+
+def test_weight_gradient_of_rows_that_overlap(cuda_device):
+    """Inputs whose rows are one row of memory (expanded), or begin inside the one before."""
+    gen = torch.Generator(cuda_device).manual_seed(5)
+    model = gcn.GCN(None, torch.zeros((1, 4), device=cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device),
+                    [torch.zeros((4, 5), device=cuda_device)], aggregate=lambda *a: None)
+    flat, g = torch.randn(600, device=cuda_device, generator=gen), torch.randn((100, 24), device=cuda_device, generator=gen)
+    for a in (flat[:40].expand(100, 40), flat.as_strided((100, 40), (3, 1))):
+        want = a.double().t() @ g.double()
+        assert (model._weight_gradient(a, g) - want).abs().max() <= 6 * 2.0 ** -24 * 130
+
+
+def test_labels_elsewhere_are_refused(cuda_device):
+    """Labels that are not one a row on the model's device do not reach the kernel: torch refuses them."""
+    def model(truth):
+        return gcn.GCN(None, torch.zeros((6, 4), device=cuda_device), truth, [torch.zeros((4, 5), device=cuda_device)],
+                       aggregate=lambda *a: None)
+    logits = torch.zeros((6, 5), device=cuda_device)
+    for truth in (torch.zeros(6, dtype=torch.int32), torch.zeros(4, dtype=torch.int32, device=cuda_device)):
+        with pytest.raises(RuntimeError):
+            model(truth)._softmax_loss(logits)
