@@ -741,6 +741,37 @@ int validate_csr(const char *who, const int *d_index, const int *d_col, int n_ro
     return DRONE_OK;
 }
 
+// counts of the rows of X, row r being gathered as often as row r of the other orientation is long
+__global__ void gather_counts_kernel(const int *__restrict__ rowptr, int n, GatherCounts *out) {
+    __shared__ GatherCounts mine;
+    for (int c = threadIdx.x; c < kGatherClasses; c += blockDim.x) mine.rows[c] = mine.gathers[c] = 0;
+    __syncthreads();
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        const int times = rowptr[r + 1] - rowptr[r];
+        if (times < 1) continue;
+        const int c = GatherCounts::class_of(times);
+        atomicAdd(&mine.rows[c], 1ull);
+        atomicAdd(&mine.gathers[c], (unsigned long long)times);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < kGatherClasses; c += blockDim.x) {
+        if (mine.rows[c] == 0) continue;
+        atomicAdd(&out->rows[c], mine.rows[c]);
+        atomicAdd(&out->gathers[c], mine.gathers[c]);
+    }
+}
+
+// `room`: device memory for one GatherCounts.
+static int count_gathers(Side &s, const int *other_rowptr, int n, GatherCounts *room, cudaStream_t st) {
+    DRONE_CUDA(cudaMemsetAsync(room, 0, sizeof(GatherCounts), st));
+    gather_counts_kernel<<<std::min(grid_for(n), 148 * 4), 256, 0, st>>>(other_rowptr, n, room);
+    DRONE_LAUNCH_CHECK("gather_counts_kernel");
+    DRONE_CUDA(cudaMemcpyAsync(&s.counts, room, sizeof(GatherCounts), cudaMemcpyDeviceToHost, st));
+    DRONE_CUDA(cudaStreamSynchronize(st));
+    s.counted = true;
+    return DRONE_OK;
+}
+
 // Nonzeros per chunk, and of a row that the short-row stream still takes.  The serial work of one warp is most of a call that
 // does not fill the GPU, and wide rows have few gathers in flight: shorter chunks and streamed rows there (us, rows up to 32 in the
 // stream and chunks of 256 / rows up to 16 and chunks of 64: R-MAT-11 F = 16 8.2 / 7.5, F = 256 40 / 15; R-MAT-12 F = 64 12.3 /
@@ -793,7 +824,8 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
         DRONE_CUDA(cudaEventCreateWithFlags(&p->fork_event, cudaEventDisableTiming));
         DRONE_CUDA(cudaEventCreateWithFlags(&p->join_event, cudaEventDisableTiming));
     }
-    DRONE_CUDA(cudaMalloc(&p->counter, sizeof(unsigned)));
+    constexpr size_t kCountsAt = 256;      // behind the counter: room for the gather counts
+    DRONE_CUDA(cudaMalloc(&p->counter, kCountsAt + sizeof(GatherCounts)));
     p->chunk_blocks_per_sm = env_int("DRONE_CHUNK_BLOCKS_PER_SM", 0);
     PlanScratch scratch;
     if (orientations & DRONE_PLAN_AT) {
@@ -826,6 +858,12 @@ static int plan_create_impl(drone_plan *p, int n_rows, int nnz, const int *d_ind
             p->hot_table_bytes = (size_t)table_mb << 20;
             DRONE_CUDA(cudaMalloc(&p->hot_table, p->hot_table_bytes));
         }
+    }
+    if (for_spmm && !p->hot_table && (orientations & DRONE_PLAN_AT) && slices_possible(n_rows, nnz)) {
+        GatherCounts *room = reinterpret_cast<GatherCounts *>(reinterpret_cast<char *>(p->counter) + kCountsAt);
+        int rc = count_gathers(p->side[DRONE_OP_AT], a.rowptr, n_rows, room, st);
+        if (rc == DRONE_OK && (orientations & DRONE_PLAN_A)) rc = count_gathers(a, p->side[DRONE_OP_AT].rowptr, n_rows, room, st);
+        if (rc) return rc;
     }
     if (orientations & DRONE_PLAN_AT) {
         const int rc = build_work_lists(p, p->side[DRONE_OP_AT], scratch, st);

@@ -23,6 +23,9 @@ constexpr int kShortRangeNnz = 64;          // stream entries per lane group (pl
 // 270,000 rows of 9: F = 8 27 / 44, F = 16 33 / 28, F = 64 114 / 87; R-MAT-18 + I: F = 16 52 / 59, F = 128 198 / 179).
 constexpr int kFineRangeNnz = 16;
 constexpr long long kFineRangeLanes = 6LL << 20;
+// Calls on such plans may run in column slices (slices_by_counts): the widest operand is larger than L2, and the rows are long enough
+// for the lists to be read once a slice.
+inline bool slices_possible(int n_rows, int nnz) { return (long long)n_rows * 4096 > 100000000 && nnz / 24 >= n_rows; }
 constexpr unsigned kLastInRow = 0x80000000u; // flag on s_col: last entry of its row
 constexpr unsigned kPlaceholder = 0x40000000u; // flag on s_col: row has no nonzeros, entry carries no data
 constexpr unsigned kColMask = 0x3fffffffu;
@@ -58,6 +61,29 @@ struct Ranges {
     int start[kMaxRowClasses + 1] = {0};   // with row classes, class c's ranges are [start[c], start[c + 1])
 };
 
+// How the gathers of an orientation are spread over the rows of X: how many rows are gathered about how often, classes of the
+// number of times being quarters of a power of two.
+constexpr int kGatherClasses = 128;
+struct GatherCounts {
+    unsigned long long rows[kGatherClasses], gathers[kGatherClasses];
+    static __host__ __device__ int class_of(int times) {      // times >= 1
+        int e = 0;
+        while (times >> e > 1) ++e;
+        return e * 4 + (e >= 2 ? times >> (e - 2) : times << (2 - e)) % 4;
+    }
+    // Share of the gathers that go to the `n` most often gathered rows.
+    double share(double n) const {
+        double reached = 0, all = 0;
+        for (int c = kGatherClasses - 1; c >= 0; --c) {
+            all += (double)gathers[c];
+            if (rows[c] == 0 || n <= 0) continue;
+            reached += (double)gathers[c] * (n < (double)rows[c] ? n / (double)rows[c] : 1.0);
+            n -= (double)rows[c];
+        }
+        return all > 0 ? reached / all : 1.0;
+    }
+};
+
 // CSR of one orientation plus the work lists of its long rows.
 struct Side {
     bool ready = false;
@@ -73,6 +99,8 @@ struct Side {
     SplitRow *split = nullptr; // [n_split_rows]
     SplitRow *wide = nullptr;  // [n_wide_rows] the split rows with more than kWideSlots slots (any order)
     int n_wide_rows = 0;
+    bool counted = false;      // `counts` is known (count_gathers)
+    GatherCounts counts;
     // Short rows (at most short_row_limit nonzeros) as one contiguous stream: their nonzeros copied
     // in row order, bit 31 of the column marking the last nonzero of a row.  A row without nonzeros
     // contributes one placeholder entry (bit 30) so that it is still written.  The stream is cut into

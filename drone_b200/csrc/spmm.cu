@@ -159,20 +159,60 @@ static bool may_allocate(cudaStream_t st) {
     return status == cudaStreamCaptureStatusNone;
 }
 
-// Width of the column slices a call is cut into (0 = no slicing).  Gathering a slice of w columns touches only
+constexpr int kSliceFloats = 64;
+constexpr double kL2Floats = 25e6;      // of gathered rows that L2 keeps
+
+// How the columns of a call are cut.
+struct Slices {
+    int width = 0;             // 0: in one piece
+    bool long_last = false;    // what is left of less than a slice goes with the slice before it
+    int next(int left) const { return width == 0 || left < width + (long_last ? width : kSliceFloats / 4) ? left : width; }
+    int widest(int F) const { return width == 0 ? F : std::min(F, width + (F % width == 0 ? 0 : long_last ? width : kSliceFloats / 4)); }
+};
+
+// Slices of 64 columns where not even a slice fits L2: by the share of the gathers that go to the rows L2 can keep (GatherCounts), at
+// the rates of gathers out of HBM and out of L2.  Graphs without popular rows gain most: of 300,000 rows of 1 KB L2 keeps a third, of
+// their slices all.  R-MAT graphs, whose popular rows are in L2 at any width, keep calls in one piece (from a third of the gathers
+// missing on; R-MAT-20 F = 256 in one piece / slices 2085 / 2297 us, R-MAT-22 F = 128 2688 / 2861).  Power law, us in one piece /
+// slices: 300,000 rows of 201 F = 256 5908 / 3997, F = 512 14202 / 8627; 400,000 of 61 F = 256 2976 / 1989; 600,000 of 101 F = 128
+// 3186 / 2532, F = 512 16370 / 11643; 150,000 of 37 F = 512 1370 / 1097; 1.2 M of 101 F = 256 16403 / 13709; 2.4 M of 51 F = 256 18120 /
+// 17350.  Rows below 24 nonzeros lose: 2.4 M of 17 F = 128 3072 / 3194.  So do slices that do not start on 128-byte lines (2.4 M of 51
+// F = 180 15246 / 18470), and rows read float by float (600,000 of 31 F = 177 2178 / 2605).
+// A rest of 32 columns is read out of HBM at 5 TB/s instead of 7: where more than half of a slice's gathers miss, it stays with the
+// slice before it (2.4 M of 51, F = 224: in one piece 16389, 3 x 64 + 32 17001).
+static Slices slices_by_counts(const drone_plan *p, const Side &s, int F) {
+    Slices cut;
+    if (!s.counted || !slices_possible(p->n_rows, p->nnz) || F < 2 * kSliceFloats) return cut;
+    const double hbm = 7, l2 = 17, stream = 6.5;      // TB/s
+    const auto picoseconds = [&](int width, double missed) { return 4.0 * width * (missed / hbm + (1 - missed) / l2) + 8 / stream; };
+    const double missed = 1 - s.counts.share(kL2Floats / F), in_slice = 1 - s.counts.share(kL2Floats / kSliceFloats);
+    if (missed < 0.35 || picoseconds(kSliceFloats, in_slice) * F / kSliceFloats > 0.95 * picoseconds(F, missed)) return cut;
+    cut.width = kSliceFloats;
+    cut.long_last = in_slice > 0.5;
+    return cut;
+}
+
+// Column slices of a call.  Gathering a slice of w columns touches only
 // n*w*4 bytes of X; when the whole operand does not fit in L2 but a slice does, running the slices one after the
 // other turns HBM gathers into L2 gathers at the price of re-reading the CSR stream once per slice.
-static int slice_width(const drone_plan *p, int F, bool vec4) {
+// on_lines: the rows of X start on 128-byte lines.
+static Slices column_slices(const drone_plan *p, const Side &s, int F, bool vec4, bool on_lines) {
+    Slices cut;
     const int forced = p->slice_forced;
-    if (forced == 0 || !vec4) return 0;
-    if (forced > 0) return (forced % 4 == 0 && forced < F && F % forced == 0) ? forced : 0;
-    if (p->hot_table) return 0;                         // tagged plan: the hot rows are kept in L2 by their table
-    const double l2_budget = 64e6;                      // about half of the 126 MB L2 for the gathered operand
-    if ((double)p->n_rows * F * 4 <= l2_budget) return 0;
-    for (int w : {128, 64}) {
-        if (w < F && F % w == 0 && (double)p->n_rows * w * 4 <= l2_budget) return w;
+    if (forced == 0 || !vec4) return cut;
+    if (forced > 0) {
+        if (forced % 4 == 0 && forced < F && F % forced == 0) cut.width = forced;
+        return cut;
     }
-    return 0;
+    if (p->hot_table) return cut;                       // tagged plan: the hot rows are kept in L2 by their table
+    const double l2_budget = 64e6;                      // about half of the 126 MB L2 for the gathered operand
+    if ((double)p->n_rows * F * 4 <= l2_budget) return cut;
+    for (int w : {128, 64})
+        if (w < F && F % w == 0 && (double)p->n_rows * w * 4 <= l2_budget) {
+            cut.width = w;
+            return cut;
+        }
+    return on_lines ? slices_by_counts(p, s, F) : cut;
 }
 
 // What a call may ask for beyond the plain product (drone_spmm_opts of the C ABI, already checked).
@@ -258,11 +298,10 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         routed = route != nullptr && vec4 && !y_copied;
         send_after = route != nullptr && !routed;
     }
-    const int slice = slice_width(p, F, vec4);
-    const int width = slice > 0 ? slice : F;
-    p->last_slice_width = slice;
+    const Slices cut = column_slices(p, s, F, vec4, ldx % 32 == 0 && (reinterpret_cast<uintptr_t>(X) & 127) == 0);
+    p->last_slice_width = cut.width;
     if (s.n_partials > 0) {
-        const int rc = ensure_scratch(p, sizeof(float) * (size_t)s.n_partials * (size_t)width);
+        const int rc = ensure_scratch(p, sizeof(float) * (size_t)s.n_partials * (size_t)cut.widest(F));
         if (rc) return rc;
     }
     SpmmArgs a;
@@ -286,11 +325,12 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         a.epi.peer_rows = peer_rows;
         a.epi.route_nvec = F / 4;
     }
-    for (int c0 = 0; c0 < F; c0 += width) {
+    for (int c0 = 0, now; c0 < F; c0 += now) {
+        now = cut.next(F - c0);
         a.gather.X = X + c0;
         a.Y = Y + c0;
         a.epi.route_col0 = c0 / 4;
-        const int rc = run_variant(p, s, a, vec4, width, opt.unit_values);
+        const int rc = run_variant(p, s, a, vec4, now, opt.unit_values);
         if (rc) return rc;
     }
     if (routed) {

@@ -784,3 +784,46 @@ def test_copied_rows_in_place_and_in_classes(cuda_device, f, lead, shift):
     for c in (0, 2):
         plan.spmm(db.OP_AT, x, out=y, row_class=c)
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("n,degree,f,slices", [(30000, 26, 608, 0),            # L2 keeps all rows
+                                               (300000, 24, 256, 64),
+                                               (300000, 24, 232, 0),            # rows that do not start on lines
+                                               (300000, 24, 224, 64),           # a slice of 32 at the end
+                                               (300000, 23, 256, 0),            # below the length from which slices pay
+                                               (900000, 24, 160, 64)])          # the last slice takes the rest with it: 64 + 96
+def test_column_slices_where_none_fits(cuda_device, n, degree, f, slices):
+    """Rows that are gathered equally often, far more of them than L2 keeps: against double, against the call in one piece, and
+    every slice against the narrow call on its columns; with the ReLU and a row scale, and from one orientation alone, which
+    does not know how often its rows are gathered."""
+    gen = torch.Generator(cuda_device).manual_seed(n + f)
+    index = (torch.arange(n + 1, device=cuda_device) * degree).int()
+    dst = torch.randint(0, n, (n, degree), device=cuda_device, generator=gen).sort(dim=1).values.int().reshape(-1)
+    val = torch.rand(n * degree, device=cuda_device, generator=gen) - 0.5
+    x = torch.randn((n, f), device=cuda_device, generator=gen)
+    scale = torch.rand(n, device=cuda_device, generator=gen)
+    plan = db.AggregationPlan(index, dst, values=val)
+    rows = torch.randint(0, n, (500,), device=cuda_device, generator=gen)
+    of = dst.reshape(n, degree)[rows].long()
+    want = (x[of].double() * val.reshape(n, degree)[rows][:, :, None].double()).sum(1)
+    got = plan.spmm(db.OP_A, x)
+    assert plan.stats().last_slice_width == slices
+    # a chain of at most `degree` additions of terms below 3 in size, whose sums stay below 8
+    assert (got[rows] - want).abs().max() <= degree * 8 * 2.0 ** -24
+    lone = db.AggregationPlan(index, dst, values=val, orientations=db.PLAN_A)
+    whole = lone.spmm(db.OP_A, x)
+    assert lone.stats().last_slice_width == 0
+    assert (got - whole).abs().max() <= degree * 8 * 2.0 ** -23
+    scaled = plan.spmm(db.OP_A, x, relu=True, row_scale=scale)
+    assert (scaled - (got * scale[:, None]).clamp(min=0)).abs().max() <= degree * 8 * 2.0 ** -24
+    if slices:
+        ends = {160: (64, 160), 224: (64, 128, 192, 224), 256: (64, 128, 192, 256)}[f]
+        for a, b in zip((0,) + ends[:-1], ends):
+            assert torch.equal(got[:, a:b], lone.spmm(db.OP_A, x[:, a:b].contiguous())), (a, b)
+    back = plan.spmm(db.OP_AT, x)
+    ones = torch.ones(n, dtype=torch.float64, device=cuda_device)
+    row_of = torch.arange(n, device=cuda_device).repeat_interleave(degree)
+    in_row = torch.zeros(n, dtype=torch.float64, device=cuda_device).index_add_(0, row_of, val.double())
+    sums = (ones[None, :] @ back.double())[0]
+    want = (in_row[None, :] @ x.double())[0]      # 1' A' X = (A 1)' X
+    assert (sums - want).abs().max() <= 1e-5 * (in_row.abs().sum() ** 0.5 * 10 + want.abs().max())
