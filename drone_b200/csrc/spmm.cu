@@ -70,6 +70,11 @@ static long long padded_stride(int n_rows, int F) {
     return (fp + 15) / 16 * 16;
 }
 
+// The same for a call that runs in column slices, each of which then starts on a line (slices_by_counts).
+static long long line_stride(int F) { return (F + 31) / 32 * 32; }
+// Nobody asked for that copy: it stays below half a gigabyte.
+static bool lines_fit(int n_rows, int F) { return line_stride(F) * n_rows <= 1 << 27; }
+
 // The copies' buffers.  drone_plan_reserve makes them ahead of time; otherwise the first call that wants them does, unless
 // that call must not allocate (its width was reserved without them, the stream is being captured), they would take more
 // than kPadBytes nobody asked for, or so much did not fit before: the next drone_plan_reserve tries again.
@@ -166,8 +171,10 @@ constexpr double kL2Floats = 25e6;      // of gathered rows that L2 keeps
 struct Slices {
     int width = 0;             // 0: in one piece
     bool long_last = false;    // what is left of less than a slice goes with the slice before it
+    bool by_counts = false;    // by the operand as well: another call of this width may run in one piece
     int next(int left) const { return width == 0 || left < width + (long_last ? width : kSliceFloats / 4) ? left : width; }
-    int widest(int F) const { return width == 0 ? F : std::min(F, width + (F % width == 0 ? 0 : long_last ? width : kSliceFloats / 4)); }
+    // Columns that partial sums are kept for: calls of a width leave room for each other, so that one of them can be captured.
+    int partial_columns(int F) const { return width == 0 || by_counts ? F : width; }
 };
 
 // Slices of 64 columns where not even a slice fits L2: by the share of the gathers that go to the rows L2 can keep (GatherCounts), at
@@ -180,17 +187,32 @@ struct Slices {
 // F = 180 15246 / 18470), and rows read float by float (600,000 of 31 F = 177 2178 / 2605).
 // A rest of 32 columns is read out of HBM at 5 TB/s instead of 7: where more than half of a slice's gathers miss, it stays with the
 // slice before it (2.4 M of 51, F = 224: in one piece 16389, 3 x 64 + 32 17001).
-static Slices slices_by_counts(const drone_plan *p, const Side &s, int F) {
+// copied: X has to be copied for it, at 3 TB/s; the slices then have to save a tenth (600,000 rows of 31, F = 232 2556 / 2294, F = 300
+// 3240 / 3172).
+static Slices slices_by_counts(const drone_plan *p, const Side &s, int F, bool copied) {
     Slices cut;
     if (!s.counted || !slices_possible(p->n_rows, p->nnz) || F < 2 * kSliceFloats) return cut;
-    const double hbm = 7, l2 = 17, stream = 6.5;      // TB/s
+    const double hbm = 7, l2 = 17, stream = 6.5, copying = 3;      // TB/s
     const auto picoseconds = [&](int width, double missed) { return 4.0 * width * (missed / hbm + (1 - missed) / l2) + 8 / stream; };
     const double missed = 1 - s.counts.share(kL2Floats / F), in_slice = 1 - s.counts.share(kL2Floats / kSliceFloats);
-    if (missed < 0.35 || picoseconds(kSliceFloats, in_slice) * F / kSliceFloats > 0.95 * picoseconds(F, missed)) return cut;
+    const double sliced = picoseconds(kSliceFloats, in_slice) * F / kSliceFloats + (copied ? 8.0 * F / copying * p->n_rows / p->nnz : 0);
+    if (missed < 0.35 || sliced > (copied ? 0.9 : 0.95) * picoseconds(F, missed)) return cut;
     cut.width = kSliceFloats;
+    cut.by_counts = true;
     cut.long_last = in_slice > 0.5;
     return cut;
 }
+
+constexpr double kL2Budget = 64e6;                      // about half of the 126 MB L2 for the gathered operand
+
+// Columns of a slice that fits L2 (0: none does).
+static int slices_that_fit(const drone_plan *p, int F) {
+    for (int w : {128, 64})
+        if (w < F && F % w == 0 && (double)p->n_rows * w * 4 <= kL2Budget) return w;
+    return 0;
+}
+
+static bool rows_on_lines(const float *X, long long ldx) { return ldx % 32 == 0 && (reinterpret_cast<uintptr_t>(X) & 127) == 0; }
 
 // Column slices of a call.  Gathering a slice of w columns touches only
 // n*w*4 bytes of X; when the whole operand does not fit in L2 but a slice does, running the slices one after the
@@ -205,14 +227,23 @@ static Slices column_slices(const drone_plan *p, const Side &s, int F, bool vec4
         return cut;
     }
     if (p->hot_table) return cut;                       // tagged plan: the hot rows are kept in L2 by their table
-    const double l2_budget = 64e6;                      // about half of the 126 MB L2 for the gathered operand
-    if ((double)p->n_rows * F * 4 <= l2_budget) return cut;
-    for (int w : {128, 64})
-        if (w < F && F % w == 0 && (double)p->n_rows * w * 4 <= l2_budget) {
-            cut.width = w;
-            return cut;
-        }
-    return on_lines ? slices_by_counts(p, s, F) : cut;
+    if ((double)p->n_rows * F * 4 <= kL2Budget) return cut;
+    cut.width = slices_that_fit(p, F);
+    if (cut.width > 0) return cut;
+    return on_lines ? slices_by_counts(p, s, F, false) : cut;
+}
+
+// Whether rows of F floats, ld apart from base, can be accessed 16 bytes at a time.
+static bool rows_of_vectors(int F, long long ld, const float *base) {
+    return F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
+}
+
+// Whether a call copies X to rows on lines for its slices.  Power law, us in one piece / with the copy: 300,000 rows of 201 F = 180
+// 4264 / 3329, F = 300 8117 / 5658; 300,000 of 41 F = 180 1088 / 920, F = 392 3153 / 2223; 600,000 of 102 F = 152 4755 / 3915, F = 180 5845 /
+// 4478; 180,000 of 101 F = 500 4183 / 2843.  Odd widths keep their route: its two forms add in the same order.
+static bool copy_x_for_slices(const drone_plan *p, const Side &s, int F, const float *X, long long ldx, int row_class) {
+    if (p->slice_forced >= 0 || p->hot_table || row_class >= 0 || rows_on_lines(X, ldx) || slices_that_fit(p, F) > 0) return false;
+    return lines_fit(p->n_rows, F) && slices_by_counts(p, s, F, true).width > 0;
 }
 
 // What a call may ask for beyond the plain product (drone_spmm_opts of the C ABI, already checked).
@@ -223,11 +254,6 @@ struct CallOptions {
     drone_xplan *push_up_to = nullptr;   // the call also sends the mirror rows of Y to their owners
     bool no_allocation = false;
 };
-
-// Whether rows of F floats, ld apart from base, can be accessed 16 bytes at a time.
-static bool rows_of_vectors(int F, long long ld, const float *base) {
-    return F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
-}
 
 // One launch sequence over columns [0, width) of the operands a.gather.X / a.Y point at.
 static int run_variant(const drone_plan *p, const Side &s, SpmmArgs &a, bool vec4, int width, bool unit_values) {
@@ -258,20 +284,29 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     const long long caller_ldy = ldy;
     const int caller_F = F;
     const bool copy_x = !rows_of_vectors(F, ldx, X), copy_y = !rows_of_vectors(F, ldy, Y);
-    bool vec4 = !copy_x && !copy_y;
-    if (!vec4 && F > 8 && worth_copying(p, F)) {
-        const int Fp = (F + 3) & ~3;
-        const long long stride = padded_stride(p->n_rows, F);
-        const size_t x_floats = copy_x ? (size_t)stride * (size_t)p->n_rows : 0, y_floats = copy_y ? (size_t)Fp * (size_t)p->n_rows : 0;
+    bool vec4 = !copy_x && !copy_y, y_copied = false;
+    // Room for the copies: there, or made by this call.
+    const auto room_for = [&](size_t x_floats, size_t y_floats) {
         const size_t missing = sizeof(float) * padding_to_make(p, x_floats, y_floats);
-        vec4 = missing == 0;
-        if (!vec4 && !opt.no_allocation && caller_F > p->reserved_features && missing < p->pad_refused_bytes &&
-            sizeof(float) * (std::max(x_floats, p->pad_x_floats) + std::max(y_floats, p->pad_y_floats)) <= kPadBytes && may_allocate(st)) {
-            vec4 = ensure_padding(p, x_floats, y_floats) == DRONE_OK;
-            if (!vec4) p->pad_refused_bytes = missing;      // rows are accessed float by float, from now on without asking again
-        }
-        if (vec4) {
-            if (copy_x) {
+        if (missing == 0) return true;
+        if (opt.no_allocation || caller_F <= p->reserved_features || missing >= p->pad_refused_bytes ||
+            sizeof(float) * (std::max(x_floats, p->pad_x_floats) + std::max(y_floats, p->pad_y_floats)) > kPadBytes || !may_allocate(st))
+            return false;
+        if (ensure_padding(p, x_floats, y_floats) == DRONE_OK) return true;
+        p->pad_refused_bytes = missing;      // the call does without, from now on without asking again
+        return false;
+    };
+    // Also copied: an X whose rows could be accessed where they lie, but not on lines, for a call that then runs in slices.  Not
+    // under capture: a wider call would replace the buffer that the graph reads.
+    const bool lines = vec4 && copy_x_for_slices(p, s, F, X, ldx, opt.row_class) && may_allocate(st);
+    if (lines || (!vec4 && F > 8 && worth_copying(p, F))) {
+        const int Fp = (F + 3) & ~3;
+        const long long stride = lines ? line_stride(F) : padded_stride(p->n_rows, F);
+        const size_t rows = (size_t)p->n_rows;
+        if (room_for(copy_x || lines ? (size_t)stride * rows : 0, copy_y ? (size_t)Fp * rows : 0)) {
+            vec4 = true;
+            y_copied = copy_y;
+            if (copy_x || lines) {
                 const long long total = (long long)p->n_rows * (Fp / 4);
                 pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
                     X, ldx, p->n_rows, F, Fp / 4, (int)stride, p->pad_x);
@@ -286,7 +321,6 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
             F = Fp;
         }
     }
-    const bool y_copied = vec4 && copy_y;
     // The upward half of the exchange inside this call: the kernels store mirror rows into their owners' memory
     // (rows read as float4 where they lie), or the copy kernel sends them afterwards (any other layout).
     bool routed = false, send_after = false;
@@ -298,10 +332,10 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         routed = route != nullptr && vec4 && !y_copied;
         send_after = route != nullptr && !routed;
     }
-    const Slices cut = column_slices(p, s, F, vec4, ldx % 32 == 0 && (reinterpret_cast<uintptr_t>(X) & 127) == 0);
+    const Slices cut = column_slices(p, s, F, vec4, rows_on_lines(X, ldx));
     p->last_slice_width = cut.width;
     if (s.n_partials > 0) {
-        const int rc = ensure_scratch(p, sizeof(float) * (size_t)s.n_partials * (size_t)cut.widest(F));
+        const int rc = ensure_scratch(p, sizeof(float) * (size_t)s.n_partials * (size_t)cut.partial_columns(F));
         if (rc) return rc;
     }
     SpmmArgs a;
@@ -533,7 +567,7 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
     }
     if ((what & DRONE_RESERVE_PADDED_ROWS) && p->n_rows > 0) {
         long long stride = 0;      // of the widths up to max_features, the one whose copy is largest
-        for (int f = 9; f <= max_features; ++f) stride = std::max(stride, padded_stride(p->n_rows, f));
+        for (int f = 9; f <= max_features; ++f) stride = std::max(stride, std::max(padded_stride(p->n_rows, f), slices_possible(p->n_rows, p->nnz) && lines_fit(p->n_rows, f) ? line_stride(f) : 0));
         rc = replace_padding(p, (size_t)stride * (size_t)p->n_rows, (size_t)copied_features * (size_t)p->n_rows);
         if (rc) return rc;
     }

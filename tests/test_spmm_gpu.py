@@ -788,7 +788,9 @@ def test_copied_rows_in_place_and_in_classes(cuda_device, f, lead, shift):
 
 @pytest.mark.parametrize("n,degree,f,slices", [(30000, 26, 608, 0),            # L2 keeps all rows
                                                (300000, 24, 256, 64),
-                                               (300000, 24, 232, 0),            # rows that do not start on lines
+                                               (300000, 24, 232, 64),           # rows that do not start on lines: X is copied
+                                               (300000, 30, 460, 0),            # for which the copy is too large
+                                               (300000, 24, 230, 0),
                                                (300000, 24, 224, 64),           # a slice of 32 at the end
                                                (300000, 23, 256, 0),            # below the length from which slices pay
                                                (900000, 24, 160, 64)])          # the last slice takes the rest with it: 64 + 96
@@ -817,9 +819,22 @@ def test_column_slices_where_none_fits(cuda_device, n, degree, f, slices):
     scaled = plan.spmm(db.OP_A, x, relu=True, row_scale=scale)
     assert (scaled - (got * scale[:, None]).clamp(min=0)).abs().max() <= degree * 8 * 2.0 ** -24
     if slices:
-        ends = {160: (64, 160), 224: (64, 128, 192, 224), 256: (64, 128, 192, 256)}[f]
+        ends = {160: (64, 160), 224: (64, 128, 192, 224), 256: (64, 128, 192, 256), 232: (64, 128, 192, 232)}[f]
         for a, b in zip((0,) + ends[:-1], ends):
             assert torch.equal(got[:, a:b], lone.spmm(db.OP_A, x[:, a:b].contiguous())), (a, b)
+    if slices and f % 32:      # a plan that must not allocate, and a call under capture, do without the copies
+        captured, graph = torch.empty_like(x), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            plan.spmm(db.OP_A, x, out=captured)
+        graph.replay()
+        assert torch.equal(captured, whole)
+        del graph
+        plan.close()
+        plan = db.AggregationPlan(index, dst, values=val)
+        plan.reserve(f)
+        assert (plan.spmm(db.OP_A, x) - whole).abs().max() <= degree * 8 * 2.0 ** -23 and plan.stats().last_slice_width == 0
+        plan.reserve(f, padded_rows=True)
+        assert torch.equal(plan.spmm(db.OP_A, x), got) and plan.stats().last_slice_width == slices
     back = plan.spmm(db.OP_AT, x)
     ones = torch.ones(n, dtype=torch.float64, device=cuda_device)
     row_of = torch.arange(n, device=cuda_device).repeat_interleave(degree)
