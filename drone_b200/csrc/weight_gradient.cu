@@ -162,7 +162,7 @@ using namespace drone;
 extern "C" {
 
 int drone_weight_gradient_scratch(int K, int M, int N, long long *n_floats) {
-    DRONE_REQUIRE(K >= 0 && M >= 1 && N >= 1 && M <= 1 << 15 && N <= 1 << 15 && n_floats, "drone_weight_gradient_scratch: K=%d M=%d N=%d", K, M, N);
+    DRONE_REQUIRE(K >= 0 && K <= 1 << 30 && M >= 1 && N >= 1 && M <= 1 << 15 && N <= 1 << 15 && n_floats, "drone_weight_gradient_scratch: K=%d M=%d N=%d", K, M, N);
     int sms = 0;
     const int rc = device_sms(&sms);
     if (rc) return rc;
@@ -173,7 +173,7 @@ int drone_weight_gradient_scratch(int K, int M, int N, long long *n_floats) {
 
 int drone_weight_gradient(int K, int M, int N, const float *d_A, int lda, const float *d_B, int ldb, float *d_C, float *d_scratch,
                           long long n_scratch, void *stream) {
-    DRONE_REQUIRE(K >= 0 && M >= 1 && N >= 1 && M <= 1 << 15 && N <= 1 << 15 && lda >= M && ldb >= N,
+    DRONE_REQUIRE(K >= 0 && K <= 1 << 30 && M >= 1 && N >= 1 && M <= 1 << 15 && N <= 1 << 15 && lda >= M && ldb >= N,
                   "drone_weight_gradient: K=%d M=%d N=%d lda=%d ldb=%d", K, M, N, lda, ldb);
     DRONE_REQUIRE(d_C && (K == 0 || (d_A && d_B)), "drone_weight_gradient: NULL argument");
     cudaStream_t st = (cudaStream_t)stream;

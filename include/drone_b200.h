@@ -334,7 +334,7 @@ int drone_softmax_loss(int n_rows, int classes, const float *d_logits, int ld, c
 int drone_relu_mask(int n_rows, int F, float *d_grad, int ld_grad, const float *d_out, int ld_out, void *stream);
 
 /* d_C[M, N] (dense rows) = A^T B for A [K, M] and B [K, N]: the weight gradient of a dense layer over K vertices
- * (CUDAMatmul::backward, cuda_module.cu:63-86), in float.  M, N <= 32768.  d_scratch: at least as many floats as
+ * (CUDAMatmul::backward, cuda_module.cu:63-86), in float.  K <= 2^30, M, N <= 32768.  d_scratch: at least as many floats as
  * drone_weight_gradient_scratch says (the same device current).  The same sums in the same order every time.  Asynchronous. */
 int drone_weight_gradient_scratch(int K, int M, int N, long long *n_floats);
 int drone_weight_gradient(int K, int M, int N, const float *d_A, int lda, const float *d_B, int ldb, float *d_C, float *d_scratch,

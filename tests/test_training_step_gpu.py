@@ -84,3 +84,12 @@ def test_labels_elsewhere_are_refused(cuda_device):
     for truth in (torch.zeros(6, dtype=torch.int32), torch.zeros(4, dtype=torch.int32, device=cuda_device)):
         with pytest.raises(RuntimeError):
             model(truth)._softmax_loss(logits)
+
+
+def test_sizes_beyond_the_row_numbers_are_refused(cuda_device):
+    """Rows are numbered in 32 bits, a share beyond the last one: more than 2^30 rows are an error before anything is launched."""
+    import ctypes as C
+    from drone_b200._lib import lib
+    size = C.c_longlong(0)
+    assert lib().drone_weight_gradient_scratch(2 ** 30 + 1, 4, 4, C.byref(size)) == -1
+    assert lib().drone_weight_gradient_scratch(2 ** 30, 4, 4, C.byref(size)) == 0 and size.value > 0
