@@ -129,7 +129,7 @@ class GCN:
         n, classes = logits.shape
         if (self._kernels and logits.is_contiguous() and self._per_row(self.labelled, torch.bool, n)
                 and self._per_row(self.safe_truth, torch.int64, n)):
-            self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), device=logits.device)
+            self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), dtype=torch.float32, device=logits.device)
             self._call("drone_softmax_loss", n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
                        self.labelled.data_ptr(), self.d_logits.data_ptr(), classes, self.loss.data_ptr(), self._scratch.data_ptr(),
                        self._stream())
@@ -164,7 +164,7 @@ class GCN:
             size = C.c_longlong(0)
             self._call("drone_weight_gradient_scratch", k, m, n, C.byref(size))
             floats = self._shares[(k, m, n)] = size.value
-        out, parts = torch.empty((m, n), device=g.device), torch.empty(floats, device=g.device)
+        out, parts = (torch.empty(shape, dtype=torch.float32, device=g.device) for shape in ((m, n), floats))
         self._call("drone_weight_gradient", k, m, n, a.data_ptr(), max(m, a.stride(0)), g.data_ptr(), n, out.data_ptr(),
                    parts.data_ptr(), floats, self._stream())
         return out

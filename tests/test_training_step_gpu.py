@@ -93,3 +93,23 @@ def test_sizes_beyond_the_row_numbers_are_refused(cuda_device):
     size = C.c_longlong(0)
     assert lib().drone_weight_gradient_scratch(2 ** 30 + 1, 4, 4, C.byref(size)) == -1
     assert lib().drone_weight_gradient_scratch(2 ** 30, 4, 4, C.byref(size)) == 0 and size.value > 0
+
+
+@pytest.mark.parametrize("default", [torch.float64, torch.bfloat16, torch.float16])
+def test_default_dtype_changed_after_the_model_was_made(cuda_device, default):
+    """What the kernels write into is float32 whatever torch makes by default when the step runs."""
+    gen = torch.Generator(cuda_device).manual_seed(11)
+    n, dims = 5003, (65, 24, 7)
+    x = torch.randn((n, dims[0]), device=cuda_device, generator=gen)
+    truth = torch.randint(-1, dims[-1], (n,), device=cuda_device, generator=gen, dtype=torch.int32)
+    weights = [torch.randn((a, b), device=cuda_device, generator=gen) / 8 for a, b in zip(dims, dims[1:])]
+    model = gcn.GCN(None, x, truth, weights, aggregate=lambda op, src, out: out.copy_(src))
+    assert model._kernels
+    want = [model.forward(), *model.backward()]
+    try:
+        torch.set_default_dtype(default)
+        got = [model.forward(), *model.backward()]
+    finally:
+        torch.set_default_dtype(torch.float32)
+    for a, b in zip(got, want):
+        assert a.dtype == torch.float32 and torch.equal(a, b)
