@@ -1084,6 +1084,11 @@ int drone_plan_destroy(drone_plan *p) {
     cudaFree(p->pad_x);
     cudaFree(p->pad_y);
     cudaFree(p->scratch);
+    while (drone_plan::Kept *k = p->kept) {
+        cudaFree(k->buffer);
+        p->kept = k->before;
+        delete k;
+    }
     cudaFree(p->stage_x);
     cudaFree(p->stage_y);
     for (int s = 0; s < 2; ++s) {

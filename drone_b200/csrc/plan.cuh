@@ -202,6 +202,11 @@ struct drone_plan {
     float *pad_x = nullptr, *pad_y = nullptr;
     size_t pad_x_floats = 0, pad_y_floats = 0;
     size_t pad_refused_bytes = ~(size_t)0;   // a call that needs this much new room for copies does without: so much did not fit
+    // A graph captured from a call goes on using the buffers that the call used: replaced by larger ones they are kept until the
+    // plan goes (give_back_replaced).
+    struct Kept { void *buffer; Kept *before; };
+    Kept *kept = nullptr;
+    bool scratch_captured = false, pad_x_captured = false, pad_y_captured = false;
     int reserved_features = 0;     // drone_plan_reserve: calls up to this width allocate nothing
     int chunk_blocks_per_sm = 0;   // cap on resident blocks of the chunk kernel per SM (0: as many as fit)
     cudaStream_t own_stream = nullptr;

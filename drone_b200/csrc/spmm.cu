@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <new>
 
 namespace drone {
 
@@ -45,11 +46,33 @@ __global__ void unpad_rows_kernel(const float *__restrict__ padded, int Fp, cons
     }
 }
 
+// Whether work put on this stream runs now; otherwise (or where the stream does not say) it becomes part of a graph, and nothing
+// may be allocated.
+static bool runs_now(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status == cudaStreamCaptureStatusNone;
+}
+
+// A buffer that has been replaced is freed, unless a captured graph uses it.
+static void give_back_replaced(drone_plan *p, float *buffer, bool *captured) {
+    if (!*captured) {
+        cudaFree(buffer);
+        return;
+    }
+    *captured = false;
+    drone_plan::Kept *k = new (std::nothrow) drone_plan::Kept{buffer, p->kept};
+    if (k) p->kept = k;      // else it outlives the plan
+}
+
 static int ensure_scratch(drone_plan *p, size_t bytes) {
     if (bytes <= p->scratch_bytes) return DRONE_OK;
     // grow: frees and reallocates, so earlier calls that use the scratch must have finished
     DRONE_CUDA(cudaDeviceSynchronize());
-    cudaFree(p->scratch);
+    give_back_replaced(p, p->scratch, &p->scratch_captured);
     p->scratch = nullptr;
     p->scratch_bytes = 0;
     DRONE_CUDA(cudaMalloc(&p->scratch, bytes));
@@ -99,25 +122,25 @@ static int ensure_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
     }
     if ((new_x && p->pad_x) || (new_y && p->pad_y)) cudaDeviceSynchronize();      // calls in flight use what is replaced
     if (new_x) {
-        cudaFree(p->pad_x);
+        give_back_replaced(p, p->pad_x, &p->pad_x_captured);
         p->pad_x = x;
         p->pad_x_floats = x_floats;
     }
     if (new_y) {
-        cudaFree(p->pad_y);
+        give_back_replaced(p, p->pad_y, &p->pad_y_captured);
         p->pad_y = y;
         p->pad_y_floats = y_floats;
     }
     return DRONE_OK;
 }
 
-// drone_plan_reserve's form: where old and new buffers do not fit together the old ones go first, and come back if the
-// new ones do not fit alone either.
+// drone_plan_reserve's form: where old and new buffers do not fit together the old ones go first (unless a graph uses them), and
+// come back if the new ones do not fit alone either.
 static int replace_padding(drone_plan *p, size_t x_floats, size_t y_floats) {
     p->pad_refused_bytes = ~(size_t)0;
     if (ensure_padding(p, x_floats, y_floats) == DRONE_OK) return DRONE_OK;
     const size_t old_x = p->pad_x_floats, old_y = p->pad_y_floats;
-    if (old_x + old_y == 0) return DRONE_E_CUDA;
+    if (old_x + old_y == 0 || p->pad_x_captured || p->pad_y_captured) return DRONE_E_CUDA;
     DRONE_CUDA(cudaDeviceSynchronize());
     cudaFree(p->pad_x);
     cudaFree(p->pad_y);
@@ -153,15 +176,6 @@ static bool worth_copying(const drone_plan *p, int F) {
     if (whole_steps && per_row >= 60) return true;
     if (per_row >= 64) return many || F <= 512 || bytes <= 100e6;
     return F > 384 && per_row >= 12 && bytes <= 40e6;
-}
-
-static bool may_allocate(cudaStream_t st) {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return status == cudaStreamCaptureStatusNone;
 }
 
 constexpr int kSliceFloats = 64;
@@ -290,15 +304,15 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         const size_t missing = sizeof(float) * padding_to_make(p, x_floats, y_floats);
         if (missing == 0) return true;
         if (opt.no_allocation || caller_F <= p->reserved_features || missing >= p->pad_refused_bytes ||
-            sizeof(float) * (std::max(x_floats, p->pad_x_floats) + std::max(y_floats, p->pad_y_floats)) > kPadBytes || !may_allocate(st))
+            sizeof(float) * (std::max(x_floats, p->pad_x_floats) + std::max(y_floats, p->pad_y_floats)) > kPadBytes || !runs_now(st))
             return false;
         if (ensure_padding(p, x_floats, y_floats) == DRONE_OK) return true;
         p->pad_refused_bytes = missing;      // the call does without, from now on without asking again
         return false;
     };
     // Also copied: an X whose rows could be accessed where they lie, but not on lines, for a call that then runs in slices.  Not
-    // under capture: a wider call would replace the buffer that the graph reads.
-    const bool lines = vec4 && copy_x_for_slices(p, s, F, X, ldx, opt.row_class) && may_allocate(st);
+    // under capture.
+    const bool lines = vec4 && copy_x_for_slices(p, s, F, X, ldx, opt.row_class) && runs_now(st);
     if (lines || (!vec4 && F > 8 && worth_copying(p, F))) {
         const int Fp = (F + 3) & ~3;
         const long long stride = lines ? line_stride(F) : padded_stride(p->n_rows, F);
@@ -306,6 +320,10 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         if (room_for(copy_x || lines ? (size_t)stride * rows : 0, copy_y ? (size_t)Fp * rows : 0)) {
             vec4 = true;
             y_copied = copy_y;
+            if (!runs_now(st)) {
+                p->pad_x_captured |= copy_x || lines;
+                p->pad_y_captured |= copy_y;
+            }
             if (copy_x || lines) {
                 const long long total = (long long)p->n_rows * (Fp / 4);
                 pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
@@ -337,6 +355,7 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     if (s.n_partials > 0) {
         const int rc = ensure_scratch(p, sizeof(float) * (size_t)s.n_partials * (size_t)cut.partial_columns(F));
         if (rc) return rc;
+        if (!opt.no_allocation && !p->scratch_captured) p->scratch_captured = !runs_now(st);      // else it is not the plan's
     }
     SpmmArgs a;
     a.side = &s;

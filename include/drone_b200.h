@@ -205,7 +205,8 @@ int drone_spmm_rows(drone_plan *plan, int orientation, int row_class, int F,
  *                                Everywhere else such rows are accessed float by float; either way adds in the same
  *                                order.
  * After it, drone_spmm / drone_spmm_rows / drone_spmm_host with F <= max_features reach neither cudaMalloc nor a
- * device-wide synchronisation.
+ * device-wide synchronisation.  A wider call may replace the plan's buffers by larger ones; a graph captured before that
+ * keeps those it was captured with, until the plan is destroyed.
  * Stands where the reference sizes its cuSPARSE workspace on the first training step,
  * cuda_gcn/src/cuda/cuda_module.cu:234-244 (cusparseSpMM_bufferSize, cudaFree + cudaMalloc of sparseBuffer).
  */

@@ -1,0 +1,52 @@
+"""Routes of an aggregation call that its operands, the plan's buffers or the stream decide, and what must not depend on them."""
+import pytest
+import torch
+
+import drone_b200 as db
+from drone_b200 import graphgen as gg
+
+pytestmark = pytest.mark.gpu
+
+
+def uniform_plan(dev, n, degree, seed):
+    """Rows of equally many columns drawn at random: forward rows are short, rows of the transpose differ in length."""
+    gen = torch.Generator(dev).manual_seed(seed)
+    index = (torch.arange(n + 1, device=dev) * degree).int()
+    dst = torch.randint(0, n, (n, degree), device=dev, generator=gen).sort(dim=1).values.int().reshape(-1)
+    val = torch.rand(n * degree, device=dev, generator=gen) - 0.5
+    return (lambda: db.AggregationPlan(index, dst, values=val)), gen
+
+
+@pytest.mark.parametrize("n,degree,first,wider", [(30000, 40, 41, 63),         # copies of X and Y, by a wider call of an odd width
+                                                  (300000, 24, 29, 232),       # the copy of X, by a call on aligned rows
+                                                  (0, 0, 32, 64)])             # partial sums
+def test_buffers_of_a_captured_call_outlive_their_replacement(cuda_device, n, degree, first, wider):
+    """A graph captured from a call runs on with what the call used, also after a wider call has replaced the plan's buffers by
+    larger ones and other tensors lie where memory came free."""
+    if n:
+        make, gen = uniform_plan(cuda_device, n, degree, n)
+        plan = make()
+    else:
+        n, u, v = gg.rmat_graph(13, 16, seed=3, device=cuda_device, symmetrise=True, self_loops="add")
+        index, dst = gg.csr_by_source(u, v, n)
+        in_deg, out_deg = gg.degrees(u, v, n)
+        plan, gen = db.AggregationPlan(index, dst, in_degree=in_deg, out_degree=out_deg), torch.Generator(cuda_device).manual_seed(1)
+        assert plan.stats().n_partials[db.OP_AT] > 0
+    x = torch.randn((n, first), device=cuda_device, generator=gen)
+    want = plan.spmm(db.OP_AT, x)
+    out, graph = torch.zeros_like(want), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.spmm(db.OP_AT, x, out=out)
+    for width in (wider, 2 * wider):
+        wide = torch.randn((n, width), device=cuda_device, generator=gen)
+        again = plan.spmm(db.OP_AT, wide)
+        torch.cuda.synchronize()
+        junk = [torch.full((size,), float("nan"), device=cuda_device) for size in [1 << 16] * 64 + [1 << 22] * 16]
+        out.zero_()
+        graph.replay()
+        assert torch.equal(out, want)
+        assert torch.equal(plan.spmm(db.OP_AT, wide), again)      # what the graph writes is not the wider call's
+        assert torch.equal(plan.spmm(db.OP_AT, x), want)
+        del junk
+    del graph
+    plan.close()
