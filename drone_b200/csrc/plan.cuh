@@ -208,6 +208,7 @@ struct drone_plan {
     Kept *kept = nullptr;
     bool scratch_captured = false, pad_x_captured = false, pad_y_captured = false;
     int reserved_features = 0;     // drone_plan_reserve: calls up to this width allocate nothing
+    int reserved_copies = 0;       // ... and up to this one have room for their copies
     int chunk_blocks_per_sm = 0;   // cap on resident blocks of the chunk kernel per SM (0: as many as fit)
     cudaStream_t own_stream = nullptr;
     // drone_spmm_host with pinned operands: second stream and one event per column half for the copy that runs ahead

@@ -252,11 +252,14 @@ static bool rows_of_vectors(int F, long long ld, const float *base) {
     return F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
 }
 
-// Whether a call copies X to rows on lines for its slices.  Power law, us in one piece / with the copy: 300,000 rows of 201 F = 180
-// 4264 / 3329, F = 300 8117 / 5658; 300,000 of 41 F = 180 1088 / 920, F = 392 3153 / 2223; 600,000 of 102 F = 152 4755 / 3915, F = 180 5845 /
-// 4478; 180,000 of 101 F = 500 4183 / 2843.  Odd widths keep their route: its two forms add in the same order.
-static bool copy_x_for_slices(const drone_plan *p, const Side &s, int F, const float *X, long long ldx, int row_class) {
-    if (p->slice_forced >= 0 || p->hot_table || row_class >= 0 || rows_on_lines(X, ldx) || slices_that_fit(p, F) > 0) return false;
+// Whether X is to be copied to rows on lines for the slices of a call (where there is room, spmm_impl).  Power law, us in one
+// piece / in slices of X where it lies / of the copy: 300,000 rows of 201 F = 180 4075 / 3455 / 2698, F = 300 7928 / 6025 / 4552; 300,000
+// of 41 F = 180 1151 / 1041 / 937, F = 392 3171 / 2188 / 2167; 600,000 of 101 F = 152 4693 / 4872 / 3713, F = 180 5739 / 5878 / 4027;
+// 690,000 of 121 F = 180 8133 / 8651 / 5742; 180,000 of 101 F = 500 4152 / 2624 / 2517.  A plan that was reserved for the width without
+// the copies keeps its calls in one piece.
+static bool copy_x_for_slices(const drone_plan *p, const Side &s, int F, const float *X, long long ldx) {
+    if (p->slice_forced >= 0 || p->hot_table || rows_on_lines(X, ldx) || slices_that_fit(p, F) > 0) return false;
+    if (F <= p->reserved_features && F > p->reserved_copies) return false;
     return lines_fit(p->n_rows, F) && slices_by_counts(p, s, F, true).width > 0;
 }
 
@@ -293,12 +296,25 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     const Side &s = p->side[orientation];
     if (p->n_rows == 0) return DRONE_OK;
     // Operands whose rows cannot be accessed as float4 where they lie are copied to where they can (X before the kernels,
-    // Y after them), where that is worth it.
+    // Y after them), where that is worth it; also an X whose rows could, but do not start on lines, for a call that then runs in
+    // slices.
     float *const caller_Y = Y;
     const long long caller_ldy = ldy;
-    const int caller_F = F;
-    const bool copy_x = !rows_of_vectors(F, ldx, X), copy_y = !rows_of_vectors(F, ldy, Y);
-    bool vec4 = !copy_x && !copy_y, y_copied = false;
+    const int caller_F = F, Fp = (F + 3) & ~3;
+    const bool x_vectors = rows_of_vectors(F, ldx, X), y_vectors = rows_of_vectors(F, ldy, Y);
+    bool vec4 = x_vectors && y_vectors;
+    const bool to_vectors = !vec4 && F > 8 && worth_copying(p, F), to_lines = vec4 && copy_x_for_slices(p, s, F, X, ldx);
+    bool copy_x = to_lines || (to_vectors && !x_vectors), copy_y = to_vectors && !y_vectors;
+    const long long stride = to_lines ? line_stride(F) : padded_stride(p->n_rows, F);
+    // The columns are cut as for the copies also where these have no room, or are left out: a row class, a call under capture and
+    // one that found no memory add in the order of the whole, eager call.
+    const Slices cut = column_slices(p, s, Fp, vec4 || to_vectors, copy_x ? stride % 32 == 0 : rows_on_lines(X, ldx));
+    // Every class of rows copies X anew, which a small class does not make up for (us for all classes, 2 / 4 / 16 equal ones, X where
+    // it lies against copied: 300,000 rows of 201 F = 180 4035 / 4161 / 6665 and 3312 / 3547 / 6878, of 41 F = 392 2462 / 3005 / 6443 and
+    // 2549 / 3432 / 8751, 690,000 of 121 F = 180 9156 / 9550 / 11661 and 6974 / 7257 / 11632).
+    if (to_lines && opt.row_class >= 0 && p->n_classes > 1 &&
+        (p->class_start[opt.row_class + 1] - p->class_start[opt.row_class]) < p->n_rows / 8)
+        copy_x = false;
     // Room for the copies: there, or made by this call.
     const auto room_for = [&](size_t x_floats, size_t y_floats) {
         const size_t missing = sizeof(float) * padding_to_make(p, x_floats, y_floats);
@@ -310,34 +326,28 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         p->pad_refused_bytes = missing;      // the call does without, from now on without asking again
         return false;
     };
-    // Also copied: an X whose rows could be accessed where they lie, but not on lines, for a call that then runs in slices.  Not
-    // under capture.
-    const bool lines = vec4 && copy_x_for_slices(p, s, F, X, ldx, opt.row_class) && runs_now(st);
-    if (lines || (!vec4 && F > 8 && worth_copying(p, F))) {
-        const int Fp = (F + 3) & ~3;
-        const long long stride = lines ? line_stride(F) : padded_stride(p->n_rows, F);
-        const size_t rows = (size_t)p->n_rows;
-        if (room_for(copy_x || lines ? (size_t)stride * rows : 0, copy_y ? (size_t)Fp * rows : 0)) {
-            vec4 = true;
-            y_copied = copy_y;
-            if (!runs_now(st)) {
-                p->pad_x_captured |= copy_x || lines;
-                p->pad_y_captured |= copy_y;
-            }
-            if (copy_x || lines) {
-                const long long total = (long long)p->n_rows * (Fp / 4);
-                pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
-                    X, ldx, p->n_rows, F, Fp / 4, (int)stride, p->pad_x);
-                DRONE_LAUNCH_CHECK("pad_rows_kernel");
-                X = p->pad_x;
-                ldx = stride;
-            }
-            if (copy_y) {
-                Y = p->pad_y;
-                ldy = Fp;
-            }
-            F = Fp;
+    const size_t rows = (size_t)p->n_rows;
+    if ((copy_x || copy_y) && room_for(copy_x ? (size_t)stride * rows : 0, copy_y ? (size_t)Fp * rows : 0)) {
+        if (!runs_now(st)) {
+            p->pad_x_captured |= copy_x;
+            p->pad_y_captured |= copy_y;
         }
+        if (copy_x) {
+            const long long total = (long long)p->n_rows * (Fp / 4);
+            pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(X, ldx, p->n_rows, F, Fp / 4,
+                                                                                                    (int)stride, p->pad_x);
+            DRONE_LAUNCH_CHECK("pad_rows_kernel");
+            X = p->pad_x;
+            ldx = stride;
+        }
+        if (copy_y) {
+            Y = p->pad_y;
+            ldy = Fp;
+        }
+        vec4 = true;
+        F = Fp;
+    } else {
+        copy_x = copy_y = false;
     }
     // The upward half of the exchange inside this call: the kernels store mirror rows into their owners' memory
     // (rows read as float4 where they lie), or the copy kernel sends them afterwards (any other layout).
@@ -347,10 +357,9 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     if (opt.push_up_to) {
         const int rc = p2p_route_begin(opt.push_up_to, p->n_rows, caller_F, &route, &peer_rows);
         if (rc) return rc;
-        routed = route != nullptr && vec4 && !y_copied;
+        routed = route != nullptr && vec4 && !copy_y;
         send_after = route != nullptr && !routed;
     }
-    const Slices cut = column_slices(p, s, F, vec4, rows_on_lines(X, ldx));
     p->last_slice_width = cut.width;
     if (s.n_partials > 0) {
         const int rc = ensure_scratch(p, sizeof(float) * (size_t)s.n_partials * (size_t)cut.partial_columns(F));
@@ -379,18 +388,18 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
         a.epi.route_nvec = F / 4;
     }
     for (int c0 = 0, now; c0 < F; c0 += now) {
-        now = cut.next(F - c0);
+        now = cut.next(Fp - c0);
         a.gather.X = X + c0;
         a.Y = Y + c0;
         a.epi.route_col0 = c0 / 4;
-        const int rc = run_variant(p, s, a, vec4, now, opt.unit_values);
+        const int rc = run_variant(p, s, a, vec4, std::min(now, F - c0), opt.unit_values);
         if (rc) return rc;
     }
     if (routed) {
         const int rc = p2p_route_publish(opt.push_up_to, st);
         if (rc) return rc;
     }
-    if (y_copied) {
+    if (copy_y) {
         const int *rows = nullptr;
         int n_out = p->n_rows;
         if (opt.row_class >= 0 && p->row_order) {      // only the rows this call computed
@@ -591,6 +600,7 @@ int drone_plan_reserve(drone_plan *p, int max_features, int what) {
         if (rc) return rc;
     }
     p->reserved_features = std::max(p->reserved_features, max_features);
+    if (what & DRONE_RESERVE_PADDED_ROWS) p->reserved_copies = std::max(p->reserved_copies, max_features);
     return DRONE_OK;
 }
 

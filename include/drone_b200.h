@@ -116,7 +116,12 @@ int drone_plan_get_csr(const drone_plan *plan, int orientation,
  * cuda_gcn/src/cuda/cuda_module.cu:233-246 (together with out->zero(), :214);
  * orientation DRONE_OP_A replaces the backward call, :323-336.
  * 1 <= F <= 1024.  fp32 data, fp32 accumulation, fixed summation order:
- * two calls on the same inputs give bit-identical results.
+ * two calls on the same inputs give bit-identical results, captured in a graph
+ * or not and whatever device memory is free.  The order of a row's additions
+ * follows from the plan, the orientation, F and the layout of the operands
+ * (whether rows can be read 16 bytes at a time, whether those of X start on
+ * 128-byte lines), and where DRONE_RESERVE_PADDED_ROWS says so from what was
+ * reserved: large operands are gathered in column slices.
  * Asynchronous on `stream`.
  */
 int drone_spmm(drone_plan *plan, int orientation, int F,
@@ -204,6 +209,13 @@ int drone_spmm_rows(drone_plan *plan, int orientation, int row_class, int F,
  *                                the stream is being captured.
  *                                Everywhere else such rows are accessed float by float; either way adds in the same
  *                                order.
+ *                                The copy of X also serves operands that can be read 16 bytes at a time but whose rows do
+ *                                not start on 128-byte lines, where the call is gathered in column slices for which that
+ *                                pays (F >= 128, 24 and more nonzeros a row, a copy of at most 512 MB).  A plan that was not
+ *                                reserved for the width makes that room too, on the first such call, and keeps it.  A plan
+ *                                reserved for it without the copies runs these calls in one piece, which adds in another
+ *                                order; a call that finds no room, or is captured before there is any, runs the slices on X
+ *                                where it lies, with the same bits as on the copy.
  * After it, drone_spmm / drone_spmm_rows / drone_spmm_host with F <= max_features reach neither cudaMalloc nor a
  * device-wide synchronisation.  A wider call may replace the plan's buffers by larger ones; a graph captured before that
  * keeps those it was captured with, until the plan is destroyed.

@@ -50,3 +50,40 @@ def test_buffers_of_a_captured_call_outlive_their_replacement(cuda_device, n, de
         del junk
     del graph
     plan.close()
+
+
+@pytest.mark.parametrize("n,degree,f", [(300000, 40, 180), (300000, 24, 232),       # X copied to rows on lines for its slices
+                                        (300000, 24, 256), (200000, 30, 128),       # slices of X where it lies: by counts, and that fit L2
+                                        (200000, 33, 127), (300000, 64, 159)])      # odd widths, whose copies run in slices
+def test_same_bits_in_classes_under_capture_and_without_room(cuda_device, n, degree, f):
+    """Calls that run in column slices: class by class, captured on a plan that has no copies yet, and where copies find no room
+    the result has the bits of the whole, eager call."""
+    make, gen = uniform_plan(cuda_device, n, degree, n + f)
+    x = torch.randn((n, f), device=cuda_device, generator=gen)
+    narrow = torch.randn((n, 9), device=cuda_device, generator=gen)
+    plan, fresh = make(), make()
+    for op in (db.OP_A, db.OP_AT):
+        want = plan.spmm(op, x)
+        assert plan.stats().last_slice_width == 64 and plan.stats().n_partials[op] == 0
+        out, graph = torch.empty_like(x), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            fresh.spmm(op, x, out=out)
+        graph.replay()
+        assert torch.equal(out, want)
+        del graph
+        if f % 4:      # copies neither reserved nor made by the call
+            bare = make()
+            bare.reserve(f)
+            assert torch.equal(bare.spmm(op, x), want)
+            bare.close()
+    for classes in (3, 16):
+        row_class = torch.randint(0, classes, (n,), device=cuda_device, generator=gen, dtype=torch.int32)
+        plan.set_row_classes(row_class, classes)
+        for op in (db.OP_A, db.OP_AT):
+            want, out = plan.spmm(op, x), torch.full_like(x, 7.0)
+            plan.spmm(op, x, out=out, row_class=1)
+            assert (out[row_class != 1] == 7.0).all()
+            for c in (0, *range(2, classes)):
+                plan.spmm(op, x, out=out, row_class=c)
+            assert torch.equal(out, want)
+    assert torch.equal(plan.spmm(db.OP_AT, narrow), fresh.spmm(db.OP_AT, narrow))
