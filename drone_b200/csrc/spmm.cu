@@ -765,20 +765,17 @@ extern "C" int drone_spmm_static_scratch(drone_plan *p, int orientation, int F, 
     float *partials = nullptr;
     rc = drone::static_partials_address(p->device, &partials);
     if (rc == DRONE_OK) {
-        // same route as drone_spmm (a padded copy where the plan already has room for it, no column slices), with the
-        // partial sums in the built-in array: the plan's own scratch pointer is swapped for the duration of the call
+        // the route of drone_spmm (copies where the plan already has room for them), with the partial sums in the built-in array: the
+        // plan's own scratch pointer is swapped for the duration of the call
         float *const plan_scratch = p->scratch;
         const size_t plan_scratch_bytes = p->scratch_bytes;
-        const int plan_slices = p->slice_forced;
         p->scratch = partials;
         p->scratch_bytes = DRONE_STATIC_SCRATCH_BYTES;
-        p->slice_forced = 0;
         drone::CallOptions opt;
         opt.no_allocation = true;
         rc = drone::spmm_impl(p, orientation, F, d_X, ldx, d_Y, ldy, (cudaStream_t)stream, opt);
         p->scratch = plan_scratch;
         p->scratch_bytes = plan_scratch_bytes;
-        p->slice_forced = plan_slices;
     }
     return rc;
 }

@@ -263,10 +263,10 @@ int drone_spmm_host_wait(drone_plan *plan, long long ticket);
  * (DRONE_STATIC_SCRATCH_BYTES, resident on every GPU that loads the library
  * until the process exits) and calls no cudaMalloc, cudaFree or any other
  * allocating routine.  Inputs, outputs, arguments and results are those of
- * drone_spmm: the same kernels run in the same order, so the output is
- * bit-identical.
+ * drone_spmm: the columns are cut and a row's nonzeros added in the same
+ * order, so the output is bit-identical.
  * Limits and rules:
- *  - a padded copy of X (see drone_plan_reserve) is made only where the plan
+ *  - a copy of X or Y (see drone_plan_reserve) is made only where the plan
  *    already has room for it;
  *  - a call whose plan needs more than DRONE_STATIC_SCRATCH_BYTES of partial
  *    sums (n_partials[orientation] * F * 4 bytes, see drone_plan_get_stats)

@@ -1,4 +1,6 @@
 """Routes of an aggregation call that its operands, the plan's buffers or the stream decide, and what must not depend on them."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -87,3 +89,33 @@ def test_same_bits_in_classes_under_capture_and_without_room(cuda_device, n, deg
                 plan.spmm(op, x, out=out, row_class=c)
             assert torch.equal(out, want)
     assert torch.equal(plan.spmm(db.OP_AT, narrow), fresh.spmm(db.OP_AT, narrow))
+
+
+@pytest.mark.parametrize("n,degree,f,split", [(300000, 40, 180, False), (300000, 24, 256, False), (200000, 30, 128, False),
+                                              (200000, 33, 127, False), (300000, 30, 256, True), (200000, 62, 255, True)])
+def test_static_scratch_runs_in_the_same_slices(cuda_device, n, degree, f, split):
+    """drone_spmm_static_scratch cuts the columns as drone_spmm does and gives its bits, before the plan has copies and after; with
+    rows of many chunks, whose partial sums lie in the built-in array."""
+    make, gen = uniform_plan(cuda_device, n, degree, n + f)
+    if split:
+        index = torch.full((n + 1,), degree, device=cuda_device, dtype=torch.int64)
+        index[0], index[1], index[7] = 0, 10000, 900
+        index = torch.cumsum(index, 0)
+        nnz = int(index[-1])
+        dst = torch.randint(0, n, (nnz,), device=cuda_device, generator=gen, dtype=torch.int32)
+        val = torch.rand(nnz, device=cuda_device, generator=gen) - 0.5
+        index = index.int()
+        make = lambda: db.AggregationPlan(index, dst, values=val)
+    x = torch.randn((n, f), device=cuda_device, generator=gen)
+    plan, fresh = make(), make()
+    for op in (db.OP_A, db.OP_AT):
+        want = plan.spmm(op, x)
+        assert plan.stats().last_slice_width == 64 and (plan.stats().n_partials[db.OP_A] > 0) == split
+        for p in (fresh, plan):
+            out = torch.full_like(x, float("nan"))
+            rc = db.lib().drone_spmm_static_scratch(p.handle, op, f, C.c_void_p(x.data_ptr()), f, C.c_void_p(out.data_ptr()), f,
+                                                    C.c_void_p(torch.cuda.current_stream().cuda_stream))
+            assert rc == 0, db.lib().drone_last_error()
+            assert p.stats().last_slice_width == 64
+            assert torch.equal(out, want)
+    assert fresh.stats().scratch_bytes == 0
