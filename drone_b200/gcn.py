@@ -124,10 +124,14 @@ class GCN:
         """Whether t is one value of this type a row, side by side on the model's device."""
         return t.dtype == dtype and t.shape == (n,) and t.device == self.x.device and t.is_contiguous()
 
+    def _float_matrix(self, t):
+        """Whether t is a matrix of floats on the model's device."""
+        return t.dtype == torch.float32 and t.dim() == 2 and t.device == self.x.device
+
     def _softmax_loss(self, logits):
         """CUDACrossEntropyLoss::forward: loss = mean over labelled rows; gradient not divided by the count."""
         n, classes = logits.shape
-        if (self._kernels and logits.is_contiguous() and self._per_row(self.labelled, torch.bool, n)
+        if (self._kernels and self._float_matrix(logits) and logits.is_contiguous() and self._per_row(self.labelled, torch.bool, n)
                 and self._per_row(self.safe_truth, torch.int64, n)):
             self.d_logits, self.loss = torch.empty_like(logits), torch.empty((), dtype=torch.float32, device=logits.device)
             self._call("drone_softmax_loss", n, classes, logits.data_ptr(), classes, self.safe_truth.data_ptr(),
@@ -147,17 +151,20 @@ class GCN:
         return self.loss
 
     def _relu_mask(self, grad, out):
-        if not self._kernels:
+        if not (self._kernels and grad.shape == out.shape and all(self._float_matrix(t) and t.is_contiguous() for t in (grad, out))):
             return grad.mul_(out > 0)
         n, f = grad.shape
         self._call("drone_relu_mask", n, f, grad.data_ptr(), f, out.data_ptr(), f, self._stream())
         return grad
 
     def _weight_gradient(self, a, g):
+        # what the kernel cannot read goes to torch, which computes or refuses it
+        if not self._kernels or not all(self._float_matrix(t) for t in (a, g)) or a.shape[0] != g.shape[0]:
+            return a.t() @ g
         (k, m), n = a.shape, g.shape[1]
         # rows one after the other: an expanded or overlapping input has none to step over
-        in_rows = a.stride(1) == 1 and (k <= 1 or m <= a.stride(0) < 1 << 31)
-        if not self._kernels or not in_rows or max(m, n) > 1 << 15:
+        in_rows = all(t.stride(1) == 1 and (k <= 1 or t.shape[1] <= t.stride(0) < 1 << 31) for t in (a, g))
+        if not in_rows or min(m, n) == 0 or max(m, n) > 1 << 15 or k > 1 << 30:
             return a.t() @ g
         floats = self._shares.get((k, m, n))
         if floats is None:      # a property of the shape
@@ -165,7 +172,8 @@ class GCN:
             self._call("drone_weight_gradient_scratch", k, m, n, C.byref(size))
             floats = self._shares[(k, m, n)] = size.value
         out, parts = (torch.empty(shape, dtype=torch.float32, device=g.device) for shape in ((m, n), floats))
-        self._call("drone_weight_gradient", k, m, n, a.data_ptr(), max(m, a.stride(0)), g.data_ptr(), n, out.data_ptr(),
+        lda, ldb = (t.stride(0) if k > 1 else t.shape[1] for t in (a, g))
+        self._call("drone_weight_gradient", k, m, n, a.data_ptr(), lda, g.data_ptr(), ldb, out.data_ptr(),
                    parts.data_ptr(), floats, self._stream())
         return out
 

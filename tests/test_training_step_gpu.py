@@ -113,3 +113,33 @@ def test_default_dtype_changed_after_the_model_was_made(cuda_device, default):
         torch.set_default_dtype(torch.float32)
     for a, b in zip(got, want):
         assert a.dtype == torch.float32 and torch.equal(a, b)
+
+
+def bare_model(device, classes=5):
+    return gcn.GCN(None, torch.zeros((6, 4), device=device), torch.zeros(6, dtype=torch.int32, device=device),
+                   [torch.zeros((4, classes), device=device)], aggregate=lambda *a: None)
+
+
+def test_what_the_kernels_cannot_read_goes_to_torch(cuda_device):
+    """Operands of a weight gradient, a mask or a loss that differ in rows, device or type, or do not lie in rows: torch's result
+    or torch's refusal."""
+    model, gen = bare_model(cuda_device), torch.Generator(cuda_device).manual_seed(13)
+    a, g = torch.randn((300, 40), device=cuda_device, generator=gen), torch.randn((300, 24), device=cuda_device, generator=gen)
+    for other in (g[:299], torch.cat([g, g]), g.cpu(), g.double(), g.half()):
+        with pytest.raises(RuntimeError) as ours:
+            model._weight_gradient(a, other)
+        with pytest.raises(RuntimeError) as torchs:
+            a.t() @ other
+        assert str(ours.value) == str(torchs.value)
+    want = a.double().t() @ g.double()
+    assert (model._weight_gradient(a, g[:, 0]) - want[:, 0]).abs().max() <= 6 * 2.0 ** -24 * 330
+    for other in (g.t().contiguous().t(), torch.cat([g, g], dim=1)[:, :24], torch.randn((600, 24), device=cuda_device)[::2].copy_(g)):
+        assert (model._weight_gradient(a, other) - want).abs().max() <= 6 * 2.0 ** -24 * 330
+    assert torch.equal(model._weight_gradient(a.double(), g.double()), want)
+    assert model._weight_gradient(a[:, :0], g).shape == (0, 24)
+    grad, out = torch.randn((9, 12), device=cuda_device, generator=gen), torch.randn((9, 12), device=cuda_device, generator=gen)
+    for x, z in ((grad.double(), out.double()), (grad.t().contiguous().t(), out), (grad.clone(), out.t().contiguous().t()), (grad.clone(), out[:1])):
+        assert torch.equal(model._relu_mask(x, z), grad.to(x.dtype) * (z > 0))
+    logits = torch.randn((6, 5), device=cuda_device, generator=gen)
+    want = model._softmax_loss(logits).clone()
+    assert abs(float(model._softmax_loss(logits.double())) - float(want)) < 1e-6 and model.d_logits.dtype == torch.float64
