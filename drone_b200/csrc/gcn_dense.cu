@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(256) softmax_loss_kernel(const float *__restri
         const float *x = logits + (long long)row * ld;
         float *g = grad + (long long)row * ld_grad;
         const long long t = __ldg(truth + row);
-        const float mask = __ldg(labelled + row) ? 1.f : 0.f;
+        // a class that does not exist: nothing plausible comes out
+        const float mask = t < 0 || t >= classes ? NAN : __ldg(labelled + row) ? 1.f : 0.f;
         constexpr int REGS = PER > 0 ? PER : 1;
         float v[REGS], m = -INFINITY, s = 0, at_truth = 0;
         if (PER > 0) {

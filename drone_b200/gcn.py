@@ -39,17 +39,30 @@ class GCN:
         self.d_h = [torch.empty((n, d), device=dev) for d in dims]      # gradients w.r.t. the Matmul outputs
         self.d_a = [torch.empty((n, d), device=dev) for d in dims[:-1]] # gradients w.r.t. the ReLU outputs (masked in place)
         self.mirror2worker = graph.mirror2worker if worker_num > 1 else None
-        self.labelled = truth >= 0
-        self.safe_truth = truth.clamp(min=0).long()
         # element-wise steps: one kernel each on the GPU, torch elsewhere
         self._kernels = x.is_cuda and all(t.dtype == torch.float32 for t in (x, *self.weights))
+        self.labelled = truth >= 0
+        self.safe_truth = truth.clamp(min=0).long()
         if self._kernels:
-            if n > 0 and int(self.safe_truth.max()) >= dims[-1]:
-                raise ValueError("a label is outside 0..%d" % (dims[-1] - 1))
             self._scratch = torch.empty(2368, dtype=torch.float64, device=dev)      # DRONE_LOSS_SCRATCH
             self._shares = {}
         self.d_w = [None] * self.n_layers
         self.loss = None
+
+    @property
+    def safe_truth(self):
+        return self._safe_truth
+
+    @safe_truth.setter
+    def safe_truth(self, classes):
+        """The rows' classes, also where they are not labelled.  They are looked at when they are set: torch would stop the step
+        at one that does not exist, the kernel makes the loss NaN (as it does when the tensor is changed in place)."""
+        most = self.weights[-1].shape[1]
+        if self._kernels and classes.numel() > 0 and not torch.cuda.is_current_stream_capturing():
+            least, largest = (int(t) for t in classes.aminmax())
+            if least < 0 or largest >= most:
+                raise ValueError("a label is outside 0..%d" % (most - 1))
+        self._safe_truth = classes
 
     # ----- pieces -----
     def sync(self, rows):

@@ -143,3 +143,21 @@ def test_what_the_kernels_cannot_read_goes_to_torch(cuda_device):
     logits = torch.randn((6, 5), device=cuda_device, generator=gen)
     want = model._softmax_loss(logits).clone()
     assert abs(float(model._softmax_loss(logits.double())) - float(want)) < 1e-6 and model.d_logits.dtype == torch.float64
+
+
+@pytest.mark.parametrize("classes", [5, 41, 300])
+def test_labels_changed_to_classes_that_do_not_exist(cuda_device, classes):
+    """Labels set on a model are looked at like those it was made with; changed in place they leave no plausible loss."""
+    for outside in (-1, classes, 2 ** 40):
+        model = bare_model(cuda_device, classes)
+        logits = torch.randn((6, classes), device=cuda_device)
+        assert torch.isfinite(model._softmax_loss(logits))
+        truth = model.safe_truth.clone()
+        truth[4] = outside
+        with pytest.raises(ValueError, match="label"):
+            model.safe_truth = truth
+        model.safe_truth = torch.full_like(truth, classes - 1)
+        assert torch.isfinite(model._softmax_loss(logits))
+        model.safe_truth[4] = outside
+        assert model._softmax_loss(logits).isnan()
+        assert model.d_logits[4].isnan().all() and torch.isfinite(model.d_logits[[0, 1, 2, 3, 5]]).all()
