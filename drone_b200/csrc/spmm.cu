@@ -186,7 +186,11 @@ struct Slices {
     int width = 0;             // 0: in one piece
     bool long_last = false;    // what is left of less than a slice goes with the slice before it
     bool by_counts = false;    // by the operand as well: another call of this width may run in one piece
-    int next(int left) const { return width == 0 || left < width + (long_last ? width : kSliceFloats / 4) ? left : width; }
+    // Widths that were forced or fit L2 divide the columns; of the others a short rest goes with the slice before it.
+    int next(int left) const {
+        const int rest = !by_counts ? 1 : long_last ? width : kSliceFloats / 4;
+        return width == 0 || left < width + rest ? left : width;
+    }
     // Columns that partial sums are kept for: calls of a width leave room for each other, so that one of them can be captured.
     int partial_columns(int F) const { return width == 0 || by_counts ? F : width; }
 };

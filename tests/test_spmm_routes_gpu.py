@@ -119,3 +119,25 @@ def test_static_scratch_runs_in_the_same_slices(cuda_device, n, degree, f, split
             assert p.stats().last_slice_width == 64
             assert torch.equal(out, want)
     assert fresh.stats().scratch_bytes == 0
+
+
+@pytest.mark.parametrize("f,width", [(16, 4), (32, 4), (32, 8), (48, 12), (60, 12), (32, 16)])
+def test_forced_slices_narrower_than_a_short_rest(cuda_device, monkeypatch, f, width):
+    """Forced slices of fewer than 16 columns are all of that width, the last one as well: partial sums have room for no more.  On
+    a fresh plan, whose partial sums no wider call has made larger; each slice has the bits of a call on its own columns."""
+    n, u, v = gg.rmat_graph(12, 16, seed=36, device=cuda_device, symmetrise=False, self_loops="add")
+    index, dst = gg.csr_by_source(u, v, n)
+    val = torch.rand(dst.numel(), device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(2)) - 0.5
+    monkeypatch.setenv("DRONE_SLICE_WIDTH", str(width))
+    sliced = db.AggregationPlan(index, dst, values=val)
+    monkeypatch.setenv("DRONE_SLICE_WIDTH", "0")
+    whole = db.AggregationPlan(index, dst, values=val)
+    x = torch.randn((n, f), device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(f))
+    for op in (db.OP_A, db.OP_AT):
+        partials = sliced.stats().n_partials[op]
+        assert partials > 0
+        got = sliced.spmm(op, x)
+        assert sliced.stats().last_slice_width == width
+        assert sliced.stats().scratch_bytes == 4 * width * max(partials, sliced.stats().n_partials[db.OP_A])
+        for c0 in range(0, f, width):
+            assert torch.equal(got[:, c0:c0 + width], whole.spmm(op, x[:, c0:c0 + width].contiguous()))
