@@ -1408,6 +1408,33 @@ static bool slices_fit_alone(drone_pr *p) {
     return slices_fit(1, &p, first_block, p->dbl ? 8 : 4, false, &room, &bytes);
 }
 
+// How large the blocks' slices would be, for the runs that keep them in shared memory.
+static int measure_slices(drone_pr *p, const Side &side) {
+    pr_slice_sizes_kernel<<<p->sms, 256>>>(side.rowptr, p->n_local, (int2 *)p->block_sums);
+    DRONE_LAUNCH_CHECK("pr_slice_sizes_kernel");
+    p->slices.resize((size_t)p->sms);
+    DRONE_CUDA(cudaMemcpy(p->slices.data(), p->block_sums, sizeof(int2) * p->slices.size(), cudaMemcpyDeviceToHost));
+    return DRONE_OK;
+}
+
+// The edges as one stream; where the device has no room for it power iterations do without (pr_run_kernel).
+static int make_stream(drone_pr *p) {
+    p->stream_block.add(&p->stream_od, sizeof(int) * (size_t)p->n_local);
+    const int warps = p->sms * (p->dbl ? stream_threads<double>() : stream_threads<float>()) / 32;
+    p->stream_block.add(&p->stream_tails, (p->dbl ? 8 : 4) * 4 * (size_t)warps);      // a piece each
+    const int rc = plan_rows_in_order(p->plan, DRONE_OP_AT, p->place, warps, &p->stream, &p->stream_block, nullptr);
+    if (rc == kNoRoom) {
+        p->stream_block.release();
+        p->stream = RowStream();
+        return DRONE_OK;
+    }
+    if (rc) return rc;
+    pr_stream_degrees_kernel<<<grid1d(p->n_local), 256>>>(p->stream.row_of, p->out_degree, p->mirror2worker, p->n_local, p->stream_od);
+    DRONE_LAUNCH_CHECK("pr_stream_degrees_kernel");
+    DRONE_CUDA(cudaDeviceSynchronize());
+    return DRONE_OK;
+}
+
 template <typename R, int MAXP, bool JOB>
 static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cudaStream_t st) {
     const int P = (int)parts.size();
@@ -1666,34 +1693,18 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
             if (e == cudaSuccess && (rc = fill_slot_split(side, p->slot_split, nullptr))) break;
         }
         if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: cudaMalloc failed: %s", cudaGetErrorString(e)); break; }
-        // how large the blocks' slices would be, for the runs that keep them in shared memory (DRONE_PR_SLICES=0: none do)
+        // (DRONE_PR_SLICES=0: no run keeps its rows in shared memory)
         const char *slices = getenv("DRONE_PR_SLICES");
-        if (e == cudaSuccess && n_local > 0 && !(slices && slices[0] == '0') && (xplan->nranks == 1 || !comm) && nnz <= (long long)p->sms * kSliceEdges && p->sms <= kBlockSums) {
-            pr_slice_sizes_kernel<<<p->sms, 256>>>(side.rowptr, n_local, (int2 *)p->block_sums);
-            count_launch();
-            p->slices.resize((size_t)p->sms);
-            e = cudaMemcpy(p->slices.data(), p->block_sums, sizeof(int2) * p->slices.size(), cudaMemcpyDeviceToHost);
-            if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: %s", cudaGetErrorString(e)); break; }
-        }
+        if (n_local > 0 && !(slices && slices[0] == '0') && (xplan->nranks == 1 || !comm) && nnz <= (long long)p->sms * kSliceEdges && p->sms <= kBlockSums &&
+            (rc = measure_slices(p, side)))
+            break;
         if (n_local > 0) {
             e = cudaMemcpy(p->out_degree, d_out_degree, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(p->mirror2worker, d_mirror2worker, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
             if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: copy failed: %s", cudaGetErrorString(e)); break; }
         }
         // one part whose slices do not fit: its edges as one stream
-        if (xplan->nranks == 1 && p->place && nnz > 0 && !slices_fit_alone(p)) {
-            p->stream_block.add(&p->stream_od, sizeof(int) * n1);
-            const int warps = p->sms * (p->dbl ? stream_threads<double>() : stream_threads<float>()) / 32;
-            p->stream_block.add(&p->stream_tails, rs * 4 * (size_t)warps);      // a piece each
-            if (plan_rows_in_order(p->plan, DRONE_OP_AT, p->place, warps, &p->stream, &p->stream_block, nullptr)) {
-                p->stream_block.release();      // no room: power iterations do without (pr_run_kernel)
-                p->stream = RowStream();
-                break;
-            }
-            pr_stream_degrees_kernel<<<grid1d(n_local), 256>>>(p->stream.row_of, p->out_degree, p->mirror2worker, n_local, p->stream_od);
-            count_launch();
-            if ((e = cudaDeviceSynchronize()) != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: %s", cudaGetErrorString(e)); break; }
-        }
+        if (xplan->nranks == 1 && p->place && nnz > 0 && !slices_fit_alone(p) && (rc = make_stream(p))) break;
     } while (0);
     if (rc) {
         drone_pr_destroy(p);

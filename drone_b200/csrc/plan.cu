@@ -972,7 +972,17 @@ int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place,
     block->add(&r.row_of, words);
     block->add(&r.first, sizeof(int) * (size_t)r.n_pieces);
     block->add(&r.col, edges);
-    DRONE_CUDA(block->make());
+    const auto make = [](DeviceBlock *of) -> int {
+        const cudaError_t e = of->make();
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return kNoRoom;
+        }
+        DRONE_CUDA(e);
+        return DRONE_OK;
+    };
+    int rc = make(block);
+    if (rc) return rc;
     struct Temp {
         int *lengths = nullptr, *filled = nullptr, *before = nullptr;
         void *scan = nullptr;
@@ -985,7 +995,7 @@ int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place,
     t.block.add(&t.filled, words);
     t.block.add(&t.before, words);
     t.block.add(&t.scan, scan_bytes);
-    DRONE_CUDA(t.block.make());
+    if ((rc = make(&t.block))) return rc;
     scatter_positions_kernel<<<grid_for(n), 256, 0, st>>>(d_place, n, r.row_of);
     DRONE_LAUNCH_CHECK("scatter_positions_kernel");
     ordered_lengths_kernel<<<grid_for(n + 1), 256, 0, st>>>(s.rowptr, r.row_of, n, t.lengths, t.filled);

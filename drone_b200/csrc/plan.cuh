@@ -166,7 +166,9 @@ struct RowStream {
     }
 #endif
 };
-// Fills in what `out` points to: `block` is made with its arrays.  `warps`: how many will share the pieces.
+// Fills in what `out` points to: `block` is made with its arrays.  `warps`: how many will share the pieces.  kNoRoom: the device has
+// no memory for it; anything else that fails is an error.
+constexpr int kNoRoom = 1;
 int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place, int warps, RowStream *out, DeviceBlock *block, cudaStream_t st);
 }  // namespace drone
 
