@@ -14,6 +14,7 @@ OP_AT = 1
 PLAN_A = 1
 PLAN_AT = 2
 PLAN_BOTH = 3
+LOSS_SCRATCH = 2368      # doubles
 
 
 class DroneError(RuntimeError):

@@ -11,7 +11,7 @@ import ctypes as C
 
 import torch
 
-from ._lib import OP_A, OP_AT, check, lib
+from ._lib import LOSS_SCRATCH, OP_A, OP_AT, check, lib
 from .graphsum import aggregate_and_exchange, clear_mirror_rows, exchange_sum
 
 
@@ -44,7 +44,7 @@ class GCN:
         self.labelled = truth >= 0
         self.safe_truth = truth.clamp(min=0).long()
         if self._kernels:
-            self._scratch = torch.empty(2368, dtype=torch.float64, device=dev)      # DRONE_LOSS_SCRATCH
+            self._scratch = torch.empty(LOSS_SCRATCH, dtype=torch.float64, device=dev)
             self._shares = {}
         self.d_w = [None] * self.n_layers
         self.loss = None

@@ -29,6 +29,14 @@ def test_library_exports_every_declared_symbol():
     assert not missing, "declared in include/ but not exported: %s" % missing
 
 
+def test_constants_are_the_headers():
+    from drone_b200 import _lib
+    text = open(os.path.join(ROOT, "include", "drone_b200.h")).read()
+    defined = {name: int(value) for name, value in re.findall(r"#define DRONE_(\w+)\s+(-?\d+)\b", text)}
+    for name in ("OP_A", "OP_AT", "PLAN_A", "PLAN_AT", "PLAN_BOTH", "EPILOGUE_NONE", "EPILOGUE_RELU", "LOSS_SCRATCH"):
+        assert getattr(_lib, name) == defined[name], name
+
+
 def test_version_and_error_string():
     import drone_b200
     lib = drone_b200.lib()
