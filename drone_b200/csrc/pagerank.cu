@@ -1524,11 +1524,12 @@ static int launch_stream(drone_pr *p, const RunRequest &rq, cudaStream_t st) {
     DRONE_CUDA(cudaMemsetAsync(p->control, 0, sizeof(RunControl), st));
     if (p->barrier_start != 0)
         DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &p->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
-    const int rc = allow_table(pr_stream_kernel<R>);
+    auto kernel = p->stream.most_spanned > kSerialPieces ? pr_stream_kernel<R, true> : pr_stream_kernel<R, false>;
+    const int rc = allow_table(kernel);
     if (rc) return rc;
     void *args[] = {&a};
-    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)pr_stream_kernel<R>, dim3(p->sms), dim3(stream_threads<R>()), args,
-                                           (size_t)a.part.table_n * sizeof(R), st));
+    DRONE_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(p->sms), dim3(stream_threads<R>()), args, (size_t)a.part.table_n * sizeof(R),
+                                           st));
     count_launch();
     return DRONE_OK;
 }

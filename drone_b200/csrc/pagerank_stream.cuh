@@ -127,14 +127,46 @@ __device__ __forceinline__ void stream_sums(const StreamArgs<R> &a, unsigned tab
     }
 }
 
-// power_vertices in stream order.
+// d and what the pieces before its last one have of row i, for the lanes in `spanning`.  A row of few pieces is its lane's, the
+// others are the warp's, one after the other.
 template <typename R>
+__device__ __forceinline__ R with_tails(const StreamArgs<R> &a, int i, unsigned spanning, R d) {
+    const int lane = threadIdx.x & 31;
+    int q0 = 0, q1 = 0;
+    if (spanning >> lane & 1) {
+        q0 = a.rows.piece_of(__ldg(a.rows.ptr + i));
+        q1 = a.rows.piece_of(__ldg(a.rows.ptr + i + 1) - 1);
+    }
+    const bool many = q1 - q0 > 16;
+    R before = 0;
+    if (!many) {
+#pragma unroll 4
+        for (int q = q0; q < q1; ++q) before += a.tails[q];
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, many); left; left &= left - 1) {
+        const int owner = __ffs(left) - 1, from = __shfl_sync(0xffffffffu, q0, owner), to = __shfl_sync(0xffffffffu, q1, owner);
+        R sum = 0;
+#pragma unroll 4
+        for (int q = from + lane; q < to; q += 32) sum += a.tails[q];
+        sum = warp_sum(sum);
+        if (lane == owner) before = sum;
+    }
+    return spanning >> lane & 1 ? before + d : d;
+}
+
+// power_vertices in stream order.  LONG: some row reaches over more than kSerialPieces pieces, which one thread alone takes too long
+// to add: us of 20 iterations, by a thread / by its warp, 65,536 vertices with one of 65,535 in-edges, 590,000 edges, float 339 / 212,
+// double 399 / 256; 4.2 M vertices with two of as many in-edges 2055 / 1442 and 2723 / 1982.  Elsewhere the other form is the better one
+// (R-MAT-18 to R-MAT-22, whose longest rows have 10 to 23 pieces, float 317 / 325, 732 / 743, 2930 / 2968).
+constexpr int kSerialPieces = 32;
+template <typename R, bool LONG>
 __device__ __forceinline__ R stream_vertices(const StreamArgs<R> &a, R dang, bool last, int first, int stride) {
     const PartView<R> &p = a.part;
     const R base = ((R)1 - a.damping) / p.global_v, share = dang / p.global_v;
     R dangling = 0;
+    const int lane = LONG ? (int)threadIdx.x & 31 : 0;      // whole warps, then
 #pragma unroll 1
-    for (int i0 = first; i0 < p.n; i0 += kVertexBatch * stride) {
+    for (int i0 = first; i0 - lane < p.n; i0 += kVertexBatch * stride) {
         int at[kVertexBatch], od[kVertexBatch];
         R d[kVertexBatch];
 #pragma unroll
@@ -145,11 +177,20 @@ __device__ __forceinline__ R stream_vertices(const StreamArgs<R> &a, R dang, boo
         }
 #pragma unroll
         for (int b = 0; b < kVertexBatch; ++b) d[b] = at[b] >= 0 ? a.sum[at[b] & ~kSpansPieces] : (R)0;
+        if constexpr (LONG) {
+            unsigned spans = 0;
+#pragma unroll
+            for (int b = 0; b < kVertexBatch; ++b) spans |= at[b] >= 0 && (at[b] & kSpansPieces) ? 1u << b : 0u;
+            if (__any_sync(0xffffffffu, spans != 0)) {
+#pragma unroll
+                for (int b = 0; b < kVertexBatch; ++b) d[b] = with_tails(a, i0 + b * stride, __ballot_sync(0xffffffffu, spans >> b & 1), d[b]);
+            }
+        }
 #pragma unroll
         for (int b = 0; b < kVertexBatch; ++b) {
             const int i = i0 + b * stride;
             if (i >= p.n) break;
-            if (at[b] >= 0 && (at[b] & kSpansPieces)) {
+            if (!LONG && at[b] >= 0 && (at[b] & kSpansPieces)) {
                 const int q0 = a.rows.piece_of(__ldg(a.rows.ptr + i)), q1 = a.rows.piece_of(__ldg(a.rows.ptr + i + 1) - 1);
                 R before = 0;
 #pragma unroll 8
@@ -170,7 +211,7 @@ __device__ __forceinline__ R stream_vertices(const StreamArgs<R> &a, R dang, boo
     return dangling;
 }
 
-template <typename R>
+template <typename R, bool LONG>
 __global__ void __launch_bounds__(stream_threads<R>(), 1) pr_stream_kernel(const __grid_constant__ StreamArgs<R> a) {
     extern __shared__ __align__(16) char table_bytes[];
     R *table_ptr = reinterpret_cast<R *>(table_bytes);
@@ -202,7 +243,7 @@ __global__ void __launch_bounds__(stream_threads<R>(), 1) pr_stream_kernel(const
         if (!grid_barrier(&a.control->barrier, phase, a.barrier_polls)) break;
         const R all = dang + (R)a.n_isolated * iso;
         const bool last = step + 1 == a.iterations;
-        dangling = stream_vertices(a, all, last, first, stride);
+        dangling = stream_vertices<R, LONG>(a, all, last, first, stride);
         iso = ((R)1 - a.damping) / p.global_v + a.damping * (all / p.global_v);
         if (last) return;
     }

@@ -933,12 +933,16 @@ __global__ void ordered_lengths_kernel(const int *__restrict__ rowptr, const int
     }
 }
 
-// at[i], from the number of rows with edges before position i
-__global__ void ordered_at_kernel(const RowStream s, const int *__restrict__ filled_before, int n) {
+// at[i], from the number of rows with edges before position i; *most_spanned, 0 before
+__global__ void ordered_at_kernel(const RowStream s, const int *__restrict__ filled_before, int n, int *most_spanned) {
+    int most = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int b = s.ptr[i], e = s.ptr[i + 1];
-        s.at[i] = e == b ? -1 : filled_before[i] | (s.piece_of(b) != s.piece_of(e - 1) ? kSpansPieces : 0);
+        const int b = s.ptr[i], e = s.ptr[i + 1], spanned = e == b ? 0 : s.piece_of(e - 1) - s.piece_of(b);
+        s.at[i] = e == b ? -1 : filled_before[i] | (spanned > 0 ? kSpansPieces : 0);
+        most = max(most, spanned);
     }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(most_spanned, most);
 }
 
 // A warp copies one row after the other, the last column marked.
@@ -984,7 +988,7 @@ int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place,
     int rc = make(block);
     if (rc) return rc;
     struct Temp {
-        int *lengths = nullptr, *filled = nullptr, *before = nullptr;
+        int *lengths = nullptr, *filled = nullptr, *before = nullptr, *most_spanned = nullptr;
         void *scan = nullptr;
         DeviceBlock block;
         ~Temp() { block.release(); }
@@ -994,6 +998,7 @@ int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place,
     t.block.add(&t.lengths, words);
     t.block.add(&t.filled, words);
     t.block.add(&t.before, words);
+    t.block.add(&t.most_spanned, sizeof(int));
     t.block.add(&t.scan, scan_bytes);
     if ((rc = make(&t.block))) return rc;
     scatter_positions_kernel<<<grid_for(n), 256, 0, st>>>(d_place, n, r.row_of);
@@ -1004,13 +1009,15 @@ int plan_rows_in_order(const drone_plan *p, int orientation, const int *d_place,
     DRONE_CUDA(cub::DeviceScan::ExclusiveSum(t.scan, scan_bytes, t.filled, t.before, n + 1, st));
     count_launch();
     count_launch();
-    ordered_at_kernel<<<grid_for(n), 256, 0, st>>>(r, t.before, n);
+    DRONE_CUDA(cudaMemsetAsync(t.most_spanned, 0, sizeof(int), st));
+    ordered_at_kernel<<<grid_for(n), 256, 0, st>>>(r, t.before, n, t.most_spanned);
     DRONE_LAUNCH_CHECK("ordered_at_kernel");
     piece_first_kernel<<<grid_for(r.n_pieces), 256, 0, st>>>(r, t.before, n);
     DRONE_LAUNCH_CHECK("piece_first_kernel");
     DRONE_CUDA(cudaMemsetAsync(r.col + (size_t)(r.n_tiles - 1) * kTileEdges, 0, sizeof(int) * kTileEdges, st));
     ordered_columns_kernel<<<grid_for((long long)n * 32), 256, 0, st>>>(s.rowptr, s.col, r.row_of, r.ptr, n, r.col);
     DRONE_LAUNCH_CHECK("ordered_columns_kernel");
+    DRONE_CUDA(cudaMemcpyAsync(&r.most_spanned, t.most_spanned, sizeof(int), cudaMemcpyDeviceToHost, st));
     DRONE_CUDA(cudaStreamSynchronize(st));
     *out = r;
     return DRONE_OK;

@@ -158,6 +158,7 @@ struct RowStream {
     int *first = nullptr;      // [n_pieces] which of the rows with edges a piece's first edge belongs to
     unsigned *col = nullptr;   // [n_tiles * kTileEdges] columns | kRowEnd; 0 beyond the last edge
     int n_pieces = 0, n_tiles = 0;
+    int most_spanned = 0;      // pieces that a row reaches over before its last one, at most
 #ifdef __CUDACC__
     // Piece q is tiles [first_tile(q), first_tile(q + 1)), one more or less than any other piece; none is empty.
     __host__ __device__ int first_tile(int q) const { return (int)((long long)n_tiles * q / n_pieces); }

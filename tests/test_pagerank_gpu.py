@@ -391,6 +391,37 @@ def test_slices_in_shared_memory(cuda_device, oracle, monkeypatch, scale, parts,
             assert np.max(np.abs(x[name] - y[name]) / np.maximum(np.abs(x[name]), 1e-3 if use_double else 1.0)) < (PR_TOL if use_double else 1e-4), name
 
 
+def hub_graph(n, edges, hubs, seed):
+    """Random edges, and for every (vertex, in-edges) of `hubs` that many sources more."""
+    rng = np.random.default_rng(seed)
+    u, v = [rng.integers(0, n, edges)], [rng.integers(0, n, edges)]
+    for vertex, count in hubs:
+        u.append(rng.permutation(n)[:count])
+        v.append(np.full(count, vertex))
+    u, v = np.concatenate(u), np.concatenate(v)
+    key = np.unique((u * n + v)[u != v])
+    return (key // n).astype(np.int32), (key % n).astype(np.int32)
+
+
+@pytest.mark.parametrize("use_double", [False, True])
+@pytest.mark.parametrize("n,edges,hubs", [(20000, 60000, [(13, 19999)]), (20000, 0, [(19999, 19000), (0, 4097), (1, 4098), (7, 300)]),
+                                          (33333, 50000, [(k, 1000 + 700 * k) for k in range(45)])])
+def test_rows_of_many_pieces(cuda_device, oracle, monkeypatch, n, edges, hubs, use_double):
+    """One part's edges as a stream with rows that reach over a few and over many of its pieces, several of them in one warp."""
+    monkeypatch.setenv("DRONE_PR_SLICES", "0")
+    u, v = hub_graph(n, edges, hubs, seed=len(hubs))
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
+    part = pt.ebv_partition(n, u, v, 1, keep_self_loops=False)
+    graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 0.0)
+    prk.power_iterate_local(prs, 20, 0.85)
+    got = prk.gather_global(prs, graphs, n)
+    touched = part.replicas > 0
+    assert np.max(np.abs(got[touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
+    prk.power_iterate_local(prs, 20, 0.85)
+    assert np.array_equal(prk.gather_global(prs, graphs, n), got)
+
+
 def device_state(job):
     """The arrays of drone_pr_device_arrays, copied."""
     ptrs = [C.c_void_p(0) for _ in range(5)]
