@@ -1373,6 +1373,19 @@ constexpr long long kSliceEdges = kSliceBytes / sizeof(unsigned);      // more e
 
 static bool all_values_or_order(const drone_pr *p, size_t value) { return p->place || p->n_local <= kTableBytes / (int)value; }
 
+// How many edges the largest slice may have above the average: a row lies in one block, and the others wait for it.  An iteration of
+// balanced slices is at least 4 us shorter than one of the other kernels, which cut long rows (R-MAT-12 to R-MAT-17, 65,536 vertices with
+// 524,000 edges: 3.4 to 7 us); what an edge costs the largest slice, in ns, depends on how much of the published values its table and L1
+// hold.  Measured with one vertex of many in-edges, us of 20 iterations on 65,536 vertices, other kernels / slices: float 16,000 in-edges
+// 219 / 201, 24,000 206 / 265, 48,000 217 / 866; double 8,000 221 / 182, 16,000 223 / 251; two parts, double, 24,000 332 / 300, 48,000 333 /
+// 401; 131,072 vertices, double, 24,000 344 / 568 (1.3 ns; R-MAT-17, whose gathers the table serves, 0.3: 318 / 269 with 5,400 edges above
+// the average); 16,384 vertices, float, 16,000 191 / 159.
+static long long edges_above_average(size_t value, long long n_local) {
+    const double ns[2][3] = {{0.20, 0.32, 0.45}, {0.29, 0.44, 0.6}};
+    const long long published = (long long)value * n_local;
+    return (long long)(4000 / ns[value == 8][published <= 128 << 10 ? 0 : published <= 512 << 10 ? 1 : 2]);
+}
+
 static bool slices_fit(int n_parts, drone_pr *const *parts, const int *first_block, size_t value, bool job, SliceRoom *room, size_t *bytes) {
     *room = SliceRoom{0, 0, 0};
     long long table = 0;
@@ -1381,6 +1394,7 @@ static bool slices_fit(int n_parts, drone_pr *const *parts, const int *first_blo
         const int blocks = first_block[q + 1] - first_block[q];
         if (p->n_local == 0 || blocks > (int)p->slices.size()) return false;
         const int2 most = p->slices[blocks - 1];
+        if (most.y - p->nnz / blocks > edges_above_average(value, p->n_local)) return false;
         room->rows = std::max(room->rows, (most.x + 3) & ~3);
         room->edges = std::max(room->edges, most.y);
         if (!all_values_or_order(p, value)) continue;

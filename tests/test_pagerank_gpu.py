@@ -422,6 +422,42 @@ def test_rows_of_many_pieces(cuda_device, oracle, monkeypatch, n, edges, hubs, u
     assert np.array_equal(prk.gather_global(prs, graphs, n), got)
 
 
+@pytest.mark.parametrize("parts,use_double,hub,kept", [(1, False, 30000, False), (1, True, 20000, False), (1, True, 2000, True),
+                                                       (2, True, 60000, False)])
+def test_slices_of_a_vertex_with_many_edges(cuda_device, oracle, monkeypatch, parts, use_double, hub, kept):
+    """A vertex whose edges would make one block's slice much larger than the others' keeps a run out of the slices, whose sums
+    add in another order: the values are bit for bit those of a handle without slices."""
+    n = 65536
+    u, v = hub_graph(n, 8 * n, [(13, hub)], seed=hub)
+    index, dst = gg.csr_by_source(torch.as_tensor(u), torch.as_tensor(v), n)
+    want = oracle.pagerank_power_f64(index.numpy(), dst.numpy(), 20, 0.85)
+    part = pt.ebv_partition(n, u, v, parts, keep_self_loops=False)
+    touched, power = part.replicas > 0, []
+    for slices in ("0", "1"):
+        monkeypatch.setenv("DRONE_PR_SLICES", slices)
+        graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+        prk.power_iterate_local(prs, 20, 0.85)
+        power.append(prk.gather_global(prs, graphs, n))
+        assert np.max(np.abs(power[-1][touched] - want[touched]) / want[touched]) < (PR_TOL if use_double else 1e-4)
+    assert np.array_equal(power[0], power[1]) == (not kept)
+
+
+def test_state_after_the_whole_job(cuda_device, monkeypatch):
+    """What a job that runs in slices to its end leaves of every part's state, against the kernel without them."""
+    n, u, v, _, part = pr_case(scale=13, seed=77, parts=3)
+    states = []
+    for slices in ("0", "1"):
+        monkeypatch.setenv("DRONE_PR_SLICES", slices)
+        _, prs = build_parts(part, n, u, v, cuda_device, True, 1e-6)
+        prk.run_job_local(prs)
+        states.append([device_state(p) for p in prs])
+    for x, y in zip(*states):
+        for name in ("active", "ubm"):
+            assert np.array_equal(x[name], y[name])
+        for name in ("pr", "acc", "diff"):
+            assert np.max(np.abs(x[name] - y[name]) / np.maximum(np.abs(x[name]), 1e-3)) < PR_TOL, name
+
+
 def device_state(job):
     """The arrays of drone_pr_device_arrays, copied."""
     ptrs = [C.c_void_p(0) for _ in range(5)]
