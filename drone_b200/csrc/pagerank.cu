@@ -1494,7 +1494,9 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
         DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &lead->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
     SliceRoom room;
     size_t bytes = 0;
-    if (slices_fit(P, parts.data(), a.first_block, sizeof(R), JOB, &room, &bytes)) {
+    // The job of one part is a single superstep, which does not repay filling the slices (float, R-MAT-16 61 / 69 us a call, R-MAT-17 68 / 82).  With several parts a
+    // superstep by itself (R-MAT-16 in two parts, double, 66 / 78) takes the kernel that the whole job takes, so that the bits are the same.
+    if ((!JOB || P > 1) && slices_fit(P, parts.data(), a.first_block, sizeof(R), JOB, &room, &bytes)) {
         for (int q = 0; q < P; ++q) a.part[q].table_n = all_values_or_order(parts[q], sizeof(R)) ? std::min(room.table, parts[q]->n_local) : 0;
         auto kernel = pr_resident_kernel<R, MAXP, JOB>;
         DRONE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSliceBytes));

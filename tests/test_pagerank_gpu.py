@@ -442,6 +442,23 @@ def test_slices_of_a_vertex_with_many_edges(cuda_device, oracle, monkeypatch, pa
     assert np.array_equal(power[0], power[1]) == (not kept)
 
 
+@pytest.mark.parametrize("use_double", [False, True])
+def test_job_of_one_part_takes_no_slices(cuda_device, monkeypatch, use_double):
+    """One superstep does not repay filling the slices: whole or step by step the job of one part has the bits of a handle without."""
+    n, u, v, _, part = pr_case(scale=14, seed=79, parts=1)
+    seen = []
+    for slices in ("0", "1"):
+        monkeypatch.setenv("DRONE_PR_SLICES", slices)
+        graphs, prs = build_parts(part, n, u, v, cuda_device, use_double, 1e-6)
+        steps, sizes = prk.run_job_local(prs)
+        seen.append((steps, sizes, prk.gather_global(prs, graphs, n)))
+        prk.step_local(prs, True)
+        prk.step_local(prs, False)
+        seen[-1] += (prk.gather_global(prs, graphs, n), device_state(prs[0])["acc"])
+    for a, b in zip(*seen):
+        assert np.array_equal(a, b)
+
+
 def test_state_after_the_whole_job(cuda_device, monkeypatch):
     """What a job that runs in slices to its end leaves of every part's state, against the kernel without them."""
     n, u, v, _, part = pr_case(scale=13, seed=77, parts=3)
