@@ -311,7 +311,9 @@ static int spmm_impl(drone_plan *p, int orientation, int F, const float *X, long
     bool copy_x = to_lines || (to_vectors && !x_vectors), copy_y = to_vectors && !y_vectors;
     const long long stride = to_lines ? line_stride(F) : padded_stride(p->n_rows, F);
     // The columns are cut as for the copies also where these have no room, or are left out: a row class, a call under capture and
-    // one that found no memory add in the order of the whole, eager call.
+    // one that found no memory add in the order of the whole, eager call.  Read float by float the slices mostly lose what they cost
+    // (us in one piece / in slices: 600,000 rows of 81 F = 177 5160 / 5740, a million of 64 F = 255 10650 / 12450, 300,000 of 201 F = 255 7600 /
+    // 6750), on plans that were reserved for an odd width without the copies.
     const Slices cut = column_slices(p, s, Fp, vec4 || to_vectors, copy_x ? stride % 32 == 0 : rows_on_lines(X, ldx));
     // Every class of rows copies X anew, which a small class does not make up for (us for all classes, 2 / 4 / 16 equal ones, X where
     // it lies against copied: 300,000 rows of 201 F = 180 4035 / 4161 / 6665 and 3312 / 3547 / 6878, of 41 F = 392 2462 / 3005 / 6443 and

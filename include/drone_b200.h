@@ -469,7 +469,10 @@ typedef struct drone_pr_response {
  * eps is the push threshold (1e-6 in DRONE/src/cuda/algorithm/pr.cu:11,
  * 0.01 in the CPU job DRONE/src/algorithm/PageRank.go:10).
  * Owns what struct PRValues holds (DRONE/src/cuda/algorithm/pr.h:7-16); all
- * buffers are allocated here once, none per superstep.
+ * buffers are allocated here once, none per superstep.  The only part of a
+ * graph whose edges do not fit the SMs' shared memory is kept a second time as
+ * one stream (4 bytes an edge, 16 a vertex), where there is room for it:
+ * drone_pr_power_iterate is slower without.
  */
 int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz,
                     const int *d_index, const int *d_dst, const int *d_out_degree,
