@@ -592,7 +592,8 @@ __device__ __forceinline__ void sum_chunk(typename Vec<VEC>::type *acc, const in
 
 // Batches of 32 entries that a warp takes together: a batch of rows that one or two lanes hold is one or two gathers a lane.
 // Four, but two in the one launch of a small plan for pairs of lanes, where four cost registers that its short rows want (us, F = 8,
-// two / four: power law, 100,000 rows of 51 51 / 75; the separate kernels: R-MAT-18 70 / 60, R-MAT-20 129 / 123).
+// two / four: power law, 100,000 rows of 51 51 / 75; the separate kernels: R-MAT-18 70 / 60, R-MAT-20 129 / 123).  Fewer where the
+// work does without (large_plan_batches, small_plan_batches); the sums and their order are the same.
 constexpr int chunk_batches(int G, int VPL, int VEC, bool one_launch) {
     return VPL > 1 || G > 2 ? 1 : G == 2 && VEC == 4 && one_launch ? 2 : 4;
 }
@@ -643,7 +644,7 @@ __device__ __forceinline__ void sum_chunk_narrow(typename Vec<VEC>::type &acc, c
     for (int o = G; o < 32; o <<= 1) Vec<VEC>::add(acc, Vec<VEC>::shfl_xor(acc, o));
 }
 
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT, int NB>
 __global__ void __launch_bounds__(256, chunk_blocks_per_sm(G, VPL, VEC, EXACT))
 spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__restrict__ col,
                    const float *__restrict__ val, Gather g, float *__restrict__ Y, long long ldy,
@@ -666,7 +667,6 @@ spmm_chunks_kernel(const Chunk *__restrict__ chunks, int n_chunks, const int *__
         if (lane == 0) next_group = atomicAdd(counter, (unsigned)kChunkGroup);   // needed only after this group
 
         // first batch of the group's first chunk
-        constexpr int NB = chunk_batches(G, VPL, VEC, false);
         int cs[NB];      // the same of several batches (NB > 1)
         float vs[NB];
         int c = 0;
@@ -851,7 +851,9 @@ __device__ __forceinline__ void store_vector(const RowDestination<VEC> &dest, in
     else st_stream(dest.ptr + vi, v, pol);
 }
 
-template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, int BLOCKS_PER_SM, int SURE = sure_vectors(G, VPL, VEC)>
+// NB = 1 for rows that one or two lanes hold: the short rows too have one entry a lane at a time, in fewer registers.
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, int BLOCKS_PER_SM, int SURE = sure_vectors(G, VPL, VEC),
+          int NB = chunk_batches(G, VPL, VEC, true)>
 __global__ void __launch_bounds__(256, BLOCKS_PER_SM)
 spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_blocks, const int *__restrict__ col,
                   const float *__restrict__ val, const SplitRow *__restrict__ split, const int *__restrict__ slot_split,
@@ -866,7 +868,7 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
     let_next_kernel_start();
     if ((int)blockIdx.x >= chunk_blocks) {
         const long long warp = (((int)blockIdx.x - chunk_blocks) * (long long)blockDim.x + threadIdx.x) >> 5;
-        if constexpr (short_entries_per_lane(G, VPL, VEC) > 1)
+        if constexpr (short_entries_per_lane(G, VPL, VEC) > 1 && NB > 1)
             walk_short_range_narrow<G, VEC, EXACT, UNIT, false, true>(warp * RPW + gi, s_range_row, n_ranges, s_rowptr, s_rows, s_col,
                                                                       s_val, g, Y, ldy, nvec, epi);
         else
@@ -878,7 +880,6 @@ spmm_small_kernel(const Chunk *__restrict__ chunks, int n_chunks, int chunk_bloc
     if (at >= n_chunks) return;
     const unsigned long long pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
     const int4 ch = __ldg(reinterpret_cast<const int4 *>(chunks) + at);      // row, first nonzero, length, slot
-    constexpr int NB = chunk_batches(G, VPL, VEC, true);
     int cs[NB];
     float vs[NB];
     int c = 0;
@@ -991,6 +992,50 @@ static int resident_grid(Kernel kernel, int cap_per_sm) {
     return per_sm * sms;
 }
 
+// Batches of a large plan's chunks.  With enough chunks every SM has gathers in flight whatever a warp has, and out of L2 more of them
+// a warp only cost registers; out of HBM they pay.  us with four / two / one: F = 8 power law 700,000 rows of 71 354 / 319 / 314, 1.4 M of 88
+// 760 / 698 / 679, 2 M of 50 836 / 784 / 716, 700,000 of 21 138 / 137 / 136, 50,000 of 500 143 / 145 / 148, of 1000 237 / 234 / 234, R-MAT-19 16 M nonzeros
+// 106 / 109 / 111, R-MAT-18 64 / 75 / 75, R-MAT-23 (X is 268 MB) 923 / 982 / 1008; value-free 2 M of 50 686 / 645 / 651, 700,000 of 36 177 / 173 / 185,
+// 50,000 of 500 131 / 134 / 142.  F = 4 700,000 of 71 326 / 307 / 306, 1.4 M of 88 688 / 669 / 660, 50,000 of 1000 192 / 197 / 194, 200,000 of 250 248 / 253 / 254,
+// of 500 466 / 457 / 458, R-MAT-24 1758 / 1663 / 1697, R-MAT-18 66 / 76 / 75; value-free 50,000 of 2000 242 / 252 / 236, 2 M of 50 620 / 601 / 595.
+// Widths of 1 and 2 keep four.
+template <int G, int VEC, bool UNIT>
+static int large_plan_batches(int nnz, int n_rows) {
+    const int most = chunk_batches(G, 1, VEC, false);
+    const bool in_l2 = 4LL * G * VEC * n_rows <= 160000000;
+    if (VEC == 4 && G == 2) return nnz > (n_rows >= 100000 ? 20000000 : 40000000) && in_l2 ? (UNIT ? 2 : 1) : most;
+    if (VEC == 4 && G == 1) return nnz > 64000000 && in_l2 ? 1 : !UNIT && nnz > 20000000 && n_rows >= 400000 ? 2 : most;
+    return most;
+}
+
+// The same for the one launch of a small plan, where one batch also halves the registers of the whole kernel: for graphs whose rows are
+// nearly all long.  us with four (F = 8: two) / one and the short rows as wide shapes have them: F = 1 20,000 rows of 300 29.2 / 26.7, 8,000 of 200
+// 9.4 / 10.1, value-free 23.7 / 19.5 and 8.7 / 7.5, 20,000 of 120 13.4 / 13.7; F = 4 12,000 of 480 34.5 / 32.8, 40,000 of 150 36.3 / 37.3, 3,000 of 300 7.2 / 8.0,
+// value-free 31.2 / 27.7 and 33.1 / 32.1; F = 8 value-free 12,000 of 480 35.0 / 33.5.  F = 4 value-free with four / two: 100,000 rows of 60 50.5 / 44.0,
+// 200,000 of 28 47.7 / 42.9, 20,000 of 40 13.2 / 14.6.
+template <int G, int VEC, bool UNIT>
+static int small_plan_batches(int nnz, int n_rows) {
+    if (nnz >= 3 << 19 && (UNIT || G == 1) && nnz / (UNIT ? 140 : 256) >= n_rows) return 1;
+    if (VEC == 4 && G == 1 && UNIT && nnz >= 3000000) return 2;
+    return chunk_batches(G, 1, VEC, true);
+}
+
+template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT, int NB>
+static int launch_chunks(const SpmmArgs &a, int chunk_lo, int n_chunks) {
+    const Side &s = *a.side;
+    auto kernel = spmm_chunks_kernel<G, VPL, VEC, 2 * U, EXACT, UNIT, HOT, NB>;
+    static int resident_all = 0;
+    if (resident_all == 0) resident_all = resident_grid(kernel, 0);
+    int resident = resident_all;
+    if (a.resident_per_sm > 0) resident = std::min(resident, a.resident_per_sm * a.sms);
+    int grid = ceil_div(ceil_div(n_chunks, kChunkGroup), 8);
+    if (resident > 0 && grid > resident) grid = resident;
+    DRONE_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), a.st));
+    kernel<<<grid, 256, 0, a.st>>>(s.chunks + chunk_lo, n_chunks, s.col, s.val, a.gather, a.Y, a.ldy, a.partials, a.nvec, a.epi, a.counter);
+    DRONE_LAUNCH_CHECK("spmm_chunks_kernel");
+    return DRONE_OK;
+}
+
 template <int G, int VPL, int VEC, int U, bool EXACT, bool UNIT, bool HOT>
 static int launch_all(const SpmmArgs &a) {
     constexpr int RPW = 32 / G;
@@ -1034,6 +1079,13 @@ static int launch_all(const SpmmArgs &a) {
         if constexpr (VEC == 1 && VPL == 4 && sure_vectors(G, VPL, VEC) > 0) {
             if (a.nnz < 1 << 20) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0, 0>;
         }
+        if constexpr (chunk_batches(G, VPL, VEC, true) > 1 && (UNIT || G == 1)) {
+            const int batches = small_plan_batches<G, VEC, UNIT>(a.nnz, a.n_rows);
+            if (batches == 1) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0, sure_vectors(G, VPL, VEC), 1>;
+            if constexpr (VEC == 4 && G == 1 && UNIT) {
+                if (batches == 2) kernel = spmm_small_kernel<G, VPL, VEC, U, EXACT, UNIT, 0, sure_vectors(G, VPL, VEC), 2>;
+            }
+        }
         DRONE_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const Chunk *)s.chunks + chunk_lo, n_chunks,
                                       chunk_blocks, (const int *)s.col, (const float *)s.val, (const SplitRow *)s.split,
                                       (const int *)s.slot_split, s.arrived, a.partials, (const int *)ranges.row + range_lo,
@@ -1064,17 +1116,19 @@ static int launch_all(const SpmmArgs &a) {
         if (overlap) DRONE_CUDA(cudaEventRecord(a.join, a.side_stream));
     }
     if (n_chunks > 0) {
-        auto kernel = spmm_chunks_kernel<G, VPL, VEC, 2 * U, EXACT, UNIT, HOT>;
-        static int resident_all = 0;
-        if (resident_all == 0) resident_all = resident_grid(kernel, 0);
-        int resident = resident_all;
-        if (a.resident_per_sm > 0) resident = std::min(resident, a.resident_per_sm * a.sms);
-        int grid = ceil_div(ceil_div(n_chunks, kChunkGroup), 8);
-        if (resident > 0 && grid > resident) grid = resident;
-        DRONE_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), a.st));
-        kernel<<<grid, 256, 0, a.st>>>(s.chunks + chunk_lo, n_chunks, s.col, s.val, a.gather, a.Y, a.ldy, a.partials,
-                                       a.nvec, a.epi, a.counter);
-        DRONE_LAUNCH_CHECK("spmm_chunks_kernel");
+        constexpr int MOST = chunk_batches(G, VPL, VEC, false);
+        auto launch = launch_chunks<G, VPL, VEC, U, EXACT, UNIT, HOT, MOST>;
+        if constexpr (MOST > 1 && VEC == 4) {
+            const int batches = large_plan_batches<G, VEC, UNIT>(a.nnz, a.n_rows);
+            if constexpr (G == 1 || !UNIT) {
+                if (batches == 1) launch = launch_chunks<G, VPL, VEC, U, EXACT, UNIT, HOT, 1>;
+            }
+            if constexpr ((G == 2) == UNIT) {
+                if (batches == 2) launch = launch_chunks<G, VPL, VEC, U, EXACT, UNIT, HOT, 2>;
+            }
+        }
+        const int rc = launch(a, chunk_lo, n_chunks);
+        if (rc) return rc;
     }
     if (n_split > 0) {
         const size_t smem = n_wide > 0 ? sizeof(float) * 8 * (size_t)a.nvec * VEC : 0;

@@ -141,3 +141,40 @@ def test_forced_slices_narrower_than_a_short_rest(cuda_device, monkeypatch, f, w
         assert sliced.stats().scratch_bytes == 4 * width * max(partials, sliced.stats().n_partials[db.OP_A])
         for c0 in range(0, f, width):
             assert torch.equal(got[:, c0:c0 + width], whole.spmm(op, x[:, c0:c0 + width].contiguous()))
+
+
+@pytest.mark.parametrize("n,per_row", [(8000, 200), (8000, 300), (100000, 31), (11000, 143),      # one launch: long rows, and not
+                                       (100000, 190), (100000, 215), (40000, 1080), (400000, 53), (40000, 1590), (40000, 1700)])   # 20, 40 and 64 M
+def test_narrow_widths_take_fewer_batches(cuda_device, n, per_row):
+    """Widths of 1 to 8 where chunks take fewer batches of gathers at a time, and beside it, against double; the same bits for the
+    rows class by class."""
+    gen = torch.Generator(cuda_device).manual_seed(n + per_row)
+    lengths = torch.randint(per_row * 9 // 10, per_row * 11 // 10 + 1, (n,), device=cuda_device, generator=gen)
+    lengths[::97], lengths[1::97], lengths[5] = 3, 0, 5000
+    index = torch.zeros(n + 1, dtype=torch.int64, device=cuda_device)
+    torch.cumsum(lengths, 0, out=index[1:])
+    nnz = int(index[-1])
+    dst = torch.randint(0, n, (nnz,), device=cuda_device, generator=gen, dtype=torch.int32)
+    val = torch.rand(nnz, device=cuda_device, generator=gen) - 0.5
+    index = index.int()
+    plan = db.AggregationPlan(index, dst, values=val, orientations=1)
+    scale = torch.rand(n, device=cuda_device, generator=gen)
+    row_class = torch.randint(0, 2, (n,), device=cuda_device, generator=gen, dtype=torch.int32)
+    x = torch.randn((n, 8), device=cuda_device, generator=gen)
+    plain = torch.sparse_csr_tensor(index.long(), dst.long(), val.double(), (n, n)) @ x.double()
+    unit = (torch.sparse_csr_tensor(index.long(), dst.long(), torch.ones_like(val).double(), (n, n)) @ x.double()) * scale[:, None]
+    results = {}
+    for f in (1, 2, 4, 8):
+        xf = x[:, :f].contiguous()
+        got = results[f, 0] = plan.spmm(db.OP_A, xf)
+        free = results[f, 1] = plan.spmm(db.OP_A, xf, unit_values=True, row_scale=scale)
+        # float sums of up to 5000 terms of size 1, in pieces of at most 256
+        for y, want in ((got, plain[:, :f]), (free, unit[:, :f])):
+            assert (y - want).abs().max() <= 2e-5 * want.abs().max()
+    plan.set_row_classes(row_class, 2)
+    for (f, form), want in results.items():
+        options = dict(unit_values=True, row_scale=scale) if form else {}
+        out = torch.empty_like(want)
+        for c in range(2):
+            plan.spmm(db.OP_A, x[:, :f].contiguous(), out=out, row_class=c, **options)
+        assert torch.equal(out, want)
