@@ -1374,12 +1374,12 @@ constexpr long long kSliceEdges = kSliceBytes / sizeof(unsigned);      // more e
 static bool all_values_or_order(const drone_pr *p, size_t value) { return p->place || p->n_local <= kTableBytes / (int)value; }
 
 // How many edges the largest slice may have above the average: a row lies in one block, and the others wait for it.  An iteration of
-// balanced slices is at least 4 us shorter than one of the other kernels, which cut long rows (R-MAT-12 to R-MAT-17, 65,536 vertices with
-// 524,000 edges: 3.4 to 7 us); what an edge costs the largest slice, in ns, depends on how much of the published values its table and L1
-// hold.  Measured with one vertex of many in-edges, us of 20 iterations on 65,536 vertices, other kernels / slices: float 16,000 in-edges
-// 219 / 201, 24,000 206 / 265, 48,000 217 / 866; double 8,000 221 / 182, 16,000 223 / 251; two parts, double, 24,000 332 / 300, 48,000 333 /
-// 401; 131,072 vertices, double, 24,000 344 / 568 (1.3 ns; R-MAT-17, whose gathers the table serves, 0.3: 318 / 269 with 5,400 edges above
-// the average); 16,384 vertices, float, 16,000 191 / 159.
+// balanced slices is at least 4 us shorter than one of the other kernels, which cut long rows (R-MAT-12 to R-MAT-17, 65,536 vertices
+// with 524,000 edges: 3.4 to 7 us); what an edge costs the largest slice, in ns, depends on how much of the published values its table
+// and L1 hold.  Measured with one vertex of many in-edges, us of 20 iterations on 65,536 vertices, other kernels / slices: float 16,000
+// in-edges 219 / 201, 24,000 206 / 265, 48,000 217 / 866; double 8,000 221 / 182, 16,000 223 / 251; two parts, double, 24,000 332 /
+// 300, 48,000 333 / 401; 131,072 vertices, double, 24,000 344 / 568 (1.3 ns; R-MAT-17, whose gathers the table serves, 0.3: 318 / 269
+// with 5,400 edges above the average); 16,384 vertices, float, 16,000 191 / 159.
 static long long edges_above_average(size_t value, long long n_local) {
     const double ns[2][3] = {{0.20, 0.32, 0.45}, {0.29, 0.44, 0.6}};
     const long long published = (long long)value * n_local;
@@ -1494,8 +1494,9 @@ static int launch_run(std::vector<drone_pr *> &parts, const RunRequest &rq, cuda
         DRONE_CUDA(cudaMemcpyAsync(&a.control->barrier.arrived, &lead->barrier_start, sizeof(unsigned), cudaMemcpyHostToDevice, st));
     SliceRoom room;
     size_t bytes = 0;
-    // The job of one part is a single superstep, which does not repay filling the slices (float, R-MAT-16 61 / 69 us a call, R-MAT-17 68 / 82).  With several parts a
-    // superstep by itself (R-MAT-16 in two parts, double, 66 / 78) takes the kernel that the whole job takes, so that the bits are the same.
+    // The job of one part is a single superstep, which does not repay filling the slices (float, R-MAT-16 61 / 69 us a call, R-MAT-17
+    // 68 / 82).  With several parts a superstep by itself (R-MAT-16 in two parts, double, 66 / 78) takes the kernel that the whole job
+    // takes, so that the bits are the same.
     if ((!JOB || P > 1) && slices_fit(P, parts.data(), a.first_block, sizeof(R), JOB, &room, &bytes)) {
         for (int q = 0; q < P; ++q) a.part[q].table_n = all_values_or_order(parts[q], sizeof(R)) ? std::min(room.table, parts[q]->n_local) : 0;
         auto kernel = pr_resident_kernel<R, MAXP, JOB>;
@@ -1712,9 +1713,8 @@ int drone_pr_create(drone_pr **out, int n_local, int global_v, int nnz, const in
         if (e != cudaSuccess) { rc = set_error(DRONE_E_CUDA, "drone_pr_create: cudaMalloc failed: %s", cudaGetErrorString(e)); break; }
         // (DRONE_PR_SLICES=0: no run keeps its rows in shared memory)
         const char *slices = getenv("DRONE_PR_SLICES");
-        if (n_local > 0 && !(slices && slices[0] == '0') && (xplan->nranks == 1 || !comm) && nnz <= (long long)p->sms * kSliceEdges && p->sms <= kBlockSums &&
-            (rc = measure_slices(p, side)))
-            break;
+        const bool may_slice = !(slices && slices[0] == '0') && (xplan->nranks == 1 || !comm);
+        if (may_slice && n_local > 0 && nnz <= (long long)p->sms * kSliceEdges && p->sms <= kBlockSums && (rc = measure_slices(p, side))) break;
         if (n_local > 0) {
             e = cudaMemcpy(p->out_degree, d_out_degree, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(p->mirror2worker, d_mirror2worker, sizeof(int) * (size_t)n_local, cudaMemcpyDeviceToDevice);

@@ -5,11 +5,12 @@
 // that all of its gathers are in flight together (a chunk of a long row has 141 edges on average, and a short row's sum took
 // a scan over 32 lanes for every 32 edges), and the vertex step reads and publishes in order.
 //
-// Bound: the LSU, one wavefront per gather that misses the table, and the lines of L1 that gathers in flight wait in: a table
-// of 128 KB is the best on R-MAT-22 and within 3 % of the best elsewhere (64 / 96 / 128 / 160 KB, ms, float: R-MAT-22 3.31 / 3.36 / 2.94 / 2.98,
-// R-MAT-18 0.324 / 0.312 / 0.316 / 0.316, a million vertices with 16 in-edges drawn uniformly 1.56 / 1.55 / 1.56 / 1.60, power law, 2.4 M of 24 4.78 /
-// 4.74 / 4.74 / 4.86; double 5.22 / 5.19 / 5.33 / 5.84, R-MAT-22 4.23 / 4.06 / 4.10 / 4.31).  ms for 20 iterations, chunks and scans / stream: R-MAT-18 float 0.54 / 0.32, double 0.60 / 0.39; R-MAT-20 1.20 /
-// 0.72 and 1.55 / 1.02; R-MAT-22 float 5.03 / 2.93.
+// Bound: the LSU, one wavefront per gather that misses the table, and the lines of L1 that gathers in flight wait in: a table of 128 KB
+// is the best on R-MAT-22 and within 3 % of the best elsewhere (64 / 96 / 128 / 160 KB, ms, float: R-MAT-22 3.31 / 3.36 / 2.94 / 2.98,
+// R-MAT-18 0.324 / 0.312 / 0.316 / 0.316, a million vertices with 16 in-edges drawn uniformly 1.56 / 1.55 / 1.56 / 1.60, power law, 2.4
+// M of 24 4.78 / 4.74 / 4.74 / 4.86; double 5.22 / 5.19 / 5.33 / 5.84, R-MAT-22 4.23 / 4.06 / 4.10 / 4.31).  ms for 20 iterations,
+// chunks and scans / stream: R-MAT-18 float 0.54 / 0.32, double 0.60 / 0.39; R-MAT-20 1.20 / 0.72 and 1.55 / 1.02; R-MAT-22 float 5.03
+// / 2.93.
 #pragma once
 
 namespace drone {

@@ -993,12 +993,12 @@ static int resident_grid(Kernel kernel, int cap_per_sm) {
 }
 
 // Batches of a large plan's chunks.  With enough chunks every SM has gathers in flight whatever a warp has, and out of L2 more of them
-// a warp only cost registers; out of HBM they pay.  us with four / two / one: F = 8 power law 700,000 rows of 71 354 / 319 / 314, 1.4 M of 88
-// 760 / 698 / 679, 2 M of 50 836 / 784 / 716, 700,000 of 21 138 / 137 / 136, 50,000 of 500 143 / 145 / 148, of 1000 237 / 234 / 234, R-MAT-19 16 M nonzeros
-// 106 / 109 / 111, R-MAT-18 64 / 75 / 75, R-MAT-23 (X is 268 MB) 923 / 982 / 1008; value-free 2 M of 50 686 / 645 / 651, 700,000 of 36 177 / 173 / 185,
-// 50,000 of 500 131 / 134 / 142.  F = 4 700,000 of 71 326 / 307 / 306, 1.4 M of 88 688 / 669 / 660, 50,000 of 1000 192 / 197 / 194, 200,000 of 250 248 / 253 / 254,
-// of 500 466 / 457 / 458, R-MAT-24 1758 / 1663 / 1697, R-MAT-18 66 / 76 / 75; value-free 50,000 of 2000 242 / 252 / 236, 2 M of 50 620 / 601 / 595.
-// Widths of 1 and 2 keep four.
+// a warp only cost registers; out of HBM they pay.  us with four / two / one: F = 8 power law 700,000 rows of 71 354 / 319 / 314, 1.4 M
+// of 88 760 / 698 / 679, 2 M of 50 836 / 784 / 716, 700,000 of 21 138 / 137 / 136, 50,000 of 500 143 / 145 / 148, of 1000 237 / 234 /
+// 234, R-MAT-19 16 M nonzeros 106 / 109 / 111, R-MAT-18 64 / 75 / 75, R-MAT-23 (X is 268 MB) 923 / 982 / 1008; value-free 2 M of 50 686
+// / 645 / 651, 700,000 of 36 177 / 173 / 185, 50,000 of 500 131 / 134 / 142.  F = 4 700,000 of 71 326 / 307 / 306, 1.4 M of 88 688 /
+// 669 / 660, 50,000 of 1000 192 / 197 / 194, 200,000 of 250 248 / 253 / 254, of 500 466 / 457 / 458, R-MAT-24 1758 / 1663 / 1697,
+// R-MAT-18 66 / 76 / 75; value-free 50,000 of 2000 242 / 252 / 236, 2 M of 50 620 / 601 / 595. Widths of 1 and 2 keep four.
 template <int G, int VEC, bool UNIT>
 static int large_plan_batches(int nnz, int n_rows) {
     const int most = chunk_batches(G, 1, VEC, false);
@@ -1009,10 +1009,10 @@ static int large_plan_batches(int nnz, int n_rows) {
 }
 
 // The same for the one launch of a small plan, where one batch also halves the registers of the whole kernel: for graphs whose rows are
-// nearly all long.  us with four (F = 8: two) / one and the short rows as wide shapes have them: F = 1 20,000 rows of 300 29.2 / 26.7, 8,000 of 200
-// 9.4 / 10.1, value-free 23.7 / 19.5 and 8.7 / 7.5, 20,000 of 120 13.4 / 13.7; F = 4 12,000 of 480 34.5 / 32.8, 40,000 of 150 36.3 / 37.3, 3,000 of 300 7.2 / 8.0,
-// value-free 31.2 / 27.7 and 33.1 / 32.1; F = 8 value-free 12,000 of 480 35.0 / 33.5.  F = 4 value-free with four / two: 100,000 rows of 60 50.5 / 44.0,
-// 200,000 of 28 47.7 / 42.9, 20,000 of 40 13.2 / 14.6.
+// nearly all long.  us with four (F = 8: two) / one and the short rows as wide shapes have them: F = 1 20,000 rows of 300 29.2 / 26.7,
+// 8,000 of 200 9.4 / 10.1, value-free 23.7 / 19.5 and 8.7 / 7.5, 20,000 of 120 13.4 / 13.7; F = 4 12,000 of 480 34.5 / 32.8, 40,000 of
+// 150 36.3 / 37.3, 3,000 of 300 7.2 / 8.0, value-free 31.2 / 27.7 and 33.1 / 32.1; F = 8 value-free 12,000 of 480 35.0 / 33.5.  F = 4
+// value-free with four / two: 100,000 rows of 60 50.5 / 44.0, 200,000 of 28 47.7 / 42.9, 20,000 of 40 13.2 / 14.6.
 template <int G, int VEC, bool UNIT>
 static int small_plan_batches(int nnz, int n_rows) {
     if (nnz >= 3 << 19 && (UNIT || G == 1) && nnz / (UNIT ? 140 : 256) >= n_rows) return 1;

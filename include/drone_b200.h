@@ -338,7 +338,8 @@ int drone_clear_mirror_rows(float *d_rows, int n_rows, int F, int ld, const int 
 /* Softmax cross-entropy over [n_rows, classes] logits with its gradient (CUDACrossEntropyLoss::forward,
  * cuda_gcn/src/cuda/cuda_kernel.cu:326-370): *d_loss = mean over the rows with d_labelled[r] != 0 (0 where there are none),
  * d_grad = (softmax - one-hot) * labelled, not divided by their number.  d_truth[r]: the row's class, 0..classes-1 (also
- * where it is not labelled); any other value makes the loss and the row's gradient NaN.  d_scratch: DRONE_LOSS_SCRATCH doubles, 16-byte aligned.  d_grad may be d_logits.  Asynchronous. */
+ * where it is not labelled); any other value makes the loss and the row's gradient NaN.  d_scratch: DRONE_LOSS_SCRATCH doubles,
+ * 16-byte aligned.  d_grad may be d_logits.  Asynchronous. */
 #define DRONE_LOSS_SCRATCH 2368
 int drone_softmax_loss(int n_rows, int classes, const float *d_logits, int ld, const long long *d_truth, const unsigned char *d_labelled,
                        float *d_grad, int ld_grad, float *d_loss, double *d_scratch, void *stream);
